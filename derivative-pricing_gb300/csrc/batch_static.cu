@@ -15,9 +15,11 @@
 // Limits: at most kStaticMaxContracts contracts and kStaticMaxSlabs slabs of
 // 4096 paths per call (about 1.07e9 paths in total); the array is about 7 MB.
 // Contracts are processed in the order given (no longest-first sort), which
-// changes load balance but not results: slab partials and their merge order
-// depend only on the slab index, so results are bitwise identical to
-// mcd_price_batch's.
+// changes load balance but not results: item partials and their merge order
+// depend only on the item index, so results are bitwise identical to
+// mcd_price_batch's.  An FP64 contract has more, smaller items (units) than
+// slabs: a batch with more of them than the partials hold runs as several
+// launches over ranges of contracts.
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -58,6 +60,7 @@ unsigned char* g_scratch_addr[kStaticMaxDevices] = {};
 int g_grid[kStaticMaxDevices][2] = {};  // persistent grid per device and precision
 DevContract g_stage_contracts[kStaticMaxContracts];
 uint32_t g_stage_prefix[kStaticMaxContracts + 1];
+const mcdg::FixedTables* g_tables[kStaticMaxDevices] = {};
 
 int report(char* msg, size_t cap, int code, const char* text) {
     if (msg && cap) std::snprintf(msg, cap, "%s", text);
@@ -79,6 +82,8 @@ int static_setup(int device, char* msg, size_t cap) {
     void* addr = nullptr;
     cudaError_t e = cudaGetSymbolAddress(&addr, g_batch_scratch);
     if (e != cudaSuccess) return report_cuda(msg, cap, e, "cudaGetSymbolAddress(scratch)");
+    e = mcdg::fixed_tables_device(&g_tables[device]);
+    if (e != cudaSuccess) return report_cuda(msg, cap, e, "fixed-point tables");
     int sms = 0;
     e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     if (e != cudaSuccess) return report_cuda(msg, cap, e, "SM count");
@@ -117,7 +122,8 @@ extern "C" int mcd_price_batch_static(const mcd_contract* contracts, size_t n, i
     int rc = static_setup(device, error_message, error_capacity);
     if (rc != MCD_OK || n == 0) return rc;
 
-    uint64_t total = 0;
+    uint64_t total = 0;   // slabs, the limit's unit
+    uint32_t items = 0;   // slabs (FP32) or units (FP64) so far, modulo 2^32
     for (size_t i = 0; i < n; ++i) {
         const char* why = mcdg::convert_contract(contracts[i], static_cast<uint32_t>(i), g_stage_contracts[i]);
         if (why) {
@@ -125,13 +131,14 @@ extern "C" int mcd_price_batch_static(const mcd_contract* contracts, size_t n, i
             std::snprintf(text, sizeof text, "contract %zu: %s", i, why);
             return report(error_message, error_capacity, MCD_ERR_INVALID_ARGUMENT, text);
         }
-        g_stage_prefix[i] = static_cast<uint32_t>(total);
+        g_stage_prefix[i] = items;
+        items += precision == MCD_PRECISION_FP64 ? g_stage_contracts[i].n_units : g_stage_contracts[i].n_slabs;
         total += g_stage_contracts[i].n_slabs;
         if (total > kStaticMaxSlabs)
             return report(error_message, error_capacity, MCD_ERR_INVALID_ARGUMENT,
                           "mcd_price_batch_static: at most 262144 slabs of 4096 paths per call");
     }
-    g_stage_prefix[n] = static_cast<uint32_t>(total);
+    g_stage_prefix[n] = items;
 
     unsigned char* base = g_scratch_addr[device];
     DevContract* d_contracts = reinterpret_cast<DevContract*>(base + kOffContracts);
@@ -147,15 +154,26 @@ extern "C" int mcd_price_batch_static(const mcd_contract* contracts, size_t n, i
     e = cudaMemcpyAsync(d_contracts, g_stage_contracts, sizeof(DevContract) * n, cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(d_prefix, g_stage_prefix, sizeof(uint32_t) * (n + 1), cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess) e = cudaMemsetAsync(d_flags, 0, 2 * sizeof(uint32_t), s);
     if (e != cudaSuccess) return report_cuda(error_message, error_capacity, e, "stage contracts");
-    if (total > 0) {
-        e = mcdg::launch_path_kernel(precision, 1, g_grid[device][precision], d_contracts, static_cast<int>(n),
-                                     d_prefix, d_flags, d_partials, d_flags + 1, s);
-        if (e != cudaSuccess) return report_cuda(error_message, error_capacity, e, "path kernel");
+    // Contracts in ranges whose items fit the partials: all at once in FP32
+    // (the slab limit); FP64 units are smaller than slabs (at most 4096 per
+    // contract below 2^23 paths, slabs above), so a large FP64 batch takes
+    // several launches on the same scratch.
+    for (size_t first = 0; first < n;) {
+        size_t end = first + 1;
+        while (end < n && g_stage_prefix[end + 1] - g_stage_prefix[first] <= kStaticMaxSlabs) ++end;
+        e = cudaMemsetAsync(d_flags, 0, (first == 0 ? 2 : 1) * sizeof(uint32_t), s);
+        if (e != cudaSuccess) return report_cuda(error_message, error_capacity, e, "reset flags");
+        const int count = static_cast<int>(end - first);
+        if (g_stage_prefix[end] != g_stage_prefix[first]) {
+            e = mcdg::launch_path_kernel(precision, 1, g_grid[device][precision], d_contracts + first, count,
+                                         d_prefix + first, d_flags, d_partials, d_flags + 1, g_tables[device], s);
+            if (e != cudaSuccess) return report_cuda(error_message, error_capacity, e, "path kernel");
+        }
+        e = mcdg::launch_merge_kernel(d_contracts + first, count, d_prefix + first, d_partials, d_results, s);
+        if (e != cudaSuccess) return report_cuda(error_message, error_capacity, e, "merge kernel");
+        first = end;
     }
-    e = mcdg::launch_merge_kernel(d_contracts, static_cast<int>(n), d_prefix, d_partials, d_results, s);
-    if (e != cudaSuccess) return report_cuda(error_message, error_capacity, e, "merge kernel");
     uint32_t flags[2] = {0, 0};
     e = cudaMemcpyAsync(results, d_results, sizeof(mcd_mc_result) * n, cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaMemcpyAsync(flags, d_flags, sizeof flags, cudaMemcpyDeviceToHost, s);

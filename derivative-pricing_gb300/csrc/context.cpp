@@ -108,6 +108,44 @@ bool finite_all(std::initializer_list<double> xs) {
     return true;
 }
 
+// A log2 step's integers: drift = (hi + lo 2^-32) 2^-frac, vs 2^(frac + 3).
+void fixed_step(double drift, double vs, int frac, int64_t* hi, uint32_t* lo, uint64_t* scale) {
+    const double d = std::ldexp(drift, frac), whole = std::floor(d);
+    *hi = static_cast<int64_t>(whole);
+    *lo = static_cast<uint32_t>(std::min((d - whole) * 4294967296.0, 4294967295.0));
+    *scale = static_cast<uint64_t>(std::ldexp(vs, frac + 3) + 0.5);
+}
+
+// ln(H / S0) in log2 units, kept within +/- 2^61 (which no path reaches).
+int64_t fixed_barrier(double log_rel, int frac) {
+    constexpr double kInvLn2 = 1.44269504088896340736;
+    const double reach = std::ldexp(1.0, 61);
+    return std::llround(std::min(std::max(std::ldexp(log_rel * kInvLn2, frac), -reach), reach));
+}
+
+// The log-spot's units (paths64.cuh).  |log2(S / S0)| stays below n times the
+// largest step (|z| < 6.34: u is at least 2^-33) and, beyond any doubt, below
+// the drift plus 40 standard deviations of the sum (probability below 1e-340
+// per path); that bound is rounded up to a power of two, 2^r, and F = 61 - r
+// fraction bits are kept, 52 to 59 of them.  Above 2^9 a double's exponent
+// range comes near: frac stays 0 and the path is stepped as the reference does.
+void fixed_scale(DevContract& c) {
+    constexpr double kInvLn2 = 1.44269504088896340736;
+    const double n = static_cast<double>(c.n_steps);
+    const double drift = c.drift * kInvLn2, vs = c.vs * kInvLn2;
+    const double bound = n * std::fabs(drift) + vs * std::min(6.35 * n, 40.0 * std::sqrt(n));
+    c.frac = 0;
+    if (!(bound < 512.0)) return;
+    int r = 2;
+    while (bound >= std::ldexp(1.0, r)) ++r;
+    c.frac = 61 - r;
+    fixed_step(drift, vs, c.frac, &c.y_drift, &c.y_drift_lo, &c.y_vs);
+    if (c.kind == kBarrier || c.kind == kBarrierBridge) {
+        c.y_barrier = fixed_barrier(c.log_h_rel, c.frac);
+        c.y_bridge = std::ldexp(-2.0 / (kInvLn2 * kInvLn2 * c.bb_denom), -2 * c.frac);
+    }
+}
+
 // Validates one contract and converts it to the kernel layout; returns null
 // or the reason the contract is rejected.  No context: mcd_price_batch's
 // planner and the allocation-free entry point (batch_static.cu) share it, so
@@ -195,6 +233,15 @@ const char* convert_contract(const mcd_contract& in, uint32_t index, DevContract
     out.drift = (in.rate - in.carry_yield - 0.5 * vol * vol) * dt;
     out.vs = vol * std::sqrt(dt);
     out.n_slabs = static_cast<uint32_t>(slabs);
+    // FP64 units: one path per lane up to 131,071 paths (a single call then has
+    // the most warps to spread over the GPU), doubling from there so that a
+    // contract keeps 2048 to 4096 units, up to a slab.
+    out.unit_log = 0;
+    while (out.unit_log < 7 && (in.path_count >> (17 + out.unit_log)) != 0) ++out.unit_log;
+    const uint64_t unit = 32ull << out.unit_log;
+    out.n_units = static_cast<uint32_t>((in.path_count + unit - 1) / unit);
+    out.inv_n = 1.0 / static_cast<double>(out.n_steps);
+    fixed_scale(out);
     return nullptr;
 }
 
@@ -213,7 +260,10 @@ double slab_cost(const DevContract& c) {
     return static_cast<double>(c.n_steps) * per_step * (c.antithetic ? 2.0 : 1.0);
 }
 
-int plan_batch(Ctx& ctx, const mcd_contract* contracts, size_t n, BatchPlan& plan) {
+// range_items: 0 for slab items, else the items are FP64 units (the pricer and
+// the Greeks in FP64), at most range_items of them in a range.
+int plan_batch(Ctx& ctx, const mcd_contract* contracts, size_t n, uint64_t range_items, BatchPlan& plan) {
+    const bool units = range_items != 0;
     if (n > 0x7FFFFFFF) return ctx.fail(MCD_ERR_INVALID_ARGUMENT, "too many contracts");
     plan.dev.resize(n);
     for (size_t i = 0; i < n; ++i) {
@@ -223,15 +273,30 @@ int plan_batch(Ctx& ctx, const mcd_contract* contracts, size_t n, BatchPlan& pla
     std::stable_sort(plan.dev.begin(), plan.dev.end(), [](const DevContract& a, const DevContract& b) {
         return slab_cost(a) > slab_cost(b);
     });
+    // The prefix counts items modulo 2^32: kernels use differences within a
+    // range of contracts, and every range holds at most range_items units (or
+    // one contract), so that the partials of a batch of many small contracts
+    // stay bounded.  A batch is one range unless it is very large.
     plan.prefix.resize(n + 1);
-    uint64_t total = 0;
+    plan.ranges.assign(1, 0);
+    uint64_t slabs = 0, in_range = 0;
+    uint32_t items = 0;
+    plan.max_items = 0;
     for (size_t i = 0; i < n; ++i) {
-        plan.prefix[i] = static_cast<uint32_t>(total);
-        total += plan.dev[i].n_slabs;
-        if (total > 0xFFFFFFF0ull) return ctx.fail(MCD_ERR_INVALID_ARGUMENT, "batch too large");
+        const uint32_t more = units ? plan.dev[i].n_units : plan.dev[i].n_slabs;
+        plan.prefix[i] = items;
+        slabs += plan.dev[i].n_slabs;
+        if (slabs > 0xFFFFFFF0ull) return ctx.fail(MCD_ERR_INVALID_ARGUMENT, "batch too large");
+        if (units && in_range > 0 && in_range + more > range_items) {
+            plan.ranges.push_back(static_cast<uint32_t>(i));
+            in_range = 0;
+        }
+        in_range += more;
+        items += more;
+        plan.max_items = std::max(plan.max_items, static_cast<uint32_t>(in_range));
     }
-    plan.prefix[n] = static_cast<uint32_t>(total);
-    plan.total_items = static_cast<uint32_t>(total);
+    plan.prefix[n] = items;
+    plan.ranges.push_back(static_cast<uint32_t>(n));
     plan.n = n;
     return MCD_OK;
 }
@@ -257,7 +322,7 @@ int upload_plan(Ctx& ctx, const BatchPlan& plan) {
     if (rc) return rc;
     rc = ctx.reserve(ctx.d_prefix, sizeof(uint32_t) * (n + 1), "prefix");
     if (rc) return rc;
-    rc = ctx.reserve(ctx.d_partials, sizeof(Welford) * std::max<uint32_t>(plan.total_items, 1), "partials");
+    rc = ctx.reserve(ctx.d_partials, sizeof(Welford) * std::max<size_t>(plan.max_items, 1), "partials");
     if (rc) return rc;
     rc = ctx.reserve(ctx.d_results, sizeof(mcd_mc_result) * std::max<size_t>(n, 1), "results");
     if (rc) return rc;
@@ -279,13 +344,34 @@ int upload_plan(Ctx& ctx, const BatchPlan& plan) {
     return MCD_OK;
 }
 
-// Captures (or reuses) the graph: reset ticket and error word, persistent
-// path kernel, merge kernel.  Timing events are recorded around the graph
-// launch on the launching stream (run_graph), not inside the graph.
-int get_graph(Ctx& ctx, int precision, const BatchPlan& plan, void* results, cudaGraphExec_t* out) {
-    int variant = 0, grid = 0;
-    int rc = launch_shape(ctx, precision, variant, grid);
-    if (rc) return rc;
+// Queues a planned batch on a stream: per range, reset ticket and error word,
+// persistent path kernel, merge kernel.  (The error word keeps the last
+// range's value; an inconsistent item shows in every run.)
+int enqueue_plan(Ctx& ctx, int precision, int variant, int grid, const BatchPlan& plan, void* results,
+                 cudaStream_t stream) {
+    cudaGetLastError();  // launches below report their own status only
+    const DevContract* dev = static_cast<const DevContract*>(ctx.d_contracts.ptr);
+    const uint32_t* prefix = static_cast<const uint32_t*>(ctx.d_prefix.ptr);
+    Welford* partials = static_cast<Welford*>(ctx.d_partials.ptr);
+    for (size_t r = 0; r + 1 < plan.ranges.size(); ++r) {
+        const uint32_t first = plan.ranges[r];
+        const int n = static_cast<int>(plan.ranges[r + 1] - first);
+        cudaError_t e = cudaMemsetAsync(ctx.d_flags, 0, (r == 0 ? 2 : 1) * sizeof(uint32_t), stream);
+        if (e != cudaSuccess) return ctx.cuda_fail(e, "reset flags");
+        e = launch_path_kernel(precision, variant, grid, dev + first, n, prefix + first, ctx.d_flags, partials,
+                               ctx.d_flags + 1, ctx.tables, stream);
+        if (e != cudaSuccess) return ctx.cuda_fail(e, "path kernel");
+        e = launch_merge_kernel(dev + first, n, prefix + first, partials, results, stream);
+        if (e != cudaSuccess) return ctx.cuda_fail(e, "merge kernel");
+    }
+    return MCD_OK;
+}
+
+// Captures (or reuses) the graph of a one-range batch.  Timing events are
+// recorded around the graph launch on the launching stream (run_plan), not
+// inside the graph.
+int get_graph(Ctx& ctx, int precision, int variant, int grid, const BatchPlan& plan, void* results,
+              cudaGraphExec_t* out) {
     GraphKey key{precision, variant, grid, plan.n, 0u, ctx.d_contracts.ptr,
                  ctx.d_prefix.ptr, ctx.d_partials.ptr, results};
     for (auto& g : ctx.graphs) {
@@ -294,32 +380,15 @@ int get_graph(Ctx& ctx, int precision, const BatchPlan& plan, void* results, cud
             return MCD_OK;
         }
     }
-    cudaGetLastError();  // launches below report their own status only
     cudaGraph_t graph = nullptr;
     cudaError_t e = cudaStreamBeginCapture(ctx.stream, cudaStreamCaptureModeThreadLocal);
     if (e != cudaSuccess) return ctx.cuda_fail(e, "begin capture");
-    uint32_t* ticket = ctx.d_flags;
-    uint32_t* err = ctx.d_flags + 1;
-    cudaError_t e1 = cudaMemsetAsync(ctx.d_flags, 0, 2 * sizeof(uint32_t), ctx.stream);
-    cudaError_t e2 = launch_path_kernel(precision, variant, grid,
-                                        static_cast<const DevContract*>(ctx.d_contracts.ptr),
-                                        static_cast<int>(plan.n),
-                                        static_cast<const uint32_t*>(ctx.d_prefix.ptr), ticket,
-                                        static_cast<Welford*>(ctx.d_partials.ptr), err, ctx.stream);
-    cudaError_t e3 = launch_merge_kernel(static_cast<const DevContract*>(ctx.d_contracts.ptr),
-                                         static_cast<int>(plan.n),
-                                         static_cast<const uint32_t*>(ctx.d_prefix.ptr),
-                                         static_cast<const Welford*>(ctx.d_partials.ptr), results,
-                                         ctx.stream);
+    const int rc = enqueue_plan(ctx, precision, variant, grid, plan, results, ctx.stream);
     e = cudaStreamEndCapture(ctx.stream, &graph);
-    const char* stage[3] = {"capture: reset flags", "capture: path kernel", "capture: merge kernel"};
-    const cudaError_t es[3] = {e1, e2, e3};
-    for (int i = 0; i < 3; ++i) {
-        if (es[i] != cudaSuccess) {
-            if (graph) cudaGraphDestroy(graph);
-            cudaGetLastError();
-            return ctx.cuda_fail(es[i], stage[i]);
-        }
+    if (rc) {
+        if (graph) cudaGraphDestroy(graph);
+        cudaGetLastError();
+        return rc;
     }
     if (e != cudaSuccess) return ctx.cuda_fail(e, "end capture");
     cudaGraphExec_t exec = nullptr;
@@ -336,12 +405,26 @@ int get_graph(Ctx& ctx, int precision, const BatchPlan& plan, void* results, cud
     return MCD_OK;
 }
 
-int run_graph(Ctx& ctx, cudaGraphExec_t exec, cudaStream_t stream) {
-    int pair = -1;
-    int rc = ctx.record_start(stream, &pair);
+// Runs an uploaded plan on a stream: one range from its graph, several (their
+// bounds depend on the batch) queued directly.
+int run_plan(Ctx& ctx, int precision, const BatchPlan& plan, void* results, cudaStream_t stream) {
+    int variant = 0, grid = 0, pair = -1;
+    int rc = launch_shape(ctx, precision, variant, grid);
     if (rc) return rc;
-    cudaError_t e = cudaGraphLaunch(exec, stream);
-    if (e != cudaSuccess) return ctx.cuda_fail(e, "graph launch");
+    cudaGraphExec_t exec = nullptr;
+    if (plan.ranges.size() == 2) {
+        rc = get_graph(ctx, precision, variant, grid, plan, results, &exec);
+        if (rc) return rc;
+    }
+    rc = ctx.record_start(stream, &pair);
+    if (rc) return rc;
+    if (exec) {
+        cudaError_t e = cudaGraphLaunch(exec, stream);
+        if (e != cudaSuccess) return ctx.cuda_fail(e, "graph launch");
+    } else {
+        rc = enqueue_plan(ctx, precision, variant, grid, plan, results, stream);
+        if (rc) return rc;
+    }
     return ctx.record_stop(stream, pair);
 }
 
@@ -359,15 +442,12 @@ int collect_after_sync(Ctx& ctx) {
 int price_batch_host(Ctx& ctx, const mcd_contract* contracts, size_t n, int precision,
                      mcd_mc_result* results) {
     BatchPlan& plan = ctx.host_plan;
-    int rc = plan_batch(ctx, contracts, n, plan);
+    int rc = plan_batch(ctx, contracts, n, precision == 0 ? kRangeItems : 0, plan);
     if (rc) return rc;
     if (n == 0) return MCD_OK;
     rc = upload_plan(ctx, plan);
     if (rc) return rc;
-    cudaGraphExec_t exec = nullptr;
-    rc = get_graph(ctx, precision, plan, ctx.d_results.ptr, &exec);
-    if (rc) return rc;
-    rc = run_graph(ctx, exec, ctx.stream);
+    rc = run_plan(ctx, precision, plan, ctx.d_results.ptr, ctx.stream);
     if (rc) return rc;
     cudaError_t e = cudaMemcpyAsync(results, ctx.d_results.ptr, sizeof(mcd_mc_result) * n,
                                     cudaMemcpyDeviceToHost, ctx.stream);
@@ -449,6 +529,7 @@ int mcd_create(int device, mcd_ctx** out) try {
     if ((e = cudaMalloc(reinterpret_cast<void**>(&ctx->d_flags), 64)) != cudaSuccess)
         return init_fail(e, "flags");
     cudaMemset(ctx->d_flags, 0, 64);
+    if ((e = fixed_tables_device(&ctx->tables)) != cudaSuccess) return init_fail(e, "fixed-point tables");
     *out = reinterpret_cast<mcd_ctx*>(ctx);
     return MCD_OK;
 } catch (...) {
@@ -515,7 +596,7 @@ int mcd_price_batch_device(mcd_ctx* handle, const mcd_contract* contracts, size_
         e = cudaMemcpyAsync(host.data(), contracts, sizeof(mcd_contract) * n, cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
         if (e != cudaSuccess) return ctx->cuda_fail(e, "read device contracts");
-        int rc = plan_batch(*ctx, host.data(), n, ctx->device_plan);
+        int rc = plan_batch(*ctx, host.data(), n, precision == 0 ? kRangeItems : 0, ctx->device_plan);
         if (rc) return rc;
         rc = upload_plan(*ctx, ctx->device_plan);
         if (rc) return rc;
@@ -524,10 +605,7 @@ int mcd_price_batch_device(mcd_ctx* handle, const mcd_contract* contracts, size_
         ctx->device_plan_key = key;
         ctx->device_plan_valid = true;
     }
-    cudaGraphExec_t exec = nullptr;
-    int rc = get_graph(*ctx, precision, ctx->device_plan, results, &exec);
-    if (rc) return rc;
-    return run_graph(*ctx, exec, s);
+    return run_plan(*ctx, precision, ctx->device_plan, results, s);
 } catch (...) {
     return abi_exception(handle);
 }
@@ -571,7 +649,7 @@ int mcd_autotune(mcd_ctx* handle, const mcd_contract* contracts, size_t n, int p
     if (precision != 0 && precision != 1) return ctx->fail(MCD_ERR_INVALID_ARGUMENT, "bad precision");
     if (n == 0 || !contracts) return ctx->fail(MCD_ERR_INVALID_ARGUMENT, "empty tuning batch");
     BatchPlan plan;
-    int rc = plan_batch(*ctx, contracts, n, plan);
+    int rc = plan_batch(*ctx, contracts, n, precision == 0 ? kRangeItems : 0, plan);
     if (rc) return rc;
     rc = upload_plan(*ctx, plan);
     if (rc) return rc;
@@ -588,12 +666,9 @@ int mcd_autotune(mcd_ctx* handle, const mcd_contract* contracts, size_t n, int p
             if (c >= 1 && std::find(cands.begin(), cands.end(), c) == cands.end()) cands.push_back(c);
         for (int c : cands) {
             ctx->shape[precision] = LaunchShape{v, c};
-            cudaGraphExec_t exec = nullptr;
-            rc = get_graph(*ctx, precision, plan, ctx->d_results.ptr, &exec);
-            if (rc) { ctx->shape[precision] = saved; return rc; }
             double total = 0.0;
             for (int rep = 0; rep < 3; ++rep) {
-                rc = run_graph(*ctx, exec, ctx->stream);
+                rc = run_plan(*ctx, precision, plan, ctx->d_results.ptr, ctx->stream);
                 if (rc) { ctx->shape[precision] = saved; return rc; }
                 e = cudaStreamSynchronize(ctx->stream);
                 if (e != cudaSuccess) { ctx->shape[precision] = saved; return ctx->cuda_fail(e, "tuning run"); }
@@ -770,8 +845,11 @@ int mcd_draws(mcd_ctx* handle, uint64_t seed, uint64_t path_begin, uint64_t n_pa
     if (total > (1ull << 31)) return ctx->fail(MCD_ERR_INVALID_ARGUMENT, "at most 2^31 draws per call");
     int rc = ctx->reserve(ctx->d_scratch, sizeof(double) * total, "draw buffer");
     if (rc) return rc;
-    cudaError_t e = launch_draws_kernel(seed, path_begin, n_paths, draw_begin, n_draws, stream_id,
-                                        precision, static_cast<double*>(ctx->d_scratch.ptr), ctx->stream);
+    double* d = static_cast<double*>(ctx->d_scratch.ptr);
+    cudaError_t e = precision == 0 && stream_id == 0
+                        ? launch_draws64_kernel(seed, path_begin, n_paths, draw_begin, n_draws, ctx->tables, d, ctx->stream)
+                        : launch_draws_kernel(seed, path_begin, n_paths, draw_begin, n_draws, stream_id, precision, d,
+                                              ctx->stream);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(out, ctx->d_scratch.ptr, sizeof(double) * total, cudaMemcpyDeviceToHost, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);

@@ -24,10 +24,12 @@ struct HostBuffer {
 
 struct BatchPlan {
     std::vector<DevContract> dev;    // longest-first
-    std::vector<uint32_t> prefix;    // n + 1 running slab counts
-    uint32_t total_items = 0;
+    std::vector<uint32_t> prefix;    // n + 1 running item counts (slabs or units)
+    std::vector<uint32_t> ranges;    // first contract of each range, then n
+    uint32_t max_items = 0;          // items of the largest range
     size_t n = 0;
 };
+constexpr uint64_t kRangeItems = 1ull << 26;  // 1.6 GB of partials
 
 struct LaunchShape {
     int variant = 1;      // __launch_bounds__ min-blocks 8
@@ -75,6 +77,7 @@ struct Ctx {
     DeviceBuffer d_contracts, d_prefix, d_partials, d_results, d_scratch, d_scratch2;
     uint32_t* d_flags = nullptr;  // [0] ticket, [1] error word, [4..5] contract digest, rest spare
     HostBuffer h_stage;
+    const FixedTables* tables = nullptr;  // this device's fixed-point tables
 
     BatchPlan host_plan, device_plan;
     DevicePlanKey device_plan_key{nullptr, 0, 0, 0};
@@ -132,7 +135,9 @@ struct Ctx {
 
 // Batch planning and execution of the path engine (context.cpp).
 int plan_contract(Ctx& ctx, const mcd_contract& in, uint32_t index, DevContract& out);
-int plan_batch(Ctx& ctx, const mcd_contract* contracts, size_t n, BatchPlan& plan);
+void fixed_step(double drift, double vs, int frac, int64_t* hi, uint32_t* lo, uint64_t* scale);
+int64_t fixed_barrier(double log_rel, int frac);
+int plan_batch(Ctx& ctx, const mcd_contract* contracts, size_t n, uint64_t range_items, BatchPlan& plan);
 int price_batch_host(Ctx& ctx, const mcd_contract* contracts, size_t n, int precision,
                      mcd_mc_result* results);
 

@@ -8,6 +8,8 @@
 
 namespace mcdg {
 
+struct FixedTables;  // fixed_math.hpp
+
 // One accumulator (include/mcd/core/stats.hpp:21-71): count, mean, M2.
 struct Welford {
     unsigned long long count;
@@ -57,6 +59,17 @@ struct DevContract {
     uint64_t seed;
     uint32_t n_slabs;
     uint32_t orig_index;   // position in the caller's array
+    // FP64 paths (gbm_paths64.cu): units of 32 << unit_log paths, and the
+    // log-spot step in base 2 as integers in units of 2^-frac.  frac = 0: the
+    // contract is outside the fixed-point range.
+    uint32_t n_units;
+    int32_t unit_log, frac;
+    uint32_t y_drift_lo;   // drift / ln 2 = (y_drift + y_drift_lo 2^-32) 2^-frac
+    int64_t y_drift;
+    uint64_t y_vs;         // vs / ln 2, 2^(frac + 3)
+    int64_t y_barrier;     // log2(H / S0), 2^frac, within +/- 2^61
+    double y_bridge;       // -2 (ln 2)^2 / (vol^2 dt), 2^(-2 frac)
+    double inv_n;          // 1 / n_steps
 };
 
 // Validates one contract and converts it to the kernel layout; null on
@@ -68,9 +81,18 @@ const char* convert_contract(const mcd_contract& in, uint32_t index, DevContract
 // The persistent path kernel over items [0, item_prefix[n_contracts]) (the
 // item count is read on the device, so one captured launch serves every path
 // count of the same number of contracts).
+// Items are slabs of kSlabPaths paths in FP32 and units of 32 << unit_log paths
+// in FP64; `tables` (fixed_tables_device) is for FP64.
 cudaError_t launch_path_kernel(int precision, int variant, int grid, const DevContract* contracts,
                                int n_contracts, const uint32_t* item_prefix, uint32_t* ticket,
-                               Welford* partials, uint32_t* error_flag, cudaStream_t stream);
+                               Welford* partials, uint32_t* error_flag, const FixedTables* tables,
+                               cudaStream_t stream);
+cudaError_t launch_path64_kernel(int variant, int grid, const DevContract* contracts, int n_contracts,
+                                 const uint32_t* item_prefix, uint32_t* ticket, Welford* partials,
+                                 uint32_t* error_flag, const FixedTables* tables, cudaStream_t stream);
+// The fixed-point tables of the current device, placed there at the first call
+// (computed once per process, 22 ms).  Not to be called during stream capture.
+cudaError_t fixed_tables_device(const FixedTables** out);
 cudaError_t launch_merge_kernel(const DevContract* contracts, int n_contracts,
                                 const uint32_t* item_prefix, const Welford* partials,
                                 void* results /* mcd_mc_result[] */, cudaStream_t stream);
@@ -82,6 +104,8 @@ cudaError_t launch_words_digest(const uint64_t* words, size_t n_words, uint64_t*
 
 cudaError_t launch_philox_kernel(const uint32_t* counters, const uint32_t* keys, size_t n,
                                  uint32_t* out, cudaStream_t stream);
+cudaError_t launch_draws64_kernel(uint64_t seed, uint64_t path_begin, uint64_t n_paths, uint32_t draw_begin,
+                                  uint32_t n_draws, const FixedTables* tables, double* out, cudaStream_t stream);
 cudaError_t launch_draws_kernel(uint64_t seed, uint64_t path_begin, uint64_t n_paths,
                                 uint32_t draw_begin, uint32_t n_draws, int stream_id,
                                 int precision, double* out, cudaStream_t stream);

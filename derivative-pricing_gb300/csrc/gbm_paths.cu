@@ -1,5 +1,6 @@
 // gbm_paths.cu -- the batched GBM path engine (European, digital, Asian,
-// barrier, lookback) as one persistent kernel per precision.
+// barrier, lookback) in FP32 as one persistent kernel, and the merge of both
+// precisions (the FP64 paths are gbm_paths64.cu).
 //
 // Work decomposition.  Every contract's paths are cut into fixed slabs of
 // kSlabPaths = 4096 paths; one (contract, slab) pair is one work item.  The
@@ -11,8 +12,8 @@
 //
 // Determinism.  A slab's Welford triple depends only on the slab: per-thread
 // accumulation in j order, then a fixed warp shuffle tree and a fixed 4-warp
-// tree.  The merge kernel folds a contract's slabs in slab order with a fixed
-// warp tree.  Grid size and kernel variant (register budget) only decide who
+// tree.  The merge kernel folds a contract's slabs in a fixed tree (merge.cuh).
+// Grid size and kernel variant (register budget) only decide who
 // computes an item, never the arithmetic, so results are bitwise identical
 // across launch shapes.
 //
@@ -26,120 +27,11 @@
 
 #include "device_common.cuh"
 #include "engine.hpp"
+#include "merge.cuh"
 
 namespace mcdg {
 
 namespace {
-
-__device__ __forceinline__ double dmax(double a, double b) { return (a < b) ? b : a; }
-__device__ __forceinline__ double dmin(double a, double b) { return (b < a) ? b : a; }
-
-// ===========================================================================
-// FP64: the reference's arithmetic (multiplicative steps, FP64 payoffs).
-// ===========================================================================
-__device__ __forceinline__ double draw64(const PhiloxPath& pp, uint32_t step, const PhiloxKeys& k,
-                                         bool neg) {
-    const double z = normal_from_bits_f64(philox_word0(pp, step, k));
-    return neg ? -z : z;
-}
-
-template <int KIND>
-__device__ double sample64(const DevContract& c, const PhiloxKeys& k, uint64_t path, bool neg) {
-    const double phi = c.type == 0 ? 1.0 : -1.0;
-    const PhiloxPath pp = philox_path(path, 0u, k);
-    if constexpr (KIND == kEuropean || KIND == kDigital) {
-        const double z = draw64(pp, 0u, k, neg);
-        const double s = c.spot * exp(c.drift + c.vs * z);
-        if constexpr (KIND == kEuropean) {
-            return c.discount * dmax(phi * (s - c.strike), 0.0);
-        } else {
-            const bool itm = phi * (s - c.strike) > 0.0;
-            return c.discount * (itm ? (c.asset ? s : c.cash) : 0.0);
-        }
-    } else if constexpr (KIND == kBarrierBridge) {
-        const PhiloxPath pu = philox_path(path, 1u, k);
-        double s = c.spot;
-        bool breached = false;
-        for (int step = 0; step < c.n_steps; ++step) {
-            const double z = draw64(pp, static_cast<uint32_t>(step), k, neg);
-            const double s_next = s * exp(c.drift + c.vs * z);
-            const bool crossed = c.up ? s_next >= c.barrier : s_next <= c.barrier;
-            breached = breached || crossed;
-            if (!breached) {
-                const double log_s = log(s);
-                const double log_s_next = log(s_next);
-                const double p_cross = exp(-2.0 * (c.log_barrier - log_s) *
-                                           (c.log_barrier - log_s_next) / c.bb_denom);
-                const double u = uniform_open01_f64(philox_word0(pu, static_cast<uint32_t>(step), k));
-                breached = u < p_cross;
-            }
-            s = s_next;
-        }
-        const double vanilla = dmax(phi * (s - c.strike), 0.0);
-        const bool pays = c.out ? !breached : breached;
-        return c.discount * (pays ? vanilla : c.rebate);
-    } else {
-        double s = c.spot;
-        double sum = 0.0, log_sum = 0.0, last = c.spot;
-        double rmax = c.spot, rmin = c.spot;
-        bool breached = false;
-        for (int step = 0; step < c.n_steps; ++step) {
-            const double z = draw64(pp, static_cast<uint32_t>(step), k, neg);
-            s = s * exp(c.drift + c.vs * z);
-            if constexpr (KIND == kAsianArith) {
-                sum += s;
-            } else if constexpr (KIND == kAsianGeo) {
-                log_sum += log(s);
-            } else if constexpr (KIND == kAsianCv) {
-                sum += s;
-                log_sum += log(s);
-            } else if constexpr (KIND == kBarrier) {
-                const bool crossed = c.up ? s >= c.barrier : s <= c.barrier;
-                breached = breached || crossed;
-            } else {
-                rmax = dmax(rmax, s);
-                rmin = dmin(rmin, s);
-            }
-            last = s;
-        }
-        const double n = static_cast<double>(c.n_steps);
-        if constexpr (KIND == kAsianArith || KIND == kAsianGeo) {
-            const double avg = KIND == kAsianArith ? sum / n : exp(log_sum / n);
-            const double ref = c.floating ? (last - avg) : (avg - c.strike);
-            return c.discount * dmax(phi * ref, 0.0);
-        } else if constexpr (KIND == kAsianCv) {
-            const double a = sum / n;
-            const double g = exp(log_sum / n);
-            const double arithmetic_payoff = c.discount * dmax(phi * (a - c.strike), 0.0);
-            const double geometric_payoff = c.discount * dmax(phi * (g - c.strike), 0.0);
-            return arithmetic_payoff - (geometric_payoff - c.kv_anchor);
-        } else if constexpr (KIND == kBarrier) {
-            const double vanilla = dmax(phi * (last - c.strike), 0.0);
-            const bool pays = c.out ? !breached : breached;
-            return c.discount * (pays ? vanilla : c.rebate);
-        } else if constexpr (KIND == kLookbackFixed) {
-            return c.discount * (c.type == 0 ? dmax(rmax - c.strike, 0.0) : dmax(c.strike - rmin, 0.0));
-        } else {
-            return c.discount * (c.type == 0 ? (last - rmin) : (rmax - last));
-        }
-    }
-}
-
-template <int KIND>
-__device__ Welford slab64(const DevContract& c, const PhiloxKeys& k, uint64_t base) {
-    Welford w{0ull, 0.0, 0.0};
-    for (int j = 0; j < kPathsPerThread; ++j) {
-        const uint64_t path = base + static_cast<uint64_t>(j * kSlabThreads) + threadIdx.x;
-        if (path >= c.path_count) break;
-        double sample = sample64<KIND>(c, k, path, false);
-        if (c.antithetic) {
-            const double sample2 = sample64<KIND>(c, k, path, true);
-            sample = 0.5 * (sample + sample2);
-        }
-        welford_add(w, sample);
-    }
-    return w;
-}
 
 // ===========================================================================
 // FP32: log-space paths x = ln(S/S0), FP32 payoffs, FP64 accumulation.
@@ -335,29 +227,22 @@ __device__ Welford slab32(const DevContract& c, const PhiloxKeys& k, uint64_t ba
     return welford_from_sums(count, s1, s2);
 }
 
-template <int PREC>
 __device__ Welford run_slab(const DevContract& c, uint64_t base) {
     const PhiloxKeys k = philox_keys(c.seed);
-#define MCD_KIND_CASE(K)                                                  \
-    case K:                                                               \
-        return PREC == 0 ? slab64<K>(c, k, base) : slab32<K>(c, k, base);
     switch (c.kind) {
-        MCD_KIND_CASE(kEuropean)
-        MCD_KIND_CASE(kDigital)
-        MCD_KIND_CASE(kAsianArith)
-        MCD_KIND_CASE(kAsianGeo)
-        MCD_KIND_CASE(kAsianCv)
-        MCD_KIND_CASE(kBarrier)
-        MCD_KIND_CASE(kBarrierBridge)
-        MCD_KIND_CASE(kLookbackFixed)
-        default:
-            return PREC == 0 ? slab64<kLookbackFloating>(c, k, base)
-                             : slab32<kLookbackFloating>(c, k, base);
+        case kEuropean: return slab32<kEuropean>(c, k, base);
+        case kDigital: return slab32<kDigital>(c, k, base);
+        case kAsianArith: return slab32<kAsianArith>(c, k, base);
+        case kAsianGeo: return slab32<kAsianGeo>(c, k, base);
+        case kAsianCv: return slab32<kAsianCv>(c, k, base);
+        case kBarrier: return slab32<kBarrier>(c, k, base);
+        case kBarrierBridge: return slab32<kBarrierBridge>(c, k, base);
+        case kLookbackFixed: return slab32<kLookbackFixed>(c, k, base);
+        default: return slab32<kLookbackFloating>(c, k, base);
     }
-#undef MCD_KIND_CASE
 }
 
-template <int PREC, int MINB>
+template <int MINB>
 __global__ void __launch_bounds__(kSlabThreads, MINB)
     path_kernel(const DevContract* __restrict__ contracts, int n_contracts,
                 const uint32_t* __restrict__ item_prefix, uint32_t* __restrict__ ticket,
@@ -395,7 +280,7 @@ __global__ void __launch_bounds__(kSlabThreads, MINB)
             __syncthreads();
             continue;
         }
-        Welford w = run_slab<PREC>(c, static_cast<uint64_t>(slab) * kSlabPaths);
+        Welford w = run_slab(c, static_cast<uint64_t>(slab) * kSlabPaths);
         w = welford_warp_reduce(w);
         if (lane == 0) s_warp[warp] = w;
         __syncthreads();
@@ -413,27 +298,14 @@ struct DevMcResult {
     unsigned long long path_count;
 };
 
-// One warp per contract: lanes fold slabs lane, lane+32, ... in slab order,
-// then a fixed shuffle tree; results go to the caller's positions.
-__global__ void merge_kernel(const DevContract* __restrict__ contracts, int n_contracts,
-                             const uint32_t* __restrict__ item_prefix,
-                             const Welford* __restrict__ partials, DevMcResult* __restrict__ results) {
-    const int warp_global = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (warp_global >= n_contracts) return;
-    const uint32_t begin = item_prefix[warp_global];
-    const uint32_t count = contracts[warp_global].n_slabs;
-    Welford w{0ull, 0.0, 0.0};
-    for (uint32_t s = lane; s < count; s += 32) w = welford_merge(w, partials[begin + s]);
-    w = welford_warp_reduce(w);
-    if (lane == 0) {
-        DevMcResult r;
-        r.price = w.mean;
-        const double var = w.count < 2 ? 0.0 : w.m2 / static_cast<double>(w.count - 1);
-        r.standard_error = w.count == 0 ? 0.0 : sqrt(var / static_cast<double>(w.count));
-        r.path_count = w.count;
-        results[contracts[warp_global].orig_index] = r;
-    }
+// One CTA per contract; results go to the caller's positions.
+__global__ void __launch_bounds__(kMergeThreads)
+    merge_kernel(const DevContract* __restrict__ contracts, const uint32_t* __restrict__ item_prefix,
+                 const Welford* __restrict__ partials, DevMcResult* __restrict__ results) {
+    const int ci = blockIdx.x;
+    const MergedResult m =
+        merge_items(partials + (item_prefix[ci] - item_prefix[0]), item_prefix[ci + 1] - item_prefix[ci], 1);
+    if (threadIdx.x == 0) results[contracts[ci].orig_index] = DevMcResult{m.mean, m.standard_error, m.count};
 }
 
 // ---- parity kernels ----------------------------------------------------------
@@ -464,35 +336,12 @@ __global__ void draws_kernel(uint64_t seed, uint64_t path_begin, uint64_t n_path
     out[i] = v;
 }
 
-template <int PREC, int MINB>
+template <int MINB>
 cudaError_t launch_one(int grid, const DevContract* c, int n, const uint32_t* prefix, uint32_t* ticket,
                        Welford* partials, uint32_t* err, cudaStream_t stream) {
     cudaGetLastError();  // report this launch only
-    path_kernel<PREC, MINB><<<grid, kSlabThreads, 0, stream>>>(c, n, prefix, ticket, partials, err);
+    path_kernel<MINB><<<grid, kSlabThreads, 0, stream>>>(c, n, prefix, ticket, partials, err);
     return cudaGetLastError();
-}
-
-template <int PREC>
-cudaError_t launch_prec(int variant, int grid, const DevContract* c, int n, const uint32_t* prefix,
-                        uint32_t* ticket, Welford* partials, uint32_t* err, cudaStream_t stream) {
-    switch (variant) {
-        case 0: return launch_one<PREC, 4>(grid, c, n, prefix, ticket, partials, err, stream);
-        case 1: return launch_one<PREC, 8>(grid, c, n, prefix, ticket, partials, err, stream);
-        case 2: return launch_one<PREC, 12>(grid, c, n, prefix, ticket, partials, err, stream);
-        case 3: return launch_one<PREC, 16>(grid, c, n, prefix, ticket, partials, err, stream);
-        default: return launch_one<PREC, 6>(grid, c, n, prefix, ticket, partials, err, stream);
-    }
-}
-
-template <int PREC>
-cudaError_t occupancy_prec(int variant, int* blocks) {
-    switch (variant) {
-        case 0: return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, path_kernel<PREC, 4>, kSlabThreads, 0);
-        case 1: return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, path_kernel<PREC, 8>, kSlabThreads, 0);
-        case 2: return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, path_kernel<PREC, 12>, kSlabThreads, 0);
-        case 3: return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, path_kernel<PREC, 16>, kSlabThreads, 0);
-        default: return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, path_kernel<PREC, 6>, kSlabThreads, 0);
-    }
 }
 
 // Digest of a word array: sum over i of splitmix64's finaliser (Steele, Lea
@@ -530,28 +379,41 @@ cudaError_t launch_words_digest(const uint64_t* words, size_t n_words, uint64_t*
 
 cudaError_t launch_path_kernel(int precision, int variant, int grid, const DevContract* contracts,
                                int n_contracts, const uint32_t* item_prefix, uint32_t* ticket,
-                               Welford* partials, uint32_t* error_flag, cudaStream_t stream) {
+                               Welford* partials, uint32_t* error_flag, const FixedTables* tables,
+                               cudaStream_t stream) {
     if (precision == 0)
-        return launch_prec<0>(variant, grid, contracts, n_contracts, item_prefix, ticket, partials,
-                              error_flag, stream);
-    return launch_prec<1>(variant, grid, contracts, n_contracts, item_prefix, ticket, partials,
-                          error_flag, stream);
+        return launch_path64_kernel(variant, grid, contracts, n_contracts, item_prefix, ticket, partials, error_flag,
+                                    tables, stream);
+    switch (variant) {
+        case 0: return launch_one<4>(grid, contracts, n_contracts, item_prefix, ticket, partials, error_flag, stream);
+        case 1: return launch_one<8>(grid, contracts, n_contracts, item_prefix, ticket, partials, error_flag, stream);
+        case 2: return launch_one<12>(grid, contracts, n_contracts, item_prefix, ticket, partials, error_flag, stream);
+        case 3: return launch_one<16>(grid, contracts, n_contracts, item_prefix, ticket, partials, error_flag, stream);
+        default: return launch_one<6>(grid, contracts, n_contracts, item_prefix, ticket, partials, error_flag, stream);
+    }
 }
 
-cudaError_t path_kernel_occupancy(int precision, int variant, int* blocks_per_sm) {
-    return precision == 0 ? occupancy_prec<0>(variant, blocks_per_sm)
-                          : occupancy_prec<1>(variant, blocks_per_sm);
+cudaError_t path_kernel_occupancy(int precision, int variant, int* blocks) {
+    if (precision == 0) {  // one CTA per SM shares the fixed-point tables
+        *blocks = 1;
+        return cudaSuccess;
+    }
+    switch (variant) {
+        case 0: return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, path_kernel<4>, kSlabThreads, 0);
+        case 1: return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, path_kernel<8>, kSlabThreads, 0);
+        case 2: return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, path_kernel<12>, kSlabThreads, 0);
+        case 3: return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, path_kernel<16>, kSlabThreads, 0);
+        default: return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, path_kernel<6>, kSlabThreads, 0);
+    }
 }
 
 cudaError_t launch_merge_kernel(const DevContract* contracts, int n_contracts,
                                 const uint32_t* item_prefix, const Welford* partials,
                                 void* results, cudaStream_t stream) {
-    const int threads = 256;
-    const int blocks = (n_contracts * 32 + threads - 1) / threads;
-    if (blocks == 0) return cudaSuccess;
+    if (n_contracts == 0) return cudaSuccess;
     cudaGetLastError();
-    merge_kernel<<<blocks, threads, 0, stream>>>(contracts, n_contracts, item_prefix, partials,
-                                                 static_cast<DevMcResult*>(results));
+    merge_kernel<<<n_contracts, kMergeThreads, 0, stream>>>(contracts, item_prefix, partials,
+                                                            static_cast<DevMcResult*>(results));
     return cudaGetLastError();
 }
 

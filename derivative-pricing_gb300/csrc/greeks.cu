@@ -19,10 +19,10 @@
 //   pathwise            src/greeks/pathwise.cpp:28-55 (European), :64-147
 //                       (Asian)
 //
-// FP64 evaluates every bumped state literally (the arithmetic of five
-// separate re-prices).  FP32 shares one log-path between the spot states
-// (only the FP64 payoff is rescaled) and carries the vol-bumped states as
-// differentials: with D_i = dx_i/dvol = sqrt(dt) W_i - vol i dt, the bumped
+// This file holds the FP32 kernel; the FP64 one, which evaluates every bumped
+// state literally (five separate re-prices on one path's draws), is
+// greeks64.cu.  FP32 shares one log-path between the spot states (only the
+// FP64 payoff is rescaled) and carries the vol-bumped states as differentials: with D_i = dx_i/dvol = sqrt(dt) W_i - vol i dt, the bumped
 // log-spot is x_i +/- h D_i - h^2 i dt / 2 exactly, and its effect on a sum
 // of spots is sum S_i expm1(+/- h D_i - h^2 i dt / 2), which FP32 resolves to
 // full relative precision even for bumps of 1e-4 (a plain FP32 re-price
@@ -34,13 +34,13 @@
 #include "device_common.cuh"
 #include "engine.hpp"
 #include "greeks.hpp"
+#include "merge.cuh"
 
 namespace mcdg {
 
 namespace {
 
 __device__ __forceinline__ double dmax(double a, double b) { return (a < b) ? b : a; }
-__device__ __forceinline__ double dmin(double a, double b) { return (b < a) ? b : a; }
 
 // expm1 for the vol-bump exponents: a short Taylor series where |a| < 1/64
 // (relative error below 2e-12 there; bumps of 1e-4 give |a| ~ 1e-4), else
@@ -59,165 +59,6 @@ __device__ __forceinline__ float expm1_small(float a) {
 // without the range test of expm1_small.
 __device__ __forceinline__ float expm1_series(float a) {
     return __fmaf_rn(__fmaf_rn(a, 1.0f / 6.0f, 0.5f) * a, a, a);
-}
-
-// Likelihood-ratio scores of the first step (likelihood_ratio.cpp:45-49,
-// :140-142), with sqrt_t = sqrt(dt) of that step.
-__device__ __forceinline__ void lr_first_step(double h, double z1, double spot, double vol, double sqrt_t, double t,
-                                              double (&o)[kNumGreeks]) {
-    const double delta_score = z1 / (spot * vol * sqrt_t);
-    const double gamma_score = (z1 * z1 - vol * sqrt_t * z1 - 1.0) / (spot * spot * vol * vol * t);
-    o[kGLrDelta] = h * delta_score;
-    o[kGLrGamma] = h * gamma_score;
-}
-
-// ===========================================================================
-// FP64: five literal states (base, spot up/down, vol up/down)
-// ===========================================================================
-template <int KIND>
-__device__ void greeks64(const DevContract& c, const DevGreeks& g, const PhiloxKeys& k, uint64_t path,
-                         double (&o)[kNumGreeks]) {
-#pragma unroll
-    for (int i = 0; i < kNumGreeks; ++i) o[i] = 0.0;
-    const double phi = c.type == 0 ? 1.0 : -1.0;
-    const PhiloxPath pp = philox_path(path, 0u, k);
-    double v[5];
-    if constexpr (KIND == kEuropean || KIND == kDigital) {
-        const double z = normal_from_bits_f64(philox_word0(pp, 0u, k));
-        const double m = exp(c.drift + c.vs * z);
-        const double st[5] = {c.spot * m, (c.spot + g.h_spot) * m, (c.spot - g.h_spot) * m,
-                              c.spot * exp(g.drift_up + g.vs_up * z), c.spot * exp(g.drift_dn + g.vs_dn * z)};
-#pragma unroll
-        for (int j = 0; j < 5; ++j) {
-            if constexpr (KIND == kEuropean) {
-                v[j] = c.discount * dmax(phi * (st[j] - c.strike), 0.0);
-            } else {
-                const bool itm = phi * (st[j] - c.strike) > 0.0;
-                v[j] = c.discount * (itm ? (c.asset ? st[j] : c.cash) : 0.0);
-            }
-        }
-        const double h = v[0];
-        // likelihood_ratio.cpp:40-64
-        const double sqrt_t = g.sqrt_dt;
-        lr_first_step(h, z, c.spot, g.vol, sqrt_t, g.time, o);
-        const double vega_score = (z * z - 1.0) / g.vol - sqrt_t * z;
-        const double rho_raw = sqrt_t * z / g.vol;
-        const double theta_raw = (z * z - 1.0) / (2.0 * g.time) + g.mu * z / (g.vol * sqrt_t);
-        o[kGLrVega] = h * vega_score;
-        o[kGLrRho] = h * (rho_raw - g.time);
-        o[kGLrTheta] = h * (g.rate - theta_raw);
-        if constexpr (KIND == kEuropean) {  // pathwise.cpp:37-50
-            const double s_t = st[0];
-            const bool itm = phi * (s_t - c.strike) > 0.0;
-            const double slope = itm ? phi : 0.0;
-            const double ds_dspot = s_t / c.spot;
-            const double ds_dvol = s_t * (sqrt_t * z - g.vol * g.time);
-            const double ds_drate = s_t * g.time;
-            o[kGPwDelta] = c.discount * slope * ds_dspot;
-            o[kGPwVega] = c.discount * slope * ds_dvol;
-            o[kGPwRho] = c.discount * slope * ds_drate - g.time * h;
-        }
-    } else {
-        double s[5] = {c.spot, c.spot + g.h_spot, c.spot - g.h_spot, c.spot, c.spot};
-        double sum[5] = {0.0, 0.0, 0.0, 0.0, 0.0}, lsum[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-        double hi[5], lo[5];
-        bool br[5] = {false, false, false, false, false};
-#pragma unroll
-        for (int j = 0; j < 5; ++j) hi[j] = lo[j] = s[j];
-        double z1 = 0.0, vega_sum = 0.0, rho_sum = 0.0, cum_z = 0.0;
-        double sum_s_dvol = 0.0, sum_dlns_dvol = 0.0, sum_s_drate = 0.0, sum_dlns_drate = 0.0;
-        double last_s_dvol = 0.0, last_s_drate = 0.0;
-        for (int step = 0; step < c.n_steps; ++step) {
-            const double z = normal_from_bits_f64(philox_word0(pp, static_cast<uint32_t>(step), k));
-            if (step == 0) z1 = z;
-            vega_sum += (z * z - 1.0) / g.vol - g.sqrt_dt * z;
-            rho_sum += g.sqrt_dt * z / g.vol;
-            const double m = exp(c.drift + c.vs * z);
-            s[0] = s[0] * m;
-            s[1] = s[1] * m;
-            s[2] = s[2] * m;
-            s[3] = s[3] * exp(g.drift_up + g.vs_up * z);
-            s[4] = s[4] * exp(g.drift_dn + g.vs_dn * z);
-#pragma unroll
-            for (int j = 0; j < 5; ++j) {
-                if constexpr (KIND == kAsianArith) {
-                    sum[j] += s[j];
-                } else if constexpr (KIND == kAsianGeo) {
-                    lsum[j] += log(s[j]);
-                } else if constexpr (KIND == kBarrier) {
-                    const bool crossed = c.up ? s[j] >= c.barrier : s[j] <= c.barrier;
-                    br[j] = br[j] || crossed;
-                } else {
-                    hi[j] = dmax(hi[j], s[j]);
-                    lo[j] = dmin(lo[j], s[j]);
-                }
-            }
-            if constexpr (KIND == kAsianArith || KIND == kAsianGeo) {  // pathwise.cpp:81-98
-                cum_z += z;
-                const double i = static_cast<double>(step + 1);
-                const double dlns_dvol = -g.vol * i * g.dt + g.sqrt_dt * cum_z;
-                const double dlns_drate = i * g.dt;
-                const double ds_dvol = s[0] * dlns_dvol;
-                const double ds_drate = s[0] * dlns_drate;
-                sum_s_dvol += ds_dvol;
-                sum_dlns_dvol += dlns_dvol;
-                sum_s_drate += ds_drate;
-                sum_dlns_drate += dlns_drate;
-                last_s_dvol = ds_dvol;
-                last_s_drate = ds_drate;
-            }
-        }
-        const double n = static_cast<double>(c.n_steps);
-        double avg0 = 0.0;
-#pragma unroll
-        for (int j = 0; j < 5; ++j) {
-            if constexpr (KIND == kAsianArith || KIND == kAsianGeo) {
-                const double avg = KIND == kAsianArith ? sum[j] / n : exp(lsum[j] / n);
-                if (j == 0) avg0 = avg;
-                const double ref = c.floating ? (s[j] - avg) : (avg - c.strike);
-                v[j] = c.discount * dmax(phi * ref, 0.0);
-            } else if constexpr (KIND == kBarrier) {
-                const double vanilla = dmax(phi * (s[j] - c.strike), 0.0);
-                const bool pays = c.out ? !br[j] : br[j];
-                v[j] = c.discount * (pays ? vanilla : c.rebate);
-            } else if constexpr (KIND == kLookbackFixed) {
-                v[j] = c.discount * (c.type == 0 ? dmax(hi[j] - c.strike, 0.0) : dmax(c.strike - lo[j], 0.0));
-            } else {
-                v[j] = c.discount * (c.type == 0 ? (s[j] - lo[j]) : (hi[j] - s[j]));
-            }
-        }
-        const double h = v[0];
-        lr_first_step(h, z1, c.spot, g.vol, g.sqrt_dt, g.dt, o);
-        o[kGLrVega] = h * vega_sum;
-        o[kGLrRho] = h * (rho_sum - g.time);
-        if constexpr (KIND == kAsianArith || KIND == kAsianGeo) {  // pathwise.cpp:100-140
-            const bool arith = KIND == kAsianArith;
-            const double d_avg_dspot = avg0 / c.spot;
-            const double d_avg_dvol = arith ? sum_s_dvol / n : avg0 * (sum_dlns_dvol / n);
-            const double d_avg_drate = arith ? sum_s_drate / n : avg0 * (sum_dlns_drate / n);
-            const double d_slast_dspot = s[0] / c.spot;
-            const double ref = c.floating ? (s[0] - avg0) : (avg0 - c.strike);
-            const bool itm = phi * ref > 0.0;
-            const double slope = itm ? phi : 0.0;
-            double delta_raw, vega_raw, rate_raw;
-            if (!c.floating) {
-                delta_raw = slope * d_avg_dspot;
-                vega_raw = slope * d_avg_dvol;
-                rate_raw = slope * d_avg_drate;
-            } else {
-                delta_raw = slope * (d_slast_dspot - d_avg_dspot);
-                vega_raw = slope * (last_s_dvol - d_avg_dvol);
-                rate_raw = slope * (last_s_drate - d_avg_drate);
-            }
-            o[kGPwDelta] = c.discount * delta_raw;
-            o[kGPwVega] = c.discount * vega_raw;
-            o[kGPwRho] = c.discount * rate_raw - g.time * h;
-        }
-    }
-    o[kGPrice] = v[0];
-    o[kGFdDelta] = (v[1] - v[2]) / (2.0 * g.h_spot);
-    o[kGFdGamma] = (v[1] - 2.0 * v[0] + v[2]) / (g.h_spot * g.h_spot);
-    o[kGFdVega] = (v[3] - v[4]) / (2.0 * g.h_vol);
 }
 
 // ===========================================================================
@@ -473,12 +314,12 @@ __device__ void greeks32(const DevContract& c, const DevGreeks& g, const PhiloxK
     o[kGFdVega] = (v[3] - v[4]) * g.inv_2hv;
 }
 
-// One slab: per-thread accumulation in path order (FP64: Welford per sample;
-// FP32: count and FP64 sums), as the path engine.  The twelve accumulator
+// One slab: per-thread accumulation in path order (count and FP64 sums), as
+// the path engine.  The twelve accumulator
 // pairs live in shared memory (acc[0][i][t], acc[1][i][t]) rather than
 // registers: they are touched once per path, and the registers go to the
 // path state instead.
-template <int PREC, int KIND, bool SER = false>
+template <int KIND, bool SER = false>
 __device__ void slab_greeks(const DevContract& c, const DevGreeks& g, const PhiloxKeys& k, uint64_t base,
                             double (*acc)[kNumGreeks][kSlabThreads], Welford (&w)[kNumGreeks]) {
     const int t = threadIdx.x;
@@ -490,54 +331,35 @@ __device__ void slab_greeks(const DevContract& c, const DevGreeks& g, const Phil
         const uint64_t path = base + static_cast<uint64_t>(j * kSlabThreads) + t;
         if (path >= c.path_count) break;
         ++count;
-        if constexpr (PREC == 0) {
-            greeks64<KIND>(c, g, k, path, o);
-            const double inv = 1.0 / static_cast<double>(count);  // welford_add, one count for all outputs
+        greeks32<KIND, SER>(c, g, k, path, o);
 #pragma unroll
-            for (int i = 0; i < kNumGreeks; ++i) {
-                const double mean = acc[0][i][t];
-                const double delta = o[i] - mean;
-                const double m = mean + delta * inv;
-                acc[0][i][t] = m;
-                acc[1][i][t] += delta * (o[i] - m);
-            }
-        } else {
-            greeks32<KIND, SER>(c, g, k, path, o);
-#pragma unroll
-            for (int i = 0; i < kNumGreeks; ++i) {
-                acc[0][i][t] += o[i];
-                acc[1][i][t] = fma(o[i], o[i], acc[1][i][t]);
-            }
+        for (int i = 0; i < kNumGreeks; ++i) {
+            acc[0][i][t] += o[i];
+            acc[1][i][t] = fma(o[i], o[i], acc[1][i][t]);
         }
     }
 #pragma unroll
-    for (int i = 0; i < kNumGreeks; ++i) {
-        if constexpr (PREC == 0)
-            w[i] = Welford{count, count ? acc[0][i][t] : 0.0, count ? acc[1][i][t] : 0.0};
-        else
-            w[i] = welford_from_sums(count, acc[0][i][t], acc[1][i][t]);
-    }
+    for (int i = 0; i < kNumGreeks; ++i) w[i] = welford_from_sums(count, acc[0][i][t], acc[1][i][t]);
 }
 
-template <int PREC>
 __device__ void run_greeks_slab(const DevContract& c, const DevGreeks& g, uint64_t base,
                                 double (*acc)[kNumGreeks][kSlabThreads], Welford (&w)[kNumGreeks]) {
     const PhiloxKeys k = philox_keys(c.seed);
     switch (c.kind) {
-        case kEuropean: slab_greeks<PREC, kEuropean>(c, g, k, base, acc, w); break;
-        case kDigital: slab_greeks<PREC, kDigital>(c, g, k, base, acc, w); break;
+        case kEuropean: slab_greeks<kEuropean>(c, g, k, base, acc, w); break;
+        case kDigital: slab_greeks<kDigital>(c, g, k, base, acc, w); break;
         case kAsianArith:
-            if (g.vol_series) slab_greeks<PREC, kAsianArith, true>(c, g, k, base, acc, w);
-            else slab_greeks<PREC, kAsianArith, false>(c, g, k, base, acc, w);
+            if (g.vol_series) slab_greeks<kAsianArith, true>(c, g, k, base, acc, w);
+            else slab_greeks<kAsianArith, false>(c, g, k, base, acc, w);
             break;
-        case kAsianGeo: slab_greeks<PREC, kAsianGeo>(c, g, k, base, acc, w); break;
-        case kBarrier: slab_greeks<PREC, kBarrier>(c, g, k, base, acc, w); break;
-        case kLookbackFixed: slab_greeks<PREC, kLookbackFixed>(c, g, k, base, acc, w); break;
-        default: slab_greeks<PREC, kLookbackFloating>(c, g, k, base, acc, w); break;
+        case kAsianGeo: slab_greeks<kAsianGeo>(c, g, k, base, acc, w); break;
+        case kBarrier: slab_greeks<kBarrier>(c, g, k, base, acc, w); break;
+        case kLookbackFixed: slab_greeks<kLookbackFixed>(c, g, k, base, acc, w); break;
+        default: slab_greeks<kLookbackFloating>(c, g, k, base, acc, w); break;
     }
 }
 
-template <int PREC, int MINB>
+template <int MINB>
 __global__ void __launch_bounds__(kSlabThreads, MINB)
     greeks_kernel(const DevContract* __restrict__ contracts, const DevGreeks* __restrict__ greeks, int n_contracts,
                   const uint32_t* __restrict__ item_prefix, uint32_t total_items, uint32_t* __restrict__ ticket,
@@ -574,7 +396,7 @@ __global__ void __launch_bounds__(kSlabThreads, MINB)
             continue;
         }
         Welford w[kNumGreeks];
-        run_greeks_slab<PREC>(s_contract, s_greeks, static_cast<uint64_t>(slab) * kSlabPaths, s_acc, w);
+        run_greeks_slab(s_contract, s_greeks, static_cast<uint64_t>(slab) * kSlabPaths, s_acc, w);
 #pragma unroll
         for (int i = 0; i < kNumGreeks; ++i) {
             const Welford r = welford_warp_reduce(w[i]);
@@ -590,34 +412,27 @@ __global__ void __launch_bounds__(kSlabThreads, MINB)
     }
 }
 
-// One warp per (contract, output): the path engine's merge.
-__global__ void greeks_merge_kernel(const DevContract* __restrict__ contracts, int n_contracts,
-                                    const uint32_t* __restrict__ item_prefix, const Welford* __restrict__ partials,
-                                    double* __restrict__ out) {
-    const int warp_global = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (warp_global >= n_contracts * kNumGreeks) return;
-    const int ci = warp_global / kNumGreeks, gi = warp_global % kNumGreeks;
-    const uint32_t begin = item_prefix[ci];
-    const uint32_t count = contracts[ci].n_slabs;
-    Welford w{0ull, 0.0, 0.0};
-    for (uint32_t s = lane; s < count; s += 32)
-        w = welford_merge(w, partials[(static_cast<size_t>(begin) + s) * kNumGreeks + gi]);
-    w = welford_warp_reduce(w);
-    if (lane == 0) {
+// One CTA per (contract, output): the path engine's merge.
+__global__ void __launch_bounds__(kMergeThreads)
+    greeks_merge_kernel(const DevContract* __restrict__ contracts, const uint32_t* __restrict__ item_prefix,
+                        const Welford* __restrict__ partials, double* __restrict__ out) {
+    const int ci = blockIdx.x, gi = blockIdx.y;
+    const size_t begin = item_prefix[ci] - item_prefix[0];
+    const MergedResult m =
+        merge_items(partials + begin * kNumGreeks + gi, item_prefix[ci + 1] - item_prefix[ci], kNumGreeks);
+    if (threadIdx.x == 0) {
         double* o = out + static_cast<size_t>(contracts[ci].orig_index) * kGreeksOutStride;
-        const double var = w.count < 2 ? 0.0 : w.m2 / static_cast<double>(w.count - 1);
-        o[2 * gi] = w.mean;
-        o[2 * gi + 1] = w.count == 0 ? 0.0 : sqrt(var / static_cast<double>(w.count));
-        if (gi == 0) o[2 * kNumGreeks] = static_cast<double>(w.count);
+        o[2 * gi] = m.mean;
+        o[2 * gi + 1] = m.standard_error;
+        if (gi == 0) o[2 * kNumGreeks] = static_cast<double>(m.count);
     }
 }
 
-template <int PREC, int MINB>
+template <int MINB>
 cudaError_t launch_one(int grid, const DevContract* c, const DevGreeks* g, int n, const uint32_t* prefix,
                        uint32_t total, uint32_t* ticket, Welford* partials, uint32_t* err, cudaStream_t stream) {
     cudaGetLastError();
-    greeks_kernel<PREC, MINB><<<grid, kSlabThreads, 0, stream>>>(c, g, n, prefix, total, ticket, partials, err);
+    greeks_kernel<MINB><<<grid, kSlabThreads, 0, stream>>>(c, g, n, prefix, total, ticket, partials, err);
     return cudaGetLastError();
 }
 
@@ -626,21 +441,16 @@ cudaError_t launch_one(int grid, const DevContract* c, const DevGreeks* g, int n
 cudaError_t launch_greeks_kernel(int precision, int variant, int grid, const DevContract* contracts,
                                  const DevGreeks* greeks, int n_contracts, const uint32_t* item_prefix,
                                  uint32_t total_items, uint32_t* ticket, Welford* partials,
-                                 uint32_t* error_flag, cudaStream_t stream) {
+                                 uint32_t* error_flag, const FixedTables* tables, cudaStream_t stream) {
+    if (precision == 0)
+        return launch_greeks64_kernel(grid, contracts, greeks, n_contracts, item_prefix, ticket, partials, error_flag,
+                                      tables, stream);
 #define MCD_GREEKS_ARGS grid, contracts, greeks, n_contracts, item_prefix, total_items, ticket, partials, error_flag, stream
-    if (precision == 0) {
-        switch (variant) {
-            case 0: return launch_one<0, 2>(MCD_GREEKS_ARGS);
-            case 1: return launch_one<0, 4>(MCD_GREEKS_ARGS);
-            case 2: return launch_one<0, 6>(MCD_GREEKS_ARGS);
-            default: return launch_one<0, 8>(MCD_GREEKS_ARGS);
-        }
-    }
     switch (variant) {
-        case 0: return launch_one<1, 2>(MCD_GREEKS_ARGS);
-        case 1: return launch_one<1, 4>(MCD_GREEKS_ARGS);
-        case 2: return launch_one<1, 6>(MCD_GREEKS_ARGS);
-        default: return launch_one<1, 8>(MCD_GREEKS_ARGS);
+        case 0: return launch_one<2>(MCD_GREEKS_ARGS);
+        case 1: return launch_one<4>(MCD_GREEKS_ARGS);
+        case 2: return launch_one<6>(MCD_GREEKS_ARGS);
+        default: return launch_one<8>(MCD_GREEKS_ARGS);
     }
 #undef MCD_GREEKS_ARGS
 }
@@ -648,29 +458,22 @@ cudaError_t launch_greeks_kernel(int precision, int variant, int grid, const Dev
 cudaError_t launch_greeks_merge(const DevContract* contracts, int n_contracts, const uint32_t* item_prefix,
                                 const Welford* partials, double* out, cudaStream_t stream) {
     cudaGetLastError();
-    const long long warps = static_cast<long long>(n_contracts) * kNumGreeks;
-    const int threads = 256;
-    const long long blocks = (warps * 32 + threads - 1) / threads;
-    if (blocks > 0)
-        greeks_merge_kernel<<<static_cast<unsigned>(blocks), threads, 0, stream>>>(contracts, n_contracts, item_prefix,
-                                                                                  partials, out);
+    if (n_contracts > 0)
+        greeks_merge_kernel<<<dim3(static_cast<unsigned>(n_contracts), kNumGreeks), kMergeThreads, 0, stream>>>(
+            contracts, item_prefix, partials, out);
     return cudaGetLastError();
 }
 
 cudaError_t greeks_kernel_occupancy(int precision, int variant, int* blocks) {
-    if (precision == 0) {
-        switch (variant) {
-            case 0: return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, greeks_kernel<0, 2>, kSlabThreads, 0);
-            case 1: return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, greeks_kernel<0, 4>, kSlabThreads, 0);
-            case 2: return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, greeks_kernel<0, 6>, kSlabThreads, 0);
-            default: return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, greeks_kernel<0, 8>, kSlabThreads, 0);
-        }
+    if (precision == 0) {  // one CTA per SM shares the fixed-point tables
+        *blocks = 1;
+        return cudaSuccess;
     }
     switch (variant) {
-        case 0: return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, greeks_kernel<1, 2>, kSlabThreads, 0);
-        case 1: return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, greeks_kernel<1, 4>, kSlabThreads, 0);
-        case 2: return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, greeks_kernel<1, 6>, kSlabThreads, 0);
-        default: return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, greeks_kernel<1, 8>, kSlabThreads, 0);
+        case 0: return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, greeks_kernel<2>, kSlabThreads, 0);
+        case 1: return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, greeks_kernel<4>, kSlabThreads, 0);
+        case 2: return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, greeks_kernel<6>, kSlabThreads, 0);
+        default: return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, greeks_kernel<8>, kSlabThreads, 0);
     }
 }
 

@@ -21,6 +21,8 @@ namespace {
 
 enum { kGDev = 21, kGConst = 22, kGPrefix = 23, kGPart = 24, kGOut = 25, kGFlags = 26 };
 
+constexpr uint64_t kGreeksRangeItems = 1ull << 23;  // 2.4 GB of FP64 partials
+
 // Bits of mcd_greeks_result::defined.
 uint32_t defined_bits(int kind) {
     uint32_t bits = 0xFu | (0xFu << kGLrDelta);  // price, finite differences, LR delta..rho
@@ -29,8 +31,8 @@ uint32_t defined_bits(int kind) {
     return bits;
 }
 
-int plan_greeks(Ctx& ctx, const mcd_contract* cs, size_t n, double spot_rel, double vol_rel, BatchPlan& plan,
-                std::vector<DevGreeks>& consts) {
+int plan_greeks(Ctx& ctx, const mcd_contract* cs, size_t n, int precision, double spot_rel, double vol_rel,
+                BatchPlan& plan, std::vector<DevGreeks>& consts) {
     if (!(spot_rel > 0.0 && spot_rel < 1.0) || !(vol_rel > 0.0 && vol_rel < 1.0))
         return ctx.fail(MCD_ERR_INVALID_ARGUMENT, "bump sizes must be in (0, 1) relative to spot and vol");
     for (size_t i = 0; i < n; ++i) {
@@ -43,11 +45,11 @@ int plan_greeks(Ctx& ctx, const mcd_contract* cs, size_t n, double spot_rel, dou
         if (c.product == MCD_PRODUCT_BARRIER && c.brownian_bridge)
             return ctx.fail(MCD_ERR_UNSUPPORTED, "contract " + std::to_string(i) + ": no Greeks for the Brownian-bridge barrier");
     }
-    int rc = plan_batch(ctx, cs, n, plan);
+    int rc = plan_batch(ctx, cs, n, precision == 0 ? kGreeksRangeItems : 0, plan);
     if (rc) return rc;
     consts.resize(n);
     for (size_t j = 0; j < n; ++j) {
-        const DevContract& d = plan.dev[j];
+        DevContract& d = plan.dev[j];
         const mcd_contract& in = cs[d.orig_index];
         DevGreeks& g = consts[j];
         std::memset(&g, 0, sizeof g);
@@ -80,6 +82,23 @@ int plan_greeks(Ctx& ctx, const mcd_contract* cs, size_t n, double spot_rel, dou
         g.inv_spot = 1.0 / in.spot;
         g.inv_2t = 1.0 / (2.0 * in.time);
         g.mu_over_vol_sqrt_t = g.mu / (in.vol * g.sqrt_dt);
+        // FP64 kernel: the vol states in the base's units.  A vol bump below
+        // 100 % makes the log-spot's bound less than four times the base's,
+        // which the two spare bits of the units take; beyond the exponent
+        // range of a double the contract leaves the fixed-point form.
+        if (d.frac != 0 && in.vol * std::sqrt(in.time) * (1.0 + vol_rel) > 8.0) d.frac = 0;
+        if (d.frac != 0) {
+            constexpr double kInvLn2 = 1.44269504088896340736;
+            fixed_step(g.drift_up * kInvLn2, g.vs_up * kInvLn2, d.frac, &g.y_drift_up, &g.y_drift_lo_up, &g.y_vs_up);
+            fixed_step(g.drift_dn * kInvLn2, g.vs_dn * kInvLn2, d.frac, &g.y_drift_dn, &g.y_drift_lo_dn, &g.y_vs_dn);
+            if (in.product == MCD_PRODUCT_BARRIER) {
+                g.y_barrier_su = fixed_barrier(g.log_h_rel_up, d.frac);
+                g.y_barrier_sd = fixed_barrier(g.log_h_rel_dn, d.frac);
+            }
+            g.x_unit = std::ldexp(1.0 / kInvLn2, -d.frac);
+            g.z_unit = 1.0 / std::ldexp(d.vs * kInvLn2, d.frac);
+            g.dvol_drift = d.drift / in.vol + in.vol * g.dt;
+        }
         // The vol-bump exponent is h_vol D - h_vol^2 i dt / 2 with |D| below
         // 8 sqrt(T) + vol T on all but > 8-sigma paths.
         g.vol_series = g.h_vol * (8.0 * std::sqrt(in.time) + in.vol * in.time) <= 1e-2 ? 1 : 0;
@@ -106,7 +125,7 @@ int prepare_greeks(Ctx& ctx, int precision, const BatchPlan& plan, const std::ve
     int rc = ctx.reserve(ctx.ext[kGDev], sizeof(DevContract) * n, "greeks contracts");
     if (!rc) rc = ctx.reserve(ctx.ext[kGConst], sizeof(DevGreeks) * n, "greeks constants");
     if (!rc) rc = ctx.reserve(ctx.ext[kGPrefix], sizeof(uint32_t) * (n + 1), "greeks prefix");
-    if (!rc) rc = ctx.reserve(ctx.ext[kGPart], sizeof(Welford) * kNumGreeks * std::max<uint32_t>(plan.total_items, 1),
+    if (!rc) rc = ctx.reserve(ctx.ext[kGPart], sizeof(Welford) * kNumGreeks * std::max<uint32_t>(plan.max_items, 1),
                               "greeks partials");
     if (!rc) rc = ctx.reserve(ctx.ext[kGOut], sizeof(double) * kGreeksOutStride * n, "greeks results");
     if (!rc) rc = ctx.reserve(ctx.ext[kGFlags], 256, "greeks flags");
@@ -123,9 +142,9 @@ int prepare_greeks(Ctx& ctx, int precision, const BatchPlan& plan, const std::ve
     int variant = 0, grid = 0;
     rc = greeks_grid(ctx, precision, variant, grid);
     if (rc) return rc;
-    const GraphKey key{precision, variant, grid, n, plan.total_items, ctx.ext[kGDev].ptr, ctx.ext[kGPrefix].ptr,
+    const GraphKey key{precision, variant, grid, n, plan.max_items, ctx.ext[kGDev].ptr, ctx.ext[kGPrefix].ptr,
                        ctx.ext[kGPart].ptr, ctx.ext[kGOut].ptr};
-    if (ctx.greeks_graph && ctx.greeks_key == key) {
+    if (ctx.greeks_graph && ctx.greeks_key == key && plan.ranges.size() == 2) {
         *out = ctx.greeks_graph;
         return MCD_OK;
     }
@@ -138,22 +157,26 @@ int prepare_greeks(Ctx& ctx, int precision, const BatchPlan& plan, const std::ve
     e = cudaStreamBeginCapture(ctx.stream, cudaStreamCaptureModeThreadLocal);
     if (e != cudaSuccess) return ctx.cuda_fail(e, "greeks begin capture");
     uint32_t* flags = static_cast<uint32_t*>(ctx.ext[kGFlags].ptr);
-    cudaError_t e1 = cudaMemsetAsync(flags, 0, 2 * sizeof(uint32_t), ctx.stream);
-    cudaError_t e2 = launch_greeks_kernel(precision, variant, grid, static_cast<const DevContract*>(ctx.ext[kGDev].ptr),
-                                          static_cast<const DevGreeks*>(ctx.ext[kGConst].ptr), static_cast<int>(n),
-                                          static_cast<const uint32_t*>(ctx.ext[kGPrefix].ptr), plan.total_items,
-                                          flags, static_cast<Welford*>(ctx.ext[kGPart].ptr), flags + 1, ctx.stream);
-    cudaError_t e3 = launch_greeks_merge(static_cast<const DevContract*>(ctx.ext[kGDev].ptr), static_cast<int>(n),
-                                         static_cast<const uint32_t*>(ctx.ext[kGPrefix].ptr),
-                                         static_cast<const Welford*>(ctx.ext[kGPart].ptr),
-                                         static_cast<double*>(ctx.ext[kGOut].ptr), ctx.stream);
+    cudaError_t el = cudaSuccess;
+    for (size_t r = 0; r + 1 < plan.ranges.size() && el == cudaSuccess; ++r) {
+        const uint32_t first = plan.ranges[r];
+        const int count = static_cast<int>(plan.ranges[r + 1] - first);
+        const DevContract* dev = static_cast<const DevContract*>(ctx.ext[kGDev].ptr) + first;
+        const uint32_t* prefix = static_cast<const uint32_t*>(ctx.ext[kGPrefix].ptr) + first;
+        Welford* partials = static_cast<Welford*>(ctx.ext[kGPart].ptr);
+        el = cudaMemsetAsync(flags, 0, (r == 0 ? 2 : 1) * sizeof(uint32_t), ctx.stream);
+        if (el == cudaSuccess)
+            el = launch_greeks_kernel(precision, variant, grid, dev,
+                                      static_cast<const DevGreeks*>(ctx.ext[kGConst].ptr) + first, count, prefix,
+                                      plan.max_items, flags, partials, flags + 1, ctx.tables, ctx.stream);
+        if (el == cudaSuccess)
+            el = launch_greeks_merge(dev, count, prefix, partials, static_cast<double*>(ctx.ext[kGOut].ptr), ctx.stream);
+    }
     e = cudaStreamEndCapture(ctx.stream, &graph);
-    for (cudaError_t ei : {e1, e2, e3}) {
-        if (ei != cudaSuccess) {
-            if (graph) cudaGraphDestroy(graph);
-            cudaGetLastError();
-            return ctx.cuda_fail(ei, "greeks capture");
-        }
+    if (el != cudaSuccess) {
+        if (graph) cudaGraphDestroy(graph);
+        cudaGetLastError();
+        return ctx.cuda_fail(el, "greeks capture");
     }
     if (e != cudaSuccess) return ctx.cuda_fail(e, "greeks end capture");
     cudaGraphExec_t exec = nullptr;
@@ -194,7 +217,7 @@ int greeks_batch(Ctx& ctx, const mcd_contract* cs, size_t n, double spot_rel, do
     if (!cs || !results) return ctx.fail(MCD_ERR_INVALID_ARGUMENT, "null array");
     BatchPlan plan;
     std::vector<DevGreeks> consts;
-    int rc = plan_greeks(ctx, cs, n, spot_rel, vol_rel, plan, consts);
+    int rc = plan_greeks(ctx, cs, n, precision, spot_rel, vol_rel, plan, consts);
     if (rc) return rc;
     cudaGraphExec_t exec = nullptr;
     rc = prepare_greeks(ctx, precision, plan, consts, &exec);
@@ -295,7 +318,7 @@ int mcd_greeks_autotune(mcd_ctx* handle, const mcd_contract* contracts, size_t n
     if (n == 0 || !contracts) return ctx->fail(MCD_ERR_INVALID_ARGUMENT, "empty tuning batch");
     BatchPlan plan;
     std::vector<DevGreeks> consts;
-    int rc = plan_greeks(*ctx, contracts, n, spot_bump_rel, vol_bump_rel, plan, consts);
+    int rc = plan_greeks(*ctx, contracts, n, precision, spot_bump_rel, vol_bump_rel, plan, consts);
     if (rc) return rc;
     const LaunchShape saved = ctx->greeks_shape[precision];
     double best = 1e300;

@@ -157,7 +157,7 @@ int plan_qmc(Ctx& ctx, const mcd_contract* cs, size_t n, BatchPlan& plan, std::v
         if (c.product >= MCD_PRODUCT_ASIAN && c.monitoring_points > kSobolDims)
             return ctx.fail(MCD_ERR_INVALID_ARGUMENT, who + "monitoring_points must be <= MCD_SOBOL_MAX_DIMS (256)");
     }
-    int rc = plan_batch(ctx, cs, n, plan);
+    int rc = plan_batch(ctx, cs, n, 0, plan);
     if (rc) return rc;
     std::map<int, uint32_t> offset_of;
     programs.clear();
@@ -203,7 +203,7 @@ int qmc_batch(Ctx& ctx, const mcd_contract* cs, size_t n, int precision, mcd_mc_
     if (!rc) rc = ctx.reserve(ctx.ext[kQConst], sizeof(DevQmc) * n, "qmc constants");
     if (!rc) rc = ctx.reserve(ctx.ext[kQDev], sizeof(DevContract) * n, "qmc contracts");
     if (!rc) rc = ctx.reserve(ctx.ext[kQPrefix], sizeof(uint32_t) * (n + 1), "qmc prefix");
-    if (!rc) rc = ctx.reserve(ctx.ext[kQPart], sizeof(Welford) * std::max<uint32_t>(plan.total_items, 1), "qmc partials");
+    if (!rc) rc = ctx.reserve(ctx.ext[kQPart], sizeof(Welford) * std::max<uint32_t>(plan.max_items, 1), "qmc partials");
     if (!rc) rc = ctx.reserve(ctx.ext[kQOut], sizeof(mcd_mc_result) * n, "qmc results");
     if (!rc) rc = ctx.reserve(ctx.ext[kQFlags], 256, "qmc flags");
     if (rc) return rc;
@@ -231,7 +231,7 @@ int qmc_batch(Ctx& ctx, const mcd_contract* cs, size_t n, int precision, mcd_mc_
     cudaError_t e1 = cudaMemsetAsync(flags, 0, 2 * sizeof(uint32_t), ctx.stream);
     cudaError_t e2 = launch_qmc_kernel(precision, grid, static_cast<const DevContract*>(ctx.ext[kQDev].ptr),
                                        static_cast<const DevQmc*>(ctx.ext[kQConst].ptr), static_cast<int>(n),
-                                       static_cast<const uint32_t*>(ctx.ext[kQPrefix].ptr), plan.total_items,
+                                       static_cast<const uint32_t*>(ctx.ext[kQPrefix].ptr), plan.max_items,
                                        static_cast<const BridgeNode*>(ctx.ext[kQProg].ptr),
                                        static_cast<const uint32_t*>(ctx.ext[kQDirs].ptr), flags,
                                        static_cast<Welford*>(ctx.ext[kQPart].ptr), flags + 1, ctx.stream);

@@ -14,17 +14,19 @@
  * instead and reports MCD_ERR_INVALID_ARGUMENT.
  *
  * Precision (mcd_precision):
- *   MCD_PRECISION_FP64  the reference's arithmetic in FP64 on the GPU (Acklam
- *                       inverse CDF with its Halley step, multiplicative GBM
- *                       steps); identical draws; prices agree with the CPU
- *                       reference to ~1e-12 relative.
+ *   MCD_PRECISION_FP64  FP64 accuracy on identical draws; prices agree with
+ *                       the CPU reference to ~1e-12 relative (GBM pricers and
+ *                       Greeks: 64-bit fixed-point paths, exact to 1e-17 per
+ *                       draw; elsewhere the reference's operations in FP64).
  *   MCD_PRECISION_FP32  the same Philox draws (same counters, word 0) turned
  *                       into FP32 normals; paths evolve in FP32 (log space);
  *                       payoffs are accumulated and merged in FP64.
  *
  * Results are bitwise identical for a given precision regardless of launch
  * configuration (grid size, kernel variant): paths are grouped into fixed
- * slabs of MCD_SLAB_PATHS and every reduction tree is fixed by slab index.
+ * slabs of MCD_SLAB_PATHS (FP64 GBM pricers: smaller units whose size depends
+ * on the contract's path count alone) and every reduction tree is fixed by
+ * slab or unit index.
  */
 #ifndef MCD_GPU_H
 #define MCD_GPU_H
@@ -197,7 +199,8 @@ int mcd_price_batch_static(const mcd_contract* contracts, size_t n, int precisio
                            size_t error_capacity);
 
 /* Launch shape of the persistent path kernel.  variant 0..4 selects the
- * register budget (__launch_bounds__ min blocks 4/8/12/16/6), ctas_per_sm the
+ * register budget (FP32: __launch_bounds__ min blocks 4/8/12/16/6; FP64:
+ * 512/1024/1024/1024/768 threads in the SM's one CTA), ctas_per_sm the
  * grid (SM count x ctas_per_sm).  0 restores the autotuned/default choice.
  * Results do not depend on either. */
 int mcd_set_launch_shape(mcd_ctx* ctx, int precision, int variant, int ctas_per_sm);
