@@ -112,7 +112,7 @@ struct Ctx {
     DeviceBuffer ext[48];
 
     // Sensitivity engine (greeks_api.cpp): launch shape and the last graph.
-    LaunchShape greeks_shape[2];
+    LaunchShape greeks_shape[2] = {{1, 0}, {3, 0}};  // FP32: 8 CTAs per SM (64 registers)
     cudaGraphExec_t greeks_graph = nullptr;
     GraphKey greeks_key{};
 

@@ -89,57 +89,11 @@ __device__ __forceinline__ double exp2_units(int64_t y, int frac, const FixedSha
     return __longlong_as_double(static_cast<long long>(double_bits(m, static_cast<int>(y >> frac))));
 }
 
-// Philox4x32-10 word 0 with round 0 and the products of round 1 taken apart:
-// of the counter {path_lo, path_hi, draw, stream} round 0 mixes the path and
-// the stream into words 2 and 3 and the draw into words 0 and 1, so round 1's
-// two products depend on the draw alone (PhiloxStep: one per warp and step,
-// path_hi being the same for a unit of paths) and on the path alone
-// (PhiloxRow: once per path).  A draw is left with rounds 2 to 9: 13 wide
-// products instead of 18.
-struct alignas(16) PhiloxStep {
-    uint32_t a, b, c;  // lo(M1 draw) ^ k0[1], hi(M0 w0) ^ k1[1], lo(M0 w0) ^ k1[2]
-    uint32_t carry;    // this step's carry of the drift's fraction below 2^-F (drift_carry)
-};
-struct PhiloxRow {
-    uint32_t a, b, c;  // hi(M1 w2), lo(M1 w2) ^ k0[2], lo(M0 path_lo)
-};
-
-__device__ __forceinline__ PhiloxStep philox_step(uint32_t draw, uint32_t path_hi, const PhiloxKeys& k) {
-    const uint64_t p = static_cast<uint64_t>(kPhiloxM1) * draw;
-    const uint32_t w0 = static_cast<uint32_t>(p >> 32) ^ path_hi ^ k.k0[0];
-    const uint64_t q = static_cast<uint64_t>(kPhiloxM0) * w0;
-    return PhiloxStep{static_cast<uint32_t>(p) ^ k.k0[1], static_cast<uint32_t>(q >> 32) ^ k.k1[1],
-                      static_cast<uint32_t>(q) ^ k.k1[2], 0u};
-}
-
 // A drift of hi + lo 2^-32 units per step: what step d adds to d whole steps'
 // hi when the running sum of lo is cut to whole units (0 or 1), so that the
 // drift's rounding does not add up over the steps.
 __device__ __forceinline__ uint32_t drift_carry(uint32_t d, uint32_t lo) {
     return static_cast<uint32_t>((static_cast<uint64_t>(d) * lo & 0xFFFFFFFFull) + lo >> 32);
-}
-
-__device__ __forceinline__ PhiloxRow philox_row(uint32_t path_lo, uint32_t stream, const PhiloxKeys& k) {
-    const uint64_t p = static_cast<uint64_t>(kPhiloxM0) * path_lo;
-    const uint32_t w2 = static_cast<uint32_t>(p >> 32) ^ stream ^ k.k1[0];
-    const uint64_t q = static_cast<uint64_t>(kPhiloxM1) * w2;
-    return PhiloxRow{static_cast<uint32_t>(q >> 32), static_cast<uint32_t>(q) ^ k.k0[2], static_cast<uint32_t>(p)};
-}
-
-__device__ __forceinline__ uint32_t philox_word0(const PhiloxRow& r, const PhiloxStep& s, const PhiloxKeys& k) {
-    uint32_t c0 = r.a ^ s.a, c2 = r.c ^ s.b;
-    uint32_t x1 = r.b, x3 = s.c;  // words 1 and 3 with the next round's keys
-#pragma unroll
-    for (int i = 2; i < 8; ++i) {
-        const uint64_t p0 = static_cast<uint64_t>(kPhiloxM0) * c0;
-        const uint64_t p1 = static_cast<uint64_t>(kPhiloxM1) * c2;
-        c0 = static_cast<uint32_t>(p1 >> 32) ^ x1;
-        c2 = static_cast<uint32_t>(p0 >> 32) ^ x3;
-        x1 = static_cast<uint32_t>(p1) ^ k.k0[i + 1];
-        x3 = static_cast<uint32_t>(p0) ^ k.k1[i + 1];
-    }
-    const uint32_t w2 = __umulhi(kPhiloxM0, c0) ^ x3;
-    return __umulhi(kPhiloxM1, w2) ^ (kPhiloxM1 * c2) ^ k.k0[9];
 }
 
 }  // namespace mcdg

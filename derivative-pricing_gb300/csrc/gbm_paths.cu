@@ -11,11 +11,20 @@
 // j = 0..31, so the Philox counters of a warp are consecutive path indices.
 //
 // Determinism.  A slab's Welford triple depends only on the slab: per-thread
-// accumulation in j order, then a fixed warp shuffle tree and a fixed 4-warp
-// tree.  The merge kernel folds a contract's slabs in a fixed tree (merge.cuh).
+// shifted sums in j order (unit_sums.cuh), then a fixed warp shuffle tree and a
+// fixed 4-warp tree.  The merge kernel folds a contract's slabs in a fixed tree (merge.cuh).
 // Grid size and kernel variant (register budget) only decide who
 // computes an item, never the arithmetic, so results are bitwise identical
 // across launch shapes.
+//
+// Bound: the FMA pipes.  A 32x32->64 product occupies them for 4.3 cycles of a
+// scheduler (measured; an FFMA 1.1, and the two do not overlap), so a
+// path-step's 12 wide products, three half products and 16 FP32 operations
+// take 82 cycles; measured 94 on the 4096-contract book.  Products that depend
+// on the draw alone come from a table per slab, those of the path alone are
+// taken once per path (PhiloxStep, PhiloxRow): 18 products -> 14.5.  The book
+// 313 -> 253 ms at 8 CTAs per SM (294 before at its best launch shape), of
+// which 7 ms from sums instead of Welford merges in the reductions.
 //
 // Reference semantics restated per kind (src/pricers/monte_carlo.cpp):
 //   terminal products :135-149, path-dependent loop :154-177, Brownian-bridge
@@ -28,6 +37,7 @@
 #include "device_common.cuh"
 #include "engine.hpp"
 #include "merge.cuh"
+#include "unit_sums.cuh"
 
 namespace mcdg {
 
@@ -36,209 +46,205 @@ namespace {
 // ===========================================================================
 // FP32: log-space paths x = ln(S/S0), FP32 payoffs, FP64 accumulation.
 // ===========================================================================
-__device__ __forceinline__ float draw32(const PhiloxPath& pp, uint32_t step, const PhiloxKeys& k,
-                                        bool neg) {
-    const float z = normal_from_bits_f32(philox_word0(pp, step, k));
-    return neg ? -z : z;
+// Philox words of the next kStepTable steps, one table per CTA: the products
+// that depend on the draw alone, computed once per slab (contracts of more
+// steps refill it along every path).
+constexpr int kStepTable = 256;
+
+__device__ __forceinline__ void fill_steps(PhiloxStep* table, int first, uint32_t path_hi, const PhiloxKeys& k) {
+    for (int d = threadIdx.x; d < kStepTable; d += kSlabThreads)
+        table[d] = philox_step(static_cast<uint32_t>(first + d), path_hi, k);
 }
 
-// Path-dependent products (Asians, discrete barrier, lookbacks), NP paths
-// (or antithetic halves) at once: their draws are independent dependency
-// chains, so interleaving them gives every warp NP-fold instruction-level
-// parallelism.  Each path's arithmetic is the single-path one, so the samples
-// do not depend on NP.
-template <int KIND, int NP>
-__device__ __forceinline__ void path_dependent32(const DevContract& c, const PhiloxKeys& k,
-                                                 const PhiloxPath (&pp)[NP], const bool (&neg)[NP],
-                                                 double (&out)[NP]) {
-    const float phi = c.type == 0 ? 1.0f : -1.0f;
-    const float mu = static_cast<float>(c.drift);
-    const float sg = static_cast<float>(c.vs);
-    const float s0 = static_cast<float>(c.spot);
-    const float strike = static_cast<float>(c.strike);
-    const float lnh = static_cast<float>(c.log_h_rel);
-    float x[NP], acc[NP], acc2[NP], xmax[NP], xmin[NP];  // log path, sum of S/S0, sum of x, extrema
-    bool breached[NP];
+// Path-dependent products (Asians, barriers, lookbacks), two paths at once (or
+// the two halves of an antithetic sample, which share their draws): two
+// independent dependency chains per thread.  Each path's arithmetic does not
+// depend on its partner.
+template <int KIND>
+struct Pair32 {
+    float x[2], acc[2], acc2[2], xmax[2], xmin[2];  // log path, sum of S/S0, sum of x, extrema
+    bool breached[2];
+
+    __device__ __forceinline__ Pair32() {
 #pragma unroll
-    for (int p = 0; p < NP; ++p) {
-        x[p] = acc[p] = acc2[p] = xmax[p] = xmin[p] = 0.0f;
-        breached[p] = false;
+        for (int p = 0; p < 2; ++p) {
+            x[p] = acc[p] = acc2[p] = xmax[p] = xmin[p] = 0.0f;
+            breached[p] = false;
+        }
     }
-    for (int step = 0; step < c.n_steps; ++step) {
-#pragma unroll
-        for (int p = 0; p < NP; ++p) {
-            const float z = draw32(pp[p], static_cast<uint32_t>(step), k, neg[p]);
-            x[p] = __fmaf_rn(sg, z, x[p] + mu);
-            if constexpr (KIND == kAsianArith) {
-                acc[p] += __expf(x[p]);
-            } else if constexpr (KIND == kAsianGeo) {
-                acc2[p] += x[p];
-            } else if constexpr (KIND == kAsianCv) {
-                acc[p] += __expf(x[p]);
-                acc2[p] += x[p];
-            } else if constexpr (KIND == kBarrier) {
-                const bool crossed = c.up ? x[p] >= lnh : x[p] <= lnh;
-                breached[p] = breached[p] || crossed;
+
+    template <bool ANTI>
+    __device__ __forceinline__ void advance(const DevContract& c, const PhiloxKeys& k, const PhiloxStep* table,
+                                            int count, const PhiloxRow (&row)[2], const PhiloxRow (&row_u)[2]) {
+        const float mu = static_cast<float>(c.drift), sg = static_cast<float>(c.vs);
+        const float lnh = static_cast<float>(c.log_h_rel);
+        const float inv_denom = KIND == kBarrierBridge ? static_cast<float>(-2.0 / c.bb_denom) : 0.0f;
+        for (int d = 0; d < count; ++d) {
+            const PhiloxStep st = table[d];
+            float z[2];
+            if constexpr (ANTI) {
+                const uint32_t bits[1] = {philox_word0(row[0], st, k)};
+                float one[1];
+                normals_from_bits_f32<1>(bits, one);
+                z[0] = one[0];
+                z[1] = -one[0];
             } else {
-                xmax[p] = fmaxf(xmax[p], x[p]);
-                xmin[p] = fminf(xmin[p], x[p]);
+                const uint32_t bits[2] = {philox_word0(row[0], st, k), philox_word0(row[1], st, k)};
+                normals_from_bits_f32<2>(bits, z);
+            }
+#pragma unroll
+            for (int p = 0; p < 2; ++p) {
+                const float x0 = x[p];
+                x[p] = __fmaf_rn(sg, z[p], x[p] + mu);
+                if constexpr (KIND == kAsianArith || KIND == kAsianCv) acc[p] += __expf(x[p]);
+                if constexpr (KIND == kAsianGeo || KIND == kAsianCv) acc2[p] += x[p];
+                if constexpr (KIND == kBarrier || KIND == kBarrierBridge) {
+                    const bool crossed = c.up ? x[p] >= lnh : x[p] <= lnh;
+                    breached[p] = breached[p] || crossed;
+                }
+                if constexpr (KIND == kBarrierBridge) {
+                    if (!breached[p]) {
+                        const float p_cross = __expf(inv_denom * (lnh - x0) * (lnh - x[p]));
+                        breached[p] = uniform_from_bits_f32(philox_word0(row_u[p], st, k)) < p_cross;
+                    }
+                }
+                if constexpr (KIND == kLookbackFixed || KIND == kLookbackFloating) {
+                    xmax[p] = fmaxf(xmax[p], x[p]);
+                    xmin[p] = fminf(xmin[p], x[p]);
+                }
             }
         }
     }
-    const float inv_n = 1.0f / static_cast<float>(c.n_steps);
-#pragma unroll
-    for (int p = 0; p < NP; ++p) {
+
+    // The discounted sample in FP64 (the payoff itself is FP32).
+    __device__ __forceinline__ double sample(const DevContract& c, int p) const {
+        const float phi = c.type == 0 ? 1.0f : -1.0f;
+        const float s0 = static_cast<float>(c.spot), strike = static_cast<float>(c.strike);
+        const float inv_n = 1.0f / static_cast<float>(c.n_steps);
         const float last = s0 * __expf(x[p]);
         if constexpr (KIND == kAsianArith || KIND == kAsianGeo) {
             const float avg = KIND == kAsianArith ? s0 * (acc[p] * inv_n) : s0 * __expf(acc2[p] * inv_n);
             const float ref = c.floating ? (last - avg) : (avg - strike);
-            out[p] = c.discount * static_cast<double>(fmaxf(phi * ref, 0.0f));
+            return c.discount * static_cast<double>(fmaxf(phi * ref, 0.0f));
         } else if constexpr (KIND == kAsianCv) {
             const float a = s0 * (acc[p] * inv_n);
             const float g = s0 * __expf(acc2[p] * inv_n);
             const double ap = c.discount * static_cast<double>(fmaxf(phi * (a - strike), 0.0f));
             const double gp = c.discount * static_cast<double>(fmaxf(phi * (g - strike), 0.0f));
-            out[p] = ap - (gp - c.kv_anchor);
-        } else if constexpr (KIND == kBarrier) {
+            return ap - (gp - c.kv_anchor);
+        } else if constexpr (KIND == kBarrier || KIND == kBarrierBridge) {
             const float vanilla = fmaxf(phi * (last - strike), 0.0f);
             const bool pays = c.out ? !breached[p] : breached[p];
-            out[p] = c.discount * static_cast<double>(pays ? vanilla : static_cast<float>(c.rebate));
+            return c.discount * static_cast<double>(pays ? vanilla : static_cast<float>(c.rebate));
         } else if constexpr (KIND == kLookbackFixed) {
             const float v = c.type == 0 ? fmaxf(s0 * __expf(xmax[p]) - strike, 0.0f)
                                         : fmaxf(strike - s0 * __expf(xmin[p]), 0.0f);
-            out[p] = c.discount * static_cast<double>(v);
+            return c.discount * static_cast<double>(v);
         } else {
             const float v = c.type == 0 ? (last - s0 * __expf(xmin[p])) : (s0 * __expf(xmax[p]) - last);
-            out[p] = c.discount * static_cast<double>(v);
+            return c.discount * static_cast<double>(v);
         }
     }
-}
+};
 
-// Returns the discounted sample in FP64 (the payoff itself is FP32).
+// European and digital: the discounted sample of one draw.
 template <int KIND>
-__device__ double sample32(const DevContract& c, const PhiloxKeys& k, uint64_t path, bool neg) {
+__device__ __forceinline__ double terminal32(const DevContract& c, uint32_t bits, bool neg) {
     const float phi = c.type == 0 ? 1.0f : -1.0f;
-    const float mu = static_cast<float>(c.drift);
-    const float sg = static_cast<float>(c.vs);
-    const float s0 = static_cast<float>(c.spot);
-    const float strike = static_cast<float>(c.strike);
-    const PhiloxPath pp = philox_path(path, 0u, k);
-    if constexpr (KIND == kEuropean || KIND == kDigital) {
-        const float z = draw32(pp, 0u, k, neg);
-        const float s = s0 * __expf(__fmaf_rn(sg, z, mu));
-        float payoff;
-        if constexpr (KIND == kEuropean) {
-            payoff = fmaxf(phi * (s - strike), 0.0f);
-        } else {
-            const bool itm = phi * (s - strike) > 0.0f;
-            payoff = itm ? (c.asset ? s : static_cast<float>(c.cash)) : 0.0f;
-        }
-        return c.discount * static_cast<double>(payoff);
-    } else if constexpr (KIND == kBarrierBridge) {
-        const PhiloxPath pu = philox_path(path, 1u, k);
-        const float lnh = static_cast<float>(c.log_h_rel);
-        const float inv_denom = static_cast<float>(-2.0 / c.bb_denom);
-        float x = 0.0f;
-        bool breached = false;
-        for (int step = 0; step < c.n_steps; ++step) {
-            const float z = draw32(pp, static_cast<uint32_t>(step), k, neg);
-            const float x_next = __fmaf_rn(sg, z, x + mu);
-            const bool crossed = c.up ? x_next >= lnh : x_next <= lnh;
-            breached = breached || crossed;
-            if (!breached) {
-                const float p_cross = __expf(inv_denom * (lnh - x) * (lnh - x_next));
-                const float u = uniform_from_bits_f32(philox_word0(pu, static_cast<uint32_t>(step), k));
-                breached = u < p_cross;
-            }
-            x = x_next;
-        }
-        const float s = s0 * __expf(x);
-        const float vanilla = fmaxf(phi * (s - strike), 0.0f);
-        const bool pays = c.out ? !breached : breached;
-        return c.discount * static_cast<double>(pays ? vanilla : static_cast<float>(c.rebate));
+    const float mu = static_cast<float>(c.drift), sg = static_cast<float>(c.vs);
+    const float s0 = static_cast<float>(c.spot), strike = static_cast<float>(c.strike);
+    const float z0 = normal_from_bits_f32(bits);
+    const float z = neg ? -z0 : z0;
+    const float s = s0 * __expf(__fmaf_rn(sg, z, mu));
+    float payoff;
+    if constexpr (KIND == kEuropean) {
+        payoff = fmaxf(phi * (s - strike), 0.0f);
     } else {
-        const PhiloxPath pps[1] = {pp};
-        const bool negs[1] = {neg};
-        double out[1];
-        path_dependent32<KIND, 1>(c, k, pps, negs, out);
-        return out[0];
+        const bool itm = phi * (s - strike) > 0.0f;
+        payoff = itm ? (c.asset ? s : static_cast<float>(c.cash)) : 0.0f;
     }
+    return c.discount * static_cast<double>(payoff);
 }
 
+// A warp's share of a slab (valid in lane 0); table: the CTA's step table.
+// Every thread runs every round (the table's refills are CTA barriers); a path
+// past the contract's last one is simulated or skipped, and not counted.
 template <int KIND>
-__device__ Welford slab32(const DevContract& c, const PhiloxKeys& k, uint64_t base) {
+__device__ Welford slab32(const DevContract& c, const PhiloxKeys& k, PhiloxStep* table, uint64_t base) {
     unsigned count = 0;
-    double s1 = 0.0, s2 = 0.0;
-    constexpr bool kPathDependent = KIND != kEuropean && KIND != kDigital && KIND != kBarrierBridge;
-    if constexpr (kPathDependent) {
-        if (c.antithetic) {  // the two halves of an antithetic sample share their draws
-            for (int j = 0; j < kPathsPerThread; ++j) {
-                const uint64_t path = base + static_cast<uint64_t>(j * kSlabThreads) + threadIdx.x;
-                if (path >= c.path_count) break;
-                const PhiloxPath pp = philox_path(path, 0u, k);
-                const PhiloxPath pps[2] = {pp, pp};
-                const bool negs[2] = {false, true};
-                double out[2];
-                path_dependent32<KIND, 2>(c, k, pps, negs, out);
-                const double sample = 0.5 * (out[0] + out[1]);
-                ++count;
-                s1 += sample;
-                s2 = fma(sample, sample, s2);
-            }
-        } else {  // two paths at a time, in path order
-            for (int j = 0; j < kPathsPerThread; j += 2) {
-                const uint64_t path = base + static_cast<uint64_t>(j * kSlabThreads) + threadIdx.x;
-                if (path >= c.path_count) break;
-                const uint64_t path2 = path + kSlabThreads;
-                double out[2];
-                if (path2 < c.path_count) {
-                    const PhiloxPath pps[2] = {philox_path(path, 0u, k), philox_path(path2, 0u, k)};
-                    const bool negs[2] = {false, false};
-                    path_dependent32<KIND, 2>(c, k, pps, negs, out);
-                } else {
-                    const PhiloxPath pps[1] = {philox_path(path, 0u, k)};
-                    const bool negs[1] = {false};
-                    double one[1];
-                    path_dependent32<KIND, 1>(c, k, pps, negs, one);
-                    out[0] = one[0];
-                }
-                const int n_here = path2 < c.path_count ? 2 : 1;
-                for (int p = 0; p < n_here; ++p) {
-                    ++count;
-                    s1 += out[p];
-                    s2 = fma(out[p], out[p], s2);
-                }
-            }
-        }
-        return welford_from_sums(count, s1, s2);
-    }
-    for (int j = 0; j < kPathsPerThread; ++j) {
-        const uint64_t path = base + static_cast<uint64_t>(j * kSlabThreads) + threadIdx.x;
-        if (path >= c.path_count) break;
-        double sample = sample32<KIND>(c, k, path, false);
-        if (c.antithetic) {
-            const double sample2 = sample32<KIND>(c, k, path, true);
-            sample = 0.5 * (sample + sample2);
-        }
+    UnitSums acc;
+    auto add = [&](double v) {
         ++count;
-        s1 += sample;
-        s2 = fma(sample, sample, s2);
+        acc.add(v);
+    };
+    const uint32_t path_hi = static_cast<uint32_t>(base >> 32);  // a slab is aligned to its size
+    const uint64_t left = c.path_count - base;
+    const int rounds = left >= kSlabPaths ? kPathsPerThread : static_cast<int>((left + kSlabThreads - 1) / kSlabThreads);
+    if constexpr (KIND == kEuropean || KIND == kDigital) {
+        const PhiloxStep st = philox_step(0u, path_hi, k);
+        for (int j = 0; j < rounds; ++j) {
+            const uint64_t path = base + static_cast<uint64_t>(j * kSlabThreads) + threadIdx.x;
+            const uint32_t bits = philox_word0(philox_row(static_cast<uint32_t>(path), 0u, k), st, k);
+            double v = terminal32<KIND>(c, bits, false);
+            if (c.antithetic) v = 0.5 * (v + terminal32<KIND>(c, bits, true));
+            if (j == 0) acc.first(v);
+            if (path < c.path_count) add(v);
+        }
+    } else {
+        const int n = c.n_steps;
+        const bool once = n <= kStepTable;
+        if (once) {
+            fill_steps(table, 0, path_hi, k);
+            __syncthreads();
+        }
+        const int stride = c.antithetic ? 1 : 2;  // paths of a thread per round, in path order
+        for (int j = 0; j < rounds; j += stride) {
+            const uint64_t path = base + static_cast<uint64_t>(j * kSlabThreads) + threadIdx.x;
+            const bool live = path < c.path_count;
+            double v0 = 0.0, v1 = 0.0;
+            if (live || !once) {
+                const uint32_t lo = static_cast<uint32_t>(path);
+                const PhiloxRow row[2] = {philox_row(lo, 0u, k), philox_row(lo + kSlabThreads, 0u, k)};
+                PhiloxRow row_u[2] = {};
+                if constexpr (KIND == kBarrierBridge) {
+                    row_u[0] = philox_row(lo, 1u, k);
+                    row_u[1] = philox_row(c.antithetic ? lo : lo + kSlabThreads, 1u, k);
+                }
+                Pair32<KIND> pair;
+                for (int d0 = 0; d0 < n; d0 += kStepTable) {
+                    if (!once) {
+                        __syncthreads();
+                        fill_steps(table, d0, path_hi, k);
+                        __syncthreads();
+                    }
+                    const int m = min(kStepTable, n - d0);
+                    if (c.antithetic) pair.template advance<true>(c, k, table, m, row, row_u);
+                    else pair.template advance<false>(c, k, table, m, row, row_u);
+                }
+                v0 = pair.sample(c, 0);
+                v1 = pair.sample(c, 1);
+                if (c.antithetic) v0 = 0.5 * (v0 + v1);
+            }
+            if (j == 0) acc.first(v0);
+            if (live) add(v0);
+            if (!c.antithetic && path + kSlabThreads < c.path_count) add(v1);
+        }
     }
-    return welford_from_sums(count, s1, s2);
+    return acc.reduce(__reduce_add_sync(0xffffffffu, count));
 }
 
-__device__ Welford run_slab(const DevContract& c, uint64_t base) {
+__device__ Welford run_slab(const DevContract& c, PhiloxStep* table, uint64_t base) {
     const PhiloxKeys k = philox_keys(c.seed);
     switch (c.kind) {
-        case kEuropean: return slab32<kEuropean>(c, k, base);
-        case kDigital: return slab32<kDigital>(c, k, base);
-        case kAsianArith: return slab32<kAsianArith>(c, k, base);
-        case kAsianGeo: return slab32<kAsianGeo>(c, k, base);
-        case kAsianCv: return slab32<kAsianCv>(c, k, base);
-        case kBarrier: return slab32<kBarrier>(c, k, base);
-        case kBarrierBridge: return slab32<kBarrierBridge>(c, k, base);
-        case kLookbackFixed: return slab32<kLookbackFixed>(c, k, base);
-        default: return slab32<kLookbackFloating>(c, k, base);
+        case kEuropean: return slab32<kEuropean>(c, k, table, base);
+        case kDigital: return slab32<kDigital>(c, k, table, base);
+        case kAsianArith: return slab32<kAsianArith>(c, k, table, base);
+        case kAsianGeo: return slab32<kAsianGeo>(c, k, table, base);
+        case kAsianCv: return slab32<kAsianCv>(c, k, table, base);
+        case kBarrier: return slab32<kBarrier>(c, k, table, base);
+        case kBarrierBridge: return slab32<kBarrierBridge>(c, k, table, base);
+        case kLookbackFixed: return slab32<kLookbackFixed>(c, k, table, base);
+        default: return slab32<kLookbackFloating>(c, k, table, base);
     }
 }
 
@@ -250,6 +256,7 @@ __global__ void __launch_bounds__(kSlabThreads, MINB)
     __shared__ uint32_t s_item, s_total;
     __shared__ Welford s_warp[kSlabThreads / 32];
     __shared__ DevContract s_contract;
+    __shared__ PhiloxStep s_step[kStepTable];
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     // The batch's item count is the prefix's last entry (read from memory, so
@@ -280,8 +287,7 @@ __global__ void __launch_bounds__(kSlabThreads, MINB)
             __syncthreads();
             continue;
         }
-        Welford w = run_slab(c, static_cast<uint64_t>(slab) * kSlabPaths);
-        w = welford_warp_reduce(w);
+        const Welford w = run_slab(c, s_step, static_cast<uint64_t>(slab) * kSlabPaths);
         if (lane == 0) s_warp[warp] = w;
         __syncthreads();
         if (threadIdx.x == 0) {

@@ -241,29 +241,6 @@ __device__ __forceinline__ void greeks_fixed(GreeksSlot& slot, const FixedShared
     }
 }
 
-// Sums v[i] over the warp for every i < 12 at once: each step halves the
-// values a lane carries while it doubles the lanes they stand for (14 additions
-// instead of 60); the additions of one value pair the same lanes as a shuffle
-// tree's.  Returns the sum of output `index` (12 or more: none).
-__device__ __forceinline__ double warp_sum12(const double (&v)[kNumGreeks], int lane, int& index) {
-    double a6[6], a3[3], a2[2];
-    const bool h16 = lane & 16, h8 = lane & 8, h4 = lane & 4, h2 = lane & 2;
-#pragma unroll
-    for (int i = 0; i < 6; ++i)
-        a6[i] = (h16 ? v[i + 6] : v[i]) + __shfl_xor_sync(0xffffffffu, h16 ? v[i] : v[i + 6], 16);
-#pragma unroll
-    for (int i = 0; i < 3; ++i)
-        a3[i] = (h8 ? a6[i + 3] : a6[i]) + __shfl_xor_sync(0xffffffffu, h8 ? a6[i] : a6[i + 3], 8);
-    // three values: lanes without bit 2 keep the first two, the others the third
-    a2[0] = (h4 ? a3[2] : a3[0]) + __shfl_xor_sync(0xffffffffu, h4 ? a3[0] : a3[2], 4);
-    const double other = __shfl_xor_sync(0xffffffffu, a3[1], 4);
-    a2[1] = a3[1] + other;
-    const double a1 = (h2 ? a2[1] : a2[0]) + __shfl_xor_sync(0xffffffffu, h2 ? a2[0] : a2[1], 2);
-    index = (h16 ? 6 : 0) + (h8 ? 3 : 0) + (h4 ? 2 : 0) + (h2 ? 1 : 0);
-    if ((h4 && h2) || (lane & 1)) index = kNumGreeks;  // a duplicate or the other half of a pair
-    return a1 + __shfl_xor_sync(0xffffffffu, a1, 1);
-}
-
 struct SharedGreeks {
     FixedShared tables;
     GreeksSlot slot[kThreads / 32];
@@ -337,8 +314,8 @@ __global__ void __launch_bounds__(kThreads, 1)
             }
         }
         int index;
-        const double a = warp_sum12(s1, lane, index);
-        const double b = warp_sum12(s2, lane, index);
+        const double a = warp_sums(s1, lane, index);
+        const double b = warp_sums(s2, lane, index);
         double p = 0.0;
 #pragma unroll
         for (int i = 0; i < kNumGreeks; ++i) p = index == i ? pivot[i] : p;

@@ -12,6 +12,7 @@
 
 #include "engine.hpp"
 #include "fixed_path.cuh"
+#include "unit_sums.cuh"
 
 namespace mcdg {
 
@@ -122,37 +123,6 @@ __device__ __forceinline__ double control_variate64(const DevContract& c, const 
     const double gp = c.discount * positive_part(put_sign(g - c.strike, c.type));
     return ap - (gp - c.kv_anchor);
 }
-
-// Shifted sums (a = sum of d, b = sum of d^2, d = sample - pivot) of a unit as
-// a Welford triple.
-__device__ __forceinline__ Welford unit_triple(uint32_t count, double pivot, double a, double b) {
-    const double m = a / static_cast<double>(count);
-    const double m2 = fma(-a, m, b);
-    return Welford{count, pivot + m, m2 > 0.0 ? m2 : 0.0};
-}
-
-// A unit's sums, shifted by the first sample of the unit: with the shift the
-// variance does not cancel, and three FP64 operations per sample replace the
-// reference's Welford update and its division (stats.hpp:29-36).  Lane 0
-// returns the triple.
-struct UnitSums {
-    double pivot = 0.0, s1 = 0.0, s2 = 0.0;
-    __device__ __forceinline__ void first(double v) { pivot = __shfl_sync(0xffffffffu, v, 0); }
-    __device__ __forceinline__ void add(double v) {
-        const double d = v - pivot;
-        s1 += d;
-        s2 = fma(d, d, s2);
-    }
-    __device__ __forceinline__ Welford reduce(uint32_t count) const {
-        double a = s1, b = s2;
-#pragma unroll
-        for (int off = 16; off >= 1; off >>= 1) {
-            a += __shfl_down_sync(0xffffffffu, a, off);
-            b += __shfl_down_sync(0xffffffffu, b, off);
-        }
-        return unit_triple(count, pivot, a, b);
-    }
-};
 
 // The contract that holds an item: the largest index whose first item is <=
 // item (empty contracts share their successor's first item and are skipped).
