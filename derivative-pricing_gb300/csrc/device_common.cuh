@@ -148,6 +148,16 @@ __device__ __forceinline__ uint32_t philox_word0(const PhiloxRow& r, const Philo
     return __umulhi(kPhiloxM1, w2) ^ (kPhiloxM1 * c2) ^ k.k0[9];
 }
 
+// Philox words of the next kStepTable steps, one table per CTA: the products
+// that depend on the draw alone, computed once per slab (contracts of more
+// steps refill it along every path).
+constexpr int kStepTable = 256;
+
+__device__ __forceinline__ void fill_steps(PhiloxStep* table, int first, uint32_t path_hi, const PhiloxKeys& k) {
+    for (unsigned d = threadIdx.x; d < kStepTable; d += blockDim.x)
+        table[d] = philox_step(static_cast<uint32_t>(first) + d, path_hi, k);
+}
+
 // ---------------------------------------------------------------------------
 // FP64 transform (src/core/rng.cpp:34-37, src/core/normal.cpp:22-82)
 //

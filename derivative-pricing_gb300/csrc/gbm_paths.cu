@@ -46,16 +46,6 @@ namespace {
 // ===========================================================================
 // FP32: log-space paths x = ln(S/S0), FP32 payoffs, FP64 accumulation.
 // ===========================================================================
-// Philox words of the next kStepTable steps, one table per CTA: the products
-// that depend on the draw alone, computed once per slab (contracts of more
-// steps refill it along every path).
-constexpr int kStepTable = 256;
-
-__device__ __forceinline__ void fill_steps(PhiloxStep* table, int first, uint32_t path_hi, const PhiloxKeys& k) {
-    for (int d = threadIdx.x; d < kStepTable; d += kSlabThreads)
-        table[d] = philox_step(static_cast<uint32_t>(first + d), path_hi, k);
-}
-
 // Path-dependent products (Asians, barriers, lookbacks), two paths at once (or
 // the two halves of an antithetic sample, which share their draws): two
 // independent dependency chains per thread.  Each path's arithmetic does not

@@ -17,65 +17,60 @@
 // terminal values in shared memory, then pays them out: thread t serves
 // strike t % K over the paths of group t / K (G = 128 / K groups), so every
 // thread is busy when K <= 128; for 128 < K <= 256, thread t serves strikes t
-// and t + 128 over all paths.  Accumulation is per thread in FP64 (FP64 path:
-// Welford; FP32 path: FP32 payoffs summed per round with Kahan compensation,
-// then added in FP64), and the groups and slabs are merged in fixed order.
+// and t + 128 over all paths.  FP32 payoffs are summed per round with Kahan
+// compensation, then added in FP64; the groups and slabs are merged in fixed
+// order.  (The FP64 paths are heston64.cu.)
+//
+// Bound: issue (72 % of the slots) and the FMA-heavy pipe (66 %), 176
+// thread-instructions per path-step.  64 sets of 64 strikes, 252 steps, 2^20
+// paths: 110 ms -> 106 with the Philox products of the draw and of the path
+// taken out of the step, 101-104 with one branch region for both paths'
+// exponential steps.
 //
 // nvcc-flags: --fmad=false
 #include <cuda_runtime.h>
 
 #include "device_common.cuh"
 #include "heston.hpp"
+#include "merge.cuh"
 
 namespace mcdg {
 
 namespace {
 
-__device__ __forceinline__ double dmax(double a, double b) { return (a < b) ? b : a; }
-
-// FP64 QE variance step in the reference's operation order (heston.cpp:91-116).
-__device__ __forceinline__ double qe_step64(double v, const HestonSet& h, uint32_t ubits) {
-    const double e = h.e;
-    const double m = h.theta + (v - h.theta) * e;
-    const double s2 = v * h.xi * h.xi * e / h.kappa * (1.0 - e) + h.s2_const;
-    const double psi = s2 / (m * m);
-    const double raw_uniform = uniform_open01_f64(ubits);
-    if (psi <= 1.5) {
-        const double inv_psi = 1.0 / psi;
-        const double b2 = 2.0 * inv_psi - 1.0 + sqrt(2.0 * inv_psi) * sqrt(2.0 * inv_psi - 1.0);
-        const double a = m / (1.0 + b2);
-        const double z_v = inv_normal_cdf_f64(raw_uniform);
-        const double b = sqrt(b2);
-        return a * (b + z_v) * (b + z_v);
-    }
-    const double p = (psi - 1.0) / (psi + 1.0);
-    const double beta = (1.0 - p) / m;
-    if (raw_uniform <= p) return 0.0;
-    return log((1.0 - p) / (1.0 - raw_uniform)) / beta;
-}
-
-// FP32 QE step: same scheme, FP32 arithmetic, 1-u formed from the bits.
-__device__ __forceinline__ float qe_step32(float v, const HestonSet32& h, uint32_t ubits) {
-    const float m = __fmaf_rn(v - h.theta, h.e, h.theta);
-    const float s2 = __fmaf_rn(v, h.s2_lin, h.s2_const);
-    const float psi = s2 * fast_rcp(m * m);
-    if (psi <= 1.5f) {
-        const float inv_psi = fast_rcp(psi);
+// FP32 QE step of two paths: the reference's scheme, 1-u formed from the bits.
+// z holds the normals of the same bits.  Both paths take the quadratic branch's
+// value, then one branch for the pair replaces it where psi > 1.5: in most
+// warps some lane has such a path, and a branch region per path would run both
+// sides one after the other.
+__device__ __forceinline__ void qe_pair32(const float (&v)[2], const HestonSet32& h, const uint32_t (&ubits)[2],
+                                          const float (&z)[2], float (&out)[2]) {
+    float m[2], psi[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        m[i] = __fmaf_rn(v[i] - h.theta, h.e, h.theta);
+        const float s2 = __fmaf_rn(v[i], h.s2_lin, h.s2_const);
+        psi[i] = s2 * fast_rcp(m[i] * m[i]);
+        const float inv_psi = fast_rcp(psi[i]);
         const float two = 2.0f * inv_psi;
         const float b2 = two - 1.0f + fast_sqrt(two) * fast_sqrt(two - 1.0f);
-        const float a = m * fast_rcp(1.0f + b2);
-        const float z_v = normal_from_bits_f32(ubits);
-        const float bz = fast_sqrt(b2) + z_v;
-        return a * bz * bz;
+        const float a = m[i] * fast_rcp(1.0f + b2);
+        const float bz = fast_sqrt(b2) + z[i];
+        out[i] = a * bz * bz;
     }
-    const float p = (psi - 1.0f) * fast_rcp(psi + 1.0f);
-    const float u = uniform_from_bits_f32(ubits);
-    if (u <= p) return 0.0f;
-    // 1 - u = (~bits + 0.5) / 2^32, exact relative precision near u = 1
-    const float one_minus_u = __fmaf_rn(__uint2float_rn(~ubits), 2.3283064365386963e-10f,
-                                        1.1641532182693481e-10f);
-    const float beta = (1.0f - p) * fast_rcp(m);
-    return __logf((1.0f - p) * fast_rcp(one_minus_u)) * fast_rcp(beta);
+    if (!(psi[0] <= 1.5f) || !(psi[1] <= 1.5f)) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const float p = (psi[i] - 1.0f) * fast_rcp(psi[i] + 1.0f);
+            const float u = uniform_from_bits_f32(ubits[i]);
+            // 1 - u = (~bits + 0.5) / 2^32, exact relative precision near u = 1
+            const float one_minus_u = __fmaf_rn(__uint2float_rn(~ubits[i]), 2.3283064365386963e-10f,
+                                                1.1641532182693481e-10f);
+            const float beta = (1.0f - p) * fast_rcp(m[i]);
+            const float e = __logf((1.0f - p) * fast_rcp(one_minus_u)) * fast_rcp(beta);
+            if (!(psi[i] <= 1.5f)) out[i] = u <= p ? 0.0f : e;
+        }
+    }
 }
 
 struct KahanF {
@@ -88,18 +83,16 @@ struct KahanF {
     }
 };
 
-// FP32: two paths per thread in flight, so a larger register budget (6 CTAs
-// of 128 threads per SM) than the FP64 kernel's (8).
-template <int PREC>
-__global__ void __launch_bounds__(128, PREC == 1 ? 6 : 8)
-    heston_kernel(const HestonSet* __restrict__ sets, int n_sets, const double* __restrict__ strikes,
+// Two paths per thread in flight: 6 CTAs of 128 threads per SM.
+__global__ void __launch_bounds__(128, 6)
+    heston_kernel(const HestonSet* __restrict__ sets, const double* __restrict__ strikes,
                   int n_strikes, int type, uint32_t items_per_set, uint32_t total_items,
                   uint32_t* __restrict__ ticket, Welford* __restrict__ partials) {
     __shared__ uint32_t s_item;
-    __shared__ double s_terminal64[128];
     __shared__ float s_terminal32[128], s_terminal32b[128];
     __shared__ Welford s_acc[256];
     __shared__ HestonSet s_set;
+    __shared__ PhiloxStep s_step[kStepTable];
     const int t = threadIdx.x;
     const int groups = n_strikes <= 128 ? 128 / n_strikes : 1;
     const int my_group = n_strikes <= 128 ? t / n_strikes : 0;
@@ -120,44 +113,19 @@ __global__ void __launch_bounds__(128, PREC == 1 ? 6 : 8)
         __syncthreads();
         const HestonSet& h = s_set;
         const PhiloxKeys k = philox_keys(h.seed);
+        const uint64_t base = static_cast<uint64_t>(slab) * 4096;
+        const uint32_t path_hi = static_cast<uint32_t>(base >> 32);
+        const bool once = h.n_steps <= kStepTable;  // the step table serves the whole slab
+        if (once) {
+            fill_steps(s_step, 0, path_hi, k);
+            __syncthreads();
+        }
         const double strike0 = serves0 ? strikes[k0] : 0.0;
         const double strike1 = serves1 ? strikes[t + 128] : 0.0;
-        Welford w0{0ull, 0.0, 0.0}, w1{0ull, 0.0, 0.0};
         unsigned cnt0 = 0, cnt1 = 0;
         double a0 = 0.0, q0 = 0.0, a1 = 0.0, q1 = 0.0;
-        HestonSet32 h32;
-        if (PREC == 1) h32 = make_set32(h);
-        if constexpr (PREC == 0) {
-            for (int j = 0; j < 32; ++j) {
-                const uint64_t path = static_cast<uint64_t>(slab) * 4096 + static_cast<uint64_t>(j * 128 + t);
-                if (path < h.path_count) {
-                    const PhiloxPath ps = philox_path(path, 0u, k);
-                    const PhiloxPath pv = philox_path(path, 1u, k);
-                    double v = h.v0;
-                    double log_s = h.log_s0;
-                    for (int step = 0; step < h.n_steps; ++step) {
-                        const uint32_t d = static_cast<uint32_t>(step);
-                        const double z_s = normal_from_bits_f64(philox_word0(ps, d, k));
-                        const double v_next = qe_step64(v, h, philox_word0(pv, d, k));
-                        const double diffusion_var = dmax(h.k3 * v + h.k4 * v_next, 0.0);
-                        log_s += h.drift + h.k0 + h.k1 * v + h.k2 * v_next + sqrt(diffusion_var) * z_s;
-                        v = v_next;
-                    }
-                    s_terminal64[t] = exp(log_s);
-                }
-                __syncthreads();
-                // Pay out the round's paths (paths of this round beyond path_count are skipped).
-                const uint64_t round_base = static_cast<uint64_t>(slab) * 4096 + static_cast<uint64_t>(j * 128);
-                const uint64_t left = round_base >= h.path_count ? 0 : h.path_count - round_base;
-                const int round_live = left > 128 ? 128 : static_cast<int>(left);
-                for (int p = my_group; p < round_live; p += groups) {
-                    const double s_t = s_terminal64[p];
-                    if (serves0) welford_add(w0, h.discount * dmax(phi * (s_t - strike0), 0.0));
-                    if (serves1) welford_add(w1, h.discount * dmax(phi * (s_t - strike1), 0.0));
-                }
-                __syncthreads();
-            }
-        } else {
+        const HestonSet32 h32 = make_set32(h);
+        {
             // Two rounds per pass: each thread simulates the paths of rounds j
             // and j + 1 together (independent dependency chains), then both
             // rounds are paid out in order, so the sums are those of one round
@@ -194,31 +162,40 @@ __global__ void __launch_bounds__(128, PREC == 1 ? 6 : 8)
                 }
             };
             for (int j = 0; j < 32; j += 2) {
-                const uint64_t path_a = static_cast<uint64_t>(slab) * 4096 + static_cast<uint64_t>(j * 128 + t);
-                const uint64_t path_b = path_a + 128;
-                if (path_a < h.path_count) {  // path_b exists only if path_a does
-                    const bool live_b = path_b < h.path_count;
-                    const PhiloxPath psa = philox_path(path_a, 0u, k), pva = philox_path(path_a, 1u, k);
-                    const PhiloxPath psb = philox_path(path_b, 0u, k), pvb = philox_path(path_b, 1u, k);
-                    float va = h32.v0, vb = h32.v0;
-                    float xa = 0.0f, xb = 0.0f;  // ln(S/S0)
-                    for (int step = 0; step < h.n_steps; ++step) {
-                        const uint32_t d = static_cast<uint32_t>(step);
-                        const float za = normal_from_bits_f32(philox_word0(psa, d, k));
-                        const float zb = normal_from_bits_f32(philox_word0(psb, d, k));
-                        const float va_next = qe_step32(va, h32, philox_word0(pva, d, k));
-                        const float vb_next = qe_step32(vb, h32, philox_word0(pvb, d, k));
-                        const float dva = fmaxf(__fmaf_rn(h32.k3, va, h32.k4 * va_next), 0.0f);
-                        const float dvb = fmaxf(__fmaf_rn(h32.k3, vb, h32.k4 * vb_next), 0.0f);
-                        const float ia = __fmaf_rn(h32.k1, va, __fmaf_rn(h32.k2, va_next, h32.c0));
-                        const float ib = __fmaf_rn(h32.k1, vb, __fmaf_rn(h32.k2, vb_next, h32.c0));
-                        xa = __fmaf_rn(fast_sqrt(dva), za, xa + ia);
-                        xb = __fmaf_rn(fast_sqrt(dvb), zb, xb + ib);
-                        va = va_next;
-                        vb = vb_next;
+                const uint64_t path_a = base + static_cast<uint64_t>(j * 128 + t);
+                // (a table refill is a CTA barrier: every thread then runs every round)
+                if (path_a < h.path_count || !once) {
+                    const uint32_t lo = static_cast<uint32_t>(path_a);
+                    const PhiloxRow ra = philox_row(lo, 0u, k), rb = philox_row(lo + 128, 0u, k);
+                    const PhiloxRow ua = philox_row(lo, 1u, k), ub = philox_row(lo + 128, 1u, k);
+                    float v[2] = {h32.v0, h32.v0}, x[2] = {0.0f, 0.0f};  // variance, ln(S/S0)
+                    for (int d0 = 0; d0 < h.n_steps; d0 += kStepTable) {
+                        if (!once) {
+                            __syncthreads();
+                            fill_steps(s_step, d0, path_hi, k);
+                            __syncthreads();
+                        }
+                        const int m = min(kStepTable, h.n_steps - d0);
+                        for (int d = 0; d < m; ++d) {
+                            const PhiloxStep st = s_step[d];
+                            const uint32_t bits[4] = {philox_word0(ra, st, k), philox_word0(rb, st, k),
+                                                      philox_word0(ua, st, k), philox_word0(ub, st, k)};
+                            float z[4], next[2];
+                            normals_from_bits_f32<4>(bits, z);
+                            const uint32_t ubits[2] = {bits[2], bits[3]};
+                            const float zv[2] = {z[2], z[3]};
+                            qe_pair32(v, h32, ubits, zv, next);
+#pragma unroll
+                            for (int i = 0; i < 2; ++i) {
+                                const float dv = fmaxf(__fmaf_rn(h32.k3, v[i], h32.k4 * next[i]), 0.0f);
+                                const float inc = __fmaf_rn(h32.k1, v[i], __fmaf_rn(h32.k2, next[i], h32.c0));
+                                x[i] = __fmaf_rn(fast_sqrt(dv), z[i], x[i] + inc);
+                                v[i] = next[i];
+                            }
+                        }
                     }
-                    s_terminal32[t] = h32.s0 * __expf(xa);
-                    if (live_b) s_terminal32b[t] = h32.s0 * __expf(xb);
+                    s_terminal32[t] = h32.s0 * __expf(x[0]);
+                    s_terminal32b[t] = h32.s0 * __expf(x[1]);
                 }
                 __syncthreads();
                 payout(j, s_terminal32);
@@ -226,12 +203,10 @@ __global__ void __launch_bounds__(128, PREC == 1 ? 6 : 8)
                 __syncthreads();
             }
         }
-        if (PREC == 1) {
-            // discount applied once: mean scales by D, M2 by D^2
-            const double d = h.discount;
-            w0 = welford_from_sums(cnt0, a0 * d, q0 * d * d);
-            w1 = welford_from_sums(cnt1, a1 * d, q1 * d * d);
-        }
+        // discount applied once: mean scales by D, M2 by D^2
+        const double disc = h.discount;
+        const Welford w0 = welford_from_sums(cnt0, a0 * disc, q0 * disc * disc);
+        const Welford w1 = welford_from_sums(cnt1, a1 * disc, q1 * disc * disc);
         // Merge the groups of each strike in group order (fixed tree).
         if (serves0) s_acc[n_strikes <= 128 ? my_group * n_strikes + k0 : k0] = w0;
         if (serves1) s_acc[t + 128] = w1;
@@ -250,54 +225,40 @@ __global__ void __launch_bounds__(128, PREC == 1 ? 6 : 8)
     }
 }
 
-// One warp per (set, strike): fold the set's slabs in slab order, fixed tree.
-__global__ void heston_merge_kernel(const HestonSet* __restrict__ sets, int n_sets, int n_strikes,
-                                    uint32_t items_per_set, const Welford* __restrict__ partials,
-                                    double* __restrict__ out /* n_sets*n_strikes x {price, se, count} */) {
-    const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (w >= n_sets * n_strikes) return;
-    const int set = w / n_strikes, kk = w % n_strikes;
-    const uint32_t n_slabs = sets[set].n_slabs;
-    Welford acc{0ull, 0.0, 0.0};
-    for (uint32_t s = lane; s < n_slabs; s += 32)
-        acc = welford_merge(acc, partials[(static_cast<size_t>(set) * items_per_set + s) * n_strikes + kk]);
-    acc = welford_warp_reduce(acc);
-    if (lane == 0) {
-        const double var = acc.count < 2 ? 0.0 : acc.m2 / static_cast<double>(acc.count - 1);
-        out[3 * static_cast<size_t>(w) + 0] = acc.mean;
-        out[3 * static_cast<size_t>(w) + 1] = acc.count == 0 ? 0.0 : sqrt(var / static_cast<double>(acc.count));
-        reinterpret_cast<unsigned long long*>(out)[3 * static_cast<size_t>(w) + 2] = acc.count;
+// One CTA per (set, strike).
+__global__ void __launch_bounds__(kMergeThreads)
+    heston_merge_kernel(int n_strikes, uint32_t items_per_set, const Welford* __restrict__ partials,
+                        double* __restrict__ out /* n_sets*n_strikes x {price, se, count} */) {
+    const size_t w = blockIdx.x, set = w / n_strikes, strike = w % n_strikes;
+    const MergedResult m = merge_items(partials + set * items_per_set * n_strikes + strike, items_per_set, n_strikes);
+    if (threadIdx.x == 0) {
+        out[3 * w] = m.mean;
+        out[3 * w + 1] = m.standard_error;
+        reinterpret_cast<unsigned long long*>(out)[3 * w + 2] = m.count;
     }
 }
 
 }  // namespace
 
-cudaError_t launch_heston(int precision, int grid, const HestonSet* sets, int n_sets,
-                          const double* strikes, int n_strikes, int type, uint32_t items_per_set,
-                          uint32_t* ticket, Welford* partials, double* out, cudaStream_t stream) {
-    const uint32_t total = items_per_set * static_cast<uint32_t>(n_sets);
+cudaError_t launch_heston32(int grid, const HestonSet* sets, int n_sets, const double* strikes, int n_strikes,
+                            int type, uint32_t items_per_set, uint32_t* ticket, Welford* partials,
+                            cudaStream_t stream) {
     cudaGetLastError();
-    if (total > 0) {
-        if (precision == 0)
-            heston_kernel<0><<<grid, 128, 0, stream>>>(sets, n_sets, strikes, n_strikes, type,
-                                                       items_per_set, total, ticket, partials);
-        else
-            heston_kernel<1><<<grid, 128, 0, stream>>>(sets, n_sets, strikes, n_strikes, type,
-                                                       items_per_set, total, ticket, partials);
-        cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) return e;
-    }
-    const int warps = n_sets * n_strikes;
-    heston_merge_kernel<<<(warps * 32 + 255) / 256, 256, 0, stream>>>(sets, n_sets, n_strikes,
-                                                                       items_per_set, partials, out);
+    heston_kernel<<<grid, 128, 0, stream>>>(sets, strikes, n_strikes, type, items_per_set,
+                                            items_per_set * static_cast<uint32_t>(n_sets), ticket, partials);
     return cudaGetLastError();
 }
 
-cudaError_t heston_occupancy(int precision, int* blocks) {
-    return precision == 0
-               ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, heston_kernel<0>, 128, 0)
-               : cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, heston_kernel<1>, 128, 0);
+cudaError_t launch_heston_merge(int n_sets, int n_strikes, uint32_t items_per_set, const Welford* partials,
+                                double* out, cudaStream_t stream) {
+    cudaGetLastError();
+    heston_merge_kernel<<<static_cast<unsigned>(n_sets) * n_strikes, kMergeThreads, 0, stream>>>(
+        n_strikes, items_per_set, partials, out);
+    return cudaGetLastError();
+}
+
+cudaError_t heston32_occupancy(int* blocks) {
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, heston_kernel, 128, 0);
 }
 
 }  // namespace mcdg

@@ -19,11 +19,15 @@ struct HestonSet {
     double discount;   // exp(-r T)
     double log_s0;     // ln S0
     double s2_lin;     // xi^2 e / kappa (1-e)   (FP32 path: s2 = v s2_lin + s2_const)
+    // FP64 path (heston64.cu): psi = r (qe_b - qe_a r) with r = 1 / E[v'], and
+    double qe_a, qe_b;  // theta xi^2 (1-e)^2 / (2 kappa), xi^2 (1-e) / kappa
+    double drift_k0;    // drift + K0
     uint64_t seed;
     uint64_t path_count;
     uint32_t n_slabs;
     int32_t n_steps;
 };
+constexpr int kHestonMaxStrikes = 256;
 
 // FP32 view used inside the FP32 kernel.
 struct HestonSet32 {
@@ -46,9 +50,17 @@ __host__ __device__ inline HestonSet32 make_set32(const HestonSet& h) {
     return r;
 }
 
-cudaError_t launch_heston(int precision, int grid, const HestonSet* sets, int n_sets,
-                          const double* strikes, int n_strikes, int type, uint32_t items_per_set,
-                          uint32_t* ticket, Welford* partials, double* out, cudaStream_t stream);
-cudaError_t heston_occupancy(int precision, int* blocks);
+// Items of a set: slabs of 4096 paths (FP32) or units of 32 << unit_log paths
+// (FP64); one Welford triple per (item, strike).  The merge folds them per
+// (set, strike) into {price, standard error, count}.
+cudaError_t launch_heston32(int grid, const HestonSet* sets, int n_sets, const double* strikes, int n_strikes,
+                            int type, uint32_t items_per_set, uint32_t* ticket, Welford* partials,
+                            cudaStream_t stream);
+cudaError_t launch_heston64(int grid, const HestonSet* sets, int n_sets, const double* strikes, int n_strikes,
+                            int type, uint32_t units_per_set, int unit_log, uint32_t* ticket, Welford* partials,
+                            const FixedTables* tables, cudaStream_t stream);
+cudaError_t launch_heston_merge(int n_sets, int n_strikes, uint32_t items_per_set, const Welford* partials,
+                                double* out, cudaStream_t stream);
+cudaError_t heston32_occupancy(int* blocks);
 
 }  // namespace mcdg

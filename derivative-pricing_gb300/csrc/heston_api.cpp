@@ -55,6 +55,9 @@ int make_set(Ctx& ctx, const mcd_heston_params& p, int steps, uint64_t paths, ui
     h.path_count = paths;
     h.n_slabs = static_cast<uint32_t>((paths + kSlabPaths - 1) / kSlabPaths);
     h.n_steps = steps;
+    h.qe_a = h.s2_const;
+    h.qe_b = p.xi * p.xi * (1.0 - h.e) / p.kappa;
+    h.drift_k0 = h.drift + h.k0;
     return MCD_OK;
 }
 
@@ -75,30 +78,50 @@ int heston_run(Ctx& ctx, const mcd_heston_params* sets, size_t n_sets, const dou
         const int rc = make_set(ctx, sets[i], steps, paths, seed, i, hs[i]);
         if (rc) return rc;
     }
-    const uint32_t items_per_set = hs[0].n_slabs;
-    const uint64_t total_items = static_cast<uint64_t>(items_per_set) * n_sets;
-    if (total_items > 0xFFFFFFF0ull) return ctx.fail(MCD_ERR_INVALID_ARGUMENT, "batch too large");
+    // FP64 units as the GBM pricer's: 32 paths per warp, doubling from 131,072
+    // paths on, up to a slab.
+    int unit_log = 0;
+    while (unit_log < 7 && (paths >> (17 + unit_log)) != 0) ++unit_log;
+    const bool fp64 = precision == 0;
+    const uint64_t unit = 32ull << unit_log;
+    const uint32_t items_per_set = fp64 ? static_cast<uint32_t>((paths + unit - 1) / unit) : hs[0].n_slabs;
+    if (static_cast<uint64_t>(hs[0].n_slabs) * n_sets > 0xFFFFFFF0ull)
+        return ctx.fail(MCD_ERR_INVALID_ARGUMENT, "batch too large");
+    // FP64 batches run in ranges of sets, so that the partials stay within 1 GB
+    // (or one set's).
+    const uint64_t set_bytes = sizeof(Welford) * std::max<uint64_t>(items_per_set, 1) * n_strikes;
+    const size_t per_range = fp64 ? std::min<size_t>(n_sets, std::max<uint64_t>((1ull << 30) / set_bytes, 1)) : n_sets;
     int rc = ctx.reserve(ctx.ext[kSets], sizeof(HestonSet) * n_sets, "heston sets");
     if (!rc) rc = ctx.reserve(ctx.ext[kStrikes], sizeof(double) * n_strikes, "strikes");
-    if (!rc) rc = ctx.reserve(ctx.ext[kPartials], sizeof(Welford) * std::max<uint64_t>(total_items, 1) * n_strikes, "heston partials");
+    if (!rc) rc = ctx.reserve(ctx.ext[kPartials], set_bytes * per_range, "heston partials");
     if (!rc) rc = ctx.reserve(ctx.ext[kOut], sizeof(mcd_mc_result) * n_sets * n_strikes, "heston results");
     if (rc) return rc;
     cudaError_t e = cudaMemcpyAsync(ctx.ext[kSets].ptr, hs.data(), sizeof(HestonSet) * n_sets, cudaMemcpyHostToDevice, ctx.stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(ctx.ext[kStrikes].ptr, strikes, sizeof(double) * n_strikes, cudaMemcpyHostToDevice, ctx.stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(ctx.d_flags, 0, sizeof(uint32_t), ctx.stream);
     if (e != cudaSuccess) return ctx.cuda_fail(e, "heston upload");
-    int blocks = 0;
-    e = heston_occupancy(precision, &blocks);
+    int blocks = 1;  // FP64: one CTA per SM shares the fixed-point tables
+    if (!fp64) e = heston32_occupancy(&blocks);
     if (e != cudaSuccess) return ctx.cuda_fail(e, "heston occupancy");
     const int grid = ctx.sm_count * std::max(blocks, 1);
     int pair = -1;
     rc = ctx.record_start(ctx.stream, &pair);
     if (rc) return rc;
-    e = launch_heston(precision, grid, static_cast<const HestonSet*>(ctx.ext[kSets].ptr),
-                      static_cast<int>(n_sets), static_cast<const double*>(ctx.ext[kStrikes].ptr),
-                      static_cast<int>(n_strikes), type, items_per_set, ctx.d_flags,
-                      static_cast<Welford*>(ctx.ext[kPartials].ptr),
-                      static_cast<double*>(ctx.ext[kOut].ptr), ctx.stream);
+    const double* d_strikes = static_cast<const double*>(ctx.ext[kStrikes].ptr);
+    Welford* partials = static_cast<Welford*>(ctx.ext[kPartials].ptr);
+    for (size_t first = 0; first < n_sets && e == cudaSuccess; first += per_range) {
+        const HestonSet* d_sets = static_cast<const HestonSet*>(ctx.ext[kSets].ptr) + first;
+        const int count = static_cast<int>(std::min(per_range, n_sets - first));
+        const int k = static_cast<int>(n_strikes);
+        e = cudaMemsetAsync(ctx.d_flags, 0, sizeof(uint32_t), ctx.stream);
+        if (e == cudaSuccess && items_per_set > 0)
+            e = fp64 ? launch_heston64(grid, d_sets, count, d_strikes, k, type, items_per_set, unit_log, ctx.d_flags,
+                                       partials, ctx.tables, ctx.stream)
+                     : launch_heston32(grid, d_sets, count, d_strikes, k, type, items_per_set, ctx.d_flags, partials,
+                                       ctx.stream);
+        if (e == cudaSuccess)
+            e = launch_heston_merge(count, k, items_per_set, partials,
+                                    static_cast<double*>(ctx.ext[kOut].ptr) + 3 * first * n_strikes, ctx.stream);
+    }
     if (e != cudaSuccess) return ctx.cuda_fail(e, "heston launch");
     rc = ctx.record_stop(ctx.stream, pair);
     if (rc) return rc;
