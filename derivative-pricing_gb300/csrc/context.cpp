@@ -108,17 +108,19 @@ bool finite_all(std::initializer_list<double> xs) {
     return true;
 }
 
-// A log2 step's integers: drift = (hi + lo 2^-32) 2^-frac, vs 2^(frac + 3).
+constexpr double kInvLn2 = 1.44269504088896340736;
+
+// The integers of a step of drift and vs (of ln S) in log2 units of 2^-frac:
+// drift = (hi + lo 2^-32), vs times 2^3.
 void fixed_step(double drift, double vs, int frac, int64_t* hi, uint32_t* lo, uint64_t* scale) {
-    const double d = std::ldexp(drift, frac), whole = std::floor(d);
+    const double d = std::ldexp(drift * kInvLn2, frac), whole = std::floor(d);
     *hi = static_cast<int64_t>(whole);
     *lo = static_cast<uint32_t>(std::min((d - whole) * 4294967296.0, 4294967295.0));
-    *scale = static_cast<uint64_t>(std::ldexp(vs, frac + 3) + 0.5);
+    *scale = static_cast<uint64_t>(std::ldexp(vs * kInvLn2, frac + 3) + 0.5);
 }
 
 // ln(H / S0) in log2 units, kept within +/- 2^61 (which no path reaches).
 int64_t fixed_barrier(double log_rel, int frac) {
-    constexpr double kInvLn2 = 1.44269504088896340736;
     const double reach = std::ldexp(1.0, 61);
     return std::llround(std::min(std::max(std::ldexp(log_rel * kInvLn2, frac), -reach), reach));
 }
@@ -129,17 +131,19 @@ int64_t fixed_barrier(double log_rel, int frac) {
 // per path); that bound is rounded up to a power of two, 2^r, and F = 61 - r
 // fraction bits are kept, 52 to 59 of them.  Above 2^9 a double's exponent
 // range comes near: frac stays 0 and the path is stepped as the reference does.
-void fixed_scale(DevContract& c) {
-    constexpr double kInvLn2 = 1.44269504088896340736;
-    const double n = static_cast<double>(c.n_steps);
-    const double drift = c.drift * kInvLn2, vs = c.vs * kInvLn2;
-    const double bound = n * std::fabs(drift) + vs * std::min(6.35 * n, 40.0 * std::sqrt(n));
-    c.frac = 0;
-    if (!(bound < 512.0)) return;
+int fixed_frac(int n_steps, double drift, double vs) {
+    const double n = static_cast<double>(n_steps);
+    const double bound = kInvLn2 * (n * std::fabs(drift) + vs * std::min(6.35 * n, 40.0 * std::sqrt(n)));
+    if (!(bound < 512.0)) return 0;
     int r = 2;
     while (bound >= std::ldexp(1.0, r)) ++r;
-    c.frac = 61 - r;
-    fixed_step(drift, vs, c.frac, &c.y_drift, &c.y_drift_lo, &c.y_vs);
+    return 61 - r;
+}
+
+void fixed_scale(DevContract& c) {
+    c.frac = fixed_frac(c.n_steps, c.drift, c.vs);
+    if (c.frac == 0) return;
+    fixed_step(c.drift, c.vs, c.frac, &c.y_drift, &c.y_drift_lo, &c.y_vs);
     if (c.kind == kBarrier || c.kind == kBarrierBridge) {
         c.y_barrier = fixed_barrier(c.log_h_rel, c.frac);
         c.y_bridge = std::ldexp(-2.0 / (kInvLn2 * kInvLn2 * c.bb_denom), -2 * c.frac);

@@ -135,6 +135,7 @@ struct Ctx {
 
 // Batch planning and execution of the path engine (context.cpp).
 int plan_contract(Ctx& ctx, const mcd_contract& in, uint32_t index, DevContract& out);
+int fixed_frac(int n_steps, double drift, double vs);
 void fixed_step(double drift, double vs, int frac, int64_t* hi, uint32_t* lo, uint64_t* scale);
 int64_t fixed_barrier(double log_rel, int frac);
 int plan_batch(Ctx& ctx, const mcd_contract* contracts, size_t n, uint64_t range_items, BatchPlan& plan);

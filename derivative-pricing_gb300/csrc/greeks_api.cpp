@@ -89,8 +89,8 @@ int plan_greeks(Ctx& ctx, const mcd_contract* cs, size_t n, int precision, doubl
         if (d.frac != 0 && in.vol * std::sqrt(in.time) * (1.0 + vol_rel) > 8.0) d.frac = 0;
         if (d.frac != 0) {
             constexpr double kInvLn2 = 1.44269504088896340736;
-            fixed_step(g.drift_up * kInvLn2, g.vs_up * kInvLn2, d.frac, &g.y_drift_up, &g.y_drift_lo_up, &g.y_vs_up);
-            fixed_step(g.drift_dn * kInvLn2, g.vs_dn * kInvLn2, d.frac, &g.y_drift_dn, &g.y_drift_lo_dn, &g.y_vs_dn);
+            fixed_step(g.drift_up, g.vs_up, d.frac, &g.y_drift_up, &g.y_drift_lo_up, &g.y_vs_up);
+            fixed_step(g.drift_dn, g.vs_dn, d.frac, &g.y_drift_dn, &g.y_drift_lo_dn, &g.y_vs_dn);
             if (in.product == MCD_PRODUCT_BARRIER) {
                 g.y_barrier_su = fixed_barrier(g.log_h_rel_up, d.frac);
                 g.y_barrier_sd = fixed_barrier(g.log_h_rel_dn, d.frac);

@@ -10,9 +10,9 @@
 //
 // Layout.  Every contract's paths live in HBM for the whole backward pass,
 // date-major (S[d-1][i], coalesced per date for the forward stores and the
-// backward column reads), FP32 or FP64; cash flows are FP64.  Paths are cut
-// into fixed chunks of 1024 (the reduction unit); a chunk is one CTA of 256
-// threads (4 paths per thread, stride 256).
+// backward column reads), FP32 or FP64; cash flows likewise.  Paths are cut
+// into fixed chunks of 1024 (the reduction unit); a chunk is one CTA of 128
+// threads (FP32, 8 paths per thread) or 256 (FP64, 4 paths per thread).
 //
 // Backward pass.  All contracts of a batch step back in lockstep: iteration k
 // handles date e = n_c - k of contract c, in one pass over the date's columns
@@ -34,7 +34,8 @@
 // conditioning (its own algorithm moves them that much when the rows are
 // reordered), and the fitted continuation values, hence the exercise
 // decisions, coincide.  Every reduction tree is fixed by chunk index.
-// Precision: the FP64 path is the reference's arithmetic throughout.  The
+// Precision: the FP64 path keeps FP64 accuracy throughout (paths in fixed point,
+// fused products, e^{-x/2} from the fixed-point tables).  The
 // FP32 path evaluates the basis, the exercise tests and the Gram products in
 // FP32 (FP64 runs at a small fraction of the FP32 rate here), keeps the cash
 // flows and continuation values in FP32 and accumulates the Gram products
@@ -45,32 +46,26 @@
 // carries a relative error below 3e-8 per date, a bias under 2e-6 of the
 // price after 50 dates.)
 //
+// Bound of a single FP64 contract: the chain of dates.  Per date of a put with
+// 131,072 paths and 50 dates: 92 us before; the FP64 pipe (about 150 -> 41
+// operations per path) and the tail (folds by transposed warp sums, the 4x4
+// algebra one element per lane: an FP64 operation holds a scheduler for 64
+// cycles with one lane or 32) -> 37 us.  Forward simulation of that put 2.9 ms
+// -> 55 us (one warp per 32 paths instead of 8 paths per thread in 128 CTAs).
+// The call 7.35 -> 1.92 ms.  FP32 pass of two contracts 62 -> 28 us, of ten
+// 100 -> 70 us, the same bits.
+//
 // nvcc-flags: --fmad=false
 #include <cuda_runtime.h>
 
 #include "device_common.cuh"
 #include "lsm.hpp"
+#include "lsm_math.cuh"
+#include "paths64.cuh"
 
 namespace mcdg {
 
 namespace {
-
-__device__ __forceinline__ double dmax(double a, double b) { return (a < b) ? b : a; }
-
-__device__ __forceinline__ double intrinsic(double s, double k, int type) {
-    return dmax((type == 0 ? 1.0 : -1.0) * (s - k), 0.0);
-}
-
-// Weighted Laguerre basis on x = S/K (src/pricers/lsm.cpp:21-25), the
-// reference's expressions (FP64 path).
-__device__ __forceinline__ void basis64(double s, double strike, double b[4]) {
-    const double x = s / strike;
-    const double e = exp(-x / 2.0);
-    b[0] = e;
-    b[1] = e * (1.0 - x);
-    b[2] = e * (1.0 - 2.0 * x + 0.5 * x * x);
-    b[3] = e * (1.0 - 3.0 * x + 1.5 * x * x - x * x * x / 6.0);
-}
 
 // FP32 path: the same basis evaluated in FP32.  FP64 arithmetic runs at a
 // small fraction of the FP32 rate on this GPU, and with FP32 paths the basis
@@ -98,10 +93,10 @@ __device__ __forceinline__ void df_add(float& hi, float& lo, float x) {
 // thread's (hi, lo) pairs go to shared memory, then warp w folds sums w,
 // w + 8, ...: lane l takes threads l, l + 32, ..., l + 224 in that order
 // (compensated), then a compensated shuffle tree; the FP64 value hi + lo of
-// each sum lands in res and, for thread 0, in out.
+// each sum lands in res.
 template <int N>
 __device__ void block_sum_df(const float (&hi)[N], const float (&lo)[N], float2 (*scratch)[kLsmThreads],
-                             double* res, double (&out)[N]) {
+                             double* res) {
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
 #pragma unroll
     for (int i = 0; i < N; ++i) scratch[i][t] = make_float2(hi[i], lo[i]);
@@ -124,10 +119,6 @@ __device__ void block_sum_df(const float (&hi)[N], const float (&lo)[N], float2 
         if (lane == 0) res[i] = static_cast<double>(h) + static_cast<double>(l);
     }
     __syncthreads();
-    if (t == 0) {
-#pragma unroll
-        for (int i = 0; i < N; ++i) out[i] = res[i];
-    }
 }
 
 // Chunk reduction of plain FP32 per-thread sums (the FP32 step's sums in a
@@ -152,91 +143,156 @@ __device__ void block_sum_f32(const float (&v)[N], float (*scratch)[kLsmThreads]
     __syncthreads();
 }
 
-template <int PREC>
-__device__ __forceinline__ double load_s(const void* store, uint64_t idx) {
-    if (PREC == 0) return static_cast<const double*>(store)[idx];
-    return static_cast<double>(static_cast<const float*>(store)[idx]);
+// The 15 sums of a chunk or fold over a warp, transposed: each step halves the
+// values a lane carries (16 additions instead of 75; an FP64 operation holds a
+// scheduler for 64 cycles, however many lanes are active).  The additions of
+// one value pair the lanes of a shuffle tree, so the bits are the tree's.
+// Lanes 2 i return sum i.
+__device__ __forceinline__ double warp_sums15(const double (&v)[15]) {
+    const int lane = threadIdx.x & 31;
+    const bool h16 = lane & 16, h8 = lane & 8, h4 = lane & 4, h2 = lane & 2;
+    auto at = [&](int i) { return i < 15 ? v[i < 15 ? i : 0] : 0.0; };
+    double a[8], b[4], c[2];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+        a[i] = (h16 ? at(i + 8) : at(i)) + __shfl_xor_sync(0xffffffffu, h16 ? at(i) : at(i + 8), 16);
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+        b[i] = (h8 ? a[i + 4] : a[i]) + __shfl_xor_sync(0xffffffffu, h8 ? a[i] : a[i + 4], 8);
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+        c[i] = (h4 ? b[i + 2] : b[i]) + __shfl_xor_sync(0xffffffffu, h4 ? b[i] : b[i + 2], 4);
+    const double d = (h2 ? c[1] : c[0]) + __shfl_xor_sync(0xffffffffu, h2 ? c[0] : c[1], 2);
+    return d + __shfl_xor_sync(0xffffffffu, d, 1);
 }
 
-// Fixed-shape block reduction of N doubles (256 threads): warp trees, then
-// warp 0 folds the 8 warp results in order.  Result valid in thread 0.
-template <int N>
-__device__ void block_sum(double (&v)[N], double (*smem)[N]) {
+// Fixed-shape block reduction of the 15 sums of the first `warps` warps (the
+// others hold zeros): warp trees, then the warps in order.  Result in res for
+// every thread after the closing barrier.
+__device__ __forceinline__ void block_sum15(const double (&v)[15], int warps, double (*smem)[15], double* res) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int i = 0; i < N; ++i) {
-        double x = v[i];
-#pragma unroll
-        for (int off = 16; off >= 1; off >>= 1) x += __shfl_down_sync(0xffffffffu, x, off);
-        v[i] = x;
-    }
-    if (lane == 0) {
-#pragma unroll
-        for (int i = 0; i < N; ++i) smem[warp][i] = v[i];
+    if (warp < warps) {
+        const double x = warp_sums15(v);
+        // lane = 16 b3 + 8 b2 + 4 b1 + 2 b0 holds sum b3 b2 b1 b0
+        if ((lane & 1) == 0 && lane < 30) smem[warp][lane >> 1] = x;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-#pragma unroll
-        for (int i = 0; i < N; ++i) {
-            double x = smem[0][i];
-            for (int w = 1; w < kLsmThreads / 32; ++w) x += smem[w][i];
-            v[i] = x;
-        }
+    if (threadIdx.x < 15) {
+        double x = smem[0][threadIdx.x];
+        for (int w = 1; w < warps; ++w) x += smem[w][threadIdx.x];
+        res[threadIdx.x] = x;
     }
+    __syncthreads();
 }
 
 // ---------------------------------------------------------------------------
 // forward simulation (src/pricers/lsm.cpp:35-58), date-major stores
 // ---------------------------------------------------------------------------
-template <int PREC>
+// FP64: one warp per 32 paths, the fixed-point tables shared by the SM's one
+// CTA; every warp takes every (number of warps)-th unit.
+struct ForwardSlot {
+    LsmDev c;
+    PhiloxStep step[32];
+};
+struct ForwardShared {
+    FixedShared tables;
+    ForwardSlot slot[32];
+};
+
+__global__ void __launch_bounds__(1024, 1)
+    lsm_forward64(const LsmDev* __restrict__ cs, const uint32_t* __restrict__ chunk_contract, uint32_t chunk_first,
+                  uint32_t chunk_end, double* __restrict__ store, const FixedTables* __restrict__ t) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    ForwardShared& sh = *reinterpret_cast<ForwardShared*>(smem);
+    load_fixed_tables(sh.tables, t);
+    const FixedShared& s = sh.tables;
+    const int lane = threadIdx.x & 31;
+    ForwardSlot& slot = sh.slot[threadIdx.x >> 5];
+    const LsmDev& c = slot.c;
+    constexpr uint32_t kUnits = kLsmChunk / 32;  // units of a chunk
+    const uint64_t units = static_cast<uint64_t>(chunk_end - chunk_first) * kUnits;
+    uint32_t have = 0xFFFFFFFFu;
+    for (uint64_t u = static_cast<uint64_t>(threadIdx.x >> 5) * gridDim.x + blockIdx.x; u < units; u += 32ull * gridDim.x) {
+        const uint32_t chunk = chunk_first + static_cast<uint32_t>(u / kUnits), ci = chunk_contract[chunk];
+        if (ci != have) {
+            have = ci;
+            __syncwarp();
+            copy_words(&slot.c, &cs[ci]);
+            __syncwarp();
+        }
+        const uint64_t base = static_cast<uint64_t>(chunk - c.chunk_begin) * kLsmChunk + (u % kUnits) * 32;
+        const uint64_t i = base + lane;
+        const bool live = i < c.path_count;
+        double* out = store + c.s_offset + i;
+        const PhiloxKeys k = philox_keys(c.seed);
+        const PhiloxRow row = philox_row(static_cast<uint32_t>(i), 0u, k);
+        int64_t y = 0;
+        double spot = c.spot;
+        for (int d0 = 0; d0 < c.n_steps; d0 += 32) {
+            __syncwarp();
+            PhiloxStep st = philox_step(static_cast<uint32_t>(d0 + lane), static_cast<uint32_t>(base >> 32), k);
+            st.carry = drift_carry(static_cast<uint32_t>(d0 + lane), c.y_drift_lo);
+            slot.step[lane] = st;
+            __syncwarp();
+            const int n = min(32, c.n_steps - d0);
+            for (int d = 0; d < n; ++d) {
+                const PhiloxStep w = slot.step[d];
+                const uint32_t bits = philox_word0(row, w, k);
+                if (c.frac > 0) {  // as LsmState64
+                    y += c.y_drift + w.carry + scaled_normal(normal_fixed(bits, s, t), c.y_vs);
+                    spot = c.spot * exp2_units(y, c.frac, s);
+                } else {
+                    spot = spot * exp(c.drift + c.vs * normal_from_bits_f64(bits));
+                }
+                if (live) *out = spot;
+                out += c.path_count;
+            }
+        }
+    }
+}
+
+// FP32: one CTA per chunk, two paths per thread at a time (independent Philox
+// chains), the step table of the path engine.
 __global__ void __launch_bounds__(kLsmThreads)
-    lsm_forward(const LsmDev* __restrict__ cs, const uint32_t* __restrict__ chunk_contract,
-                uint32_t chunk_first, uint32_t chunk_end, void* __restrict__ store) {
+    lsm_forward32(const LsmDev* __restrict__ cs, const uint32_t* __restrict__ chunk_contract, uint32_t chunk_first,
+                  uint32_t chunk_end, float* __restrict__ store) {
+    __shared__ PhiloxStep s_step[kStepTable];
     const uint32_t chunk = chunk_first + blockIdx.x;
     if (chunk >= chunk_end) return;
     const LsmDev c = cs[chunk_contract[chunk]];
-    const uint32_t local = chunk - c.chunk_begin;
     const PhiloxKeys k = philox_keys(c.seed);
-    const float mu = static_cast<float>(c.drift), sg = static_cast<float>(c.vs);
-    const float s0 = static_cast<float>(c.spot);
-    for (int j = 0; j < kLsmChunk / kLsmThreads; ++j) {
-        const uint64_t i = static_cast<uint64_t>(local) * kLsmChunk + j * kLsmThreads + threadIdx.x;
-        if (i >= c.path_count) break;
-        const PhiloxPath pp = philox_path(i, 0u, k);
-        if (PREC == 0) {
-            double* S = static_cast<double*>(store) + c.s_offset;
-            double s = c.spot;
-            for (int d = 0; d < c.n_steps; ++d) {
-                const double z = normal_from_bits_f64(philox_word0(pp, static_cast<uint32_t>(d), k));
-                s = gbm_step_f64(s, z, c.drift, c.vs);
-                S[static_cast<uint64_t>(d) * c.path_count + i] = s;
-            }
-        } else {
-            // two paths per iteration when both exist: independent Philox
-            // chains for instruction-level parallelism, the same values
-            float* S = static_cast<float*>(store) + c.s_offset;
-            const uint64_t i2 = i + kLsmThreads;
-            if ((j & 1) == 0 && j + 1 < kLsmChunk / kLsmThreads && i2 < c.path_count) {
-                const PhiloxPath pp2 = philox_path(i2, 0u, k);
-                float x = 0.0f, x2 = 0.0f;
-                float* out = S + i;  // date d's column, advanced by one column per date
-                for (int d = 0; d < c.n_steps; ++d) {
-                    const float z = normal_from_bits_f32(philox_word0(pp, static_cast<uint32_t>(d), k));
-                    const float z2 = normal_from_bits_f32(philox_word0(pp2, static_cast<uint32_t>(d), k));
-                    x = gbm_log_step_f32(x, z, mu, sg);
-                    x2 = gbm_log_step_f32(x2, z2, mu, sg);
-                    out[0] = gbm_spot_f32(s0, x);
-                    out[kLsmThreads] = gbm_spot_f32(s0, x2);
-                    out += c.path_count;
-                }
-                ++j;  // the partner path is done
-                continue;
-            }
-            float x = 0.0f;
-            for (int d = 0; d < c.n_steps; ++d) {
-                const float z = normal_from_bits_f32(philox_word0(pp, static_cast<uint32_t>(d), k));
-                x = gbm_log_step_f32(x, z, mu, sg);
-                S[static_cast<uint64_t>(d) * c.path_count + i] = gbm_spot_f32(s0, x);
+    const float mu = static_cast<float>(c.drift), sg = static_cast<float>(c.vs), s0 = static_cast<float>(c.spot);
+    const uint64_t base = static_cast<uint64_t>(chunk - c.chunk_begin) * kLsmChunk;
+    float* S = store + c.s_offset;
+    // dates outermost when the table has to be refilled: a chunk's log-paths
+    // stay in registers (8 per thread)
+    constexpr int kPer = kLsmChunk / kLsmThreads;
+    float x[kPer];
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) x[j] = 0.0f;
+    for (int d0 = 0; d0 < c.n_steps; d0 += kStepTable) {
+        if (d0 > 0) __syncthreads();
+        fill_steps(s_step, d0, static_cast<uint32_t>(base >> 32), k);
+        __syncthreads();
+        const int n = min(kStepTable, c.n_steps - d0);
+#pragma unroll
+        for (int j = 0; j < kPer; j += 2) {
+            const uint64_t i = base + j * kLsmThreads + threadIdx.x;
+            if (i >= c.path_count) continue;
+            const bool both = i + kLsmThreads < c.path_count;
+            const PhiloxRow row[2] = {philox_row(static_cast<uint32_t>(i), 0u, k),
+                                      philox_row(static_cast<uint32_t>(i) + kLsmThreads, 0u, k)};
+            float* out = S + static_cast<uint64_t>(d0) * c.path_count + i;  // advanced by one column per date
+            for (int d = 0; d < n; ++d) {
+                const PhiloxStep st = s_step[d];
+                const uint32_t bits[2] = {philox_word0(row[0], st, k), philox_word0(row[1], st, k)};
+                float z[2];
+                normals_from_bits_f32<2>(bits, z);
+                x[j] = gbm_log_step_f32(x[j], z[0], mu, sg);
+                x[j + 1] = gbm_log_step_f32(x[j + 1], z[1], mu, sg);
+                out[0] = gbm_spot_f32(s0, x[j]);
+                if (both) out[kLsmThreads] = gbm_spot_f32(s0, x[j + 1]);
+                out += c.path_count;
             }
         }
     }
@@ -373,7 +429,7 @@ __device__ __forceinline__ void store_T(LsmReg& r, const double T[4][4]) {
 // basis X P of preconditioner P (upper triangular).  Solves G beta = h by
 // the 4x4 Householder QR and returns gamma = P beta, the coefficients in the
 // Laguerre basis (the reference's policy layout).
-__device__ void solve_preconditioned(const double s[15], const double P[4][4], double gamma[4]) {
+__device__ void solve_preconditioned(const double* s, const double P[4][4], double gamma[4]) {
     double G[4][4], y[4], beta[4] = {0, 0, 0, 0};
     for (int a = 0; a < 4; ++a)
         for (int b2 = a; b2 < 4; ++b2) G[a][b2] = G[b2][a] = s[1 + tri(a, b2)];
@@ -399,7 +455,7 @@ __device__ void solve_preconditioned(const double s[15], const double P[4][4], d
 // factorisation is retried with a diagonal shift of 1e-10 of the trace --
 // shifted Cholesky QR (Fukaya, Kannan, Nakatsukasa, Zhang and Yamamoto, SIAM
 // J. Sci. Comput. 42 (2020)) -- and the second pass fits the unshifted problem.
-__device__ void solve_lagged(const double s[15], const double L[4][4], double kappa_max, LsmReg& r,
+__device__ void solve_lagged(const double* s, const double L[4][4], double kappa_max, LsmReg& r,
                              uint32_t* need_second_pass) {
     if (s[0] < 4.0) {  // too few in-the-money paths (src/pricers/lsm.cpp:102-104)
         r.has = -1;
@@ -460,7 +516,7 @@ __device__ void solve_lagged(const double s[15], const double L[4][4], double ka
             r.gamma[a] = x;
             r.gamma_f[a] = static_cast<float>(x);
         }
-        laguerre_poly(r.gamma, r.poly_f);
+        laguerre_poly(r.gamma, r.poly, r.poly_f);
         r.has = 1;
     } else {
         r.has = 2;
@@ -468,20 +524,154 @@ __device__ void solve_lagged(const double s[15], const double L[4][4], double ka
     }
 }
 
-// Fixed-order fold of a contract's chunk partials by the whole CTA: thread t
-// takes chunks t, t + 256, ... in order, then the fixed block tree; the
-// result is valid in thread 0.
-template <int N>
-__device__ void fold_partials(const LsmPartial* __restrict__ part, uint32_t begin, uint32_t count,
-                              double (&v)[N], double (*smem)[N]) {
+// solve_lagged by one warp, the same operations on the same operands (so the
+// same bits) with one matrix element per lane: lane 4a + b of each half-warp
+// holds element (a, b).  An FP64 operation holds the scheduler for 64 cycles
+// with one lane active or with 32, and the serial form is a chain of about 300
+// of them; this is about 115.  Only the form without a diagonal shift: a
+// matrix that is not positive definite goes to the serial routine.
+__device__ void solve_lagged_warp(const double* s /* shared, 15 */, const double* lag /* packed T, or null */,
+                                  double kappa_max, LsmReg& r, uint32_t* need_second_pass) {
+    constexpr unsigned kAll = 0xffffffffu;
+    const int lane = threadIdx.x & 31, a = (lane >> 2) & 3, b = lane & 3;
+    const bool writer = lane < 16 && a <= b;  // the upper triangle, first half-warp
+    double l[4];                              // row a of the lag
 #pragma unroll
-    for (int q = 0; q < N; ++q) v[q] = 0.0;
-    for (uint32_t ch = threadIdx.x; ch < count; ch += kLsmThreads) {
-        const double* p = part[begin + ch].v;
-#pragma unroll
-        for (int q = 0; q < N; ++q) v[q] += __ldcg(p + q);
+    for (int p = 0; p < 4; ++p) l[p] = lag ? (p >= a ? lag[tri(a, p)] : 0.0) : (p == a ? 1.0 : 0.0);
+    if (s[0] < 4.0) {  // too few in-the-money paths: the lag passes through
+        if (lane == 0) {
+            r.has = -1;
+            r.degenerate = 0;
+        }
+        if (writer) {
+            const double x = b == 0 ? l[0] : b == 1 ? l[1] : b == 2 ? l[2] : l[3];
+            r.T[tri(a, b)] = x;
+            r.T_f[tri(a, b)] = static_cast<float>(x);
+        }
+        return;
     }
-    block_sum<N>(v, smem);
+    // Cholesky G = R^T R, one row per step
+    double x = s[1 + (a <= b ? tri(a, b) : tri(b, a))], R = 0.0, rinv[4];
+    bool ok = true;
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+        const double d = __shfl_sync(kAll, x, 5 * p);
+        ok = ok && d > 0.0;
+        rinv[p] = rsqrt(d);
+        if (a == p) R = b == p ? d * rinv[p] : x * rinv[p];
+        const double ra = __shfl_sync(kAll, R, 4 * p + a), rb = __shfl_sync(kAll, R, 4 * p + b);
+        if (a > p && b >= a) x -= ra * rb;
+    }
+    if (!ok) {
+        if (lane == 0) {
+            double L[4][4];
+            for (int i = 0; i < 4; ++i)
+                for (int j = 0; j < 4; ++j) L[i][j] = lag ? (j >= i ? lag[tri(i, j)] : 0.0) : (i == j ? 1.0 : 0.0);
+            solve_lagged(s, L, kappa_max, r, need_second_pass);
+        }
+        return;
+    }
+    if (b < a) R = 0.0;
+    // row a of R^{-1}
+    double t[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) t[q] = q == a ? rinv[q] : 0.0;
+#pragma unroll
+    for (int q = 1; q < 4; ++q) {
+        double y = 0.0;
+#pragma unroll
+        for (int p = 0; p < q; ++p) {
+            const double rpq = __shfl_sync(kAll, R, 4 * p + q);
+            if (p >= a) y += t[p] * rpq;
+        }
+        if (q > a) t[q] = -y * rinv[q];
+    }
+    const double ri = b == 0 ? t[0] : b == 1 ? t[1] : b == 2 ? t[2] : t[3];
+    // ||R||^2 in the first half-warp, ||R^{-1}||^2 in the second
+    const double sq = lane < 16 ? R * R : ri * ri;
+    double norm = 0.0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = i; j < 4; ++j) norm += __shfl_sync(kAll, sq, (lane & 16) + 4 * i + j);
+    const double kappa = __shfl_sync(kAll, norm, 0) * __shfl_sync(kAll, norm, 16);
+    // T = L R^{-1}
+    double tab = 0.0;
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+        const double rpb = __shfl_sync(kAll, ri, 4 * p + b);
+        if (p >= a && p <= b) tab += l[p] * rpb;
+    }
+    if (writer) {
+        r.T[tri(a, b)] = tab;
+        r.T_f[tri(a, b)] = static_cast<float>(tab);
+    }
+    if (lane == 0) r.degenerate = 0;
+    if (!(kappa <= kappa_max)) {
+        if (lane == 0) {
+            r.has = 2;
+            atomicAdd(need_second_pass, 1u);
+        }
+        return;
+    }
+    double w = 0.0, beta = 0.0, gamma = 0.0;  // R^{-T} h by column b; R^{-1} w and L beta by row a
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+        const double rpb = __shfl_sync(kAll, ri, 4 * p + b);
+        if (p <= b) w += rpb * s[11 + p];
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const double wq = __shfl_sync(kAll, w, q);
+        if (q >= a) beta += t[q] * wq;
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const double bq = __shfl_sync(kAll, beta, 4 * q);
+        if (q >= a) gamma += l[q] * bq;
+    }
+    // laguerre_poly, coefficient a in row a
+    const double g[4] = {__shfl_sync(kAll, gamma, 0), __shfl_sync(kAll, gamma, 4), __shfl_sync(kAll, gamma, 8),
+                         __shfl_sync(kAll, gamma, 12)};
+    const double m1 = a == 0 ? 1.0 : a == 1 ? -1.0 : 0.0, m2 = a == 0 ? 1.0 : a == 1 ? -2.0 : 0.5;
+    const double m3 = a == 0 ? 1.0 : a == 1 ? -3.0 : 1.5;
+    double poly = a == 0 ? g[0] : 0.0;
+    poly += m1 * g[1];
+    poly += m2 * g[2];
+    poly += m3 * g[3];
+    const double q0 = -g[3] * (1.0 / 6.0);  // -g3 / 6, correctly rounded
+    const double sixth = fma(fma(-q0, 6.0, -g[3]), 1.0 / 6.0, q0);
+    if (a == 3) poly = sixth;
+    if (lane < 16 && b == 0) {
+        r.gamma[a] = gamma;
+        r.gamma_f[a] = static_cast<float>(gamma);
+        r.poly[a] = poly;
+        r.poly_f[a] = static_cast<float>(poly);
+    }
+    if (lane == 0) r.has = 1;
+}
+
+// Fixed-order fold of a contract's chunk partials by the whole CTA: thread t
+// takes rows t, t + blockDim, ... in order, then the fixed block tree; the result is
+// in res (shared) for every thread.
+__device__ __forceinline__ void fold_partials(const LsmPartial* __restrict__ part, uint32_t begin, uint32_t count,
+                                              double (*smem)[15], double* res) {
+    double v[15];
+#pragma unroll
+    for (int q = 0; q < 15; ++q) v[q] = 0.0;
+    for (uint32_t ch = threadIdx.x; ch < count; ch += blockDim.x) {
+        const double2* p = reinterpret_cast<const double2*>(part[begin + ch].v);
+        double row[16];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            const double2 x = __ldcg(p + q);
+            row[2 * q] = x.x;
+            row[2 * q + 1] = x.y;
+        }
+#pragma unroll
+        for (int q = 0; q < 15; ++q) v[q] = ch == threadIdx.x ? row[q] : v[q] + row[q];
+    }
+    block_sum15(v, static_cast<int>(min((count + 31u) / 32u, blockDim.x / 32u)), smem, res);
 }
 
 // One arrival at a completion counter; true in the CTA that arrives last.
@@ -502,31 +692,30 @@ __device__ __forceinline__ bool last_arrival(uint32_t* counter, uint32_t expecte
     return last;
 }
 
-// Publishes this CTA's chunk partial (thread 0 wrote part[chunk]) and climbs
-// the two-level tree of the contract's sums: the last chunk of a group of
-// LsmDev::fold_chunks chunks folds the group's partials in chunk order into
+// Publishes this CTA's chunk partial (in res; thread q < 15 writes entry q) and
+// climbs the two-level tree of the contract's sums: the last chunk of a group
+// of LsmDev::fold_chunks chunks folds the group's partials in chunk order into
 // the group partial, the last group of the contract folds the group partials
 // in group order.  Every fold is short (a few dozen to a few hundred rows over
 // the whole CTA), so the contract's totals are ready soon after its last
-// chunk.  Returns true in the CTA holding the totals (valid in thread 0).
+// chunk.  Returns true in the CTA holding the totals, then in res.
 // counters: the group counter of group g at group_counters[2 g], the
 // contract's at *contract_counter.
-__device__ bool publish_and_fold(uint32_t chunk, const LsmDev& c, const LsmPartial* __restrict__ part,
+__device__ bool publish_and_fold(uint32_t chunk, const LsmDev& c, LsmPartial* __restrict__ part,
                                  LsmPartial* __restrict__ gpart, uint32_t* group_counters,
-                                 uint32_t* contract_counter, double (&tot)[15], double (*smem)[15],
-                                 int* s_flag) {
+                                 uint32_t* contract_counter, double (*smem)[15], double* res, int* s_flag) {
     const uint32_t local = chunk - c.chunk_begin;
     const uint32_t g = local / c.fold_chunks;
     const uint32_t first = g * c.fold_chunks;
     const uint32_t count = min(c.fold_chunks, c.n_chunks - first);
+    if (threadIdx.x < 15) part[chunk].v[threadIdx.x] = res[threadIdx.x];
+    __syncthreads();
     if (!last_arrival(&group_counters[2 * (c.fold_begin + g)], count, s_flag)) return false;
-    fold_partials<15>(part, c.chunk_begin + first, count, tot, smem);
-    if (threadIdx.x == 0) {
-#pragma unroll
-        for (int q = 0; q < 15; ++q) gpart[c.fold_begin + g].v[q] = tot[q];
-    }
+    fold_partials(part, c.chunk_begin + first, count, smem, res);
+    if (threadIdx.x < 15) gpart[c.fold_begin + g].v[threadIdx.x] = res[threadIdx.x];
+    __syncthreads();
     if (!last_arrival(contract_counter, c.n_folds, s_flag)) return false;
-    fold_partials<15>(gpart, c.fold_begin, c.n_folds, tot, smem);
+    fold_partials(gpart, c.fold_begin, c.n_folds, smem, res);
     return true;
 }
 
@@ -535,22 +724,49 @@ __device__ bool publish_and_fold(uint32_t chunk, const LsmDev& c, const LsmParti
 // e-1 in the lagged basis -- or, when e = 1, the final Welford partial.  The
 // contract's last CTA folds the sums and solves date e-1.
 // ---------------------------------------------------------------------------
+// One in-the-money path's share of the regression sums in the basis b T
+// (b'_l = sum_{j <= l} b_j T[j][l]), FP64; entry 0, the count, is the caller's.
+__device__ __forceinline__ void add_sums64(double s, double inv_strike, const double (&T)[10], double v,
+                                           const GlobalTables& tables, double (&acc)[15]) {
+    double b[4];
+    basis64(s, inv_strike, tables, b);
+    const double q0 = b[0] * T[0];
+    const double q1 = fma(b[1], T[4], b[0] * T[1]);
+    const double q2 = fma(b[2], T[7], fma(b[1], T[5], b[0] * T[2]));
+    const double q3 = fma(b[3], T[9], fma(b[2], T[8], fma(b[1], T[6], b[0] * T[3])));
+    acc[1] = fma(q0, q0, acc[1]);
+    acc[2] = fma(q0, q1, acc[2]);
+    acc[3] = fma(q0, q2, acc[3]);
+    acc[4] = fma(q0, q3, acc[4]);
+    acc[5] = fma(q1, q1, acc[5]);
+    acc[6] = fma(q1, q2, acc[6]);
+    acc[7] = fma(q1, q3, acc[7]);
+    acc[8] = fma(q2, q2, acc[8]);
+    acc[9] = fma(q2, q3, acc[9]);
+    acc[10] = fma(q3, q3, acc[10]);
+    acc[11] = fma(q0, v, acc[11]);
+    acc[12] = fma(q1, v, acc[12]);
+    acc[13] = fma(q2, v, acc[13]);
+    acc[14] = fma(q3, v, acc[14]);
+}
+
 // COMP (FP32 path): the sums are compensated FP32 per thread and chunk (the
 // first iteration, whose basis is the raw Laguerre one); otherwise plain FP32
 // per thread and chunk -- the lagged basis is close to orthonormal, where
 // FP32 sums lose nothing the FP32 path data does not already carry.
 template <int PREC, bool COMP>
-__global__ void __launch_bounds__(kLsmThreads, PREC == 0 ? 1 : 8)
+__global__ void __launch_bounds__(kChunkThreads<PREC>, PREC == 0 ? 1 : 8)
     lsm_step(int k, const LsmDev* __restrict__ cs, const uint32_t* __restrict__ chunk_contract,
              uint32_t chunk_first, uint32_t chunk_end, const void* __restrict__ store, double* __restrict__ cf,
              LsmReg* __restrict__ reg, LsmPartial* __restrict__ part, LsmPartial* __restrict__ gpart,
              Welford* __restrict__ final_part, uint32_t* __restrict__ counters,
-             uint32_t* __restrict__ group_counters, uint32_t* __restrict__ need_second_pass, double kappa_max) {
-    __shared__ double smem[kLsmThreads / 32][15];
+             uint32_t* __restrict__ group_counters, uint32_t* __restrict__ need_second_pass, double kappa_max,
+             const FixedTables* __restrict__ fixed) {
+    __shared__ double smem[kChunkThreads<PREC> / 32][15];
     __shared__ float2 scratch[COMP ? 15 : 1][kLsmThreads];  // compensated sums' per-thread pairs
     __shared__ float pscratch[COMP ? 1 : 15][kLsmThreads];  // plain sums' per-thread values
     __shared__ double sres[15];
-    __shared__ Welford swf[kLsmThreads / 32];
+    __shared__ Welford swf[kChunkThreads<PREC> / 32];
     __shared__ Sum64 s64[kLsmThreads / 32];
     __shared__ int s_last;
     const uint32_t chunk = chunk_first + blockIdx.x;
@@ -565,17 +781,15 @@ __global__ void __launch_bounds__(kLsmThreads, PREC == 0 ? 1 : 8)
     const bool gram = !last;
     const LsmReg* re = (!init && e <= n - 1) ? &reg[c.reg_offset + e] : nullptr;
     const bool exercise = re != nullptr && re->has == 1;
-    double g0 = 0, g1 = 0, g2 = 0, g3 = 0;
-    if (exercise) {
-        g0 = re->gamma[0];
-        g1 = re->gamma[1];
-        g2 = re->gamma[2];
-        g3 = re->gamma[3];
-    }
     const uint32_t local = chunk - c.chunk_begin;
     Welford w{0ull, 0.0, 0.0};
-    double out[15];
     if constexpr (PREC == 0) {
+        const GlobalTables tables{fixed};
+        double poly[4] = {0.0, 0.0, 0.0, 0.0};
+        if (exercise) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) poly[q] = re->poly[q];
+        }
         // lagged preconditioner: date e's T (identity before the first regression)
         double T[10];
 #pragma unroll
@@ -583,66 +797,46 @@ __global__ void __launch_bounds__(kLsmThreads, PREC == 0 ? 1 : 8)
         double acc[15];
 #pragma unroll
         for (int q = 0; q < 15; ++q) acc[q] = 0.0;
-        for (int j = 0; j < kLsmChunk / kLsmThreads; ++j) {
-            const uint64_t i = static_cast<uint64_t>(local) * kLsmChunk + j * kLsmThreads + threadIdx.x;
-            if (i >= c.path_count) break;
-            double v;
-            if (init) {
-                v = intrinsic(load_s<PREC>(store, c.s_offset + static_cast<uint64_t>(n - 1) * c.path_count + i),
-                              c.strike, c.type);
-            } else {
-                v = cf[c.cf_offset + i];
-                if (exercise) {
-                    const double s = load_s<PREC>(store, c.s_offset + static_cast<uint64_t>(e - 1) * c.path_count + i);
-                    const double ex = intrinsic(s, c.strike, c.type);
-                    if (ex > 0.0) {
-                        double b[4];
-                        basis64(s, c.strike, b);
-                        double cont = 0.0;
-                        cont += g0 * b[0];
-                        cont += g1 * b[1];
-                        cont += g2 * b[2];
-                        cont += g3 * b[3];
-                        if (ex > cont) v = ex;
-                    }
-                }
+        const double* S = static_cast<const double*>(store) + c.s_offset;
+        const double* col_e = S + static_cast<uint64_t>(init ? n - 1 : e - 1) * c.path_count;
+        const double* col_d = S + static_cast<uint64_t>(gram ? e - 2 : 0) * c.path_count;
+        double* cash = cf + c.cf_offset;
+        // all loads of this thread's paths first (independent, in flight together)
+        constexpr int kPer = kLsmChunk / kLsmThreads64;
+        const uint64_t i0 = static_cast<uint64_t>(local) * kLsmChunk + threadIdx.x;
+        double vv[kPer], se[kPer], sd[kPer];
+#pragma unroll
+        for (int j = 0; j < kPer; ++j) {
+            const uint64_t i = i0 + j * kLsmThreads64;
+            const bool live = i < c.path_count;
+            vv[j] = live && !init ? cash[i] : 0.0;
+            se[j] = live && (init || exercise) ? col_e[i] : c.strike;
+            sd[j] = live && gram ? col_d[i] : c.strike;
+        }
+        uint32_t in_money = 0;
+#pragma unroll
+        for (int j = 0; j < kPer; ++j) {
+            const uint64_t i = i0 + j * kLsmThreads64;
+            if (i >= c.path_count) continue;
+            double v = vv[j];
+            if (in_the_money64(se[j], c.strike, c.type)) {
+                const double ex = put_sign(se[j] - c.strike, c.type);
+                if (init || ex > continuation64(se[j], c.inv_strike, poly, tables)) v = ex;
             }
             v *= c.disc;
             if (last) {
                 welford_add(w, v);
             } else {
-                cf[c.cf_offset + i] = v;
-                const double s = load_s<PREC>(store, c.s_offset + static_cast<uint64_t>(e - 2) * c.path_count + i);
-                if (intrinsic(s, c.strike, c.type) > 0.0) {
-                    double b[4];
-                    basis64(s, c.strike, b);
-                    // b'_l = sum_{j <= l} b_j T[j][l]
-                    const double q0 = b[0] * T[0];
-                    const double q1 = b[0] * T[1] + b[1] * T[4];
-                    const double q2 = b[0] * T[2] + b[1] * T[5] + b[2] * T[7];
-                    const double q3 = b[0] * T[3] + b[1] * T[6] + b[2] * T[8] + b[3] * T[9];
-                    acc[0] += 1.0;
-                    acc[1] += q0 * q0;
-                    acc[2] += q0 * q1;
-                    acc[3] += q0 * q2;
-                    acc[4] += q0 * q3;
-                    acc[5] += q1 * q1;
-                    acc[6] += q1 * q2;
-                    acc[7] += q1 * q3;
-                    acc[8] += q2 * q2;
-                    acc[9] += q2 * q3;
-                    acc[10] += q3 * q3;
-                    acc[11] += q0 * v;
-                    acc[12] += q1 * v;
-                    acc[13] += q2 * v;
-                    acc[14] += q3 * v;
+                cash[i] = v;
+                if (in_the_money64(sd[j], c.strike, c.type)) {
+                    ++in_money;
+                    add_sums64(sd[j], c.inv_strike, T, v, tables, acc);
                 }
             }
         }
         if (gram) {
-            block_sum<15>(acc, smem);
-#pragma unroll
-            for (int q = 0; q < 15; ++q) out[q] = acc[q];
+            acc[0] = static_cast<double>(in_money);
+            block_sum15(acc, kLsmThreads64 / 32, smem, sres);
         }
     } else {
         // FP32 paths: FP32 cash flows (stored in the FP64 buffer's space),
@@ -752,11 +946,9 @@ __global__ void __launch_bounds__(kLsmThreads, PREC == 0 ? 1 : 8)
         }
         if (gram) {
             if constexpr (COMP) {
-                block_sum_df<15>(hi, lo, scratch, sres, out);
+                block_sum_df<15>(hi, lo, scratch, sres);
             } else {
                 block_sum_f32<15>(hi, pscratch, sres);
-#pragma unroll
-                for (int q = 0; q < 15; ++q) out[q] = sres[q];
             }
         }
     }
@@ -767,7 +959,7 @@ __global__ void __launch_bounds__(kLsmThreads, PREC == 0 ? 1 : 8)
             __syncthreads();
             if (threadIdx.x == 0) {
                 Welford m = swf[0];
-                for (int q = 1; q < kLsmThreads / 32; ++q) m = welford_merge(m, swf[q]);
+                for (int q = 1; q < kLsmThreads64 / 32; ++q) m = welford_merge(m, swf[q]);
                 final_part[chunk] = m;
             }
         } else {
@@ -776,22 +968,9 @@ __global__ void __launch_bounds__(kLsmThreads, PREC == 0 ? 1 : 8)
         }
         return;
     }
-    if (threadIdx.x == 0) {
-#pragma unroll
-        for (int q = 0; q < 15; ++q) part[chunk].v[q] = out[q];
-    }
-    double tot[15];
-    if (!publish_and_fold(chunk, c, part, gpart, group_counters, &counters[2 * ci], tot, smem, &s_last)) return;
-    if (threadIdx.x == 0) {
-        double L[4][4];
-        if (init) {
-            for (int a = 0; a < 4; ++a)
-                for (int b2 = 0; b2 < 4; ++b2) L[a][b2] = a == b2 ? 1.0 : 0.0;
-        } else {
-            unpack_upper(re->T, L);
-        }
-        solve_lagged(tot, L, kappa_max, reg[c.reg_offset + e - 1], need_second_pass + k);
-    }
+    if (!publish_and_fold(chunk, c, part, gpart, group_counters, &counters[2 * ci], smem, sres, &s_last)) return;
+    if (threadIdx.x < 32)
+        solve_lagged_warp(sres, init ? nullptr : re->T, kappa_max, reg[c.reg_offset + e - 1], need_second_pass + k);
 }
 
 // Second pass for the dates solve_lagged marked (has = 2): the sums in the
@@ -799,13 +978,13 @@ __global__ void __launch_bounds__(kLsmThreads, PREC == 0 ? 1 : 8)
 // path), then the contract's last chunk solves (has = 1).  A small
 // persistent grid walks the chunks and skips those of other contracts.
 template <int PREC>
-__global__ void __launch_bounds__(kLsmThreads, PREC == 0 ? 1 : 4)
+__global__ void __launch_bounds__(kChunkThreads<PREC>, PREC == 0 ? 1 : 4)
     lsm_refine(int k, const LsmDev* __restrict__ cs, const uint32_t* __restrict__ chunk_contract,
                uint32_t chunk_first, uint32_t chunk_end, const void* __restrict__ store, const double* __restrict__ cf,
                LsmReg* __restrict__ reg, LsmPartial* __restrict__ part, LsmPartial* __restrict__ gpart,
                uint32_t* __restrict__ counters, uint32_t* __restrict__ group_counters,
-               const uint32_t* __restrict__ need_second_pass) {
-    __shared__ double smem[kLsmThreads / 32][15];
+               const uint32_t* __restrict__ need_second_pass, const FixedTables* __restrict__ fixed) {
+    __shared__ double smem[kChunkThreads<PREC> / 32][15];
     __shared__ float2 scratch[15][kLsmThreads];  // FP32 path: the sums' per-thread pairs
     __shared__ double sres[15];
     __shared__ int s_last;
@@ -818,45 +997,26 @@ __global__ void __launch_bounds__(kLsmThreads, PREC == 0 ? 1 : 4)
     LsmReg& r = reg[c.reg_offset + date];
     if (r.has != 2) continue;  // solved by the first pass, or no regression at this date
     const uint32_t local = chunk - c.chunk_begin;
-    double out[15];
     if constexpr (PREC == 0) {
+        const GlobalTables tables{fixed};
         double T[10];
 #pragma unroll
         for (int q = 0; q < 10; ++q) T[q] = r.T[q];
         double acc[15];
 #pragma unroll
         for (int q = 0; q < 15; ++q) acc[q] = 0.0;
-        for (int j = 0; j < kLsmChunk / kLsmThreads; ++j) {
-            const uint64_t i = static_cast<uint64_t>(local) * kLsmChunk + j * kLsmThreads + threadIdx.x;
+        const double* S = static_cast<const double*>(store) + c.s_offset + static_cast<uint64_t>(date - 1) * c.path_count;
+        uint32_t in_money = 0;
+        for (int j = 0; j < kLsmChunk / kLsmThreads64; ++j) {
+            const uint64_t i = static_cast<uint64_t>(local) * kLsmChunk + j * kLsmThreads64 + threadIdx.x;
             if (i >= c.path_count) break;
-            const double s = load_s<PREC>(store, c.s_offset + static_cast<uint64_t>(date - 1) * c.path_count + i);
-            if (!(intrinsic(s, c.strike, c.type) > 0.0)) continue;
-            double b[4];
-            basis64(s, c.strike, b);
-            const double q0 = b[0] * T[0];
-            const double q1 = b[0] * T[1] + b[1] * T[4];
-            const double q2 = b[0] * T[2] + b[1] * T[5] + b[2] * T[7];
-            const double q3 = b[0] * T[3] + b[1] * T[6] + b[2] * T[8] + b[3] * T[9];
-            const double y = cf[c.cf_offset + i];
-            acc[0] += 1.0;
-            acc[1] += q0 * q0;
-            acc[2] += q0 * q1;
-            acc[3] += q0 * q2;
-            acc[4] += q0 * q3;
-            acc[5] += q1 * q1;
-            acc[6] += q1 * q2;
-            acc[7] += q1 * q3;
-            acc[8] += q2 * q2;
-            acc[9] += q2 * q3;
-            acc[10] += q3 * q3;
-            acc[11] += q0 * y;
-            acc[12] += q1 * y;
-            acc[13] += q2 * y;
-            acc[14] += q3 * y;
+            const double s = S[i];
+            if (!in_the_money64(s, c.strike, c.type)) continue;
+            ++in_money;
+            add_sums64(s, c.inv_strike, T, cf[c.cf_offset + i], tables, acc);
         }
-        block_sum<15>(acc, smem);
-#pragma unroll
-        for (int q = 0; q < 15; ++q) out[q] = acc[q];
+        acc[0] = static_cast<double>(in_money);
+        block_sum15(acc, kLsmThreads64 / 32, smem, sres);
     } else {
         float T[10];
 #pragma unroll
@@ -903,23 +1063,18 @@ __global__ void __launch_bounds__(kLsmThreads, PREC == 0 ? 1 : 4)
             df_add(hi[13], lo[13], q2 * y);
             df_add(hi[14], lo[14], q3 * y);
         }
-        block_sum_df<15>(hi, lo, scratch, sres, out);
+        block_sum_df<15>(hi, lo, scratch, sres);
     }
-    if (threadIdx.x == 0) {
-#pragma unroll
-        for (int q = 0; q < 15; ++q) part[chunk].v[q] = out[q];
-    }
-    double tot[15];
-    if (publish_and_fold(chunk, c, part, gpart, group_counters + 1, &counters[2 * ci + 1], tot, smem, &s_last)) {
+    if (publish_and_fold(chunk, c, part, gpart, group_counters + 1, &counters[2 * ci + 1], smem, sres, &s_last)) {
         if (threadIdx.x == 0) {
             double T[4][4], gamma[4];
             unpack_upper(r.T, T);
-            solve_preconditioned(tot, T, gamma);
+            solve_preconditioned(sres, T, gamma);
             for (int a = 0; a < 4; ++a) {
                 r.gamma[a] = gamma[a];
                 r.gamma_f[a] = static_cast<float>(gamma[a]);
             }
-            laguerre_poly(r.gamma, r.poly_f);
+            laguerre_poly(r.gamma, r.poly, r.poly_f);
             r.has = 1;
         }
     }
@@ -951,17 +1106,22 @@ __global__ void lsm_finish(const LsmDev* __restrict__ cs, int n_contracts,
 
 }  // namespace
 
-cudaError_t launch_lsm_forward(int precision, const LsmDev* c, int n_contracts,
-                               const uint32_t* chunk_contract, uint32_t chunk_first, uint32_t chunk_count,
-                               void* s_store, cudaStream_t stream) {
-    (void)n_contracts;
+cudaError_t launch_lsm_forward(int precision, int sm_count, const LsmDev* c, const uint32_t* chunk_contract,
+                               uint32_t chunk_first, uint32_t chunk_count, void* s_store, const FixedTables* tables,
+                               cudaStream_t stream) {
     cudaGetLastError();
     if (chunk_count == 0) return cudaSuccess;
     const uint32_t end = chunk_first + chunk_count;
-    if (precision == 0)
-        lsm_forward<0><<<chunk_count, kLsmThreads, 0, stream>>>(c, chunk_contract, chunk_first, end, s_store);
-    else
-        lsm_forward<1><<<chunk_count, kLsmThreads, 0, stream>>>(c, chunk_contract, chunk_first, end, s_store);
+    if (precision == 0) {
+        constexpr int bytes = static_cast<int>(sizeof(ForwardShared));
+        cudaError_t e = cudaFuncSetAttribute(lsm_forward64, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+        if (e != cudaSuccess) return e;
+        lsm_forward64<<<sm_count, 1024, bytes, stream>>>(c, chunk_contract, chunk_first, end,
+                                                         static_cast<double*>(s_store), tables);
+    } else {
+        lsm_forward32<<<chunk_count, kLsmThreads, 0, stream>>>(c, chunk_contract, chunk_first, end,
+                                                               static_cast<float*>(s_store));
+    }
     return cudaGetLastError();
 }
 
@@ -969,7 +1129,7 @@ cudaError_t launch_lsm_iteration(int precision, int k, const LsmDev* c, int n_co
                                  const uint32_t* chunk_contract, uint32_t chunk_first, uint32_t chunk_count,
                                  uint32_t total_folds, const void* s_store, double* cf, LsmReg* reg,
                                  LsmPartial* part, LsmPartial* gpart, Welford* final_part, uint32_t* counters,
-                                 cudaStream_t stream) {
+                                 const FixedTables* tables, cudaStream_t stream) {
     cudaGetLastError();
     if (chunk_count == 0) return cudaSuccess;
     const uint32_t end = chunk_first + chunk_count;
@@ -992,26 +1152,28 @@ cudaError_t launch_lsm_iteration(int precision, int k, const LsmDev* c, int n_co
     // FP32 basis values carry anyway.
     if (precision == 0) {
         if (k == 0)
-            lsm_step<0, true><<<chunk_count, kLsmThreads, 0, stream>>>(
+            lsm_step<0, true><<<chunk_count, kLsmThreads64, 0, stream>>>(
                 k, c, chunk_contract, chunk_first, end, s_store, cf, reg, part, gpart, final_part, counters,
-                group_counters, need, 1e2);
+                group_counters, need, 1e2, tables);
         else
-            lsm_step<0, false><<<chunk_count, kLsmThreads, 0, stream>>>(
+            lsm_step<0, false><<<chunk_count, kLsmThreads64, 0, stream>>>(
                 k, c, chunk_contract, chunk_first, end, s_store, cf, reg, part, gpart, final_part, counters,
-                group_counters, need, 1e2);
-        lsm_refine<0><<<refine_grid, kLsmThreads, 0, stream>>>(k, c, chunk_contract, chunk_first, end, s_store, cf,
-                                                               reg, part, gpart, counters, group_counters, need);
+                group_counters, need, 1e2, tables);
+        lsm_refine<0><<<refine_grid, kLsmThreads64, 0, stream>>>(k, c, chunk_contract, chunk_first, end, s_store, cf,
+                                                               reg, part, gpart, counters, group_counters, need,
+                                                               tables);
     } else {
         if (k == 0)
             lsm_step<1, true><<<chunk_count, kLsmThreads, 0, stream>>>(
                 k, c, chunk_contract, chunk_first, end, s_store, cf, reg, part, gpart, final_part, counters,
-                group_counters, need, 1e3);
+                group_counters, need, 1e3, tables);
         else
             lsm_step<1, false><<<chunk_count, kLsmThreads, 0, stream>>>(
                 k, c, chunk_contract, chunk_first, end, s_store, cf, reg, part, gpart, final_part, counters,
-                group_counters, need, 1e3);
+                group_counters, need, 1e3, tables);
         lsm_refine<1><<<refine_grid, kLsmThreads, 0, stream>>>(k, c, chunk_contract, chunk_first, end, s_store, cf,
-                                                               reg, part, gpart, counters, group_counters, need);
+                                                               reg, part, gpart, counters, group_counters, need,
+                                                               tables);
     }
     return cudaGetLastError();
 }

@@ -9,7 +9,10 @@
 namespace mcdg {
 
 constexpr int kLsmChunk = 1024;      // paths per chunk (fixed reduction unit)
-constexpr int kLsmThreads = 128;     // 8 paths per thread per chunk
+constexpr int kLsmThreads = 128;     // FP32: 8 paths per thread per chunk
+constexpr int kLsmThreads64 = 256;   // FP64: 4 paths per thread (two warps per scheduler cover each other's loads)
+template <int PREC>
+constexpr int kChunkThreads = PREC == 0 ? kLsmThreads64 : kLsmThreads;
 constexpr unsigned kRefineGrid = 1216;  // CTAs of the second regression pass (8 per SM)
 constexpr int kLsmBasis = 4;         // weighted Laguerre, degree 3 (src/pricers/lsm.cpp:16-25)
 
@@ -32,6 +35,13 @@ struct LsmDev {
     uint32_t fold_begin, n_folds;    // QR regression: second level of the chunk-sum tree,
     uint32_t fold_chunks;            // groups of fold_chunks chunks
     float strike_f, inv_strike_f, disc_f, phi_f;  // FP32 copies for the FP32-path kernels
+    // FP64 paths: the log2 step in units of 2^-frac (frac = 0: outside the
+    // fixed-point range) and 1 / K
+    int32_t frac;
+    uint32_t y_drift_lo;
+    int64_t y_drift;
+    uint64_t y_vs;
+    double inv_strike;
 };
 
 constexpr int kLsmMaxGroups = 256;  // learned-regression CTAs per contract at most
@@ -47,12 +57,13 @@ constexpr int kGramPacked = 66 * 67 / 2;  // upper triangle of the 66 x 66 Gram 
 struct LsmReg {
     double T[10];
     double gamma[4];
+    double poly[4];       // the continuation value e^{-x/2} (p0 + p1 x + p2 x^2 + p3 x^3), x = S/K: the
+                          // Laguerre combination gamma expanded in FP64 (laguerre_poly)
     int32_t has;          // 1 coefficients valid (>= 4 ITM paths), -1 no regression, 2 second pass pending
     int32_t degenerate;   // Cholesky of the lagged Gram matrix: 0 plain, 2 with a diagonal shift, 1 failed
     float T_f[10];        // FP32 copies for the FP32-path kernels (written with T and gamma)
     float gamma_f[4];
-    float poly_f[4];      // FP32 path: the continuation value e^{-x/2} (p0 + p1 x + p2 x^2 + p3 x^3),
-                          // x = S/K, the Laguerre combination gamma expanded in FP64 (laguerre_poly)
+    float poly_f[4];
 };
 
 // Per-chunk partial sums of one date's regression: count + 10 Gram entries +
@@ -68,6 +79,9 @@ struct LsmPartial {
 struct FrozenScenario {
     double spot, drift, vs;
     float spot_f, mu_f, sg_f, pad;
+    int64_t y_drift;      // FP64: the scenario's log2 step in the contract's units (LsmDev::frac)
+    uint64_t y_vs;
+    uint32_t y_drift_lo, pad2;
 };
 constexpr int kFrozenScenarios = 5;  // base, spot+h, spot-h, vol+h, vol-h
 constexpr int kFrozenOutputs = 8;    // five scenario averages, then the CRN delta, gamma, vega
@@ -77,24 +91,23 @@ struct FrozenDev {
     float inv_2hs_f, inv_hs2_f, inv_2hv_f, pad;
 };
 
-// Forward simulation of chunks [chunk_first, chunk_first + chunk_count).
 // Monomial coefficients of gamma_0 L_0 + ... + gamma_3 L_3 (the weighted
 // Laguerre polynomials of src/pricers/lsm.cpp:21-25 without their common
-// factor e^{-x/2}), computed in FP64 and rounded once.
-__host__ __device__ inline void laguerre_poly(const double gamma[4], float poly[4]) {
-    poly[0] = static_cast<float>(gamma[0] + gamma[1] + gamma[2] + gamma[3]);
-    poly[1] = static_cast<float>(-gamma[1] - 2.0 * gamma[2] - 3.0 * gamma[3]);
-    poly[2] = static_cast<float>(0.5 * gamma[2] + 1.5 * gamma[3]);
-    poly[3] = static_cast<float>(-gamma[3] / 6.0);
+// factor e^{-x/2}).
+__host__ __device__ inline void laguerre_poly(const double gamma[4], double poly[4], float poly_f[4]) {
+    poly[0] = gamma[0] + gamma[1] + gamma[2] + gamma[3];
+    poly[1] = -gamma[1] - 2.0 * gamma[2] - 3.0 * gamma[3];
+    poly[2] = 0.5 * gamma[2] + 1.5 * gamma[3];
+    poly[3] = -gamma[3] / 6.0;
+    for (int i = 0; i < 4; ++i) poly_f[i] = static_cast<float>(poly[i]);
 }
 
 #ifdef __CUDACC__
-// One date of a stored GBM path: FP32 paths step ln(S/S0) and store
-// S0 exp(x); FP64 paths multiply S by exp(drift + vs z).  Every kernel that
-// regenerates stored path values uses these, so they agree bit for bit.
+// One date of a stored FP32 GBM path: ln(S/S0) is stepped, S0 exp(x) stored.
+// Every kernel that regenerates stored path values uses these, so they agree
+// bit for bit (FP64: lsm_math.cuh).
 __device__ __forceinline__ float gbm_log_step_f32(float x, float z, float mu, float sg) { return __fmaf_rn(sg, z, x + mu); }
 __device__ __forceinline__ float gbm_spot_f32(float s0, float x) { return s0 * __expf(x); }
-__device__ __forceinline__ double gbm_step_f64(double s, double z, double drift, double vs) { return s * exp(drift + vs * z); }
 // FP32 continuation value at S from poly (the FP32 backward pass and the
 // FP32 frozen replay both use this, so their decisions coincide).
 __device__ __forceinline__ float continuation_poly32(float s, float inv_strike, const float p[4]) {
@@ -104,9 +117,10 @@ __device__ __forceinline__ float continuation_poly32(float s, float inv_strike, 
 }
 #endif
 
-cudaError_t launch_lsm_forward(int precision, const LsmDev* c, int n_contracts,
-                               const uint32_t* chunk_contract, uint32_t chunk_first, uint32_t chunk_count,
-                               void* s_store, cudaStream_t stream);
+// Forward simulation of chunks [chunk_first, chunk_first + chunk_count).
+cudaError_t launch_lsm_forward(int precision, int sm_count, const LsmDev* c, const uint32_t* chunk_contract,
+                               uint32_t chunk_first, uint32_t chunk_count, void* s_store, const FixedTables* tables,
+                               cudaStream_t stream);
 // One backward iteration k (see lsm.cu) of the contracts whose chunks are
 // [chunk_first, chunk_first + chunk_count) -- whole contracts.  part: one
 // partial per chunk, gpart: one per fold group (LsmDev::fold_begin/n_folds),
@@ -117,7 +131,7 @@ cudaError_t launch_lsm_iteration(int precision, int k, const LsmDev* c, int n_co
                                  const uint32_t* chunk_contract, uint32_t chunk_first, uint32_t chunk_count,
                                  uint32_t total_folds, const void* s_store, double* cf, LsmReg* reg,
                                  LsmPartial* part, LsmPartial* gpart, Welford* final_part, uint32_t* counters,
-                                 cudaStream_t stream);
+                                 const FixedTables* tables, cudaStream_t stream);
 cudaError_t launch_lsm_finish(const LsmDev* c, int n_contracts, const Welford* final_part,
                               double* out /* n x 6: price, se, count, inception, mean, se */,
                               cudaStream_t stream);
@@ -128,6 +142,7 @@ cudaError_t launch_lsm_finish(const LsmDev* c, int n_contracts, const Welford* f
 // outputs = 1 for one scenario, kFrozenOutputs for five).
 cudaError_t launch_lsm_frozen(int precision, int n_scenarios, const LsmDev* c, const FrozenDev* f,
                               int n_contracts, const uint32_t* chunk_contract, uint32_t total_chunks,
-                              const LsmReg* reg, Welford* partials, double* out, cudaStream_t stream);
+                              const LsmReg* reg, Welford* partials, double* out, const FixedTables* tables,
+                              cudaStream_t stream);
 
 }  // namespace mcdg

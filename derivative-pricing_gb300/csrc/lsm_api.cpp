@@ -69,6 +69,11 @@ int plan_lsm(Ctx& ctx, const mcd_lsm_contract* cs, size_t n, LsmPlan& p) {
         d.inv_strike_f = static_cast<float>(1.0 / c.strike);
         d.disc_f = static_cast<float>(d.disc);
         d.phi_f = c.type == 0 ? 1.0f : -1.0f;
+        d.inv_strike = 1.0 / c.strike;
+        // Fixed point leaves room for a replay at up to twice the volatility
+        // (four times the log-spot's bound) within a double's exponents.
+        d.frac = c.vol * std::sqrt(c.time) <= 4.0 ? fixed_frac(c.monitoring_points, d.drift, d.vs) : 0;
+        if (d.frac) fixed_step(d.drift, d.vs, d.frac, &d.y_drift, &d.y_drift_lo, &d.y_vs);
         d.seed = c.seed;
         d.path_count = c.path_count;
         d.n_steps = c.monitoring_points;
@@ -189,9 +194,12 @@ int upload_and_run(Ctx& ctx, const LsmPlan& p, int precision, bool frozen, std::
     if (e != cudaSuccess) return ctx.cuda_fail(e, "lsm upload");
     const MlpConfig cfg{ctx.mlp_steps_first, ctx.mlp_steps, ctx.mlp_lr_first, ctx.mlp_lr};
 
-    // Capture forward pass + every backward iteration + finish into one graph.
+    // Forward pass, every backward iteration and the finish, queued directly: a
+    // call's launches are enqueued while its first kernels run, where a graph
+    // would have to be instantiated before the first of them (the launches
+    // depend on the batch, so it would serve one call only).
     // The contracts run as up to kLsmChains independent chains (contiguous
-    // ranges of about equal chunk counts), each captured on its own stream: a
+    // ranges of about equal chunk counts), each on its own stream: a
     // date ends with a tail of little parallelism -- the QR pass's last chunk
     // folds and per-contract solve, the learned fit's Gram slices and
     // per-contract solve -- and another chain's work fills the GPU meanwhile.
@@ -229,9 +237,9 @@ int upload_and_run(Ctx& ctx, const LsmPlan& p, int precision, bool frozen, std::
         }
     }
     cudaGetLastError();
-    cudaGraph_t graph = nullptr;
-    e = cudaStreamBeginCapture(ctx.stream, cudaStreamCaptureModeThreadLocal);
-    if (e != cudaSuccess) return ctx.cuda_fail(e, "lsm begin capture");
+    int pair = -1;
+    rc = ctx.record_start(ctx.stream, &pair);
+    if (rc) return rc;
     const LsmDev* d_dev = static_cast<const LsmDev*>(ctx.ext[kDev].ptr);
     const uint32_t* d_map = static_cast<const uint32_t*>(ctx.ext[kChunkMap].ptr);
     // The chains start one after another: chain j+1's forward simulation
@@ -259,7 +267,7 @@ int upload_and_run(Ctx& ctx, const LsmPlan& p, int precision, bool frozen, std::
                                                    static_cast<float*>(ctx.ext[kFeats].ptr),
                                                    static_cast<double*>(ctx.ext[kPreS].ptr),
                                                    static_cast<double*>(ctx.ext[kPreCf].ptr), cfg,
-                                                   static_cast<uint32_t*>(ctx.ext[kErr].ptr), ts);
+                                                   static_cast<uint32_t*>(ctx.ext[kErr].ptr), ctx.tables, ts);
             if (le == cudaSuccess) le = cudaEventRecord(ctx.ev_train[j], ts);
         }
     }
@@ -268,8 +276,8 @@ int upload_and_run(Ctx& ctx, const LsmPlan& p, int precision, bool frozen, std::
         cudaStream_t cs = j == 0 ? ctx.stream : ctx.aux_stream[j - 1];
         if (j > 0) le = cudaStreamWaitEvent(cs, ctx.ev_stage[j - 1], 0);
         if (le == cudaSuccess)
-            le = launch_lsm_forward(precision, d_dev, static_cast<int>(n), d_map, ch.chunk_first, ch.chunk_count,
-                                    ctx.ext[kStore].ptr, cs);
+            le = launch_lsm_forward(precision, ctx.sm_count, d_dev, d_map, ch.chunk_first, ch.chunk_count,
+                                    ctx.ext[kStore].ptr, ctx.tables, cs);
         if (le == cudaSuccess && j + 1 < chains.size()) le = cudaEventRecord(ctx.ev_stage[j], cs);
         for (int k = 0; k < ch.max_steps && le == cudaSuccess; ++k) {
             if (mlp)
@@ -295,7 +303,7 @@ int upload_and_run(Ctx& ctx, const LsmPlan& p, int precision, bool frozen, std::
                                           static_cast<LsmPartial*>(ctx.ext[kPartA].ptr),
                                           static_cast<LsmPartial*>(ctx.ext[kPartB].ptr),
                                           static_cast<Welford*>(ctx.ext[kFinal].ptr),
-                                          static_cast<uint32_t*>(ctx.ext[kCounters].ptr), cs);
+                                          static_cast<uint32_t*>(ctx.ext[kCounters].ptr), ctx.tables, cs);
         }
         if (j > 0 && le == cudaSuccess) le = cudaEventRecord(ctx.ev_join[j - 1], cs);
     }
@@ -304,31 +312,18 @@ int upload_and_run(Ctx& ctx, const LsmPlan& p, int precision, bool frozen, std::
     if (le == cudaSuccess)
         le = launch_lsm_finish(d_dev, static_cast<int>(n), static_cast<const Welford*>(ctx.ext[kFinal].ptr),
                                static_cast<double*>(ctx.ext[kOut].ptr), ctx.stream);
-    e = cudaStreamEndCapture(ctx.stream, &graph);
-    if (le != cudaSuccess) {
-        if (graph) cudaGraphDestroy(graph);
+    if (le != cudaSuccess) {  // let what was queued finish before the buffers are used again
         cudaGetLastError();
-        return ctx.cuda_fail(le, "lsm capture");
+        cudaDeviceSynchronize();
+        return ctx.cuda_fail(le, "lsm launch");
     }
-    if (e != cudaSuccess) return ctx.cuda_fail(e, "lsm end capture");
-    cudaGraphExec_t exec = nullptr;
-    e = cudaGraphInstantiate(&exec, graph, 0);
-    cudaGraphDestroy(graph);
-    if (e != cudaSuccess) return ctx.cuda_fail(e, "lsm instantiate");
-    int pair = -1;
-    rc = ctx.record_start(ctx.stream, &pair);
-    if (!rc) {
-        e = cudaGraphLaunch(exec, ctx.stream);
-        if (e != cudaSuccess) rc = ctx.cuda_fail(e, "lsm graph launch");
-    }
-    if (!rc) rc = ctx.record_stop(ctx.stream, pair);
+    rc = ctx.record_stop(ctx.stream, pair);
     out.assign(6 * n, 0.0);
     if (!rc) {
         e = cudaMemcpyAsync(out.data(), ctx.ext[kOut].ptr, sizeof(double) * 6 * n, cudaMemcpyDeviceToHost, ctx.stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(ctx.stream);
         if (e != cudaSuccess) rc = ctx.cuda_fail(e, "lsm execution");
     }
-    cudaGraphExecDestroy(exec);
     ctx.collect_timing(false);
     if (!rc && mlp) {
         uint32_t werr = 0;
@@ -402,7 +397,7 @@ int lsm_batch(Ctx& ctx, const mcd_lsm_contract* cs, size_t n, int precision, int
 
 // One scenario's inputs: the GBM step constants of `vol` in the order of
 // plan_lsm (src/models/gbm.cpp:8-10), plus the FP32 kernel's copies.
-FrozenScenario scenario(double spot, const mcd_lsm_contract& c, double vol) {
+FrozenScenario scenario(double spot, const mcd_lsm_contract& c, double vol, int frac) {
     const double dt = c.time / static_cast<double>(c.monitoring_points);
     FrozenScenario s{};
     s.spot = spot;
@@ -411,19 +406,20 @@ FrozenScenario scenario(double spot, const mcd_lsm_contract& c, double vol) {
     s.spot_f = static_cast<float>(spot);
     s.mu_f = static_cast<float>(s.drift);
     s.sg_f = static_cast<float>(s.vs);
+    if (frac) fixed_step(s.drift, s.vs, frac, &s.y_drift, &s.y_drift_lo, &s.y_vs);
     return s;
 }
 
 // Scenarios base, spot +/- hs, vol +/- hv (hs = hv = 0: the base alone).
 // The kernel shares the base's growth factors with the two spot scenarios,
 // so those must keep the base volatility.
-FrozenDev frozen_dev(const mcd_lsm_contract& c, double hs, double hv) {
+FrozenDev frozen_dev(const mcd_lsm_contract& c, int frac, double hs, double hv) {
     FrozenDev f{};
-    f.sc[0] = scenario(c.spot, c, c.vol);
-    f.sc[1] = scenario(c.spot + hs, c, c.vol);
-    f.sc[2] = scenario(c.spot - hs, c, c.vol);
-    f.sc[3] = scenario(c.spot, c, c.vol + hv);
-    f.sc[4] = scenario(c.spot, c, c.vol - hv);
+    f.sc[0] = scenario(c.spot, c, c.vol, frac);
+    f.sc[1] = scenario(c.spot + hs, c, c.vol, frac);
+    f.sc[2] = scenario(c.spot - hs, c, c.vol, frac);
+    f.sc[3] = scenario(c.spot, c, c.vol + hv, frac);
+    f.sc[4] = scenario(c.spot, c, c.vol - hv, frac);
     f.inv_2hs = hs > 0.0 ? 0.5 / hs : 0.0;
     f.inv_hs2 = hs > 0.0 ? 1.0 / (hs * hs) : 0.0;
     f.inv_2hv = hv > 0.0 ? 0.5 / hv : 0.0;
@@ -464,7 +460,7 @@ int frozen_run(Ctx& ctx, const LsmPlan& p, const std::vector<FrozenDev>& fz, int
                           static_cast<const FrozenDev*>(ctx.ext[kFzDev].ptr), static_cast<int>(n),
                           static_cast<const uint32_t*>(ctx.ext[kChunkMap].ptr), p.total_chunks,
                           static_cast<const LsmReg*>(ctx.ext[kReg].ptr), static_cast<Welford*>(ctx.ext[kFzPart].ptr),
-                          static_cast<double*>(ctx.ext[kFzOut].ptr), ctx.stream);
+                          static_cast<double*>(ctx.ext[kFzOut].ptr), ctx.tables, ctx.stream);
     if (e != cudaSuccess) return ctx.cuda_fail(e, "frozen launch");
     rc = ctx.record_stop(ctx.stream, pair);
     if (rc) return rc;
@@ -488,7 +484,7 @@ std::vector<LsmReg> policy_table(const LsmPlan& p, int monitoring_points, const 
             reg[d].gamma[b] = coefficients[4 * d + b];
             reg[d].gamma_f[b] = static_cast<float>(coefficients[4 * d + b]);
         }
-        laguerre_poly(reg[d].gamma, reg[d].poly_f);
+        laguerre_poly(reg[d].gamma, reg[d].poly, reg[d].poly_f);
     }
     return reg;
 }
@@ -562,7 +558,7 @@ int mcd_lsm_reprice_frozen(mcd_ctx* handle, double spot, double strike, double r
     int rc = plan_lsm(*ctx, &c, 1, p);
     if (rc) return rc;
     const std::vector<LsmReg> reg = policy_table(p, monitoring_points, coefficients, has_coefficients);
-    const std::vector<FrozenDev> fz{frozen_dev(c, 0.0, 0.0)};
+    const std::vector<FrozenDev> fz{frozen_dev(c, p.dev[0].frac, 0.0, 0.0)};
     std::vector<double> out;
     rc = frozen_run(*ctx, p, fz, precision, 1, &reg, out);
     if (rc) return rc;
@@ -590,7 +586,7 @@ int mcd_lsm_frozen_greeks(mcd_ctx* handle, double spot, double strike, double ra
     int rc = plan_lsm(*ctx, &c, 1, p);
     if (rc) return rc;
     const std::vector<LsmReg> reg = policy_table(p, monitoring_points, coefficients, has_coefficients);
-    const std::vector<FrozenDev> fz{frozen_dev(c, spot_bump, vol_bump)};
+    const std::vector<FrozenDev> fz{frozen_dev(c, p.dev[0].frac, spot_bump, vol_bump)};
     std::vector<double> res;
     rc = frozen_run(*ctx, p, fz, precision, kFrozenScenarios, &reg, res);
     if (rc) return rc;
@@ -617,7 +613,7 @@ int mcd_lsm_greeks_batch(mcd_ctx* handle, const mcd_lsm_contract* contracts, siz
     if (rc) return rc;
     std::vector<FrozenDev> fz(n);
     for (size_t i = 0; i < n; ++i)
-        fz[i] = frozen_dev(contracts[i], spot_bump_rel * contracts[i].spot, vol_bump_rel * contracts[i].vol);
+        fz[i] = frozen_dev(contracts[i], p.dev[i].frac, spot_bump_rel * contracts[i].spot, vol_bump_rel * contracts[i].vol);
     std::vector<double> res;
     rc = frozen_run(*ctx, p, fz, precision, kFrozenScenarios, nullptr, res);
     if (rc) return rc;

@@ -25,6 +25,7 @@
 
 #include "device_common.cuh"
 #include "lsm.hpp"
+#include "lsm_math.cuh"
 
 namespace mcdg {
 
@@ -33,19 +34,6 @@ namespace {
 __device__ __forceinline__ double intrinsic(double s, double k, int type) {
     const double x = (type == 0 ? 1.0 : -1.0) * (s - k);
     return (x < 0.0) ? 0.0 : x;
-}
-
-// Weighted Laguerre basis (src/pricers/lsm.cpp:21-25), FP64, and the FP32
-// path's version; both as in the backward pass, so decisions agree with it.
-__device__ __forceinline__ double continuation64(double s, double strike, const double g[4]) {
-    const double x = s / strike;
-    const double e = exp(-x / 2.0);
-    double cont = 0.0;
-    cont += g[0] * e;
-    cont += g[1] * (e * (1.0 - x));
-    cont += g[2] * (e * (1.0 - 2.0 * x + 0.5 * x * x));
-    cont += g[3] * (e * (1.0 - 3.0 * x + 1.5 * x * x - x * x * x / 6.0));
-    return cont;
 }
 
 // Scenarios by volatility: {base, spot+h, spot-h} share the base's GBM step
@@ -64,11 +52,19 @@ __device__ __forceinline__ bool group_live(const bool (&live)[NS], int gi) {
 
 // One path, NS scenarios: cash flow of each scenario, discounted to t = 0.
 template <int NS>
-__device__ void replay64(const LsmDev& c, const FrozenDev& f, const LsmReg* __restrict__ rg, const PhiloxPath& pp,
-                         const PhiloxKeys& k, double (&v)[NS]) {
-    double s[NS];
+__device__ void replay64(const LsmDev& c, const FrozenDev& f, const LsmReg* __restrict__ rg, uint64_t path,
+                         const PhiloxKeys& k, const GlobalTables& tables, double (&v)[NS]) {
+    // per volatility group: the log-spot (units of 2^-frac), or the product of
+    // growth factors outside the fixed-point range
+    int64_t y[kGroups<NS>];
+    double growth[kGroups<NS>], s[NS];
     int stop[NS];
     bool live[NS];
+#pragma unroll
+    for (int gi = 0; gi < kGroups<NS>; ++gi) {
+        y[gi] = 0;
+        growth[gi] = 1.0;
+    }
 #pragma unroll
     for (int q = 0; q < NS; ++q) {
         s[q] = f.sc[q].spot;
@@ -76,34 +72,40 @@ __device__ void replay64(const LsmDev& c, const FrozenDev& f, const LsmReg* __re
         live[q] = true;
         v[q] = 0.0;
     }
+    const uint32_t path_hi = static_cast<uint32_t>(path >> 32);
+    const PhiloxRow row = philox_row(static_cast<uint32_t>(path), 0u, k);
     int n_live = NS;
     for (int d = 0; d < c.n_steps && n_live > 0; ++d) {
-        const double z = normal_from_bits_f64(philox_word0(pp, static_cast<uint32_t>(d), k));
+        const uint32_t du = static_cast<uint32_t>(d);
+        const uint32_t bits = philox_word0(row, philox_step(du, path_hi, k), k);
         const int date = d + 1;
         const bool test = date < c.n_steps && rg[date].has == 1;
-        double g[4] = {0.0, 0.0, 0.0, 0.0};
+        double p[4] = {0.0, 0.0, 0.0, 0.0};
         if (test) {
-            g[0] = rg[date].gamma[0];
-            g[1] = rg[date].gamma[1];
-            g[2] = rg[date].gamma[2];
-            g[3] = rg[date].gamma[3];
-        }
-        // one growth factor per volatility group (src/models/gbm.cpp:7-12):
-        // the spot scenarios share the base's, bit for bit
-        double gr[kGroups<NS>];
 #pragma unroll
-        for (int gi = 0; gi < kGroups<NS>; ++gi) {
-            gr[gi] = 1.0;
-            if (group_live<NS>(live, gi))
-                gr[gi] = exp(f.sc[group_lead(gi)].drift + f.sc[group_lead(gi)].vs * z);
+            for (int q = 0; q < 4; ++q) p[q] = rg[date].poly[q];
+        }
+        if (c.frac > 0) {  // the spot scenarios share the base's growth
+            const FixedNormal z = tables.normal(bits);
+#pragma unroll
+            for (int gi = 0; gi < kGroups<NS>; ++gi) {
+                const FrozenScenario& sc = f.sc[group_lead(gi)];
+                y[gi] += sc.y_drift + drift_carry(du, sc.y_drift_lo) + scaled_normal(z, sc.y_vs);
+                growth[gi] = tables.exp2(y[gi], c.frac);
+            }
+        } else {
+            const double z = normal_from_bits_f64(bits);
+#pragma unroll
+            for (int gi = 0; gi < kGroups<NS>; ++gi)
+                if (group_live<NS>(live, gi)) growth[gi] = exp(f.sc[group_lead(gi)].drift + f.sc[group_lead(gi)].vs * z);
         }
 #pragma unroll
         for (int q = 0; q < NS; ++q) {
             if (!live[q]) continue;
-            s[q] = s[q] * gr[group_of(q)];
+            s[q] = (c.frac > 0 ? f.sc[q].spot : s[q]) * growth[group_of(q)];
             if (test) {
                 const double ex = intrinsic(s[q], c.strike, c.type);
-                if (ex > 0.0 && ex > continuation64(s[q], c.strike, g)) {
+                if (ex > 0.0 && ex > continuation64(s[q], c.inv_strike, p, tables)) {
                     v[q] = ex;
                     stop[q] = date;
                     live[q] = false;
@@ -187,12 +189,13 @@ __device__ void replay32(const LsmDev& c, const FrozenDev& f, const LsmReg* __re
 // each (measured 1.3x faster than 512 threads at 106 registers on the 20-put
 // grid: paths that exercise early leave the pass latency-bound).
 template <int PREC, int NS>
-__global__ void __launch_bounds__(kLsmThreads, ((PREC == 1 && NS > 1) ? 3 : 2) * (256 / kLsmThreads))
+__global__ void __launch_bounds__(kChunkThreads<PREC>, ((PREC == 1 && NS > 1) ? 3 : 2) * (256 / kChunkThreads<PREC>))
     lsm_frozen_stream(const LsmDev* __restrict__ cs, const FrozenDev* __restrict__ fz,
                       const uint32_t* __restrict__ chunk_contract, uint32_t total_chunks,
-                      const LsmReg* __restrict__ reg, Welford* __restrict__ part) {
+                      const LsmReg* __restrict__ reg, Welford* __restrict__ part,
+                      const FixedTables* __restrict__ fixed) {
     constexpr int NW = NS == 1 ? 1 : kFrozenOutputs;
-    __shared__ Welford swf[kLsmThreads / 32][NW];
+    __shared__ Welford swf[kLsmThreads64 / 32][NW];
     __shared__ Sum64 s64[NW][kLsmThreads / 32];
     const uint32_t chunk = blockIdx.x;
     if (chunk >= total_chunks) return;
@@ -206,11 +209,11 @@ __global__ void __launch_bounds__(kLsmThreads, ((PREC == 1 && NS > 1) ? 3 : 2) *
         Welford w[NW];
 #pragma unroll
         for (int q = 0; q < NW; ++q) w[q] = Welford{0ull, 0.0, 0.0};
-        for (int j = 0; j < kLsmChunk / kLsmThreads; ++j) {
-            const uint64_t i = static_cast<uint64_t>(local) * kLsmChunk + j * kLsmThreads + threadIdx.x;
+        for (int j = 0; j < kLsmChunk / kLsmThreads64; ++j) {
+            const uint64_t i = static_cast<uint64_t>(local) * kLsmChunk + j * kLsmThreads64 + threadIdx.x;
             if (i >= c.path_count) break;
             double v[NS];
-            replay64<NS>(c, f, rg, philox_path(i, 0u, k), k, v);
+            replay64<NS>(c, f, rg, i, k, GlobalTables{fixed}, v);
 #pragma unroll
             for (int q = 0; q < NS; ++q) welford_add(w[q], v[q]);
             if constexpr (NS == kFrozenScenarios) {
@@ -228,7 +231,7 @@ __global__ void __launch_bounds__(kLsmThreads, ((PREC == 1 && NS > 1) ? 3 : 2) *
         if (threadIdx.x < NW) {
             const int q = threadIdx.x;
             Welford m = swf[0][q];
-            for (int wi = 1; wi < kLsmThreads / 32; ++wi) m = welford_merge(m, swf[wi][q]);
+            for (int wi = 1; wi < kLsmThreads64 / 32; ++wi) m = welford_merge(m, swf[wi][q]);
             part[static_cast<uint64_t>(chunk) * NW + q] = m;
         }
     } else {
@@ -287,17 +290,18 @@ __global__ void lsm_frozen_finish(const LsmDev* __restrict__ cs, int n_contracts
 
 cudaError_t launch_lsm_frozen(int precision, int n_scenarios, const LsmDev* c, const FrozenDev* f,
                               int n_contracts, const uint32_t* chunk_contract, uint32_t total_chunks,
-                              const LsmReg* reg, Welford* partials, double* out, cudaStream_t stream) {
+                              const LsmReg* reg, Welford* partials, double* out, const FixedTables* tables,
+                              cudaStream_t stream) {
     cudaGetLastError();
     if (n_scenarios != 1 && n_scenarios != kFrozenScenarios) return cudaErrorInvalidValue;
     if (total_chunks) {
         const bool five = n_scenarios == kFrozenScenarios;
         if (precision == 0) {
-            if (five) lsm_frozen_stream<0, kFrozenScenarios><<<total_chunks, kLsmThreads, 0, stream>>>(c, f, chunk_contract, total_chunks, reg, partials);
-            else lsm_frozen_stream<0, 1><<<total_chunks, kLsmThreads, 0, stream>>>(c, f, chunk_contract, total_chunks, reg, partials);
+            if (five) lsm_frozen_stream<0, kFrozenScenarios><<<total_chunks, kLsmThreads64, 0, stream>>>(c, f, chunk_contract, total_chunks, reg, partials, tables);
+            else lsm_frozen_stream<0, 1><<<total_chunks, kLsmThreads64, 0, stream>>>(c, f, chunk_contract, total_chunks, reg, partials, tables);
         } else {
-            if (five) lsm_frozen_stream<1, kFrozenScenarios><<<total_chunks, kLsmThreads, 0, stream>>>(c, f, chunk_contract, total_chunks, reg, partials);
-            else lsm_frozen_stream<1, 1><<<total_chunks, kLsmThreads, 0, stream>>>(c, f, chunk_contract, total_chunks, reg, partials);
+            if (five) lsm_frozen_stream<1, kFrozenScenarios><<<total_chunks, kLsmThreads, 0, stream>>>(c, f, chunk_contract, total_chunks, reg, partials, tables);
+            else lsm_frozen_stream<1, 1><<<total_chunks, kLsmThreads, 0, stream>>>(c, f, chunk_contract, total_chunks, reg, partials, tables);
         }
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;

@@ -46,6 +46,7 @@
 #include "cp_async.cuh"
 #include "device_common.cuh"
 #include "lsm.hpp"
+#include "lsm_math.cuh"
 #include "lsm_mlp_dev.hpp"
 #include "mlp.cuh"
 #include "umma.cuh"
@@ -400,7 +401,7 @@ __device__ __forceinline__ uint64_t train_sample_path(const LsmDev& c, int date,
 // Training samples of the first (latest) regression date, drawn without the
 // path store: sample s of step st is path i of the contract, regenerated from
 // its Philox stream up to date n with the forward simulation's arithmetic
-// (gbm_log_step_f32 / gbm_step_f64), so its spot at date n-1 and its terminal
+// (gbm_log_step_f32 / LsmState64), so its spot at date n-1 and its terminal
 // cash flow (the payoff at date n, discounted once, rounded as the cash-flow
 // store holds it) equal what the stores will hold bit for bit.  The training
 // then needs neither the forward simulation nor the terminal step and runs
@@ -410,7 +411,8 @@ __device__ __forceinline__ uint64_t train_sample_path(const LsmDev& c, int date,
 template <int PREC>
 __global__ void __launch_bounds__(128)
     lsm_mlp_train_samples(const LsmDev* __restrict__ cs, int c_first, int n_contracts, int steps,
-                          double* __restrict__ pre_s, double* __restrict__ pre_cf) {
+                          double* __restrict__ pre_s, double* __restrict__ pre_cf,
+                          const FixedTables* __restrict__ fixed) {
     const int ci = c_first + static_cast<int>(blockIdx.x), s = threadIdx.x;
     if (ci >= n_contracts) return;
     const LsmDev c = cs[ci];
@@ -422,13 +424,12 @@ __global__ void __launch_bounds__(128)
         const PhiloxPath pp = philox_path(i, 0u, key);
         double s_prev = 0.0, s_last = 0.0;
         if (PREC == 0) {
-            double sp = c.spot;
+            LsmState64 p(c);
             for (int d = 0; d < n; ++d) {
-                const double z = normal_from_bits_f64(philox_word0(pp, static_cast<uint32_t>(d), key));
-                sp = gbm_step_f64(sp, z, c.drift, c.vs);
-                if (d == n - 2) s_prev = sp;
+                p.advance(c, philox_word0(pp, static_cast<uint32_t>(d), key), static_cast<uint32_t>(d), GlobalTables{fixed});
+                if (d == n - 2) s_prev = p.s;
             }
-            s_last = sp;
+            s_last = p.s;
         } else {
             const float mu = static_cast<float>(c.drift), sg = static_cast<float>(c.vs), s0 = static_cast<float>(c.spot);
             float x = 0.0f;
@@ -1327,16 +1328,16 @@ cudaError_t mlp_prepare() {
 cudaError_t launch_lsm_mlp_first_training(int precision, const LsmDev* c, int c_first, int c_end, int max_steps,
                                           float* nets, float* snaps, int* snap_ok, int* adam_t, float* feats,
                                           double* pre_s, double* pre_cf, const MlpConfig& cfg, uint32_t* err,
-                                          cudaStream_t stream) {
+                                          const FixedTables* tables, cudaStream_t stream) {
     cudaGetLastError();
     if (c_end <= c_first) return cudaSuccess;
     const int n_contracts = c_end - c_first;
     if (cfg.steps_first > 0) {
         const dim3 grid(static_cast<unsigned>(n_contracts), static_cast<unsigned>(std::min(cfg.steps_first, 1024)));
         if (precision == 0)
-            lsm_mlp_train_samples<0><<<grid, 128, 0, stream>>>(c, c_first, c_end, cfg.steps_first, pre_s, pre_cf);
+            lsm_mlp_train_samples<0><<<grid, 128, 0, stream>>>(c, c_first, c_end, cfg.steps_first, pre_s, pre_cf, tables);
         else
-            lsm_mlp_train_samples<1><<<grid, 128, 0, stream>>>(c, c_first, c_end, cfg.steps_first, pre_s, pre_cf);
+            lsm_mlp_train_samples<1><<<grid, 128, 0, stream>>>(c, c_first, c_end, cfg.steps_first, pre_s, pre_cf, tables);
     }
     // the trainer reads no store at k = 0 when the samples are given
     if (precision == 0)

@@ -100,6 +100,7 @@ cudaError_t mlp_prepare();  // opts the kernels into their dynamic shared memory
 cudaError_t launch_lsm_mlp_first_training(int precision, const LsmDev* c, int c_first, int c_end, int max_steps,
                                           float* nets, float* snaps, int* snap_ok, int* adam_t, float* feats,
                                           double* pre_s, double* pre_cf, const MlpConfig& cfg, uint32_t* err,
+                                          const FixedTables* tables,
                                           cudaStream_t stream);
 // One backward iteration k: exercise at date n-k, discount, and (train =
 // true) the Gram matrix and output-layer fit of date n-k-1 on node tables; at
