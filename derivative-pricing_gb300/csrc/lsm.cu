@@ -55,12 +55,13 @@
 // The call 7.35 -> 1.92 ms.  FP32 pass of two contracts 62 -> 28 us, of ten
 // 100 -> 70 us, the same bits.
 //
-// nvcc-flags: --fmad=false
+// nvcc-flags: --fmad=false --ftz=true
 #include <cuda_runtime.h>
 
 #include "device_common.cuh"
 #include "lsm.hpp"
 #include "lsm_math.cuh"
+#include "merge.cuh"
 #include "paths64.cuh"
 
 namespace mcdg {
@@ -71,13 +72,18 @@ namespace {
 // small fraction of the FP32 rate on this GPU, and with FP32 paths the basis
 // carries FP32 inputs anyway; the regression is fitted to exactly this
 // evaluated basis and the sums that need the range stay compensated (below).
-__device__ __forceinline__ void basis32(float s, float inv_strike, float b[4]) {
+__device__ __forceinline__ float sixth(float x) {  // x / 6, correctly rounded (Markstein), without the division's slow path
+    constexpr float y = 1.0f / 6.0f;
+    const float q = x * y;
+    return __fmaf_rn(__fmaf_rn(-6.0f, q, x), y, q);
+}
+__device__ __forceinline__ void basis32(float s, float inv_strike, bool use, float b[4]) {  // use: else zeros
     const float x = s * inv_strike;
-    const float e = __expf(-0.5f * x);
+    const float e = use ? __expf(-0.5f * x) : 0.0f;
     b[0] = e;
     b[1] = e * (1.0f - x);
     b[2] = e * __fmaf_rn(0.5f * x, x, __fmaf_rn(-2.0f, x, 1.0f));
-    b[3] = e * __fmaf_rn(__fmaf_rn(-x / 6.0f, x, 1.5f * x), x, __fmaf_rn(-3.0f, x, 1.0f));
+    b[3] = e * __fmaf_rn(__fmaf_rn(-sixth(x), x, 1.5f * x), x, __fmaf_rn(-3.0f, x, 1.0f));
 }
 
 // Compensated FP32 accumulation (Knuth's TwoSum): hi + lo carries ~44 bits,
@@ -251,48 +257,59 @@ __global__ void __launch_bounds__(1024, 1)
     }
 }
 
+// Two paths from table step 0 to n, from log-spots x, storing S0 e^x per date.
+__device__ __forceinline__ void forward_pair32(const PhiloxStep* table, int n, const PhiloxKeys& k, uint32_t path_lo,
+                                               float mu, float sg, float s0, uint64_t column, bool both,
+                                               float (&x)[2], float* __restrict__ out) {
+    const PhiloxRow row[2] = {philox_row(path_lo, 0u, k), philox_row(path_lo + kLsmThreads, 0u, k)};
+    for (int d = 0; d < n; ++d) {
+        const PhiloxStep st = table[d];
+        const uint32_t bits[2] = {philox_word0(row[0], st, k), philox_word0(row[1], st, k)};
+        float z[2];
+        normals_from_bits_f32<2>(bits, z);
+        x[0] = gbm_log_step_f32(x[0], z[0], mu, sg);
+        x[1] = gbm_log_step_f32(x[1], z[1], mu, sg);
+        out[0] = gbm_spot_f32(s0, x[0]);
+        if (both) out[kLsmThreads] = gbm_spot_f32(s0, x[1]);
+        out += column;  // one column per date
+    }
+}
+
 // FP32: one CTA per chunk, two paths per thread at a time (independent Philox
-// chains), the step table of the path engine.
-__global__ void __launch_bounds__(kLsmThreads)
+// chains), the step table of the path engine.  A contract of more dates than
+// the table holds keeps its chunk's log-spots in shared memory between refills.
+__global__ void __launch_bounds__(kLsmThreads, 8)
     lsm_forward32(const LsmDev* __restrict__ cs, const uint32_t* __restrict__ chunk_contract, uint32_t chunk_first,
                   uint32_t chunk_end, float* __restrict__ store) {
     __shared__ PhiloxStep s_step[kStepTable];
+    __shared__ float s_x[kLsmChunk];
     const uint32_t chunk = chunk_first + blockIdx.x;
     if (chunk >= chunk_end) return;
-    const LsmDev c = cs[chunk_contract[chunk]];
+    const LsmDev& c = cs[chunk_contract[chunk]];
     const PhiloxKeys k = philox_keys(c.seed);
     const float mu = static_cast<float>(c.drift), sg = static_cast<float>(c.vs), s0 = static_cast<float>(c.spot);
-    const uint64_t base = static_cast<uint64_t>(chunk - c.chunk_begin) * kLsmChunk;
+    const uint64_t base = static_cast<uint64_t>(chunk - c.chunk_begin) * kLsmChunk, paths = c.path_count;
     float* S = store + c.s_offset;
-    // dates outermost when the table has to be refilled: a chunk's log-paths
-    // stay in registers (8 per thread)
-    constexpr int kPer = kLsmChunk / kLsmThreads;
-    float x[kPer];
-#pragma unroll
-    for (int j = 0; j < kPer; ++j) x[j] = 0.0f;
-    for (int d0 = 0; d0 < c.n_steps; d0 += kStepTable) {
+    const int n = c.n_steps;
+    for (int d0 = 0; d0 < n; d0 += kStepTable) {
         if (d0 > 0) __syncthreads();
         fill_steps(s_step, d0, static_cast<uint32_t>(base >> 32), k);
         __syncthreads();
-        const int n = min(kStepTable, c.n_steps - d0);
-#pragma unroll
-        for (int j = 0; j < kPer; j += 2) {
-            const uint64_t i = base + j * kLsmThreads + threadIdx.x;
-            if (i >= c.path_count) continue;
-            const bool both = i + kLsmThreads < c.path_count;
-            const PhiloxRow row[2] = {philox_row(static_cast<uint32_t>(i), 0u, k),
-                                      philox_row(static_cast<uint32_t>(i) + kLsmThreads, 0u, k)};
-            float* out = S + static_cast<uint64_t>(d0) * c.path_count + i;  // advanced by one column per date
-            for (int d = 0; d < n; ++d) {
-                const PhiloxStep st = s_step[d];
-                const uint32_t bits[2] = {philox_word0(row[0], st, k), philox_word0(row[1], st, k)};
-                float z[2];
-                normals_from_bits_f32<2>(bits, z);
-                x[j] = gbm_log_step_f32(x[j], z[0], mu, sg);
-                x[j + 1] = gbm_log_step_f32(x[j + 1], z[1], mu, sg);
-                out[0] = gbm_spot_f32(s0, x[j]);
-                if (both) out[kLsmThreads] = gbm_spot_f32(s0, x[j + 1]);
-                out += c.path_count;
+        const int m = min(kStepTable, n - d0);
+        for (int j = 0; j < kLsmChunk; j += 2 * kLsmThreads) {
+            const int at = j + threadIdx.x;
+            const uint64_t i = base + at;
+            if (i >= paths) break;
+            float x[2] = {0.0f, 0.0f};
+            if (d0 > 0) {
+                x[0] = s_x[at];
+                x[1] = s_x[at + kLsmThreads];
+            }
+            forward_pair32(s_step, m, k, static_cast<uint32_t>(i), mu, sg, s0, paths, i + kLsmThreads < paths, x,
+                           S + static_cast<uint64_t>(d0) * paths + i);
+            if (m < n) {
+                s_x[at] = x[0];
+                s_x[at + kLsmThreads] = x[1];
             }
         }
     }
@@ -884,59 +901,82 @@ __global__ void __launch_bounds__(kChunkThreads<PREC>, PREC == 0 ? 1 : 8)
                 if (gram) sd[j] = col_d[o];
             }
         }
+        if constexpr (!COMP) {
+            // Branch-free, so that the paths of a thread interleave: a path that
+            // is not in the money enters with e = 0, x = 1 and no cash flow, and
+            // adds zeros (the sums keep their bits).  Nearly every warp holds
+            // in-the-money lanes, so a branch would skip nothing.
 #pragma unroll
-        for (int j = 0; j < kPer; ++j) {
-            if (!live[j]) continue;
-            float v = init ? fmaxf(phi * (vv[j] - strike), 0.0f) : vv[j];
-            if (exercise) {
+            for (int j = 0; j < kPer; ++j) {
                 const float ex = phi * (se[j] - strike);
-                if (ex > 0.0f && ex > continuation_poly32(se[j], inv_kf, poly)) v = ex;
+                float v = exercise && ex > 0.0f && ex > continuation_poly32(se[j], inv_kf, poly) ? ex : vv[j];
+                v *= disc;
+                if (last) {
+                    if (live[j]) sum32_add(fin, v);
+                    continue;
+                }
+                if (live[j]) cf_t[j * kLsmThreads] = v;
+                const bool itm = live[j] && phi * (sd[j] - strike) > 0.0f;
+                float b[4];
+                basis32(itm ? sd[j] : strike, inv_kf, itm, b);
+                v = itm ? v : 0.0f;
+                const float q0 = b[0] * T[0];
+                const float q1 = __fmaf_rn(b[1], T[4], b[0] * T[1]);
+                const float q2 = __fmaf_rn(b[2], T[7], __fmaf_rn(b[1], T[5], b[0] * T[2]));
+                const float q3 = __fmaf_rn(b[3], T[9], __fmaf_rn(b[2], T[8], __fmaf_rn(b[1], T[6], b[0] * T[3])));
+                hi[0] += itm ? 1.0f : 0.0f;  // exact: a chunk holds fewer than 2^24 paths
+                hi[1] = __fmaf_rn(q0, q0, hi[1]);
+                hi[2] = __fmaf_rn(q0, q1, hi[2]);
+                hi[3] = __fmaf_rn(q0, q2, hi[3]);
+                hi[4] = __fmaf_rn(q0, q3, hi[4]);
+                hi[5] = __fmaf_rn(q1, q1, hi[5]);
+                hi[6] = __fmaf_rn(q1, q2, hi[6]);
+                hi[7] = __fmaf_rn(q1, q3, hi[7]);
+                hi[8] = __fmaf_rn(q2, q2, hi[8]);
+                hi[9] = __fmaf_rn(q2, q3, hi[9]);
+                hi[10] = __fmaf_rn(q3, q3, hi[10]);
+                hi[11] = __fmaf_rn(q0, v, hi[11]);
+                hi[12] = __fmaf_rn(q1, v, hi[12]);
+                hi[13] = __fmaf_rn(q2, v, hi[13]);
+                hi[14] = __fmaf_rn(q3, v, hi[14]);
             }
-            v *= disc;
-            if (last) {
-                sum32_add(fin, v);
-            } else {
-                cf_t[j * kLsmThreads] = v;
-                if (phi * (sd[j] - strike) > 0.0f) {
-                    float b[4];
-                    basis32(sd[j], inv_kf, b);
-                    const float q0 = b[0] * T[0];
-                    const float q1 = __fmaf_rn(b[1], T[4], b[0] * T[1]);
-                    const float q2 = __fmaf_rn(b[2], T[7], __fmaf_rn(b[1], T[5], b[0] * T[2]));
-                    const float q3 = __fmaf_rn(b[3], T[9], __fmaf_rn(b[2], T[8], __fmaf_rn(b[1], T[6], b[0] * T[3])));
-                    if constexpr (!COMP) {
-                        hi[0] += 1.0f;  // exact: a chunk holds fewer than 2^24 paths
-                        hi[1] = __fmaf_rn(q0, q0, hi[1]);
-                        hi[2] = __fmaf_rn(q0, q1, hi[2]);
-                        hi[3] = __fmaf_rn(q0, q2, hi[3]);
-                        hi[4] = __fmaf_rn(q0, q3, hi[4]);
-                        hi[5] = __fmaf_rn(q1, q1, hi[5]);
-                        hi[6] = __fmaf_rn(q1, q2, hi[6]);
-                        hi[7] = __fmaf_rn(q1, q3, hi[7]);
-                        hi[8] = __fmaf_rn(q2, q2, hi[8]);
-                        hi[9] = __fmaf_rn(q2, q3, hi[9]);
-                        hi[10] = __fmaf_rn(q3, q3, hi[10]);
-                        hi[11] = __fmaf_rn(q0, v, hi[11]);
-                        hi[12] = __fmaf_rn(q1, v, hi[12]);
-                        hi[13] = __fmaf_rn(q2, v, hi[13]);
-                        hi[14] = __fmaf_rn(q3, v, hi[14]);
-                        continue;
+        } else {
+#pragma unroll
+            for (int j = 0; j < kPer; ++j) {
+                if (!live[j]) continue;
+                float v = init ? fmaxf(phi * (vv[j] - strike), 0.0f) : vv[j];
+                if (exercise) {
+                    const float ex = phi * (se[j] - strike);
+                    if (ex > 0.0f && ex > continuation_poly32(se[j], inv_kf, poly)) v = ex;
+                }
+                v *= disc;
+                if (last) {
+                    sum32_add(fin, v);
+                } else {
+                    cf_t[j * kLsmThreads] = v;
+                    if (phi * (sd[j] - strike) > 0.0f) {
+                        float b[4];
+                        basis32(sd[j], inv_kf, true, b);
+                        const float q0 = b[0] * T[0];
+                        const float q1 = __fmaf_rn(b[1], T[4], b[0] * T[1]);
+                        const float q2 = __fmaf_rn(b[2], T[7], __fmaf_rn(b[1], T[5], b[0] * T[2]));
+                        const float q3 = __fmaf_rn(b[3], T[9], __fmaf_rn(b[2], T[8], __fmaf_rn(b[1], T[6], b[0] * T[3])));
+                        df_add(hi[0], lo[0], 1.0f);
+                        df_add(hi[1], lo[1], q0 * q0);
+                        df_add(hi[2], lo[2], q0 * q1);
+                        df_add(hi[3], lo[3], q0 * q2);
+                        df_add(hi[4], lo[4], q0 * q3);
+                        df_add(hi[5], lo[5], q1 * q1);
+                        df_add(hi[6], lo[6], q1 * q2);
+                        df_add(hi[7], lo[7], q1 * q3);
+                        df_add(hi[8], lo[8], q2 * q2);
+                        df_add(hi[9], lo[9], q2 * q3);
+                        df_add(hi[10], lo[10], q3 * q3);
+                        df_add(hi[11], lo[11], q0 * v);
+                        df_add(hi[12], lo[12], q1 * v);
+                        df_add(hi[13], lo[13], q2 * v);
+                        df_add(hi[14], lo[14], q3 * v);
                     }
-                    df_add(hi[0], lo[0], 1.0f);
-                    df_add(hi[1], lo[1], q0 * q0);
-                    df_add(hi[2], lo[2], q0 * q1);
-                    df_add(hi[3], lo[3], q0 * q2);
-                    df_add(hi[4], lo[4], q0 * q3);
-                    df_add(hi[5], lo[5], q1 * q1);
-                    df_add(hi[6], lo[6], q1 * q2);
-                    df_add(hi[7], lo[7], q1 * q3);
-                    df_add(hi[8], lo[8], q2 * q2);
-                    df_add(hi[9], lo[9], q2 * q3);
-                    df_add(hi[10], lo[10], q3 * q3);
-                    df_add(hi[11], lo[11], q0 * v);
-                    df_add(hi[12], lo[12], q1 * v);
-                    df_add(hi[13], lo[13], q2 * v);
-                    df_add(hi[14], lo[14], q3 * v);
                 }
             }
         }
@@ -1041,7 +1081,7 @@ __global__ void __launch_bounds__(kChunkThreads<PREC>, PREC == 0 ? 1 : 4)
         for (int j = 0; j < kPer; ++j) {
             if (!live[j] || !(phi * (sv[j] - strike) > 0.0f)) continue;
             float b[4];
-            basis32(sv[j], inv_kf, b);
+            basis32(sv[j], inv_kf, true, b);
             const float q0 = b[0] * T[0];
             const float q1 = __fmaf_rn(b[1], T[4], b[0] * T[1]);
             const float q2 = __fmaf_rn(b[2], T[7], __fmaf_rn(b[1], T[5], b[0] * T[2]));
@@ -1082,18 +1122,14 @@ __global__ void __launch_bounds__(kChunkThreads<PREC>, PREC == 0 ? 1 : 4)
     }
 }
 
-__global__ void lsm_finish(const LsmDev* __restrict__ cs, int n_contracts,
-                           const Welford* __restrict__ final_part, double* __restrict__ out) {
-    const int ci = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (ci >= n_contracts) return;
-    const LsmDev c = cs[ci];
-    Welford w{0ull, 0.0, 0.0};
-    for (uint32_t ch = lane; ch < c.n_chunks; ch += 32) w = welford_merge(w, final_part[c.chunk_begin + ch]);
-    w = welford_warp_reduce(w);
-    if (lane != 0) return;
-    const double var = w.count < 2 ? 0.0 : w.m2 / static_cast<double>(w.count - 1);
-    const double se = w.count == 0 ? 0.0 : sqrt(var / static_cast<double>(w.count));
+// One CTA per contract.
+__global__ void __launch_bounds__(kMergeThreads)
+    lsm_finish(const LsmDev* __restrict__ cs, const Welford* __restrict__ final_part, double* __restrict__ out) {
+    const int ci = blockIdx.x;
+    const LsmDev& c = cs[ci];
+    const MergedResult w = merge_items(final_part + c.chunk_begin, c.n_chunks, 1);
+    if (threadIdx.x != 0) return;
+    const double se = w.standard_error;
     // inception decision (src/pricers/lsm.cpp:141-148)
     const bool ex0 = c.inception > w.mean;
     out[6 * ci + 0] = ex0 ? c.inception : w.mean;
@@ -1181,7 +1217,7 @@ cudaError_t launch_lsm_iteration(int precision, int k, const LsmDev* c, int n_co
 cudaError_t launch_lsm_finish(const LsmDev* c, int n_contracts, const Welford* final_part,
                               double* out, cudaStream_t stream) {
     cudaGetLastError();
-    lsm_finish<<<(n_contracts * 32 + 127) / 128, 128, 0, stream>>>(c, n_contracts, final_part, out);
+    if (n_contracts > 0) lsm_finish<<<n_contracts, kMergeThreads, 0, stream>>>(c, final_part, out);
     return cudaGetLastError();
 }
 

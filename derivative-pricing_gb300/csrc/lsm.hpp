@@ -139,8 +139,9 @@ cudaError_t launch_lsm_finish(const LsmDev* c, int n_contracts, const Welford* f
 // `reg` (rows per contract at LsmDev::reg_offset), in n_scenarios (1 or
 // kFrozenScenarios) scenarios, and writes per contract and output the path
 // average, its standard error and the path count (out: n x outputs x 3;
-// outputs = 1 for one scenario, kFrozenOutputs for five).
-cudaError_t launch_lsm_frozen(int precision, int n_scenarios, const LsmDev* c, const FrozenDev* f,
+// outputs = 1 for one scenario, kFrozenOutputs for five).  max_steps: the most
+// dates of any contract.
+cudaError_t launch_lsm_frozen(int precision, int n_scenarios, int max_steps, const LsmDev* c, const FrozenDev* f,
                               int n_contracts, const uint32_t* chunk_contract, uint32_t total_chunks,
                               const LsmReg* reg, Welford* partials, double* out, const FixedTables* tables,
                               cudaStream_t stream);

@@ -456,7 +456,7 @@ int frozen_run(Ctx& ctx, const LsmPlan& p, const std::vector<FrozenDev>& fz, int
     int pair = -1;
     rc = ctx.record_start(ctx.stream, &pair);
     if (rc) return rc;
-    e = launch_lsm_frozen(precision, n_scenarios, static_cast<const LsmDev*>(ctx.ext[kDev].ptr),
+    e = launch_lsm_frozen(precision, n_scenarios, p.max_steps, static_cast<const LsmDev*>(ctx.ext[kDev].ptr),
                           static_cast<const FrozenDev*>(ctx.ext[kFzDev].ptr), static_cast<int>(n),
                           static_cast<const uint32_t*>(ctx.ext[kChunkMap].ptr), p.total_chunks,
                           static_cast<const LsmReg*>(ctx.ext[kReg].ptr), static_cast<Welford*>(ctx.ext[kFzPart].ptr),

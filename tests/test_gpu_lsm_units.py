@@ -48,10 +48,15 @@ def test_fit_against_oracle_and_replay(engine, orc, args):
     assert g["price"][0] == res.price
 
 
-@pytest.mark.parametrize("steps", [255, 256, 257, 300])
-def test_fp32_forward_around_the_step_table(engine, steps):
-    """Stored FP32 paths past the 256-step table: the streaming replay, which draws
-    step by step, gives the fitted price bit for bit."""
-    args = (40.0, 40.0, .06, 0.0, .3, 1.0, 1, steps, 3000, 11)
+@pytest.mark.parametrize("kind", [0, 1])
+@pytest.mark.parametrize("steps", [2, 251, 252, 253, 255, 256, 257, 300])
+def test_fp32_forward_and_replay_around_the_tables(engine, steps, kind):
+    """Stored FP32 paths past the 256-step table, and the replay's two kernels (up to 252
+    dates each lane takes its own paths): the fitted price bit for bit."""
+    args = (40.0, 40.0, .06, .02, .3, 1.0, kind, steps, 3000, 11)
     res, co, has = engine.monte_carlo_lsm_american(*args, precision="fp32", policy=True)
     assert engine.reprice_against_frozen_policy(*args, co, has, bool(res.exercise_at_inception), "fp32") == res.price
+    g = engine.lsm_frozen_greeks(*args, co, has, bool(res.exercise_at_inception), 0.4, 0.003, precision="fp32")
+    assert g["price"][0] == res.price
+    up = (40.4, *args[1:])  # a bumped scenario is the single replay at the bumped spot
+    assert g["scenario"][0] == engine.reprice_against_frozen_policy(*up, co, has, False, "fp32")
