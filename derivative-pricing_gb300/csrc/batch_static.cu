@@ -89,7 +89,7 @@ int static_setup(int device, char* msg, size_t cap) {
     if (e != cudaSuccess) return report_cuda(msg, cap, e, "SM count");
     for (int precision = 0; precision < 2; ++precision) {
         int blocks = 0;
-        e = mcdg::path_kernel_occupancy(precision, 1, &blocks);
+        e = mcdg::path_kernel_occupancy(precision, mcdg::kDefaultVariant[precision], &blocks);
         if (e != cudaSuccess) return report_cuda(msg, cap, e, "occupancy");
         g_grid[device][precision] = sms * (blocks > 0 ? blocks : 1);
     }
@@ -166,7 +166,7 @@ extern "C" int mcd_price_batch_static(const mcd_contract* contracts, size_t n, i
         if (e != cudaSuccess) return report_cuda(error_message, error_capacity, e, "reset flags");
         const int count = static_cast<int>(end - first);
         if (g_stage_prefix[end] != g_stage_prefix[first]) {
-            e = mcdg::launch_path_kernel(precision, 1, g_grid[device][precision], d_contracts + first, count,
+            e = mcdg::launch_path_kernel(precision, mcdg::kDefaultVariant[precision], g_grid[device][precision], d_contracts + first, count,
                                          d_prefix + first, d_flags, d_partials, d_flags + 1, g_tables[device], s);
             if (e != cudaSuccess) return report_cuda(error_message, error_capacity, e, "path kernel");
         }

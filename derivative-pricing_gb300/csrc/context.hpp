@@ -32,7 +32,7 @@ struct BatchPlan {
 constexpr uint64_t kRangeItems = 1ull << 26;  // 1.6 GB of partials
 
 struct LaunchShape {
-    int variant = 1;      // __launch_bounds__ min-blocks 8
+    int variant = 1;
     int ctas_per_sm = 0;  // 0: occupancy limit
 };
 
@@ -83,7 +83,7 @@ struct Ctx {
     DevicePlanKey device_plan_key{nullptr, 0, 0, 0};
     bool device_plan_valid = false;
 
-    LaunchShape shape[2];
+    LaunchShape shape[2] = {{kDefaultVariant[0], 0}, {kDefaultVariant[1], 0}};
     std::vector<CachedGraph> graphs;
 
     // Extra streams and events for graphs captured as concurrent chains

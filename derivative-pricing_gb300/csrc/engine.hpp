@@ -20,7 +20,8 @@ struct Welford {
 constexpr int kSlabPaths = 4096;       // MCD_SLAB_PATHS
 constexpr int kSlabThreads = 128;      // one CTA = one slab lane group
 constexpr int kPathsPerThread = kSlabPaths / kSlabThreads;
-constexpr int kNumVariants = 5;        // __launch_bounds__ min-blocks 4, 8, 12, 16, 6
+constexpr int kNumVariants = 5;        // FP32: __launch_bounds__ min-blocks 4, 8, 12, 16, 7
+constexpr int kDefaultVariant[2] = {1, 4};  // per precision (FP64: 1024 threads; FP32: 7 CTAs per SM)
 
 // Internal product kinds: one loop body per kind (the switch is outside the
 // step loop and uniform over a CTA).

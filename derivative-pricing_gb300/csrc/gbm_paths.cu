@@ -24,14 +24,18 @@
 // on the draw alone come from a table per slab, those of the path alone are
 // taken once per path (PhiloxStep, PhiloxRow): 18 products -> 14.5.  The book
 // 313 -> 253 ms at 8 CTAs per SM (294 before at its best launch shape), of
-// which 7 ms from sums instead of Welford merges in the reductions.
+// which 7 ms from sums instead of Welford merges in the reductions.  Flushing
+// denormals (--ftz) takes the range tests out of the logarithm and the
+// exponentials (arguments here are normal numbers, the bits stay); the
+// compiler then wants 72 registers: at 5, 6, 7 and 8 CTAs per SM 260, 256, 253
+// and 266 ms on one GPU.
 //
 // Reference semantics restated per kind (src/pricers/monte_carlo.cpp):
 //   terminal products :135-149, path-dependent loop :154-177, Brownian-bridge
 //   barrier :184-230, control-variate Asian :275-302, antithetic pairing
 //   :73-79; payoffs include/mcd/payoffs/{european,digital,asian,barrier,
 //   lookback}.hpp.
-// nvcc-flags: --fmad=false
+// nvcc-flags: --fmad=false --ftz=true
 #include <cuda_runtime.h>
 
 #include "device_common.cuh"
@@ -69,6 +73,7 @@ struct Pair32 {
         const float mu = static_cast<float>(c.drift), sg = static_cast<float>(c.vs);
         const float lnh = static_cast<float>(c.log_h_rel);
         const float inv_denom = KIND == kBarrierBridge ? static_cast<float>(-2.0 / c.bb_denom) : 0.0f;
+#pragma unroll 1
         for (int d = 0; d < count; ++d) {
             const PhiloxStep st = table[d];
             float z[2];
@@ -385,7 +390,7 @@ cudaError_t launch_path_kernel(int precision, int variant, int grid, const DevCo
         case 1: return launch_one<8>(grid, contracts, n_contracts, item_prefix, ticket, partials, error_flag, stream);
         case 2: return launch_one<12>(grid, contracts, n_contracts, item_prefix, ticket, partials, error_flag, stream);
         case 3: return launch_one<16>(grid, contracts, n_contracts, item_prefix, ticket, partials, error_flag, stream);
-        default: return launch_one<6>(grid, contracts, n_contracts, item_prefix, ticket, partials, error_flag, stream);
+        default: return launch_one<7>(grid, contracts, n_contracts, item_prefix, ticket, partials, error_flag, stream);
     }
 }
 
@@ -399,7 +404,7 @@ cudaError_t path_kernel_occupancy(int precision, int variant, int* blocks) {
         case 1: return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, path_kernel<8>, kSlabThreads, 0);
         case 2: return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, path_kernel<12>, kSlabThreads, 0);
         case 3: return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, path_kernel<16>, kSlabThreads, 0);
-        default: return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, path_kernel<6>, kSlabThreads, 0);
+        default: return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, path_kernel<7>, kSlabThreads, 0);
     }
 }
 

@@ -34,7 +34,7 @@
 // the path taken out of the step, transposed warp sums instead of twelve
 // Welford trees, and 8 CTAs per SM as the default.
 //
-// nvcc-flags: --fmad=false
+// nvcc-flags: --fmad=false --ftz=true
 #include <cuda_runtime.h>
 
 #include "device_common.cuh"

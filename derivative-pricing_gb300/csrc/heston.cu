@@ -27,7 +27,7 @@
 // taken out of the step, 101-104 with one branch region for both paths'
 // exponential steps.
 //
-// nvcc-flags: --fmad=false
+// nvcc-flags: --fmad=false --ftz=true
 #include <cuda_runtime.h>
 
 #include "device_common.cuh"

@@ -42,7 +42,7 @@
 // below the BF16 rounding of the network's own hidden layer.  Every mbarrier
 // wait is bounded (umma.cuh).
 //
-// nvcc-flags: --fmad=false
+// nvcc-flags: --fmad=false --ftz=true
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 

@@ -21,7 +21,7 @@
 // aggregates at once (sum, log-sum, extrema, barrier test, terminal spot), so
 // no path array is kept: one value per tree depth.
 //
-// nvcc-flags: --fmad=false
+// nvcc-flags: --fmad=false --ftz=true
 #include <cuda_runtime.h>
 
 #include <type_traits>

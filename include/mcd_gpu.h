@@ -199,7 +199,7 @@ int mcd_price_batch_static(const mcd_contract* contracts, size_t n, int precisio
                            size_t error_capacity);
 
 /* Launch shape of the persistent path kernel.  variant 0..4 selects the
- * register budget (FP32: __launch_bounds__ min blocks 4/8/12/16/6; FP64:
+ * register budget (FP32: __launch_bounds__ min blocks 4/8/12/16/7; FP64:
  * 512/1024/1024/1024/768 threads in the SM's one CTA), ctas_per_sm the
  * grid (SM count x ctas_per_sm).  0 restores the autotuned/default choice.
  * Results do not depend on either. */
