@@ -292,18 +292,16 @@ __device__ __forceinline__ float normal_from_bits_f32(uint32_t bits) {
     return upper ? z : -z;
 }
 
-// NP draws at once, the bits of normal_from_bits_f32: every draw takes the
-// central polynomial, then one branch for all of them replaces the tail draws'
-// values (one branch region per NP draws instead of one each: 3.8e11 ->
-// 4.2e11 path-steps/s with the hoisted Philox products, two paths).
+// NP quantiles at once: q in (0, 1/2], negative where upper is false.  Every
+// draw takes the central polynomial, then one branch for all of them replaces
+// the tail draws' values (one branch region per NP draws instead of one each:
+// 3.8e11 -> 4.2e11 path-steps/s with the hoisted Philox products, two paths).
 template <int NP>
-__device__ __forceinline__ void normals_from_bits_f32(const uint32_t (&bits)[NP], float (&z)[NP]) {
-    float q[NP], w[NP], p[NP];
+__device__ __forceinline__ void normals_from_q(const float (&q)[NP], const bool (&upper)[NP], float (&z)[NP]) {
+    float w[NP], p[NP];
     bool tail = false;
 #pragma unroll
     for (int i = 0; i < NP; ++i) {
-        const uint32_t m = bits[i] ^ static_cast<uint32_t>(static_cast<int32_t>(bits[i]) >> 31);
-        q[i] = __fmaf_rn(__uint2float_rn(m), 2.3283064365386963e-10f, 1.1641532182693481e-10f);
         w[i] = upper_arg(q[i]);
         p[i] = upper_central(w[i]);
         tail = tail || !(w[i] < 5.0f);
@@ -316,8 +314,22 @@ __device__ __forceinline__ void normals_from_bits_f32(const uint32_t (&bits)[NP]
 #pragma unroll
     for (int i = 0; i < NP; ++i) {
         const float v = p[i] * __fmaf_rn(-2.0f, q[i], 1.0f);
-        z[i] = __uint_as_float(__float_as_uint(v) ^ (~bits[i] & 0x80000000u));
+        z[i] = upper[i] ? v : -v;
     }
+}
+
+// The bits of normal_from_bits_f32.
+template <int NP>
+__device__ __forceinline__ void normals_from_bits_f32(const uint32_t (&bits)[NP], float (&z)[NP]) {
+    float q[NP];
+    bool upper[NP];
+#pragma unroll
+    for (int i = 0; i < NP; ++i) {
+        upper[i] = static_cast<int32_t>(bits[i]) < 0;
+        const uint32_t m = bits[i] ^ static_cast<uint32_t>(static_cast<int32_t>(bits[i]) >> 31);
+        q[i] = __fmaf_rn(__uint2float_rn(m), 2.3283064365386963e-10f, 1.1641532182693481e-10f);
+    }
+    normals_from_q<NP>(q, upper, z);
 }
 
 // Standard normal of a Sobol coordinate u = x / 2^32 (x > 0), in FP32: the
@@ -327,6 +339,19 @@ __device__ __forceinline__ float normal_from_sobol_f32(uint32_t x) {
     const uint32_t m = upper ? (0u - x) : x;
     const float z = inv_normal_upper(__uint2float_rn(m) * 2.3283064365386963e-10f);
     return upper ? z : -z;
+}
+
+// The bits of normal_from_sobol_f32.
+template <int NP>
+__device__ __forceinline__ void normals_from_sobol_f32(const uint32_t (&x)[NP], float (&z)[NP]) {
+    float q[NP];
+    bool upper[NP];
+#pragma unroll
+    for (int i = 0; i < NP; ++i) {
+        upper[i] = x[i] > 0x80000000u;
+        q[i] = __uint2float_rn(upper[i] ? (0u - x[i]) : x[i]) * 2.3283064365386963e-10f;
+    }
+    normals_from_q<NP>(q, upper, z);
 }
 
 // Uniform (bits+0.5)/2^32 in FP32 (for comparisons against probabilities).

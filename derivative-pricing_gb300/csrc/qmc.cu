@@ -29,6 +29,7 @@
 #include "device_common.cuh"
 #include "engine.hpp"
 #include "qmc.hpp"
+#include "unit_sums.cuh"
 
 namespace mcdg {
 
@@ -66,6 +67,8 @@ struct SobolLane {
 };
 
 constexpr int kSxStride = kSobolDims + 1;  // +1 word: the last lane's row sits in another bank
+template <int PREC>
+constexpr int kSxPerWarp = (PREC == 0 ? 2 : 4) * kSxStride;  // FP32: two groups of 32 paths at a time
 
 // Bridge coefficients of one contract in program order, FP64 kernel.
 struct QmcTables64 {
@@ -79,7 +82,6 @@ struct QmcTables64 {
 struct QmcTables32 {
     float4 node[kSobolDims];  // {a, sd, drift, bits(meta)}
 };
-constexpr uint32_t kMetaRoot = 1u << 20;  // the terminal point (no ancestors)
 __device__ __forceinline__ uint32_t meta_dim(uint32_t m) { return m & 0xFFu; }
 __device__ __forceinline__ uint32_t meta_left(uint32_t m) { return (m >> 8) & 0xFu; }
 __device__ __forceinline__ uint32_t meta_right(uint32_t m) { return (m >> 12) & 0xFu; }
@@ -119,7 +121,7 @@ __device__ void fill_tables(const DevContract& c, const DevQmc& q, const BridgeN
         } else {
             const uint32_t meta = static_cast<uint32_t>(b.dim) | (static_cast<uint32_t>(b.slot_left) << 8) |
                                   (static_cast<uint32_t>(b.slot_right) << 12) |
-                                  (static_cast<uint32_t>(b.slot_out) << 16) | (root ? kMetaRoot : 0u);
+                                  (static_cast<uint32_t>(b.slot_out) << 16);
             S.node[e] = make_float4(static_cast<float>(a), static_cast<float>(sd), static_cast<float>(drift),
                                     __uint_as_float(meta));
         }
@@ -185,131 +187,215 @@ __device__ double sample_qmc64(const DevContract& c, const DevQmc& q, const QmcT
     }
 }
 
-// FP32: log-space spots x = ln(S/S0), FP32 payoff, FP64 accumulation.  The
-// bridge values live in shared memory, one column per thread (w[slot * 128]):
-// a node's slots are known only at run time, so a register array would be
-// spilled to local memory.
+// FP32: log-space spots x = ln(S/S0), FP32 payoff, FP64 accumulation.
+__device__ __forceinline__ double terminal_qmc32(const DevContract& c, uint32_t x) {  // European, digital
+    const float phi = c.type == 0 ? 1.0f : -1.0f;
+    const float s0 = static_cast<float>(c.spot), strike = static_cast<float>(c.strike);
+    const float z = normal_from_sobol_f32(x);
+    const float s = s0 * __expf(__fmaf_rn(static_cast<float>(c.vs), z, static_cast<float>(c.drift)));
+    float payoff;
+    if (c.kind == kEuropean) {
+        payoff = fmaxf(phi * (s - strike), 0.0f);
+    } else {
+        const bool itm = phi * (s - strike) > 0.0f;
+        payoff = itm ? (c.asset ? s : static_cast<float>(c.cash)) : 0.0f;
+    }
+    return c.discount * static_cast<double>(payoff);
+}
+
+// Two paths of a thread, 128 indices apart: they share the program's records,
+// their slots' addresses and the lane's Y word, and their chains interleave.
+// Bound by issue (89 % of the cycles at 7 CTAs per SM, 67 registers).  A
+// book of 4096 mixed contracts of 1e4 to 1e6 paths: one path at a time 282 ms,
+// two 277 (both waiting on bank conflicts of the directions, see add_x), with
+// the bit-major directions and the node fetched one ahead 173, the root taken
+// out of the loop 165.
+// The bridge values live in shared memory, one column per thread and path
+// (w[slot * 256], w[slot * 256 + 128]): a node's slots are known only at run
+// time, so a register array would be spilled to local memory.
 template <int KIND>
-__device__ double sample_qmc32(const DevContract& c, const DevQmc& q, const QmcTables32& S, const SobolLane& sob,
-                               float* __restrict__ w) {
+__device__ __forceinline__ void pair_qmc32(const DevContract& c, const DevQmc& q, const QmcTables32& S,
+                                           const uint32_t* x0, const uint32_t* x1, const uint32_t* __restrict__ y,
+                                           float* __restrict__ w, double (&out)[2]) {
     const float phi = c.type == 0 ? 1.0f : -1.0f;
     const float s0 = static_cast<float>(c.spot);
     const float strike = static_cast<float>(c.strike);
-    if constexpr (KIND == kEuropean || KIND == kDigital) {
-        const float z = normal_from_sobol_f32(sob(0u));
-        const float s = s0 * __expf(__fmaf_rn(static_cast<float>(c.vs), z, static_cast<float>(c.drift)));
-        float payoff;
-        if constexpr (KIND == kEuropean) {
-            payoff = fmaxf(phi * (s - strike), 0.0f);
+    const int n = c.n_steps;
+    const float vol = static_cast<float>(q.vol);
+    const float lnh = static_cast<float>(c.log_h_rel);
+    w[0] = w[kSlabThreads] = 0.0f;
+    float acc[2] = {0.0f, 0.0f}, xlast[2], xmax[2] = {0.0f, 0.0f}, xmin[2] = {0.0f, 0.0f};
+    bool breached[2] = {false, false};
+    auto observe = [&](int p, float x) {
+        if constexpr (KIND == kAsianArith) {
+            acc[p] += __expf(x);
+        } else if constexpr (KIND == kAsianGeo) {
+            acc[p] += x;
+        } else if constexpr (KIND == kBarrier) {
+            breached[p] = breached[p] || (c.up ? x >= lnh : x <= lnh);
         } else {
-            const bool itm = phi * (s - strike) > 0.0f;
-            payoff = itm ? (c.asset ? s : static_cast<float>(c.cash)) : 0.0f;
+            xmax[p] = fmaxf(xmax[p], x);
+            xmin[p] = fminf(xmin[p], x);
         }
-        return c.discount * static_cast<double>(payoff);
-    } else {
-        const int n = c.n_steps;
-        const float vol = static_cast<float>(q.vol);
-        const float lnh = static_cast<float>(c.log_h_rel);
-        w[0] = 0.0f;
-        float acc = 0.0f, acc2 = 0.0f, xlast = 0.0f, xmax = 0.0f, xmin = 0.0f;
-        bool breached = false;
-        for (int e = 0; e < n; ++e) {
-            const float4 nd = S.node[e];
-            const uint32_t meta = __float_as_uint(nd.w);
-            const float z = normal_from_sobol_f32(sob(meta_dim(meta)));
-            float val;
-            const bool root = (meta & kMetaRoot) != 0u;
-            if (root) {
-                val = nd.y * z;
-            } else {
-                const float wl = w[meta_left(meta) * kSlabThreads], wr = w[meta_right(meta) * kSlabThreads];
-                val = __fmaf_rn(nd.y, z, __fmaf_rn(nd.x, wr - wl, wl));
-            }
-            w[meta_out(meta) * kSlabThreads] = val;
-            const float x = __fmaf_rn(vol, val, nd.z);
-            if (root) xlast = x;  // the terminal point is the bridge's root
-            if constexpr (KIND == kAsianArith) {
-                acc += __expf(x);
-            } else if constexpr (KIND == kAsianGeo) {
-                acc2 += x;
-            } else if constexpr (KIND == kBarrier) {
-                breached = breached || (c.up ? x >= lnh : x <= lnh);
-            } else {
-                xmax = fmaxf(xmax, x);
-                xmin = fminf(xmin, x);
-            }
+    };
+    auto offset = [&](uint32_t slot) { return w + slot * (2 * kSlabThreads); };
+    // the next node's record and draws are fetched a node ahead
+    float4 ahead;
+    uint32_t yw, xa, xb;
+    auto fetch = [&](int e) {
+        ahead = S.node[e];
+        const uint32_t dim = meta_dim(__float_as_uint(ahead.w));
+        yw = __ldg(y + dim * 32u);
+        xa = x0[dim];
+        xb = x1[dim];
+    };
+    fetch(0);
+    {  // the program starts at its root, the terminal point, which has no ancestors
+        const float4 nd = ahead;
+        const uint32_t bits[2] = {xa ^ yw, xb ^ yw};
+        fetch(n > 1 ? 1 : 0);
+        float z[2];
+        normals_from_sobol_f32<2>(bits, z);
+        float* at = offset(meta_out(__float_as_uint(nd.w)));
+#pragma unroll
+        for (int p = 0; p < 2; ++p) {
+            const float val = nd.y * z[p];
+            at[p * kSlabThreads] = val;
+            xlast[p] = __fmaf_rn(vol, val, nd.z);
+            observe(p, xlast[p]);
         }
-        const float inv_n = 1.0f / static_cast<float>(n);
-        const float last = s0 * __expf(xlast);
+    }
+    for (int e = 1; e < n; ++e) {
+        const float4 nd = ahead;
+        const uint32_t meta = __float_as_uint(nd.w);
+        const uint32_t bits[2] = {xa ^ yw, xb ^ yw};
+        fetch(min(e + 1, n - 1));
+        float z[2];
+        normals_from_sobol_f32<2>(bits, z);
+        const float *left = offset(meta_left(meta)), *right = offset(meta_right(meta));
+        float* at = offset(meta_out(meta));
+#pragma unroll
+        for (int p = 0; p < 2; ++p) {
+            const float wl = left[p * kSlabThreads], wr = right[p * kSlabThreads];
+            const float val = __fmaf_rn(nd.y, z[p], __fmaf_rn(nd.x, wr - wl, wl));
+            at[p * kSlabThreads] = val;
+            observe(p, __fmaf_rn(vol, val, nd.z));
+        }
+    }
+    const float inv_n = 1.0f / static_cast<float>(n);
+#pragma unroll
+    for (int p = 0; p < 2; ++p) {
+        const float last = s0 * __expf(xlast[p]);
+        float v;
         if constexpr (KIND == kAsianArith || KIND == kAsianGeo) {
-            const float avg = KIND == kAsianArith ? s0 * (acc * inv_n) : s0 * __expf(acc2 * inv_n);
-            const float ref = c.floating ? (last - avg) : (avg - strike);
-            return c.discount * static_cast<double>(fmaxf(phi * ref, 0.0f));
+            const float avg = KIND == kAsianArith ? s0 * (acc[p] * inv_n) : s0 * __expf(acc[p] * inv_n);
+            v = fmaxf(phi * (c.floating ? (last - avg) : (avg - strike)), 0.0f);
         } else if constexpr (KIND == kBarrier) {
             const float vanilla = fmaxf(phi * (last - strike), 0.0f);
-            const bool pays = c.out ? !breached : breached;
-            return c.discount * static_cast<double>(pays ? vanilla : static_cast<float>(c.rebate));
+            v = (c.out ? !breached[p] : breached[p]) ? vanilla : static_cast<float>(c.rebate);
         } else if constexpr (KIND == kLookbackFixed) {
-            const float v = c.type == 0 ? fmaxf(s0 * __expf(xmax) - strike, 0.0f)
-                                        : fmaxf(strike - s0 * __expf(xmin), 0.0f);
-            return c.discount * static_cast<double>(v);
+            v = c.type == 0 ? fmaxf(s0 * __expf(xmax[p]) - strike, 0.0f) : fmaxf(strike - s0 * __expf(xmin[p]), 0.0f);
         } else {
-            const float v = c.type == 0 ? (last - s0 * __expf(xmin)) : (s0 * __expf(xmax) - last);
-            return c.discount * static_cast<double>(v);
+            v = c.type == 0 ? (last - s0 * __expf(xmin[p])) : (s0 * __expf(xmax[p]) - last);
         }
+        out[p] = c.discount * static_cast<double>(v);
     }
 }
 
+// Adds (over GF(2)) the directions of the set bits of `gray` to a row of X, the
+// dimensions spread over the lanes; start: from zero.  From one group of paths
+// to the next only one to three bits of the Gray code change, so the rows are
+// updated rather than computed anew.  The directions are read bit-major: from
+// the dimension-major table a warp's 32 loads were 128 bytes apart, and their
+// wavefronts held the L1 for half of the kernel's cycles.
+__device__ __forceinline__ void add_x(uint32_t* row, const uint32_t* __restrict__ by_bit, uint32_t ndims, uint32_t gray,
+                                      bool start) {
+    for (uint32_t d = threadIdx.x & 31; d < ndims; d += 32) {
+        uint32_t x = start ? 0u : row[d];
+        for (uint32_t g = gray; g != 0u; g &= g - 1u) x ^= __ldg(by_bit + (__ffs(g) - 1) * kSobolDims + d);
+        row[d] = x;
+    }
+}
+
+__device__ __forceinline__ uint32_t gray_code(uint64_t i) { return static_cast<uint32_t>(i ^ (i >> 1)); }
+
+// X of the warp's 32 paths from b0 on: row 0 for index base B = b0 (lanes 0..30),
+// row 1 for B + 32 (lane 31).  The rows hold those of the paths from `before` on,
+// or nothing yet.
+__device__ __forceinline__ void fill_x(uint32_t* xw, const uint32_t* __restrict__ by_bit, uint32_t ndims, uint64_t b0,
+                                       uint64_t before, bool start) {
+    const uint32_t g0 = gray_code(b0), g1 = gray_code(b0 + 32);
+    add_x(xw, by_bit, ndims, start ? g0 : g0 ^ gray_code(before), start);
+    add_x(xw + kSxStride, by_bit, ndims, start ? g1 : g1 ^ gray_code(before + 32), start);
+}
+
+// A warp's share of a slab; valid in lane 0 (FP32: shifted sums, FP64: a
+// Welford triple per lane, merged in a fixed tree).
 template <int PREC, int KIND>
 __device__ Welford slab_qmc(const DevContract& c, const DevQmc& q, const QmcTables<PREC>& S,
-                            const uint32_t* __restrict__ dirs, const uint32_t* __restrict__ ytab, uint32_t* sx,
+                            const uint32_t* __restrict__ by_bit, const uint32_t* __restrict__ ytab, uint32_t* sx,
                             float* bridge_w, uint64_t base) {
+    constexpr bool kTerminal = KIND == kEuropean || KIND == kDigital;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint32_t ndims = (KIND == kEuropean || KIND == kDigital) ? 1u : static_cast<uint32_t>(c.n_steps);
-    uint32_t* xw = sx + warp * 2 * kSxStride;
-    const SobolLane sob{xw + (lane == 31 ? kSxStride : 0), ytab + lane};
-    Welford w{0ull, 0.0, 0.0};
-    unsigned count = 0;
-    double s1 = 0.0, s2 = 0.0;
-    for (int j = 0; j < kPathsPerThread; ++j) {
-        const uint64_t b0 = base + static_cast<uint64_t>(j * kSlabThreads) + 32u * warp;  // this warp's first path
-        if (b0 >= c.path_count) break;  // uniform per warp
-        // X for index bases B = b0 (lanes 0..30) and B + 32 (lane 31), dimensions spread over the lanes
-        const uint32_t g0 = static_cast<uint32_t>(b0 ^ (b0 >> 1));
-        const uint32_t g1 = static_cast<uint32_t>((b0 + 32) ^ ((b0 + 32) >> 1));
-        __syncwarp();
-        for (uint32_t d = lane; d < ndims; d += 32) {
-            xw[d] = sobol_x(dirs, d, g0);
-            xw[kSxStride + d] = sobol_x(dirs, d, g1);
+    const uint32_t ndims = kTerminal ? 1u : static_cast<uint32_t>(c.n_steps);
+    uint32_t* xw = sx + warp * kSxPerWarp<PREC>;
+    const uint32_t* my_x = xw + (lane == 31 ? kSxStride : 0);
+    if constexpr (PREC == 0) {
+        const SobolLane sob{my_x, ytab + lane};
+        Welford w{0ull, 0.0, 0.0};
+        for (int j = 0; j < kPathsPerThread; ++j) {
+            const uint64_t b0 = base + static_cast<uint64_t>(j * kSlabThreads) + 32u * warp;  // this warp's first path
+            if (b0 >= c.path_count) break;  // uniform per warp
+            __syncwarp();
+            fill_x(xw, by_bit, ndims, b0, b0 - kSlabThreads, j == 0);
+            __syncwarp();
+            if (b0 + lane < c.path_count) welford_add(w, sample_qmc64<KIND>(c, q, S, sob));
         }
-        __syncwarp();
-        const uint64_t path = b0 + lane;
-        if (path >= c.path_count) continue;
-        if constexpr (PREC == 0) {
-            welford_add(w, sample_qmc64<KIND>(c, q, S, sob));
-        } else {
-            const double v = sample_qmc32<KIND>(c, q, S, sob, bridge_w + threadIdx.x);
-            ++count;
-            s1 += v;
-            s2 = fma(v, v, s2);
+        return welford_warp_reduce(w);
+    } else {
+        UnitSums acc;
+        unsigned count = 0;
+        for (int j = 0; j < kPathsPerThread; j += 2) {
+            const uint64_t b0 = base + static_cast<uint64_t>(j * kSlabThreads) + 32u * warp;
+            if (b0 >= c.path_count) break;  // uniform per warp
+            __syncwarp();
+            fill_x(xw, by_bit, ndims, b0, b0 - 2 * kSlabThreads, j == 0);
+            fill_x(xw + 2 * kSxStride, by_bit, ndims, b0 + kSlabThreads, b0 - kSlabThreads, j == 0);
+            __syncwarp();
+            const uint64_t path = b0 + lane;
+            double v[2];
+            if constexpr (kTerminal) {
+                const uint32_t y = __ldg(ytab + lane);
+                v[0] = terminal_qmc32(c, my_x[0] ^ y);
+                v[1] = terminal_qmc32(c, my_x[2 * kSxStride] ^ y);
+            } else {
+                pair_qmc32<KIND>(c, q, S, my_x, my_x + 2 * kSxStride, ytab + lane, bridge_w + threadIdx.x, v);
+            }
+            if (j == 0) acc.first(v[0]);
+#pragma unroll
+            for (int p = 0; p < 2; ++p) {
+                if (path + p * kSlabThreads < c.path_count) {
+                    ++count;
+                    acc.add(v[p]);
+                }
+            }
         }
+        return acc.reduce(__reduce_add_sync(0xffffffffu, count));
     }
-    if constexpr (PREC == 1) w = welford_from_sums(count, s1, s2);
-    return w;
 }
 
 template <int PREC>
 __device__ Welford run_qmc_slab(const DevContract& c, const DevQmc& q, const QmcTables<PREC>& S,
-                                const uint32_t* __restrict__ dirs, const uint32_t* __restrict__ ytab, uint32_t* sx,
+                                const uint32_t* __restrict__ by_bit, const uint32_t* __restrict__ ytab, uint32_t* sx,
                                 float* bridge_w, uint64_t base) {
     switch (c.kind) {
-        case kEuropean: return slab_qmc<PREC, kEuropean>(c, q, S, dirs, ytab, sx, bridge_w, base);
-        case kDigital: return slab_qmc<PREC, kDigital>(c, q, S, dirs, ytab, sx, bridge_w, base);
-        case kAsianArith: return slab_qmc<PREC, kAsianArith>(c, q, S, dirs, ytab, sx, bridge_w, base);
-        case kAsianGeo: return slab_qmc<PREC, kAsianGeo>(c, q, S, dirs, ytab, sx, bridge_w, base);
-        case kBarrier: return slab_qmc<PREC, kBarrier>(c, q, S, dirs, ytab, sx, bridge_w, base);
-        case kLookbackFixed: return slab_qmc<PREC, kLookbackFixed>(c, q, S, dirs, ytab, sx, bridge_w, base);
-        default: return slab_qmc<PREC, kLookbackFloating>(c, q, S, dirs, ytab, sx, bridge_w, base);
+        case kEuropean: return slab_qmc<PREC, kEuropean>(c, q, S, by_bit, ytab, sx, bridge_w, base);
+        case kDigital: return slab_qmc<PREC, kDigital>(c, q, S, by_bit, ytab, sx, bridge_w, base);
+        case kAsianArith: return slab_qmc<PREC, kAsianArith>(c, q, S, by_bit, ytab, sx, bridge_w, base);
+        case kAsianGeo: return slab_qmc<PREC, kAsianGeo>(c, q, S, by_bit, ytab, sx, bridge_w, base);
+        case kBarrier: return slab_qmc<PREC, kBarrier>(c, q, S, by_bit, ytab, sx, bridge_w, base);
+        case kLookbackFixed: return slab_qmc<PREC, kLookbackFixed>(c, q, S, by_bit, ytab, sx, bridge_w, base);
+        default: return slab_qmc<PREC, kLookbackFloating>(c, q, S, by_bit, ytab, sx, bridge_w, base);
     }
 }
 
@@ -319,14 +405,15 @@ __global__ void __launch_bounds__(kSlabThreads)
                const uint32_t* __restrict__ item_prefix, uint32_t total_items,
                const BridgeNode* __restrict__ programs, const uint32_t* __restrict__ dirs,
                uint32_t* __restrict__ ticket, Welford* __restrict__ partials, uint32_t* __restrict__ error_flag) {
-    const uint32_t* ytab = dirs + kSobolDims * kSobolBits;  // Y table follows the directions
-    __shared__ uint32_t s_sx[(kSlabThreads / 32) * 2 * kSxStride];
+    const uint32_t* ytab = dirs + kSobolDims * kSobolBits;  // Y table, then the directions bit-major
+    const uint32_t* by_bit = ytab + kSobolDims * 32;
+    __shared__ uint32_t s_sx[(kSlabThreads / 32) * kSxPerWarp<PREC>];
     __shared__ uint32_t s_item;
     __shared__ Welford s_warp[kSlabThreads / 32];
     __shared__ DevContract s_c;
     __shared__ DevQmc s_q;
     __shared__ QmcTables<PREC> S;
-    __shared__ float s_bridge[PREC == 0 ? 1 : kBridgeSlots * kSlabThreads];  // FP32 bridge values, per thread
+    __shared__ float s_bridge[PREC == 0 ? 1 : 2 * kBridgeSlots * kSlabThreads];  // FP32 bridge values, per thread and path
     __shared__ int s_loaded;  // sorted index of the contract whose tables are in S
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
@@ -365,8 +452,7 @@ __global__ void __launch_bounds__(kSlabThreads)
             if (threadIdx.x == 0) atomicOr(error_flag, 1u);
             continue;
         }
-        Welford w = run_qmc_slab<PREC>(s_c, s_q, S, dirs, ytab, s_sx, s_bridge, static_cast<uint64_t>(slab) * kSlabPaths);
-        w = welford_warp_reduce(w);
+        const Welford w = run_qmc_slab<PREC>(s_c, s_q, S, by_bit, ytab, s_sx, s_bridge, static_cast<uint64_t>(slab) * kSlabPaths);
         if (lane == 0) s_warp[warp] = w;
         __syncthreads();
         if (threadIdx.x == 0)

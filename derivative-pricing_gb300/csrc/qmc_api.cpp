@@ -48,8 +48,8 @@ bool primitive(unsigned s, uint32_t interior) {
     return false;
 }
 
-// Direction numbers (kSobolDims x 32, dims-major) followed by the warp
-// decomposition's Y table (kSobolDims x 32 lanes).
+// Direction numbers (kSobolDims x 32, dims-major), the warp decomposition's Y
+// table (kSobolDims x 32 lanes), and the directions bit-major.
 std::vector<uint32_t> sobol_directions() {
     std::vector<std::pair<unsigned, uint32_t>> polys;
     for (int d = 0; d < 7; ++d) polys.emplace_back(kRefDegree[d], kRefInterior[d]);
@@ -82,7 +82,7 @@ std::vector<uint32_t> sobol_directions() {
     // Y table of the warp decomposition (qmc.cu, SobolLane): for lane l the
     // low index part is (l + 1) mod 32; Y[d][l] = the coordinate bits of its
     // Gray code in dimension d.
-    dirs.resize(static_cast<size_t>(kSobolDims) * kSobolBits * 2);
+    dirs.resize(static_cast<size_t>(kSobolDims) * kSobolBits * 3);
     uint32_t* y = dirs.data() + static_cast<size_t>(kSobolDims) * kSobolBits;
     for (int d = 0; d < kSobolDims; ++d)
         for (uint32_t l = 0; l < 32; ++l) {
@@ -92,6 +92,12 @@ std::vector<uint32_t> sobol_directions() {
                 if ((g >> b) & 1u) x ^= dirs[static_cast<size_t>(d) * kSobolBits + b];
             y[static_cast<size_t>(d) * 32 + l] = x;
         }
+    // The directions once more, bit-major: a warp that takes one bit of 32
+    // consecutive dimensions reads 32 consecutive words.
+    uint32_t* by_bit = y + static_cast<size_t>(kSobolDims) * 32;
+    for (int d = 0; d < kSobolDims; ++d)
+        for (int b = 0; b < kSobolBits; ++b)
+            by_bit[static_cast<size_t>(b) * kSobolDims + d] = dirs[static_cast<size_t>(d) * kSobolBits + b];
     return dirs;
 }
 
