@@ -55,11 +55,16 @@ struct alignas(16) QuantHi {
 constexpr int kExpBits = 10;  // 2^x by two tables of 2^10 entries and a quadratic
 constexpr int kExpEntries = 1 << kExpBits;
 
+constexpr int kLogBits = 10;  // logarithm: intervals of [1, 2) (fixed_root.hpp)
+constexpr int kLogEntries = 1 << kLogBits;
+
 struct FixedTables {
     QuantLo lo[kQuantEntries];
     QuantHi hi[kQuantEntries];
     uint64_t exp_a[kExpEntries];  // 2^(i / 2^10), units of 2^-63
     uint64_t exp_b[kExpEntries];  // 2^(i / 2^20) - 1, units of 2^-64
+    alignas(16) uint64_t log_l[kLogEntries];  // -ln(c 2^-31), units of 2^-59
+    uint32_t log_c[kLogEntries];              // 1 / (1 + i / 2^10) rounded up, units of 2^-31
 };
 
 MCD_HD uint32_t mul_hi32(uint32_t a, uint32_t b) {

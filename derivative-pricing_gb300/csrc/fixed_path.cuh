@@ -11,33 +11,41 @@
 
 namespace mcdg {
 
-// Tables of the CTA: the quantile's first kQuantSharedOctaves octaves and both
-// exponential tables (176 KB).
-struct FixedShared {
+// Tables of the CTA: the quantile's first kQuantSharedOctaves octaves (160 KB)
+// and both exponential tables (16 KB).
+struct QuantTables {
     QuantLo lo[kQuantShared];
     QuantHi hi[kQuantShared];
+};
+struct FixedShared : QuantTables {
     uint64_t exp_a[kExpEntries];
     uint64_t exp_b[kExpEntries];
 };
 
-// Copies the tables into shared memory (asynchronous 16-byte copies by the
-// whole CTA; ends with a barrier).
-__device__ __forceinline__ void load_fixed_tables(FixedShared& s, const FixedTables* __restrict__ g) {
-    auto copy = [](void* to, const void* from, int bytes) {
-        for (int o = threadIdx.x * 16; o < bytes; o += blockDim.x * 16)
-            cp_async16(static_cast<char*>(to) + o, static_cast<const char*>(from) + o);
-    };
-    copy(s.lo, g->lo, sizeof s.lo);
-    copy(s.hi, g->hi, sizeof s.hi);
-    copy(s.exp_a, g->exp_a, sizeof s.exp_a);
-    copy(s.exp_b, g->exp_b, sizeof s.exp_b);
+// Starts a table's copy into shared memory (asynchronous 16-byte copies by the
+// whole CTA).
+__device__ __forceinline__ void copy_table(void* to, const void* from, int bytes) {
+    for (int o = threadIdx.x * 16; o < bytes; o += blockDim.x * 16)
+        cp_async16(static_cast<char*>(to) + o, static_cast<const char*>(from) + o);
+}
+__device__ __forceinline__ void copy_quantile(QuantTables& s, const FixedTables* __restrict__ g) {
+    copy_table(s.lo, g->lo, sizeof s.lo);
+    copy_table(s.hi, g->hi, sizeof s.hi);
+}
+__device__ __forceinline__ void wait_tables() {
     cp_async_commit();
     cp_async_wait_all();
     __syncthreads();
 }
+__device__ __forceinline__ void load_fixed_tables(FixedShared& s, const FixedTables* __restrict__ g) {
+    copy_quantile(s, g);
+    copy_table(s.exp_a, g->exp_a, sizeof s.exp_a);
+    copy_table(s.exp_b, g->exp_b, sizeof s.exp_b);
+    wait_tables();
+}
 
 // -Phi^-1(w / 2^33) in units of 2^-61, 1 <= w < 2^32.
-__device__ __forceinline__ uint64_t quantile_units(uint32_t w, const FixedShared& s,
+__device__ __forceinline__ uint64_t quantile_units(uint32_t w, const QuantTables& s,
                                                    const FixedTables* __restrict__ g) {
     const QuantArg a = quant_arg(w);
     const uint32_t i = min(a.entry, static_cast<uint32_t>(kQuantShared - 1));
@@ -59,7 +67,7 @@ struct FixedNormal {
     uint64_t mag;
     int32_t neg;
 };
-__device__ __forceinline__ FixedNormal normal_fixed(uint32_t bits, const FixedShared& s,
+__device__ __forceinline__ FixedNormal normal_fixed(uint32_t bits, const QuantTables& s,
                                                     const FixedTables* __restrict__ g) {
     const int32_t upper = static_cast<int32_t>(bits) >> 31;
     const uint32_t m = bits ^ static_cast<uint32_t>(upper);

@@ -109,17 +109,32 @@ void fill_quantile(FixedTables& t) {
 }
 
 // 2^(i / 2^10) and 2^(i / 2^20) - 1 by the exponential series of i ln 2 / 2^k.
+DD expm1(DD x) {
+    DD r{0.0, 0.0};
+    for (int k = 30; k >= 1; --k) r = div_small(mul(x, add(r, DD{1.0, 0.0})), k);
+    return r;
+}
+
 void fill_exp(FixedTables& t) {
     const DD ln2{0.693147180559945286226764, 2.319046813846299558417771e-17};
-    auto expm1 = [](DD x) {
-        DD r{0.0, 0.0};
-        for (int k = 30; k >= 1; --k) r = div_small(mul(x, add(r, DD{1.0, 0.0})), k);
-        return r;
-    };
     for (int i = 0; i < kExpEntries; ++i) {
         const DD x = mul(ln2, DD{static_cast<double>(i), 0.0});
         t.exp_a[i] = to_units(add(DD{1.0, 0.0}, expm1(scale(x, 1.0 / (1 << kExpBits)))), 63);
         t.exp_b[i] = to_units(expm1(scale(x, 1.0 / (1 << (2 * kExpBits)))), 64);
+    }
+}
+
+// Reciprocals of the intervals' left ends, rounded up, and their logarithms:
+// one Newton step of exp(x) = c from the library's logarithm (its error squared
+// is below 10^-31).
+void fill_log(FixedTables& t) {
+    for (uint32_t i = 0; i < kLogEntries; ++i) {
+        const uint64_t left = kLogEntries + i;
+        t.log_c[i] = static_cast<uint32_t>(((1ull << (31 + kLogBits)) + left - 1) / left);
+        const double c = std::ldexp(static_cast<double>(t.log_c[i]), -31), x = -std::log(c);  // x >= 0
+        // c exp(x) - 1 = (c - 1) + c expm1(x)
+        const DD d = add(DD{c - 1.0, 0.0}, mul(DD{c, 0.0}, expm1(DD{x, 0.0})));
+        t.log_l[i] = to_units(add(DD{x, 0.0}, DD{-d.h, -d.l}), 59);
     }
 }
 
@@ -132,6 +147,7 @@ const FixedTables& fixed_tables() {
         auto t = std::make_unique<FixedTables>();
         fill_quantile(*t);
         fill_exp(*t);
+        fill_log(*t);
         tables = std::move(t);
     });
     return *tables;

@@ -21,7 +21,9 @@ struct HestonSet {
     double s2_lin;     // xi^2 e / kappa (1-e)   (FP32 path: s2 = v s2_lin + s2_const)
     // FP64 path (heston64.cu): psi = r (qe_b - qe_a r) with r = 1 / E[v'], and
     double qe_a, qe_b;  // theta xi^2 (1-e)^2 / (2 kappa), xi^2 (1-e) / kappa
-    double drift_k0;    // drift + K0
+    double reversion;   // theta (1-e): E[v'] = v e + reversion
+    // ln(S_T / S_0) = drift_sum + k12 sum(v) + k2 (v_n - v_0) + root_k3 sum(z sqrt(v + v'))
+    double drift_sum, k12, root_k3;
     uint64_t seed;
     uint64_t path_count;
     uint32_t n_slabs;

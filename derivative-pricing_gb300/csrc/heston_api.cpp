@@ -57,7 +57,10 @@ int make_set(Ctx& ctx, const mcd_heston_params& p, int steps, uint64_t paths, ui
     h.n_steps = steps;
     h.qe_a = h.s2_const;
     h.qe_b = p.xi * p.xi * (1.0 - h.e) / p.kappa;
-    h.drift_k0 = h.drift + h.k0;
+    h.reversion = p.theta * (1.0 - h.e);
+    h.drift_sum = (h.drift + h.k0) * static_cast<double>(steps);
+    h.k12 = dt * (p.kappa * p.rho / p.xi - 0.5);
+    h.root_k3 = std::sqrt(h.k3);
     return MCD_OK;
 }
 
