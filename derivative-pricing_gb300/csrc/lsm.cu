@@ -50,15 +50,18 @@
 // 131,072 paths and 50 dates: 92 us before; the FP64 pipe (about 150 -> 41
 // operations per path) and the tail (folds by transposed warp sums, the 4x4
 // algebra one element per lane: an FP64 operation holds a scheduler for 64
-// cycles with one lane or 32) -> 37 us.  Forward simulation of that put 2.9 ms
+// cycles with one lane or 32) -> 37 us; every date in one launch with the cash
+// flows and basis values kept on the SM (lsm_chain64) and in-the-money paths
+// packed before the products -> 17 us.  Forward simulation of that put 2.9 ms
 // -> 55 us (one warp per 32 paths instead of 8 paths per thread in 128 CTAs).
-// The call 7.35 -> 1.92 ms.  FP32 pass of two contracts 62 -> 28 us, of ten
-// 100 -> 70 us, the same bits.
+// The call 7.35 -> 1.92 -> 1.0 ms.  FP32 pass of two contracts 62 -> 28 us, of
+// ten 100 -> 70 us.
 //
 // nvcc-flags: --fmad=false --ftz=true
 #include <cuda_runtime.h>
 
 #include "device_common.cuh"
+#include "fp64_fast.cuh"
 #include "lsm.hpp"
 #include "lsm_math.cuh"
 #include "merge.cuh"
@@ -541,14 +544,32 @@ __device__ void solve_lagged(const double* s, const double L[4][4], double kappa
     }
 }
 
-// solve_lagged by one warp, the same operations on the same operands (so the
-// same bits) with one matrix element per lane: lane 4a + b of each half-warp
-// holds element (a, b).  An FP64 operation holds the scheduler for 64 cycles
-// with one lane active or with 32, and the serial form is a chain of about 300
-// of them; this is about 115.  Only the form without a diagonal shift: a
-// matrix that is not positive definite goes to the serial routine.
+// 1 / sqrt(d), d > 0: an FP32 seed and one cubic iteration (fp64_fast.cuh), five
+// FP64 operations in a row where the library's routine takes 427 cycles.
+__device__ __forceinline__ double pivot_rsqrt(double d) {
+    if (!seed_range(d)) return rsqrt(d);
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(seed_of(d)));
+    const double y = seed_wide(r);
+    const double e = fma(-d * y, y, 1.0);
+    return fma(y * e, fma(0.375, e, 0.5), y);
+}
+
+// solve_lagged by one warp with one matrix element per lane: lane 4a + b of
+// each half-warp holds element (a, b).  An FP64 operation holds the scheduler
+// for 64 cycles with one lane active or with 32, and the serial form is a chain
+// of about 300 of them.  PREC 1: the serial form's operations on the same
+// operands, about 105; on FP32 paths a continuation value one bit off moves
+// exercise decisions (those of paths within FP32 rounding of the boundary) and
+// with them the price by 1e-5.  PREC 0: 65 (fused products, the pivots' own
+// rsqrt, gamma = T R^{-T} h), 12,400 -> 6,000 cycles from the sums to the
+// coefficients; decisions there would have to tie to 1e-16.  Only the form
+// without a diagonal shift: a matrix that is not positive definite goes to the
+// serial routine.
+template <int PREC>
 __device__ void solve_lagged_warp(const double* s /* shared, 15 */, const double* lag /* packed T, or null */,
                                   double kappa_max, LsmReg& r, uint32_t* need_second_pass) {
+    auto madd = [](double x, double y, double z) { return PREC == 0 ? fma(x, y, z) : z + x * y; };
     constexpr unsigned kAll = 0xffffffffu;
     const int lane = threadIdx.x & 31, a = (lane >> 2) & 3, b = lane & 3;
     const bool writer = lane < 16 && a <= b;  // the upper triangle, first half-warp
@@ -574,10 +595,12 @@ __device__ void solve_lagged_warp(const double* s /* shared, 15 */, const double
     for (int p = 0; p < 4; ++p) {
         const double d = __shfl_sync(kAll, x, 5 * p);
         ok = ok && d > 0.0;
-        rinv[p] = rsqrt(d);
-        if (a == p) R = b == p ? d * rinv[p] : x * rinv[p];
-        const double ra = __shfl_sync(kAll, R, 4 * p + a), rb = __shfl_sync(kAll, R, 4 * p + b);
-        if (a > p && b >= a) x -= ra * rb;
+        rinv[p] = PREC == 0 ? pivot_rsqrt(d) : rsqrt(d);
+        if (a == p) R = x * rinv[p];
+        if (p < 3) {
+            const double ra = __shfl_sync(kAll, R, 4 * p + a), rb = __shfl_sync(kAll, R, 4 * p + b);
+            if (a > p && b >= a) x = madd(-ra, rb, x);
+        }
     }
     if (!ok) {
         if (lane == 0) {
@@ -589,7 +612,7 @@ __device__ void solve_lagged_warp(const double* s /* shared, 15 */, const double
         return;
     }
     if (b < a) R = 0.0;
-    // row a of R^{-1}
+    // row a of R^{-1} (zero left of the diagonal)
     double t[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) t[q] = q == a ? rinv[q] : 0.0;
@@ -597,27 +620,23 @@ __device__ void solve_lagged_warp(const double* s /* shared, 15 */, const double
     for (int q = 1; q < 4; ++q) {
         double y = 0.0;
 #pragma unroll
-        for (int p = 0; p < q; ++p) {
-            const double rpq = __shfl_sync(kAll, R, 4 * p + q);
-            if (p >= a) y += t[p] * rpq;
-        }
+        for (int p = 0; p < q; ++p) y = madd(t[p], __shfl_sync(kAll, R, 4 * p + q), y);
         if (q > a) t[q] = -y * rinv[q];
     }
     const double ri = b == 0 ? t[0] : b == 1 ? t[1] : b == 2 ? t[2] : t[3];
     // ||R||^2 in the first half-warp, ||R^{-1}||^2 in the second
-    const double sq = lane < 16 ? R * R : ri * ri;
-    double norm = 0.0;
+    const double el = lane < 16 ? R : ri;
+    double norm = el * el;
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = i; j < 4; ++j) norm += __shfl_sync(kAll, sq, (lane & 16) + 4 * i + j);
-    const double kappa = __shfl_sync(kAll, norm, 0) * __shfl_sync(kAll, norm, 16);
-    // T = L R^{-1}
-    double tab = 0.0;
+    for (int off = 8; off >= 1; off >>= 1) norm += __shfl_xor_sync(kAll, norm, off);
+    const double kappa = norm * __shfl_xor_sync(kAll, norm, 16);
+    // T = L R^{-1}, and R^{-T} h by column b
+    double tab = 0.0, w = 0.0;
 #pragma unroll
     for (int p = 0; p < 4; ++p) {
         const double rpb = __shfl_sync(kAll, ri, 4 * p + b);
-        if (p >= a && p <= b) tab += l[p] * rpb;
+        tab = madd(l[p], rpb, tab);
+        w = madd(rpb, s[11 + p], w);
     }
     if (writer) {
         r.T[tri(a, b)] = tab;
@@ -631,31 +650,24 @@ __device__ void solve_lagged_warp(const double* s /* shared, 15 */, const double
         }
         return;
     }
-    double w = 0.0, beta = 0.0, gamma = 0.0;  // R^{-T} h by column b; R^{-1} w and L beta by row a
+    double gamma = 0.0;  // by row a
+    if constexpr (PREC == 0) {
+        gamma = tab * w;  // T R^{-T} h
+        gamma += __shfl_xor_sync(kAll, gamma, 1);
+        gamma += __shfl_xor_sync(kAll, gamma, 2);
+    } else {
+        double beta = 0.0;  // R^{-1} w, then L beta
 #pragma unroll
-    for (int p = 0; p < 4; ++p) {
-        const double rpb = __shfl_sync(kAll, ri, 4 * p + b);
-        if (p <= b) w += rpb * s[11 + p];
-    }
+        for (int q = 0; q < 4; ++q) beta = madd(t[q], __shfl_sync(kAll, w, q), beta);
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        const double wq = __shfl_sync(kAll, w, q);
-        if (q >= a) beta += t[q] * wq;
+        for (int q = 0; q < 4; ++q) gamma = madd(l[q], __shfl_sync(kAll, beta, 4 * q), gamma);
     }
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        const double bq = __shfl_sync(kAll, beta, 4 * q);
-        if (q >= a) gamma += l[q] * bq;
-    }
-    // laguerre_poly, coefficient a in row a
+    // laguerre_poly, coefficient a in row a (the products of +-1, -2 and 1/2 are exact)
     const double g[4] = {__shfl_sync(kAll, gamma, 0), __shfl_sync(kAll, gamma, 4), __shfl_sync(kAll, gamma, 8),
                          __shfl_sync(kAll, gamma, 12)};
     const double m1 = a == 0 ? 1.0 : a == 1 ? -1.0 : 0.0, m2 = a == 0 ? 1.0 : a == 1 ? -2.0 : 0.5;
     const double m3 = a == 0 ? 1.0 : a == 1 ? -3.0 : 1.5;
-    double poly = a == 0 ? g[0] : 0.0;
-    poly += m1 * g[1];
-    poly += m2 * g[2];
-    poly += m3 * g[3];
+    double poly = fma(m2, g[2], fma(m1, g[1], a == 0 ? g[0] : 0.0)) + m3 * g[3];
     const double q0 = -g[3] * (1.0 / 6.0);  // -g3 / 6, correctly rounded
     const double sixth = fma(fma(-q0, 6.0, -g[3]), 1.0 / 6.0, q0);
     if (a == 3) poly = sixth;
@@ -709,6 +721,10 @@ __device__ __forceinline__ bool last_arrival(uint32_t* counter, uint32_t expecte
     return last;
 }
 
+// FP64: group sums of a contract up to this many are added in order, one sum per
+// lane (15 FP64 additions at most, against 16 and 32 shuffles of the warp's tree).
+constexpr uint32_t kSerialFolds = 16;
+
 // Publishes this CTA's chunk partial (in res; thread q < 15 writes entry q) and
 // climbs the two-level tree of the contract's sums: the last chunk of a group
 // of LsmDev::fold_chunks chunks folds the group's partials in chunk order into
@@ -718,6 +734,7 @@ __device__ __forceinline__ bool last_arrival(uint32_t* counter, uint32_t expecte
 // chunk.  Returns true in the CTA holding the totals, then in res.
 // counters: the group counter of group g at group_counters[2 g], the
 // contract's at *contract_counter.
+template <int PREC>
 __device__ bool publish_and_fold(uint32_t chunk, const LsmDev& c, LsmPartial* __restrict__ part,
                                  LsmPartial* __restrict__ gpart, uint32_t* group_counters,
                                  uint32_t* contract_counter, double (*smem)[15], double* res, int* s_flag) {
@@ -732,7 +749,16 @@ __device__ bool publish_and_fold(uint32_t chunk, const LsmDev& c, LsmPartial* __
     if (threadIdx.x < 15) gpart[c.fold_begin + g].v[threadIdx.x] = res[threadIdx.x];
     __syncthreads();
     if (!last_arrival(contract_counter, c.n_folds, s_flag)) return false;
-    fold_partials(gpart, c.fold_begin, c.n_folds, smem, res);
+    if (PREC == 0 && c.n_folds <= kSerialFolds) {
+        if (threadIdx.x < 15) {
+            double x = __ldcg(&gpart[c.fold_begin].v[threadIdx.x]);
+            for (uint32_t i = 1; i < c.n_folds; ++i) x += __ldcg(&gpart[c.fold_begin + i].v[threadIdx.x]);
+            res[threadIdx.x] = x;
+        }
+        __syncthreads();
+    } else {
+        fold_partials(gpart, c.fold_begin, c.n_folds, smem, res);
+    }
     return true;
 }
 
@@ -743,10 +769,8 @@ __device__ bool publish_and_fold(uint32_t chunk, const LsmDev& c, LsmPartial* __
 // ---------------------------------------------------------------------------
 // One in-the-money path's share of the regression sums in the basis b T
 // (b'_l = sum_{j <= l} b_j T[j][l]), FP64; entry 0, the count, is the caller's.
-__device__ __forceinline__ void add_sums64(double s, double inv_strike, const double (&T)[10], double v,
-                                           const GlobalTables& tables, double (&acc)[15]) {
-    double b[4];
-    basis64(s, inv_strike, tables, b);
+__device__ __forceinline__ void add_products64(const double (&b)[4], const double (&T)[10], double v,
+                                               double (&acc)[15]) {
     const double q0 = b[0] * T[0];
     const double q1 = fma(b[1], T[4], b[0] * T[1]);
     const double q2 = fma(b[2], T[7], fma(b[1], T[5], b[0] * T[2]));
@@ -767,6 +791,46 @@ __device__ __forceinline__ void add_sums64(double s, double inv_strike, const do
     acc[14] = fma(q3, v, acc[14]);
 }
 
+// FP64: a warp's in-the-money paths, packed.  The products of a path take 24
+// FP64 operations, each of which holds a scheduler for 64 cycles however many
+// lanes need it, so the warp's 128 paths are packed before them: near the money
+// two or three rounds of 32 instead of four.
+constexpr int kWarpPaths = kLsmChunk / (kLsmThreads64 / 32);  // 128
+constexpr int kPer64 = kLsmChunk / kLsmThreads64;             // paths per thread
+struct MoneyRank {
+    uint32_t at[kPer64];  // a path's position among the packed, or kWarpPaths
+    uint32_t count;
+};
+__device__ __forceinline__ MoneyRank rank_money(const double (&s)[kPer64], double strike, int type) {
+    MoneyRank r;
+    r.count = 0;
+    const uint32_t below = (1u << (threadIdx.x & 31)) - 1u;
+#pragma unroll
+    for (int j = 0; j < kPer64; ++j) {
+        const bool in = in_the_money64(s[j], strike, type);
+        const uint32_t mask = __ballot_sync(0xffffffffu, in);
+        r.at[j] = in ? r.count + __popc(mask & below) : kWarpPaths;
+        r.count += __popc(mask);
+    }
+    return r;
+}
+struct PackedPaths {
+    double s[kWarpPaths], v[kWarpPaths];
+};
+// The sums of a warp's packed paths (entry 0, their number, in lane 0).
+__device__ __forceinline__ void packed_sums64(const PackedPaths& p, uint32_t count, double inv_strike,
+                                              const double (&T)[10], const GlobalTables& tables, double (&acc)[15]) {
+    const uint32_t lane = threadIdx.x & 31;
+#pragma unroll
+    for (int q = 0; q < 15; ++q) acc[q] = 0.0;
+    if (lane == 0) acc[0] = static_cast<double>(count);
+    for (uint32_t at = lane; at < count; at += 32) {
+        double b[4];
+        basis64(p.s[at], inv_strike, tables, b);
+        add_products64(b, T, p.v[at], acc);
+    }
+}
+
 // COMP (FP32 path): the sums are compensated FP32 per thread and chunk (the
 // first iteration, whose basis is the raw Laguerre one); otherwise plain FP32
 // per thread and chunk -- the lagged basis is close to orthonormal, where
@@ -785,6 +849,7 @@ __global__ void __launch_bounds__(kChunkThreads<PREC>, PREC == 0 ? 1 : 8)
     __shared__ double sres[15];
     __shared__ Welford swf[kChunkThreads<PREC> / 32];
     __shared__ Sum64 s64[kLsmThreads / 32];
+    __shared__ PackedPaths s_packed[PREC == 0 ? kLsmThreads64 / 32 : 1];
     __shared__ int s_last;
     const uint32_t chunk = chunk_first + blockIdx.x;
     if (chunk >= chunk_end) return;
@@ -811,28 +876,25 @@ __global__ void __launch_bounds__(kChunkThreads<PREC>, PREC == 0 ? 1 : 8)
         double T[10];
 #pragma unroll
         for (int q = 0; q < 10; ++q) T[q] = init ? ((q == 0 || q == 4 || q == 7 || q == 9) ? 1.0 : 0.0) : re->T[q];
-        double acc[15];
-#pragma unroll
-        for (int q = 0; q < 15; ++q) acc[q] = 0.0;
         const double* S = static_cast<const double*>(store) + c.s_offset;
         const double* col_e = S + static_cast<uint64_t>(init ? n - 1 : e - 1) * c.path_count;
         const double* col_d = S + static_cast<uint64_t>(gram ? e - 2 : 0) * c.path_count;
         double* cash = cf + c.cf_offset;
         // all loads of this thread's paths first (independent, in flight together)
-        constexpr int kPer = kLsmChunk / kLsmThreads64;
         const uint64_t i0 = static_cast<uint64_t>(local) * kLsmChunk + threadIdx.x;
-        double vv[kPer], se[kPer], sd[kPer];
+        double vv[kPer64], se[kPer64], sd[kPer64];
 #pragma unroll
-        for (int j = 0; j < kPer; ++j) {
+        for (int j = 0; j < kPer64; ++j) {
             const uint64_t i = i0 + j * kLsmThreads64;
             const bool live = i < c.path_count;
             vv[j] = live && !init ? cash[i] : 0.0;
             se[j] = live && (init || exercise) ? col_e[i] : c.strike;
             sd[j] = live && gram ? col_d[i] : c.strike;
         }
-        uint32_t in_money = 0;
+        const MoneyRank rank = rank_money(sd, c.strike, c.type);
+        PackedPaths& packed = s_packed[threadIdx.x >> 5];
 #pragma unroll
-        for (int j = 0; j < kPer; ++j) {
+        for (int j = 0; j < kPer64; ++j) {
             const uint64_t i = i0 + j * kLsmThreads64;
             if (i >= c.path_count) continue;
             double v = vv[j];
@@ -845,14 +907,16 @@ __global__ void __launch_bounds__(kChunkThreads<PREC>, PREC == 0 ? 1 : 8)
                 welford_add(w, v);
             } else {
                 cash[i] = v;
-                if (in_the_money64(sd[j], c.strike, c.type)) {
-                    ++in_money;
-                    add_sums64(sd[j], c.inv_strike, T, v, tables, acc);
+                if (rank.at[j] < kWarpPaths) {
+                    packed.s[rank.at[j]] = sd[j];
+                    packed.v[rank.at[j]] = v;
                 }
             }
         }
         if (gram) {
-            acc[0] = static_cast<double>(in_money);
+            __syncwarp();
+            double acc[15];
+            packed_sums64(packed, rank.count, c.inv_strike, T, tables, acc);
             block_sum15(acc, kLsmThreads64 / 32, smem, sres);
         }
     } else {
@@ -1008,9 +1072,9 @@ __global__ void __launch_bounds__(kChunkThreads<PREC>, PREC == 0 ? 1 : 8)
         }
         return;
     }
-    if (!publish_and_fold(chunk, c, part, gpart, group_counters, &counters[2 * ci], smem, sres, &s_last)) return;
+    if (!publish_and_fold<PREC>(chunk, c, part, gpart, group_counters, &counters[2 * ci], smem, sres, &s_last)) return;
     if (threadIdx.x < 32)
-        solve_lagged_warp(sres, init ? nullptr : re->T, kappa_max, reg[c.reg_offset + e - 1], need_second_pass + k);
+        solve_lagged_warp<PREC>(sres, init ? nullptr : re->T, kappa_max, reg[c.reg_offset + e - 1], need_second_pass + k);
 }
 
 // Second pass for the dates solve_lagged marked (has = 2): the sums in the
@@ -1027,6 +1091,7 @@ __global__ void __launch_bounds__(kChunkThreads<PREC>, PREC == 0 ? 1 : 4)
     __shared__ double smem[kChunkThreads<PREC> / 32][15];
     __shared__ float2 scratch[15][kLsmThreads];  // FP32 path: the sums' per-thread pairs
     __shared__ double sres[15];
+    __shared__ PackedPaths s_packed[PREC == 0 ? kLsmThreads64 / 32 : 1];
     __shared__ int s_last;
     if (__ldcg(need_second_pass + k) == 0) return;  // no date of this iteration needs it
     for (uint32_t chunk = chunk_first + blockIdx.x; chunk < chunk_end; chunk += gridDim.x) {
@@ -1042,20 +1107,26 @@ __global__ void __launch_bounds__(kChunkThreads<PREC>, PREC == 0 ? 1 : 4)
         double T[10];
 #pragma unroll
         for (int q = 0; q < 10; ++q) T[q] = r.T[q];
-        double acc[15];
-#pragma unroll
-        for (int q = 0; q < 15; ++q) acc[q] = 0.0;
         const double* S = static_cast<const double*>(store) + c.s_offset + static_cast<uint64_t>(date - 1) * c.path_count;
-        uint32_t in_money = 0;
-        for (int j = 0; j < kLsmChunk / kLsmThreads64; ++j) {
-            const uint64_t i = static_cast<uint64_t>(local) * kLsmChunk + j * kLsmThreads64 + threadIdx.x;
-            if (i >= c.path_count) break;
-            const double s = S[i];
-            if (!in_the_money64(s, c.strike, c.type)) continue;
-            ++in_money;
-            add_sums64(s, c.inv_strike, T, cf[c.cf_offset + i], tables, acc);
+        const uint64_t i0 = static_cast<uint64_t>(local) * kLsmChunk + threadIdx.x;
+        double s[kPer64], v[kPer64];
+#pragma unroll
+        for (int j = 0; j < kPer64; ++j) {
+            const uint64_t i = i0 + j * kLsmThreads64;
+            s[j] = i < c.path_count ? S[i] : c.strike;
+            v[j] = i < c.path_count ? cf[c.cf_offset + i] : 0.0;
         }
-        acc[0] = static_cast<double>(in_money);
+        const MoneyRank rank = rank_money(s, c.strike, c.type);
+        PackedPaths& packed = s_packed[threadIdx.x >> 5];
+#pragma unroll
+        for (int j = 0; j < kPer64; ++j)
+            if (rank.at[j] < kWarpPaths) {
+                packed.s[rank.at[j]] = s[j];
+                packed.v[rank.at[j]] = v[j];
+            }
+        __syncwarp();
+        double acc[15];
+        packed_sums64(packed, rank.count, c.inv_strike, T, tables, acc);
         block_sum15(acc, kLsmThreads64 / 32, smem, sres);
     } else {
         float T[10];
@@ -1105,7 +1176,7 @@ __global__ void __launch_bounds__(kChunkThreads<PREC>, PREC == 0 ? 1 : 4)
         }
         block_sum_df<15>(hi, lo, scratch, sres);
     }
-    if (publish_and_fold(chunk, c, part, gpart, group_counters + 1, &counters[2 * ci + 1], smem, sres, &s_last)) {
+    if (publish_and_fold<PREC>(chunk, c, part, gpart, group_counters + 1, &counters[2 * ci + 1], smem, sres, &s_last)) {
         if (threadIdx.x == 0) {
             double T[4][4], gamma[4];
             unpack_upper(r.T, T);
@@ -1119,6 +1190,256 @@ __global__ void __launch_bounds__(kChunkThreads<PREC>, PREC == 0 ? 1 : 4)
         }
     }
     __syncthreads();  // shared memory is reused by the next chunk
+    }
+}
+
+// ---------------------------------------------------------------------------
+// FP64 batches whose chunks all fit on the GPU at once: every date in one
+// cooperative launch, one CTA per chunk.
+// ---------------------------------------------------------------------------
+// The lockstep form spends a date of a single contract mostly on latencies: two
+// launches, the contract's and the date's records, two columns and the cash
+// flows read again.  Here a CTA keeps its chunk's cash flows and the basis
+// values of its in-the-money paths in shared memory.  The contract's last CTA
+// folds and solves a date and publishes its number; meanwhile the others pack
+// the next date's column and evaluate its basis.  Every operation on a path and
+// every sum is the lockstep form's (the basis is evaluated once for both uses),
+// so prices and policies have its bits.  A CTA waits for its own contract's
+// CTAs only, all of them resident; a wait that runs out (kChainPolls) is
+// recorded and ends the CTA.
+//
+// Bound: a date is a serial chain of products (about 8,000 cycles, the FP64
+// pipe), the CTA's and the contract's folds (9,000), the solve (6,000), two
+// trips through L2 and the exercise tests (5,000).  A put of 131,072 paths and
+// 50 dates: 37 -> 17 us a date, the call 1.92 -> 1.0 ms.  Two CTAs fit an SM,
+// so batches of up to 304 chunks come here; larger ones go date by date, where
+// the chunks of one date fill the GPU and the launches' share is small.
+constexpr int kChainSlots = 5;  // s and the four basis values of a packed path
+struct ChainWarp {
+    double f[2][kChainSlots][kWarpPaths];  // packed paths of this date and of the next
+    uint8_t path[2][kWarpPaths];           // their place in the warp's 128
+    double cash[kWarpPaths];
+};
+struct ChainShared {
+    ChainWarp warp[kLsmThreads64 / 32];
+    double T[10], poly[4];
+    int has;
+};
+constexpr uint32_t kChainPolls = 1u << 22;  // of at least 0.1 us each
+
+__device__ __forceinline__ uint32_t load_acquire(const uint32_t* p) {
+    uint32_t v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void store_release(uint32_t* p, uint32_t v) {
+    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+
+// Packs a column's in-the-money paths and evaluates their basis; returns their number.
+__device__ __forceinline__ uint32_t pack_date(ChainWarp& w, int side, const double* __restrict__ col, uint64_t i0,
+                                              const LsmDev& c, const GlobalTables& tables) {
+    const uint32_t lane = threadIdx.x & 31;
+    double s[kPer64];
+#pragma unroll
+    for (int j = 0; j < kPer64; ++j) {
+        const uint64_t i = i0 + j * kLsmThreads64;
+        s[j] = i < c.path_count ? __ldg(col + i) : c.strike;
+    }
+    const MoneyRank rank = rank_money(s, c.strike, c.type);
+    __syncwarp();
+#pragma unroll
+    for (int j = 0; j < kPer64; ++j)
+        if (rank.at[j] < kWarpPaths) {
+            w.f[side][0][rank.at[j]] = s[j];
+            w.path[side][rank.at[j]] = static_cast<uint8_t>(j * 32 + lane);
+        }
+    __syncwarp();
+    for (uint32_t at = lane; at < rank.count; at += 32) {
+        double b[4];
+        basis64(w.f[side][0][at], c.inv_strike, tables, b);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) w.f[side][1 + q][at] = b[q];
+    }
+    return rank.count;
+}
+
+// A chunk's sums over its packed paths, published; in the contract's last CTA
+// the totals are in sres.  The two-level tree of publish_and_fold, a group of
+// chunks per warp.
+__device__ bool chain_sums(const ChainWarp& w, int side, uint32_t count, const double* T_shared, uint32_t chunk,
+                           const LsmDev& c, LsmPartial* __restrict__ part, uint32_t* counter, double (*smem)[15],
+                           double (*group)[15], double* sres, int* s_flag) {
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    double T[10], acc[15];
+#pragma unroll
+    for (int q = 0; q < 10; ++q) T[q] = T_shared[q];
+#pragma unroll
+    for (int q = 0; q < 15; ++q) acc[q] = 0.0;
+    if (lane == 0) acc[0] = static_cast<double>(count);
+    for (uint32_t at = lane; at < count; at += 32) {
+        double b[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) b[q] = w.f[side][1 + q][at];
+        add_products64(b, T, w.cash[w.path[side][at]], acc);
+    }
+    block_sum15(acc, kLsmThreads64 / 32, smem, sres);
+    if (threadIdx.x < 15) part[chunk].v[threadIdx.x] = sres[threadIdx.x];
+    __syncthreads();
+    if (!last_arrival(counter, c.n_chunks, s_flag)) return false;
+    for (uint32_t g = warp; g < c.n_folds; g += kLsmThreads64 / 32) {
+        const uint32_t at = g * c.fold_chunks + lane;
+        double v[16] = {};
+        if (at < c.n_chunks) {
+            const double2* p = reinterpret_cast<const double2*>(part[c.chunk_begin + at].v);
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                const double2 x = __ldcg(p + q);
+                v[2 * q] = x.x;
+                v[2 * q + 1] = x.y;
+            }
+        }
+        double u[15];
+#pragma unroll
+        for (int q = 0; q < 15; ++q) u[q] = v[q];
+        const double x = warp_sums15(u);
+        if ((lane & 1) == 0 && lane < 30) group[g][lane >> 1] = x;
+    }
+    __syncthreads();
+    if (threadIdx.x < 15) {
+        double x = group[0][threadIdx.x];
+        for (uint32_t i = 1; i < c.n_folds; ++i) x += group[i][threadIdx.x];
+        sres[threadIdx.x] = x;
+    }
+    __syncwarp();
+    return true;
+}
+
+__global__ void __launch_bounds__(kLsmThreads64, 2)
+    lsm_chain64(const LsmDev* __restrict__ cs, const uint32_t* __restrict__ chunk_contract,
+                const double* __restrict__ store, LsmReg* __restrict__ reg, LsmPartial* __restrict__ part,
+                Welford* __restrict__ final_part, uint32_t* __restrict__ counters /* arrivals, epoch */,
+                uint32_t* __restrict__ need, double kappa_max, double* __restrict__ error,
+                const FixedTables* __restrict__ fixed) {
+    extern __shared__ __align__(16) unsigned char chain_smem[];
+    ChainShared& sh = *reinterpret_cast<ChainShared*>(chain_smem);
+    __shared__ double smem[kLsmThreads64 / 32][15];
+    __shared__ double group[kSerialFolds][15];
+    __shared__ double sres[15];
+    __shared__ Welford swf[kLsmThreads64 / 32];
+    __shared__ int s_flag, s_waited;
+    const uint32_t chunk = blockIdx.x, ci = chunk_contract[chunk];
+    const LsmDev c = cs[ci];
+    const GlobalTables tables{fixed};
+    const uint32_t lane = threadIdx.x & 31;
+    ChainWarp& w = sh.warp[threadIdx.x >> 5];
+    uint32_t* arrivals = &counters[2 * ci];
+    uint32_t* epoch = &counters[2 * ci + 1];
+    uint32_t seen = 0;
+    const uint64_t i0 = static_cast<uint64_t>(chunk - c.chunk_begin) * kLsmChunk + threadIdx.x;
+    const double* S = store + c.s_offset;
+    auto column = [&](int date) { return S + static_cast<uint64_t>(date - 1) * c.path_count; };
+    auto publish = [&] {  // warp 0 of the contract's last CTA
+        __syncwarp();
+        if (lane == 0) {
+            __threadfence();
+            store_release(epoch, seen + 1);
+        }
+    };
+    // Waits for the next epoch and takes the date's record; false: gave up.
+    auto await = [&](int date) {
+        ++seen;
+        if (threadIdx.x == 0) {
+            uint32_t polls = 0;
+            while (load_acquire(epoch) < seen && ++polls < kChainPolls) {}
+            s_waited = polls < kChainPolls;
+        }
+        __syncthreads();
+        const bool ok = s_waited != 0;
+        const LsmReg& r = reg[c.reg_offset + date];
+        if (threadIdx.x < 10) sh.T[threadIdx.x] = __ldcg(&r.T[threadIdx.x]);
+        else if (threadIdx.x < 14) sh.poly[threadIdx.x - 10] = __ldcg(&r.poly[threadIdx.x - 10]);
+        else if (threadIdx.x == 14) sh.has = __ldcg(&r.has);
+        __syncthreads();
+        if (!ok && threadIdx.x == 0) *error = 1.0;
+        return ok;
+    };
+    // the terminal date
+    const int n = c.n_steps;
+#pragma unroll
+    for (int j = 0; j < kPer64; ++j) {
+        const uint64_t i = i0 + j * kLsmThreads64;
+        const double s = i < c.path_count ? column(n)[i] : c.strike;
+        const double v = in_the_money64(s, c.strike, c.type) ? put_sign(s - c.strike, c.type) : 0.0;
+        w.cash[j * 32 + lane] = v * c.disc;
+    }
+    if (threadIdx.x < 10) {
+        const int q = threadIdx.x;
+        sh.T[q] = q == 0 || q == 4 || q == 7 || q == 9 ? 1.0 : 0.0;
+    }
+    __syncthreads();
+    int side = 0;
+    uint32_t count = n > 1 ? pack_date(w, side, column(n - 1), i0, c, tables) : 0u;
+    __syncwarp();
+    for (int e = n; e > 1; --e) {
+        // the sums of date e - 1 in the basis of date e, whose T is in sh
+        if (chain_sums(w, side, count, sh.T, chunk, c, part, arrivals, smem, group, sres, &s_flag) && threadIdx.x < 32) {
+            solve_lagged_warp<0>(sres, e == n ? nullptr : sh.T, kappa_max, reg[c.reg_offset + e - 1], need);
+            publish();
+        }
+        // meanwhile the date before it
+        uint32_t next = 0;
+        if (e > 2) next = pack_date(w, side ^ 1, column(e - 2), i0, c, tables);
+        if (!await(e - 1)) return;
+        if (sh.has == 2) {  // second pass in the basis of the date's own T (lsm_refine)
+            if (chain_sums(w, side, count, sh.T, chunk, c, part, arrivals, smem, group, sres, &s_flag) &&
+                threadIdx.x < 32) {
+                if (lane == 0) {
+                    LsmReg& r = reg[c.reg_offset + e - 1];
+                    double T[4][4], gamma[4];
+                    unpack_upper(sh.T, T);
+                    solve_preconditioned(sres, T, gamma);
+                    for (int a = 0; a < 4; ++a) {
+                        r.gamma[a] = gamma[a];
+                        r.gamma_f[a] = static_cast<float>(gamma[a]);
+                    }
+                    laguerre_poly(r.gamma, r.poly, r.poly_f);
+                    r.has = 1;
+                }
+                publish();
+            }
+            if (!await(e - 1)) return;
+        }
+        // exercise at date e - 1, discount
+        if (sh.has == 1) {
+#pragma unroll
+            for (int j = 0; j < kPer64; ++j) {
+                const uint32_t at = j * 32 + lane;
+                if (at >= count) break;
+                const double s = w.f[side][0][at], x = s * c.inv_strike;
+                const double ex = put_sign(s - c.strike, c.type);
+                const double go = w.f[side][1][at] * fma(fma(fma(sh.poly[3], x, sh.poly[2]), x, sh.poly[1]), x, sh.poly[0]);
+                if (ex > go) w.cash[w.path[side][at]] = ex;
+            }
+        }
+        __syncwarp();
+#pragma unroll
+        for (int j = 0; j < kPer64; ++j) w.cash[j * 32 + lane] *= c.disc;
+        __syncwarp();
+        side ^= 1;
+        count = next;
+    }
+    Welford f{0ull, 0.0, 0.0};
+#pragma unroll
+    for (int j = 0; j < kPer64; ++j)
+        if (i0 + j * kLsmThreads64 < c.path_count) welford_add(f, w.cash[j * 32 + lane]);
+    f = welford_warp_reduce(f);
+    if (lane == 0) swf[threadIdx.x >> 5] = f;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        Welford m = swf[0];
+        for (int q = 1; q < kLsmThreads64 / 32; ++q) m = welford_merge(m, swf[q]);
+        final_part[chunk] = m;
     }
 }
 
@@ -1212,6 +1533,28 @@ cudaError_t launch_lsm_iteration(int precision, int k, const LsmDev* c, int n_co
                                                                tables);
     }
     return cudaGetLastError();
+}
+
+cudaError_t lsm_chain64_capacity(int sm_count, uint32_t* chunks) {
+    constexpr int bytes = static_cast<int>(sizeof(ChainShared));
+    cudaError_t e = cudaFuncSetAttribute(lsm_chain64, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    int blocks = 0;
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, lsm_chain64, kLsmThreads64, bytes);
+    *chunks = e == cudaSuccess ? static_cast<uint32_t>(blocks) * static_cast<uint32_t>(sm_count) : 0u;
+    return e;
+}
+
+cudaError_t launch_lsm_chain64(const LsmDev* c, int n_contracts, const uint32_t* chunk_contract, uint32_t chunk_count,
+                               uint32_t total_folds, const double* s_store, LsmReg* reg, LsmPartial* part,
+                               Welford* final_part, uint32_t* counters, double* error, const FixedTables* tables,
+                               cudaStream_t stream) {
+    cudaGetLastError();
+    if (chunk_count == 0) return cudaSuccess;
+    uint32_t* need = counters + 2 * static_cast<size_t>(n_contracts) + 2 * static_cast<size_t>(total_folds);
+    double kappa_max = 1e2;  // as launch_lsm_iteration
+    void* args[] = {&c, &chunk_contract, &s_store, &reg, &part, &final_part, &counters, &need, &kappa_max, &error, &tables};
+    return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(lsm_chain64), dim3(chunk_count),
+                                       dim3(kLsmThreads64), args, sizeof(ChainShared), stream);
 }
 
 cudaError_t launch_lsm_finish(const LsmDev* c, int n_contracts, const Welford* final_part,

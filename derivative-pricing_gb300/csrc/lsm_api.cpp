@@ -143,7 +143,7 @@ int upload_and_run(Ctx& ctx, const LsmPlan& p, int precision, bool frozen, std::
     if (!rc) rc = ctx.reserve(ctx.ext[kPartA], sizeof(LsmPartial) * std::max<size_t>(p.total_chunks, 1), "lsm partials");
     if (!rc) rc = ctx.reserve(ctx.ext[kPartB], sizeof(LsmPartial) * std::max<size_t>(p.total_folds, 1), "lsm group partials");
     if (!rc) rc = ctx.reserve(ctx.ext[kFinal], sizeof(Welford) * std::max<size_t>(p.total_chunks, 1), "lsm final partials");
-    if (!rc) rc = ctx.reserve(ctx.ext[kOut], sizeof(double) * 6 * n, "lsm results");
+    if (!rc) rc = ctx.reserve(ctx.ext[kOut], sizeof(double) * (6 * n + 1), "lsm results");
     const size_t n_counters = 2 * n + 2 * static_cast<size_t>(p.total_folds) + static_cast<size_t>(p.max_steps) + 1;
     if (!rc) rc = ctx.reserve(ctx.ext[kCounters], sizeof(uint32_t) * n_counters, "lsm chunk counters");
     if (!rc && mlp) {
@@ -237,6 +237,22 @@ int upload_and_run(Ctx& ctx, const LsmPlan& p, int precision, bool frozen, std::
         }
     }
     cudaGetLastError();
+    // An FP64 batch whose chunks are all resident at once walks its dates in one
+    // cooperative launch (lsm.cu).
+    uint32_t resident = 0;
+    if (precision == 0 && !mlp) {
+        e = lsm_chain64_capacity(ctx.sm_count, &resident);
+        if (e != cudaSuccess) return ctx.cuda_fail(e, "lsm occupancy");
+    }
+    const bool one_launch = p.total_chunks > 0 && p.total_chunks <= std::min(resident, kLsmChainChunks);
+    double* d_out = static_cast<double*>(ctx.ext[kOut].ptr);
+    if (one_launch) {
+        e = cudaMemsetAsync(d_out + 6 * n, 0, sizeof(double), ctx.stream);
+        if (e != cudaSuccess) return ctx.cuda_fail(e, "lsm error word");
+        Chain all;
+        all.chunk_count = p.total_chunks;
+        chains.assign(1, all);
+    }
     int pair = -1;
     rc = ctx.record_start(ctx.stream, &pair);
     if (rc) return rc;
@@ -279,6 +295,13 @@ int upload_and_run(Ctx& ctx, const LsmPlan& p, int precision, bool frozen, std::
             le = launch_lsm_forward(precision, ctx.sm_count, d_dev, d_map, ch.chunk_first, ch.chunk_count,
                                     ctx.ext[kStore].ptr, ctx.tables, cs);
         if (le == cudaSuccess && j + 1 < chains.size()) le = cudaEventRecord(ctx.ev_stage[j], cs);
+        if (le == cudaSuccess && one_launch)
+            le = launch_lsm_chain64(d_dev, static_cast<int>(n), d_map, p.total_chunks, p.total_folds,
+                                    static_cast<const double*>(ctx.ext[kStore].ptr),
+                                    static_cast<LsmReg*>(ctx.ext[kReg].ptr),
+                                    static_cast<LsmPartial*>(ctx.ext[kPartA].ptr),
+                                    static_cast<Welford*>(ctx.ext[kFinal].ptr),
+                                    static_cast<uint32_t*>(ctx.ext[kCounters].ptr), d_out + 6 * n, ctx.tables, cs);
         for (int k = 0; k < ch.max_steps && le == cudaSuccess; ++k) {
             if (mlp)
                 le = launch_lsm_mlp_iteration(precision, k, !frozen, d_dev, ch.c_first, ch.c_end, ch.max_steps,
@@ -318,13 +341,15 @@ int upload_and_run(Ctx& ctx, const LsmPlan& p, int precision, bool frozen, std::
         return ctx.cuda_fail(le, "lsm launch");
     }
     rc = ctx.record_stop(ctx.stream, pair);
-    out.assign(6 * n, 0.0);
+    out.assign(6 * n + 1, 0.0);
     if (!rc) {
-        e = cudaMemcpyAsync(out.data(), ctx.ext[kOut].ptr, sizeof(double) * 6 * n, cudaMemcpyDeviceToHost, ctx.stream);
+        e = cudaMemcpyAsync(out.data(), d_out, sizeof(double) * (6 * n + (one_launch ? 1 : 0)), cudaMemcpyDeviceToHost,
+                            ctx.stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(ctx.stream);
         if (e != cudaSuccess) rc = ctx.cuda_fail(e, "lsm execution");
     }
     ctx.collect_timing(false);
+    if (!rc && one_launch && out[6 * n] != 0.0) return ctx.fail(MCD_ERR_TIMEOUT, "a wait for a date's regression gave up");
     if (!rc && mlp) {
         uint32_t werr = 0;
         e = cudaMemcpy(&werr, ctx.ext[kErr].ptr, sizeof werr, cudaMemcpyDeviceToHost);
