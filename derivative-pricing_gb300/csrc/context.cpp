@@ -76,7 +76,7 @@ Ctx::~Ctx() {
         if (g.exec) cudaGraphExecDestroy(g.exec);
     }
     if (greeks_graph) cudaGraphExecDestroy(greeks_graph);
-    for (DeviceBuffer* b : {&d_contracts, &d_prefix, &d_partials, &d_results, &d_scratch, &d_scratch2}) {
+    for (DeviceBuffer* b : {&d_plan, &d_partials, &d_scratch, &d_scratch2}) {
         if (b->ptr) cudaFree(b->ptr);
     }
     if (d_flags) cudaFree(d_flags);
@@ -317,55 +317,69 @@ int launch_shape(Ctx& ctx, int precision, int& variant, int& grid) {
     return MCD_OK;
 }
 
-// Uploads a plan into the context's device buffers (async on ctx.stream).
+// A plan's buffers, one allocation: the contracts, the prefix, the ticket and
+// error words and the results, so that a call uploads the first three in one
+// copy and reads the last two back in one.
+struct PlanBuffers {
+    char* base;
+    size_t prefix_at, flags_at, results_at, bytes;
+    PlanBuffers(void* p, size_t n) : base(static_cast<char*>(p)) {
+        auto up = [](size_t x) { return (x + 15) & ~size_t(15); };
+        prefix_at = up(sizeof(DevContract) * n);
+        flags_at = up(prefix_at + sizeof(uint32_t) * (n + 1));
+        results_at = flags_at + 16;
+        bytes = results_at + sizeof(mcd_mc_result) * n;
+    }
+    const DevContract* contracts() const { return reinterpret_cast<const DevContract*>(base); }
+    const uint32_t* prefix() const { return reinterpret_cast<const uint32_t*>(base + prefix_at); }
+    uint32_t* flags() const { return reinterpret_cast<uint32_t*>(base + flags_at); }
+    void* results() const { return base + results_at; }
+};
+
+// Uploads a plan (its ticket and error words zero) into the context's device
+// buffers (async on ctx.stream).
 int upload_plan(Ctx& ctx, const BatchPlan& plan) {
     // The device-resident plan shares these buffers; any upload retires it.
     ctx.device_plan_valid = false;
     const size_t n = plan.n;
-    int rc = ctx.reserve(ctx.d_contracts, sizeof(DevContract) * std::max<size_t>(n, 1), "contracts");
-    if (rc) return rc;
-    rc = ctx.reserve(ctx.d_prefix, sizeof(uint32_t) * (n + 1), "prefix");
+    PlanBuffers at(nullptr, n);
+    int rc = ctx.reserve(ctx.d_plan, at.bytes, "contracts and results");
     if (rc) return rc;
     rc = ctx.reserve(ctx.d_partials, sizeof(Welford) * std::max<size_t>(plan.max_items, 1), "partials");
     if (rc) return rc;
-    rc = ctx.reserve(ctx.d_results, sizeof(mcd_mc_result) * std::max<size_t>(n, 1), "results");
-    if (rc) return rc;
-    // Stage through pinned memory so the copies are truly asynchronous.
-    const size_t cbytes = sizeof(DevContract) * n, pbytes = sizeof(uint32_t) * (n + 1);
-    rc = ctx.reserve_host(ctx.h_stage, cbytes + pbytes, "pinned staging");
+    // Stage through pinned memory so the copy is truly asynchronous.
+    rc = ctx.reserve_host(ctx.h_stage, at.bytes, "pinned staging");
     if (rc) return rc;
     cudaError_t e = cudaStreamSynchronize(ctx.stream);  // staging buffer reuse
     if (e != cudaSuccess) return ctx.cuda_fail(e, "stream sync");
     char* stage = static_cast<char*>(ctx.h_stage.ptr);
-    if (n) std::memcpy(stage, plan.dev.data(), cbytes);
-    std::memcpy(stage + cbytes, plan.prefix.data(), pbytes);
-    if (n) {
-        e = cudaMemcpyAsync(ctx.d_contracts.ptr, stage, cbytes, cudaMemcpyHostToDevice, ctx.stream);
-        if (e != cudaSuccess) return ctx.cuda_fail(e, "copy contracts");
-    }
-    e = cudaMemcpyAsync(ctx.d_prefix.ptr, stage + cbytes, pbytes, cudaMemcpyHostToDevice, ctx.stream);
-    if (e != cudaSuccess) return ctx.cuda_fail(e, "copy prefix");
+    if (n) std::memcpy(stage, plan.dev.data(), sizeof(DevContract) * n);
+    std::memcpy(stage + at.prefix_at, plan.prefix.data(), sizeof(uint32_t) * (n + 1));
+    std::memset(stage + at.flags_at, 0, at.results_at - at.flags_at);
+    e = cudaMemcpyAsync(ctx.d_plan.ptr, stage, at.results_at, cudaMemcpyHostToDevice, ctx.stream);
+    if (e != cudaSuccess) return ctx.cuda_fail(e, "copy contracts");
     return MCD_OK;
 }
 
-// Queues a planned batch on a stream: per range, reset ticket and error word,
-// persistent path kernel, merge kernel.  (The error word keeps the last
-// range's value; an inconsistent item shows in every run.)
+// Queues a planned batch on a stream: per range, reset ticket and error word
+// (the first range's are zero already when `fresh`), persistent path kernel,
+// merge kernel.  (The error word keeps the last range's value; an inconsistent
+// item shows in every run.)
 int enqueue_plan(Ctx& ctx, int precision, int variant, int grid, const BatchPlan& plan, void* results,
-                 cudaStream_t stream) {
+                 uint32_t* flags, bool fresh, cudaStream_t stream) {
     cudaGetLastError();  // launches below report their own status only
-    const DevContract* dev = static_cast<const DevContract*>(ctx.d_contracts.ptr);
-    const uint32_t* prefix = static_cast<const uint32_t*>(ctx.d_prefix.ptr);
+    const PlanBuffers at(ctx.d_plan.ptr, plan.n);
     Welford* partials = static_cast<Welford*>(ctx.d_partials.ptr);
     for (size_t r = 0; r + 1 < plan.ranges.size(); ++r) {
         const uint32_t first = plan.ranges[r];
         const int n = static_cast<int>(plan.ranges[r + 1] - first);
-        cudaError_t e = cudaMemsetAsync(ctx.d_flags, 0, (r == 0 ? 2 : 1) * sizeof(uint32_t), stream);
+        cudaError_t e = cudaSuccess;
+        if (r > 0 || !fresh) e = cudaMemsetAsync(flags, 0, (r == 0 ? 2 : 1) * sizeof(uint32_t), stream);
         if (e != cudaSuccess) return ctx.cuda_fail(e, "reset flags");
-        e = launch_path_kernel(precision, variant, grid, dev + first, n, prefix + first, ctx.d_flags, partials,
-                               ctx.d_flags + 1, ctx.tables, stream);
+        e = launch_path_kernel(precision, variant, grid, at.contracts() + first, n, at.prefix() + first, flags,
+                               partials, flags + 1, ctx.tables, stream);
         if (e != cudaSuccess) return ctx.cuda_fail(e, "path kernel");
-        e = launch_merge_kernel(dev + first, n, prefix + first, partials, results, stream);
+        e = launch_merge_kernel(at.contracts() + first, n, at.prefix() + first, partials, results, stream);
         if (e != cudaSuccess) return ctx.cuda_fail(e, "merge kernel");
     }
     return MCD_OK;
@@ -376,8 +390,7 @@ int enqueue_plan(Ctx& ctx, int precision, int variant, int grid, const BatchPlan
 // inside the graph.
 int get_graph(Ctx& ctx, int precision, int variant, int grid, const BatchPlan& plan, void* results,
               cudaGraphExec_t* out) {
-    GraphKey key{precision, variant, grid, plan.n, 0u, ctx.d_contracts.ptr,
-                 ctx.d_prefix.ptr, ctx.d_partials.ptr, results};
+    GraphKey key{precision, variant, grid, plan.n, 0u, ctx.d_plan.ptr, nullptr, ctx.d_partials.ptr, results};
     for (auto& g : ctx.graphs) {
         if (g.key == key && g.exec) {
             *out = g.exec;
@@ -387,7 +400,7 @@ int get_graph(Ctx& ctx, int precision, int variant, int grid, const BatchPlan& p
     cudaGraph_t graph = nullptr;
     cudaError_t e = cudaStreamBeginCapture(ctx.stream, cudaStreamCaptureModeThreadLocal);
     if (e != cudaSuccess) return ctx.cuda_fail(e, "begin capture");
-    const int rc = enqueue_plan(ctx, precision, variant, grid, plan, results, ctx.stream);
+    const int rc = enqueue_plan(ctx, precision, variant, grid, plan, results, ctx.d_flags, false, ctx.stream);
     e = cudaStreamEndCapture(ctx.stream, &graph);
     if (rc) {
         if (graph) cudaGraphDestroy(graph);
@@ -426,7 +439,7 @@ int run_plan(Ctx& ctx, int precision, const BatchPlan& plan, void* results, cuda
         cudaError_t e = cudaGraphLaunch(exec, stream);
         if (e != cudaSuccess) return ctx.cuda_fail(e, "graph launch");
     } else {
-        rc = enqueue_plan(ctx, precision, variant, grid, plan, results, stream);
+        rc = enqueue_plan(ctx, precision, variant, grid, plan, results, ctx.d_flags, false, stream);
         if (rc) return rc;
     }
     return ctx.record_stop(stream, pair);
@@ -451,14 +464,31 @@ int price_batch_host(Ctx& ctx, const mcd_contract* contracts, size_t n, int prec
     if (n == 0) return MCD_OK;
     rc = upload_plan(ctx, plan);
     if (rc) return rc;
-    rc = run_plan(ctx, precision, plan, ctx.d_results.ptr, ctx.stream);
+    // One upload, two launches, one read-back into pinned memory: launched
+    // directly, their inputs (and the zeroed ticket) having just been queued.
+    int variant = 0, grid = 0, pair = -1;
+    rc = launch_shape(ctx, precision, variant, grid);
+    if (!rc) rc = ctx.record_start(ctx.stream, &pair);
     if (rc) return rc;
-    cudaError_t e = cudaMemcpyAsync(results, ctx.d_results.ptr, sizeof(mcd_mc_result) * n,
-                                    cudaMemcpyDeviceToHost, ctx.stream);
+    const PlanBuffers at(ctx.d_plan.ptr, n);
+    rc = enqueue_plan(ctx, precision, variant, grid, plan, at.results(), at.flags(), true, ctx.stream);
+    if (!rc) rc = ctx.record_stop(ctx.stream, pair);
+    if (rc) {  // let what was queued finish before the buffers are used again
+        cudaStreamSynchronize(ctx.stream);
+        cudaGetLastError();
+        return rc;
+    }
+    char* stage = static_cast<char*>(ctx.h_stage.ptr) + at.flags_at;
+    cudaError_t e = cudaMemcpyAsync(stage, at.flags(), at.bytes - at.flags_at, cudaMemcpyDeviceToHost, ctx.stream);
     if (e != cudaSuccess) return ctx.cuda_fail(e, "copy results");
     e = cudaStreamSynchronize(ctx.stream);
     if (e != cudaSuccess) return ctx.cuda_fail(e, "batch execution");
-    return collect_after_sync(ctx);
+    ctx.collect_timing(false);
+    uint32_t error_word;
+    std::memcpy(&error_word, stage + sizeof error_word, sizeof error_word);
+    if (error_word != 0) return ctx.fail(MCD_ERR_CUDA, "path kernel reported an inconsistent work item");
+    std::memcpy(results, stage + 16, sizeof(mcd_mc_result) * n);
+    return MCD_OK;
 }
 
 }  // namespace mcdg
@@ -672,7 +702,7 @@ int mcd_autotune(mcd_ctx* handle, const mcd_contract* contracts, size_t n, int p
             ctx->shape[precision] = LaunchShape{v, c};
             double total = 0.0;
             for (int rep = 0; rep < 3; ++rep) {
-                rc = run_plan(*ctx, precision, plan, ctx->d_results.ptr, ctx->stream);
+                rc = run_plan(*ctx, precision, plan, PlanBuffers(ctx->d_plan.ptr, n).results(), ctx->stream);
                 if (rc) { ctx->shape[precision] = saved; return rc; }
                 e = cudaStreamSynchronize(ctx->stream);
                 if (e != cudaSuccess) { ctx->shape[precision] = saved; return ctx->cuda_fail(e, "tuning run"); }

@@ -74,7 +74,7 @@ struct Ctx {
     cudaStream_t stream = nullptr;
     std::string error;
 
-    DeviceBuffer d_contracts, d_prefix, d_partials, d_results, d_scratch, d_scratch2;
+    DeviceBuffer d_plan, d_partials, d_scratch, d_scratch2;
     uint32_t* d_flags = nullptr;  // [0] ticket, [1] error word, [4..5] contract digest, rest spare
     HostBuffer h_stage;
     const FixedTables* tables = nullptr;  // this device's fixed-point tables
