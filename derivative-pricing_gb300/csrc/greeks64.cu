@@ -13,11 +13,16 @@
 // sum i S_i from the prefix sums of S_i.
 //
 // Bound: issue and the FMA-heavy pipe for barriers, lookbacks and geometric
-// Asians; the FP64 pipe for arithmetic Asians (five operations per step).  512
-// threads per CTA: the twelve outputs' sums and the path state take 128
-// registers.  Measured: finite-difference European, likelihood-ratio barrier
-// and pathwise Asian of 1e5 paths and 52 dates, one call each, 130 -> 0.51 ms
-// in all; largest error against 64-bit values 4.7e-13 -> 2.2e-14.
+// Asians; the FP64 pipe for arithmetic Asians (five operations per step).  1024
+// threads per CTA (64 registers): the twelve outputs' sums are then spilled
+// between the rounds of a unit, but a call of 1e5 paths (3125 units) is one
+// round of the 4864 resident warps, where 512 threads and 128 registers took
+// two.  Measured: finite-difference European, likelihood-ratio barrier and
+// pathwise Asian of 1e5 paths and 52 dates, one call each, 130 -> 0.39 ms in all
+// (512, 640, 768, 1024 threads: 0.48, 0.48, 0.42, 0.41 before the units' sums
+// lost their division); 16 contracts of 2e5 paths, Asian 3.09 -> 2.91 ms, barrier
+// 1.91 -> 1.65, lookback 1.66 -> 1.61, European 0.81; largest error against
+// 64-bit values 4.7e-13 -> 2.2e-14.
 //
 // nvcc-flags: --fmad=false
 #include <cuda_runtime.h>
@@ -30,7 +35,7 @@ namespace mcdg {
 
 namespace {
 
-constexpr int kThreads = 512;
+constexpr int kThreads = 1024;
 
 __device__ __forceinline__ double dmax(double a, double b) { return (a < b) ? b : a; }
 
