@@ -83,8 +83,10 @@ struct KahanF {
     }
 };
 
-// Two paths per thread in flight: 6 CTAs of 128 threads per SM.
-__global__ void __launch_bounds__(128, 6)
+// Two paths per thread in flight, 5 CTAs of 128 threads per SM (92 registers): 64
+// sets of 2^20 paths and 252 steps at 3, 4, 5, 6, 7, 8 CTAs: 107.7, 99.7, 97.5,
+// 99.9, 104.4, 105.8 ms.
+__global__ void __launch_bounds__(128, 5)
     heston_kernel(const HestonSet* __restrict__ sets, const double* __restrict__ strikes,
                   int n_strikes, int type, uint32_t items_per_set, uint32_t total_items,
                   uint32_t* __restrict__ ticket, Welford* __restrict__ partials) {
