@@ -456,12 +456,41 @@ int collect_after_sync(Ctx& ctx) {
     return MCD_OK;
 }
 
+// Up to this many slabs (4.2 million paths) a European or digital contract by
+// itself is one launch (quote64_kernel, where both forms' times stand).
+constexpr uint32_t kQuoteSlabs = 1024;
+
+int price_quote(Ctx& ctx, const DevContract& c, mcd_mc_result* result) {
+    static_assert(sizeof(DevMcResult) == sizeof(mcd_mc_result), "the result is copied as it is");
+    int rc = ctx.reserve(ctx.d_partials, sizeof(Welford) * std::max<size_t>(c.n_units, 1), "partials");
+    if (!rc) rc = ctx.reserve_host(ctx.h_stage, sizeof(DevMcResult), "pinned staging");
+    if (rc) return rc;
+    cudaError_t e = cudaStreamSynchronize(ctx.stream);  // staging buffer reuse
+    if (e != cudaSuccess) return ctx.cuda_fail(e, "stream sync");
+    int pair = -1;
+    rc = ctx.record_start(ctx.stream, &pair);
+    if (rc) return rc;
+    e = launch_quote64(ctx.sm_count, c, static_cast<Welford*>(ctx.d_partials.ptr), ctx.d_flags + 8,
+                       static_cast<DevMcResult*>(ctx.h_stage.ptr), ctx.tables, ctx.stream);
+    if (e != cudaSuccess) return ctx.cuda_fail(e, "quote kernel");
+    rc = ctx.record_stop(ctx.stream, pair);
+    e = cudaStreamSynchronize(ctx.stream);
+    if (e != cudaSuccess) return ctx.cuda_fail(e, "batch execution");
+    ctx.collect_timing(false);
+    if (rc) return rc;
+    std::memcpy(result, ctx.h_stage.ptr, sizeof *result);
+    return MCD_OK;
+}
+
 int price_batch_host(Ctx& ctx, const mcd_contract* contracts, size_t n, int precision,
                      mcd_mc_result* results) {
     BatchPlan& plan = ctx.host_plan;
     int rc = plan_batch(ctx, contracts, n, precision == 0 ? kRangeItems : 0, plan);
     if (rc) return rc;
     if (n == 0) return MCD_OK;
+    const DevContract& c0 = plan.dev[0];
+    if (precision == 0 && n == 1 && (c0.kind == kEuropean || c0.kind == kDigital) && c0.n_slabs <= kQuoteSlabs)
+        return price_quote(ctx, c0, results);
     rc = upload_plan(ctx, plan);
     if (rc) return rc;
     // One upload, two launches, one read-back into pinned memory: launched

@@ -75,7 +75,7 @@ struct Ctx {
     std::string error;
 
     DeviceBuffer d_plan, d_partials, d_scratch, d_scratch2;
-    uint32_t* d_flags = nullptr;  // [0] ticket, [1] error word, [4..5] contract digest, rest spare
+    uint32_t* d_flags = nullptr;  // [0] ticket, [1] error word, [4..5] contract digest, [8] CTAs done (quote64_kernel), rest spare
     HostBuffer h_stage;
     const FixedTables* tables = nullptr;  // this device's fixed-point tables
 

@@ -17,6 +17,12 @@ struct Welford {
     double m2;
 };
 
+struct DevMcResult {  // mcd_mc_result
+    double price;
+    double standard_error;
+    unsigned long long path_count;
+};
+
 constexpr int kSlabPaths = 4096;       // MCD_SLAB_PATHS
 constexpr int kSlabThreads = 128;      // one CTA = one slab lane group
 constexpr int kPathsPerThread = kSlabPaths / kSlabThreads;
@@ -91,6 +97,10 @@ cudaError_t launch_path_kernel(int precision, int variant, int grid, const DevCo
 cudaError_t launch_path64_kernel(int variant, int grid, const DevContract* contracts, int n_contracts,
                                  const uint32_t* item_prefix, uint32_t* ticket, Welford* partials,
                                  uint32_t* error_flag, const FixedTables* tables, cudaStream_t stream);
+// An FP64 call of one European or digital contract: the result goes to pinned
+// host memory; one partial per unit, *done zero before and after.
+cudaError_t launch_quote64(int sm_count, const DevContract& c, Welford* partials, uint32_t* done, DevMcResult* result,
+                           const FixedTables* tables, cudaStream_t stream);
 // The fixed-point tables of the current device, placed there at the first call
 // (computed once per process, 22 ms).  Not to be called during stream capture.
 cudaError_t fixed_tables_device(const FixedTables** out);

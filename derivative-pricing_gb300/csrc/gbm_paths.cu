@@ -293,12 +293,6 @@ __global__ void __launch_bounds__(kSlabThreads, MINB)
     }
 }
 
-struct DevMcResult {
-    double price;
-    double standard_error;
-    unsigned long long path_count;
-};
-
 // One CTA per contract; results go to the caller's positions.
 __global__ void __launch_bounds__(kMergeThreads)
     merge_kernel(const DevContract* __restrict__ contracts, const uint32_t* __restrict__ item_prefix,

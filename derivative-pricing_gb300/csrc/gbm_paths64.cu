@@ -23,10 +23,13 @@
 // nvcc-flags: --fmad=false
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <mutex>
 
 #include "engine.hpp"
 #include "fixed_tables.hpp"
+#include "lsm_math.cuh"
+#include "merge.cuh"
 #include "paths64.cuh"
 
 namespace mcdg {
@@ -34,6 +37,8 @@ namespace mcdg {
 namespace {
 
 __device__ FixedTables g_fixed_tables;
+
+constexpr int kQuoteThreads = 128, kQuoteCtas = 6;
 
 // ---------------------------------------------------------------------------
 // Contracts whose log-spot does not fit the fixed-point range (|log2(S/S0)|
@@ -155,6 +160,69 @@ struct Shared64 {
     WarpSlot slot[1];  // one per warp
 };
 
+// A call of one European or digital contract, latency above all: the contract is
+// a launch parameter, the tables are read through the L1 cache (a CTA would copy
+// 176 KB of them for a few hundred lookups), and the last CTA folds the units
+// and writes the result to pinned host memory.  So a call is one launch, without
+// copies.  Microseconds per call by number of paths, against upload, path
+// kernel, merge kernel and read-back: 32: 36.3 -> 23.4, 1e4: 35.9 -> 27.5, 1e5:
+// 48.3 -> 38.2, 1e6: 60.6 -> 57.8, 3e6: 85 -> 79, 1e7: 196 -> 203 (where the
+// table in shared memory pays).  With several contracts the last CTA's folds
+// follow one another: nine of 1e5 paths took 70 us longer.
+__global__ void __launch_bounds__(kQuoteThreads, kQuoteCtas)
+    quote64_kernel(const __grid_constant__ DevContract c, Welford* __restrict__ partials,
+                    uint32_t* __restrict__ done, DevMcResult* __restrict__ result,
+                    const FixedTables* __restrict__ g) {
+    __shared__ bool s_last;
+    const int lane = threadIdx.x & 31;
+    const uint32_t warps = gridDim.x * (kQuoteThreads / 32);
+    const GlobalTables tables{g};
+    for (uint32_t item = (threadIdx.x >> 5) * gridDim.x + blockIdx.x; item < c.n_units; item += warps) {
+        const uint64_t base = static_cast<uint64_t>(item) << (5 + c.unit_log);
+        const uint64_t left = c.path_count - base;
+        const uint32_t size = 32u << c.unit_log;
+        const uint32_t count = left < size ? static_cast<uint32_t>(left) : size;
+        const int rounds = static_cast<int>((count + 31u) / 32u);
+        Welford r;
+        if (c.frac == 0) {
+            r = unit_wide(c, base, count, rounds);
+        } else {  // unit_fixed of one step
+            const PhiloxKeys k = philox_keys(c.seed);
+            const PhiloxStep st = philox_step(0u, static_cast<uint32_t>(base >> 32), k);
+            UnitSums acc;
+            for (int j = 0; j < rounds; ++j) {
+                const uint32_t o = static_cast<uint32_t>(j) * 32u + lane;
+                const PhiloxRow row = philox_row(static_cast<uint32_t>(base) + o, 0u, k);
+                const int64_t x = scaled_normal(tables.normal(philox_word0(row, st, k)), c.y_vs);
+                auto sample = [&](int64_t y) {
+                    const double last = c.spot * tables.exp2(y, c.frac), v = put_sign(last - c.strike, c.type);
+                    const double pay = c.kind == kDigital ? (v > 0.0 ? (c.asset ? last : c.cash) : 0.0) : positive_part(v);
+                    return c.discount * pay;
+                };
+                double v = sample(c.y_drift + x);
+                if (c.antithetic) v = 0.5 * (v + sample(c.y_drift - x));
+                if (j == 0) acc.first(v);
+                if (o < count) acc.add(v);
+            }
+            r = acc.reduce(count);
+        }
+        if (lane == 0) partials[item] = r;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        s_last = atomicAdd(done, 1u) == gridDim.x - 1u;
+    }
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    const MergedResult m = merge_items(partials, c.n_units, 1);
+    if (threadIdx.x == 0) {
+        *result = DevMcResult{m.mean, m.standard_error, m.count};
+        *done = 0u;  // for the next call
+    }
+}
+
 template <int THREADS>
 __global__ void __launch_bounds__(THREADS, 1)
     path64_kernel(const DevContract* __restrict__ contracts, int n_contracts, const uint32_t* __restrict__ prefix,
@@ -273,6 +341,15 @@ cudaError_t launch_path64_kernel(int variant, int grid, const DevContract* contr
         default: return launch_threads<1024>(grid, contracts, n_contracts, item_prefix, ticket, partials, error_flag,
                                              tables, stream);
     }
+}
+
+cudaError_t launch_quote64(int sm_count, const DevContract& c, Welford* partials, uint32_t* done, DevMcResult* result,
+                           const FixedTables* tables, cudaStream_t stream) {
+    constexpr uint32_t kWarps = kQuoteThreads / 32;
+    const uint32_t ctas = std::max(1u, std::min((c.n_units + kWarps - 1) / kWarps, static_cast<uint32_t>(sm_count) * kQuoteCtas));
+    cudaGetLastError();
+    quote64_kernel<<<ctas, kQuoteThreads, 0, stream>>>(c, partials, done, result, tables);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_draws64_kernel(uint64_t seed, uint64_t path_begin, uint64_t n_paths, uint32_t draw_begin,

@@ -17,23 +17,28 @@ struct MergedResult {
     unsigned long long count;
 };
 
-// One CTA of kMergeThreads folds the Welford triples items[i * stride],
-// i < count: thread t takes t, t + kMergeThreads, ... in order, as sums shifted by the
+// The first kMergeThreads threads of a CTA fold the Welford triples
+// items[i * stride], i < count (every thread calls; read past the L1): thread t takes t, t + kMergeThreads, ... in order, as sums shifted by the
 // first item's mean (four FP64 operations per item and no division: a chain of
 // Welford merges takes about forty), then a fixed tree.  Valid in thread 0.
 __device__ __forceinline__ MergedResult merge_items(const Welford* __restrict__ items, uint32_t count, int stride) {
     __shared__ double s_sum[2][kMergeThreads / 32];
     __shared__ unsigned long long s_count[kMergeThreads / 32];
-    const double shift = count ? items[0].mean : 0.0;
+    static_assert(sizeof(Welford) == 24 && offsetof(Welford, mean) == 8 && offsetof(Welford, m2) == 16, "three words");
+    auto load = [&](uint32_t i) {
+        const double* p = reinterpret_cast<const double*>(items + static_cast<size_t>(i) * stride);
+        return Welford{static_cast<unsigned long long>(__double_as_longlong(__ldcg(p))), __ldcg(p + 1), __ldcg(p + 2)};
+    };
+    const double shift = count ? load(0).mean : 0.0;
     unsigned long long n = 0;
     double s1 = 0.0, s2 = 0.0;
     constexpr int kAhead = 4;
-    for (uint32_t i0 = threadIdx.x; i0 < count; i0 += kAhead * kMergeThreads) {
+    for (uint32_t i0 = threadIdx.x; threadIdx.x < kMergeThreads && i0 < count; i0 += kAhead * kMergeThreads) {
         Welford w[kAhead];
 #pragma unroll
         for (int j = 0; j < kAhead; ++j) {
             const uint32_t i = i0 + j * kMergeThreads;
-            if (i < count) w[j] = items[static_cast<size_t>(i) * stride];
+            if (i < count) w[j] = load(i);
         }
 #pragma unroll
         for (int j = 0; j < kAhead; ++j) {
@@ -50,7 +55,7 @@ __device__ __forceinline__ MergedResult merge_items(const Welford* __restrict__ 
         s1 += __shfl_down_sync(0xffffffffu, s1, off);
         s2 += __shfl_down_sync(0xffffffffu, s2, off);
     }
-    if ((threadIdx.x & 31) == 0) {
+    if ((threadIdx.x & 31) == 0 && threadIdx.x < kMergeThreads) {
         s_count[threadIdx.x >> 5] = n;
         s_sum[0][threadIdx.x >> 5] = s1;
         s_sum[1][threadIdx.x >> 5] = s2;
