@@ -67,8 +67,8 @@ struct SobolLane {
 };
 
 constexpr int kSxStride = kSobolDims + 1;  // +1 word: the last lane's row sits in another bank
-template <int PREC>
-constexpr int kSxPerWarp = (PREC == 0 ? 2 : 4) * kSxStride;  // FP32: two groups of 32 paths at a time
+constexpr int kSxPerWarp = 2 * kSxStride;
+constexpr int kQuad = 4;  // FP32: paths per thread at a time
 
 // Bridge coefficients of one contract in program order, FP64 kernel.
 struct QmcTables64 {
@@ -80,7 +80,8 @@ struct QmcTables64 {
 // (the same address across the warp): the FP32 coefficients and the node's
 // Sobol dimension and slots packed into the last word.
 struct QmcTables32 {
-    float4 node[kSobolDims];  // {a, sd, drift, bits(meta)}
+    float4 node[kSobolDims];     // {a, sd, drift, bits(meta)}
+    uint4 mask[kSobolDims][2];   // quad_qmc32: of lanes 0..30, of lane 31
 };
 __device__ __forceinline__ uint32_t meta_dim(uint32_t m) { return m & 0xFFu; }
 __device__ __forceinline__ uint32_t meta_left(uint32_t m) { return (m >> 8) & 0xFu; }
@@ -90,11 +91,22 @@ __device__ __forceinline__ uint32_t meta_out(uint32_t m) { return (m >> 16) & 0x
 template <int PREC>
 using QmcTables = typename std::conditional<PREC == 0, QmcTables64, QmcTables32>::type;
 
+// FP32: a thread's four paths are 32 indices apart, B + 32 p + lane with B a
+// multiple of 128, so the indices' high parts differ in bits 5 and 6 only:
+// X(B + 32 p) = X(B) ^ M_p, M_p the directions of the bits of gray(32 p), one
+// row X(B) for all four.  Lane 31's low part is 0 of the next 32: its masks are
+// M_1, M_2, M_3 and, for its last path, the row X(B + 128).
+__device__ __forceinline__ uint3 quad_masks(const uint32_t* __restrict__ by_bit, uint32_t dim) {
+    const uint32_t v4 = __ldg(by_bit + 4 * kSobolDims + dim), v5 = __ldg(by_bit + 5 * kSobolDims + dim),
+                   v6 = __ldg(by_bit + 6 * kSobolDims + dim);
+    return make_uint3(v4 ^ v5, v5 ^ v6, v4 ^ v6);  // gray(32), gray(64), gray(96)
+}
+
 // Bridge coefficients of one contract in program order, with the reference's
 // operations (brownian_bridge_path.cpp:29-31, :52-62, :71-74): t_i = i T / n.
 template <int PREC>
 __device__ void fill_tables(const DevContract& c, const DevQmc& q, const BridgeNode* __restrict__ programs,
-                            QmcTables<PREC>& S) {
+                            const uint32_t* __restrict__ by_bit, QmcTables<PREC>& S) {
     const int n = c.n_steps;
     const double nd = static_cast<double>(n);
     auto t_of = [&](int i) { return static_cast<double>(i) * q.time / nd; };
@@ -124,6 +136,9 @@ __device__ void fill_tables(const DevContract& c, const DevQmc& q, const BridgeN
                                   (static_cast<uint32_t>(b.slot_out) << 16);
             S.node[e] = make_float4(static_cast<float>(a), static_cast<float>(sd), static_cast<float>(drift),
                                     __uint_as_float(meta));
+            const uint3 m = quad_masks(by_bit, b.dim);
+            S.mask[e][0] = make_uint4(0u, m.x, m.y, m.z);
+            S.mask[e][1] = make_uint4(m.x, m.y, m.z, 0u);
         }
     }
 }
@@ -203,29 +218,35 @@ __device__ __forceinline__ double terminal_qmc32(const DevContract& c, uint32_t 
     return c.discount * static_cast<double>(payoff);
 }
 
-// Two paths of a thread, 128 indices apart: they share the program's records,
-// their slots' addresses and the lane's Y word, and their chains interleave.
-// Bound by issue (89 % of the cycles at 7 CTAs per SM, 67 registers).  A
-// book of 4096 mixed contracts of 1e4 to 1e6 paths: one path at a time 282 ms,
-// two 277 (both waiting on bank conflicts of the directions, see add_x), with
-// the bit-major directions and the node fetched one ahead 173, the root taken
-// out of the loop 165.
+// The four paths of a thread: they share the program's records, their slots'
+// addresses, the row X and the lane's Y word, and their chains interleave.
+// Bound by issue.  A book of 4096 mixed contracts of 1e4 to 1e6 paths: one path
+// at a time 282 ms, two 277 (both waiting on bank conflicts of the directions,
+// see add_x), with the bit-major directions and the node fetched one ahead 173,
+// the root taken out of the loop 165, four paths from one row 149 (47
+// instructions per path-step instead of 59, issue 83 % at 5 CTAs per SM).
 // The bridge values live in shared memory, one column per thread and path
-// (w[slot * 256], w[slot * 256 + 128]): a node's slots are known only at run
-// time, so a register array would be spilled to local memory.
+// (w[slot * 512 + 128 p]): a node's slots are known only at run time, so a
+// register array would be spilled to local memory.
 template <int KIND>
-__device__ __forceinline__ void pair_qmc32(const DevContract& c, const DevQmc& q, const QmcTables32& S,
-                                           const uint32_t* x0, const uint32_t* x1, const uint32_t* __restrict__ y,
-                                           float* __restrict__ w, double (&out)[2]) {
+__device__ __forceinline__ void quad_qmc32(const DevContract& c, const DevQmc& q, const QmcTables32& S,
+                                           const uint32_t* row, const uint32_t* row_last,
+                                           const uint32_t* __restrict__ y, float* __restrict__ w,
+                                           double (&out)[kQuad]) {
     const float phi = c.type == 0 ? 1.0f : -1.0f;
     const float s0 = static_cast<float>(c.spot);
     const float strike = static_cast<float>(c.strike);
     const int n = c.n_steps;
     const float vol = static_cast<float>(q.vol);
     const float lnh = static_cast<float>(c.log_h_rel);
-    w[0] = w[kSlabThreads] = 0.0f;
-    float acc[2] = {0.0f, 0.0f}, xlast[2], xmax[2] = {0.0f, 0.0f}, xmin[2] = {0.0f, 0.0f};
-    bool breached[2] = {false, false};
+    float acc[kQuad], xlast[kQuad], xmax[kQuad], xmin[kQuad];
+    bool breached[kQuad];
+#pragma unroll
+    for (int p = 0; p < kQuad; ++p) {
+        w[p * kSlabThreads] = 0.0f;
+        acc[p] = xmax[p] = xmin[p] = 0.0f;
+        breached[p] = false;
+    }
     auto observe = [&](int p, float x) {
         if constexpr (KIND == kAsianArith) {
             acc[p] += __expf(x);
@@ -238,27 +259,28 @@ __device__ __forceinline__ void pair_qmc32(const DevContract& c, const DevQmc& q
             xmin[p] = fminf(xmin[p], x);
         }
     };
-    auto offset = [&](uint32_t slot) { return w + slot * (2 * kSlabThreads); };
+    auto offset = [&](uint32_t slot) { return w + slot * (kQuad * kSlabThreads); };
+    const uint4* mask = &S.mask[0][(threadIdx.x & 31) == 31 ? 1 : 0];
     // the next node's record and draws are fetched a node ahead
     float4 ahead;
-    uint32_t yw, xa, xb;
+    uint4 bits;
     auto fetch = [&](int e) {
         ahead = S.node[e];
         const uint32_t dim = meta_dim(__float_as_uint(ahead.w));
-        yw = __ldg(y + dim * 32u);
-        xa = x0[dim];
-        xb = x1[dim];
+        const uint32_t yw = __ldg(y + dim * 32u), x = row[dim];
+        const uint4 m = mask[2 * e];
+        bits = make_uint4(x ^ yw ^ m.x, x ^ yw ^ m.y, x ^ yw ^ m.z, row_last[dim] ^ yw ^ m.w);
     };
     fetch(0);
     {  // the program starts at its root, the terminal point, which has no ancestors
         const float4 nd = ahead;
-        const uint32_t bits[2] = {xa ^ yw, xb ^ yw};
+        const uint32_t u[kQuad] = {bits.x, bits.y, bits.z, bits.w};
         fetch(n > 1 ? 1 : 0);
-        float z[2];
-        normals_from_sobol_f32<2>(bits, z);
+        float z[kQuad];
+        normals_from_sobol_f32<kQuad>(u, z);
         float* at = offset(meta_out(__float_as_uint(nd.w)));
 #pragma unroll
-        for (int p = 0; p < 2; ++p) {
+        for (int p = 0; p < kQuad; ++p) {
             const float val = nd.y * z[p];
             at[p * kSlabThreads] = val;
             xlast[p] = __fmaf_rn(vol, val, nd.z);
@@ -268,14 +290,14 @@ __device__ __forceinline__ void pair_qmc32(const DevContract& c, const DevQmc& q
     for (int e = 1; e < n; ++e) {
         const float4 nd = ahead;
         const uint32_t meta = __float_as_uint(nd.w);
-        const uint32_t bits[2] = {xa ^ yw, xb ^ yw};
+        const uint32_t u[kQuad] = {bits.x, bits.y, bits.z, bits.w};
         fetch(min(e + 1, n - 1));
-        float z[2];
-        normals_from_sobol_f32<2>(bits, z);
+        float z[kQuad];
+        normals_from_sobol_f32<kQuad>(u, z);
         const float *left = offset(meta_left(meta)), *right = offset(meta_right(meta));
         float* at = offset(meta_out(meta));
 #pragma unroll
-        for (int p = 0; p < 2; ++p) {
+        for (int p = 0; p < kQuad; ++p) {
             const float wl = left[p * kSlabThreads], wr = right[p * kSlabThreads];
             const float val = __fmaf_rn(nd.y, z[p], __fmaf_rn(nd.x, wr - wl, wl));
             at[p * kSlabThreads] = val;
@@ -284,7 +306,7 @@ __device__ __forceinline__ void pair_qmc32(const DevContract& c, const DevQmc& q
     }
     const float inv_n = 1.0f / static_cast<float>(n);
 #pragma unroll
-    for (int p = 0; p < 2; ++p) {
+    for (int p = 0; p < kQuad; ++p) {
         const float last = s0 * __expf(xlast[p]);
         float v;
         if constexpr (KIND == kAsianArith || KIND == kAsianGeo) {
@@ -319,14 +341,13 @@ __device__ __forceinline__ void add_x(uint32_t* row, const uint32_t* __restrict_
 
 __device__ __forceinline__ uint32_t gray_code(uint64_t i) { return static_cast<uint32_t>(i ^ (i >> 1)); }
 
-// X of the warp's 32 paths from b0 on: row 0 for index base B = b0 (lanes 0..30),
-// row 1 for B + 32 (lane 31).  The rows hold those of the paths from `before` on,
-// or nothing yet.
+// Rows X(b0) and X(b0 + span) of a warp's paths from b0 on (the second for the
+// last lane).  They hold those of the paths from `before` on, or nothing yet.
 __device__ __forceinline__ void fill_x(uint32_t* xw, const uint32_t* __restrict__ by_bit, uint32_t ndims, uint64_t b0,
-                                       uint64_t before, bool start) {
-    const uint32_t g0 = gray_code(b0), g1 = gray_code(b0 + 32);
+                                       uint64_t span, uint64_t before, bool start) {
+    const uint32_t g0 = gray_code(b0), g1 = gray_code(b0 + span);
     add_x(xw, by_bit, ndims, start ? g0 : g0 ^ gray_code(before), start);
-    add_x(xw + kSxStride, by_bit, ndims, start ? g1 : g1 ^ gray_code(before + 32), start);
+    add_x(xw + kSxStride, by_bit, ndims, start ? g1 : g1 ^ gray_code(before + span), start);
 }
 
 // A warp's share of a slab; valid in lane 0 (FP32: shifted sums, FP64: a
@@ -338,7 +359,7 @@ __device__ Welford slab_qmc(const DevContract& c, const DevQmc& q, const QmcTabl
     constexpr bool kTerminal = KIND == kEuropean || KIND == kDigital;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t ndims = kTerminal ? 1u : static_cast<uint32_t>(c.n_steps);
-    uint32_t* xw = sx + warp * kSxPerWarp<PREC>;
+    uint32_t* xw = sx + warp * kSxPerWarp;
     const uint32_t* my_x = xw + (lane == 31 ? kSxStride : 0);
     if constexpr (PREC == 0) {
         const SobolLane sob{my_x, ytab + lane};
@@ -347,7 +368,7 @@ __device__ Welford slab_qmc(const DevContract& c, const DevQmc& q, const QmcTabl
             const uint64_t b0 = base + static_cast<uint64_t>(j * kSlabThreads) + 32u * warp;  // this warp's first path
             if (b0 >= c.path_count) break;  // uniform per warp
             __syncwarp();
-            fill_x(xw, by_bit, ndims, b0, b0 - kSlabThreads, j == 0);
+            fill_x(xw, by_bit, ndims, b0, 32, b0 - kSlabThreads, j == 0);
             __syncwarp();
             if (b0 + lane < c.path_count) welford_add(w, sample_qmc64<KIND>(c, q, S, sob));
         }
@@ -355,26 +376,29 @@ __device__ Welford slab_qmc(const DevContract& c, const DevQmc& q, const QmcTabl
     } else {
         UnitSums acc;
         unsigned count = 0;
-        for (int j = 0; j < kPathsPerThread; j += 2) {
-            const uint64_t b0 = base + static_cast<uint64_t>(j * kSlabThreads) + 32u * warp;
+        uint3 m0 = make_uint3(0u, 0u, 0u);
+        if constexpr (kTerminal) m0 = quad_masks(by_bit, 0u);
+        for (int j = 0; j < kPathsPerThread; j += kQuad) {  // 128 paths of a warp at a time
+            const uint64_t b0 = base + static_cast<uint64_t>(j * kSlabThreads) + kQuad * 32u * warp;
             if (b0 >= c.path_count) break;  // uniform per warp
             __syncwarp();
-            fill_x(xw, by_bit, ndims, b0, b0 - 2 * kSlabThreads, j == 0);
-            fill_x(xw + 2 * kSxStride, by_bit, ndims, b0 + kSlabThreads, b0 - kSlabThreads, j == 0);
+            fill_x(xw, by_bit, ndims, b0, kQuad * 32u, b0 - kQuad * kSlabThreads, j == 0);
             __syncwarp();
-            const uint64_t path = b0 + lane;
-            double v[2];
+            double v[kQuad];
             if constexpr (kTerminal) {
-                const uint32_t y = __ldg(ytab + lane);
-                v[0] = terminal_qmc32(c, my_x[0] ^ y);
-                v[1] = terminal_qmc32(c, my_x[2 * kSxStride] ^ y);
+                const uint32_t x = xw[0] ^ __ldg(ytab + lane);
+                const bool end = lane == 31;
+                v[0] = terminal_qmc32(c, end ? x ^ m0.x : x);
+                v[1] = terminal_qmc32(c, x ^ (end ? m0.y : m0.x));
+                v[2] = terminal_qmc32(c, x ^ (end ? m0.z : m0.y));
+                v[3] = terminal_qmc32(c, end ? xw[kSxStride] ^ __ldg(ytab + lane) : x ^ m0.z);
             } else {
-                pair_qmc32<KIND>(c, q, S, my_x, my_x + 2 * kSxStride, ytab + lane, bridge_w + threadIdx.x, v);
+                quad_qmc32<KIND>(c, q, S, xw, my_x, ytab + lane, bridge_w + threadIdx.x, v);
             }
             if (j == 0) acc.first(v[0]);
 #pragma unroll
-            for (int p = 0; p < 2; ++p) {
-                if (path + p * kSlabThreads < c.path_count) {
+            for (int p = 0; p < kQuad; ++p) {
+                if (b0 + 32u * p + lane < c.path_count) {
                     ++count;
                     acc.add(v[p]);
                 }
@@ -407,13 +431,13 @@ __global__ void __launch_bounds__(kSlabThreads)
                uint32_t* __restrict__ ticket, Welford* __restrict__ partials, uint32_t* __restrict__ error_flag) {
     const uint32_t* ytab = dirs + kSobolDims * kSobolBits;  // Y table, then the directions bit-major
     const uint32_t* by_bit = ytab + kSobolDims * 32;
-    __shared__ uint32_t s_sx[(kSlabThreads / 32) * kSxPerWarp<PREC>];
+    __shared__ uint32_t s_sx[(kSlabThreads / 32) * kSxPerWarp];
     __shared__ uint32_t s_item;
     __shared__ Welford s_warp[kSlabThreads / 32];
     __shared__ DevContract s_c;
     __shared__ DevQmc s_q;
     __shared__ QmcTables<PREC> S;
-    __shared__ float s_bridge[PREC == 0 ? 1 : 2 * kBridgeSlots * kSlabThreads];  // FP32 bridge values, per thread and path
+    __shared__ float s_bridge[PREC == 0 ? 1 : kQuad * kBridgeSlots * kSlabThreads];  // FP32 bridge values, per thread and path
     __shared__ int s_loaded;  // sorted index of the contract whose tables are in S
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
@@ -442,7 +466,7 @@ __global__ void __launch_bounds__(kSlabThreads)
                     if (threadIdx.x == 0) atomicOr(error_flag, 2u);
                     continue;
                 }
-                fill_tables<PREC>(s_c, s_q, programs, S);
+                fill_tables<PREC>(s_c, s_q, programs, by_bit, S);
             }
             if (threadIdx.x == 0) s_loaded = lo;
             __syncthreads();

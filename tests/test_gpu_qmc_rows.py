@@ -1,5 +1,5 @@
-"""GPU checks of the FP32 Sobol kernel's pairs of paths and incremental Gray-code rows
-(derivative-pricing_gb300/csrc/qmc.cu) at the edges of warps, pairs and slabs.
+"""GPU checks of the FP32 Sobol kernel's four paths per thread and incremental Gray-code
+rows (derivative-pricing_gb300/csrc/qmc.cu) at the edges of warps, CTAs and slabs.
 
 Oracle: the FP64 kernel of the same paths (tied to the reference in test_gpu_qmc.py).
 Bar per path, relative to the spot: quantile and bridge rounding through the volatility
@@ -16,7 +16,7 @@ import mcd_gpu as G
 
 pytestmark = pytest.mark.gpu
 
-PATHS = (1, 31, 32, 33, 127, 128, 129, 255, 256, 257, 4095, 4096, 4097, 4097 + 128, 12289)
+PATHS = (1, 31, 32, 33, 63, 64, 65, 96, 97, 127, 128, 129, 255, 256, 257, 511, 512, 513, 4095, 4096, 4097, 4097 + 128, 12289)
 STEPS = (1, 2, 3, 31, 32, 33, 255, 256)
 PRODUCTS = (
     dict(product=G.EUROPEAN, type=0, strike=90.0),
@@ -29,7 +29,7 @@ PRODUCTS = (
 
 
 @pytest.mark.parametrize("kw", PRODUCTS, ids=lambda k: f"{k['product']}-{k['type']}")
-def test_pairs_match_fp64(engine, kw):
+def test_rows_match_fp64(engine, kw):
     sizes = [(p, n) for p in PATHS for n in STEPS]
     arr = np.zeros(len(sizes), dtype=G.CONTRACT_DTYPE)
     for i, (p, n) in enumerate(sizes):
