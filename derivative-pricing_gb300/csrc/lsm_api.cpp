@@ -4,6 +4,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -123,9 +124,10 @@ int plan_lsm(Ctx& ctx, const mcd_lsm_contract* cs, size_t n, LsmPlan& p) {
 // regression, fitted, or (frozen) replaying the networks in frozen_nets, one
 // kParamStride block per (contract, date) row.  Frozen QR policies are
 // replayed by the streaming kernel instead (frozen_run).
+// chained: an FP64 QR batch may take the form of one cooperative launch.
 int upload_and_run(Ctx& ctx, const LsmPlan& p, int precision, bool frozen, std::vector<double>& out,
                    bool mlp = false, const std::vector<float>* frozen_nets = nullptr,
-                   const std::vector<int>* frozen_ok = nullptr) {
+                   const std::vector<int>* frozen_ok = nullptr, bool chained = true) {
     const size_t n = p.dev.size();
     const size_t elem = precision == 0 ? sizeof(double) : sizeof(float);
     if (mlp && !frozen)  // training samples paths; the bin moments of one CTA are exact up to 2^23 paths
@@ -238,13 +240,18 @@ int upload_and_run(Ctx& ctx, const LsmPlan& p, int precision, bool frozen, std::
     }
     cudaGetLastError();
     // An FP64 batch whose chunks are all resident at once walks its dates in one
-    // cooperative launch (lsm.cu).
+    // cooperative launch (lsm.cu).  One such launch at a time in the process:
+    // another thread's batch meanwhile goes date by date, with the same bits, and
+    // so does this one again if its CTAs gave up waiting for one another.
+    static std::mutex chain_lock;
+    std::unique_lock<std::mutex> chain_hold(chain_lock, std::defer_lock);
     uint32_t resident = 0;
-    if (precision == 0 && !mlp) {
+    if (precision == 0 && !mlp && chained && p.total_chunks > 0 && chain_hold.try_lock()) {
         e = lsm_chain64_capacity(ctx.sm_count, &resident);
         if (e != cudaSuccess) return ctx.cuda_fail(e, "lsm occupancy");
     }
-    const bool one_launch = p.total_chunks > 0 && p.total_chunks <= std::min(resident, kLsmChainChunks);
+    const bool one_launch = p.total_chunks <= std::min(resident, kLsmChainChunks) && resident > 0;
+    if (!one_launch && chain_hold.owns_lock()) chain_hold.unlock();
     double* d_out = static_cast<double*>(ctx.ext[kOut].ptr);
     if (one_launch) {
         e = cudaMemsetAsync(d_out + 6 * n, 0, sizeof(double), ctx.stream);
@@ -349,7 +356,10 @@ int upload_and_run(Ctx& ctx, const LsmPlan& p, int precision, bool frozen, std::
         if (e != cudaSuccess) rc = ctx.cuda_fail(e, "lsm execution");
     }
     ctx.collect_timing(false);
-    if (!rc && one_launch && out[6 * n] != 0.0) return ctx.fail(MCD_ERR_TIMEOUT, "a wait for a date's regression gave up");
+    if (!rc && one_launch && out[6 * n] != 0.0) {
+        chain_hold.unlock();
+        return upload_and_run(ctx, p, precision, frozen, out, mlp, frozen_nets, frozen_ok, false);
+    }
     if (!rc && mlp) {
         uint32_t werr = 0;
         e = cudaMemcpy(&werr, ctx.ext[kErr].ptr, sizeof werr, cudaMemcpyDeviceToHost);

@@ -8,6 +8,7 @@ the oracle's price on identical draws.
 from __future__ import annotations
 
 import ctypes as C
+import threading
 
 import numpy as np
 import pytest
@@ -46,6 +47,23 @@ def test_one_launch_has_the_bits_of_a_launch_per_date(engine):
         assert engine.lsm_batch(arr[i:i + 1], "fp64").tobytes() == batch[i:i + 1].tobytes(), ROWS[i]
     some = engine.lsm_batch(arr[:8], "fp64")  # several contracts in one launch
     assert some.tobytes() == batch[:8].tobytes()
+
+
+def test_threads_take_turns(engine):
+    """One cooperative launch at a time: the other threads' calls go date by date, same bytes."""
+    arr = _record([(40.0, 40.0, .2, 1, 20, 200 * 1024)])
+    want, bad = engine.lsm_batch(arr, "fp64").tobytes(), []
+
+    def work():
+        e = G.Engine(0)
+        bad.extend(1 for _ in range(6) if e.lsm_batch(arr, "fp64").tobytes() != want)
+
+    threads = [threading.Thread(target=work) for _ in range(3)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad
 
 
 @pytest.mark.parametrize("groups", [16, 17])  # group sums added in order, or by the warp's tree
