@@ -109,12 +109,12 @@ PATH_KERNEL_SOURCES = ("derivative-pricing_gb300/csrc/gbm_paths.cu",
                        "derivative-pricing_gb300/csrc/device_common.cuh",
                        "derivative-pricing_gb300/csrc/engine.hpp")
 PATH_KERNEL_PROFILE = {
-    "sources": "bd4a0512aa792e85",
+    "sources": "e907cc1bbe6addaf",
     "case_path_steps": 6807363601.0,
     # variant -> smsp__inst_executed.sum of one launch
-    "warp_inst": {"0": 15205895145, "1": 16932465571, "2": 19960539871, "3": 15461878018, "4": 15332180663},
+    "warp_inst": {"0": 14007048935, "1": 14022687499, "2": 14730401002, "3": 14114297334, "4": 14020495026},
     # variant -> dram__bytes_read.sum + dram__bytes_write.sum of one launch
-    "dram_bytes": {"0": 514560, "1": 525312, "2": 698880, "3": 3397120, "4": 473856},
+    "dram_bytes": {"0": 201984, "1": 253440, "2": 498944, "3": 1787392, "4": 162304},
 }
 
 

@@ -16,8 +16,8 @@
 // Measured on one GB300 against the reference's operations in FP64 (about 200
 // FP64 operations per path-step, slabs of 4096 paths as items): a
 // control-variate antithetic Asian of 1e5 paths and 252 dates 842-1035 ms ->
-// 0.335 ms per call, a European of 1e4 paths 0.55 -> 0.060 ms, a mixed book of
-// 64 contracts (1e4 to 3e5 paths, 12 to 252 dates) 750-990 -> 3.5 ms; error
+// 0.31 ms per call, a European of 1e4 paths 0.55 -> 0.026 ms, a mixed book of
+// 64 contracts (1e4 to 3e5 paths, 12 to 252 dates) 750-990 -> 3.3-3.9 ms; error
 // of the book's prices against 64-bit values 5.9e-16 -> 2.7e-16 relative.
 //
 // nvcc-flags: --fmad=false

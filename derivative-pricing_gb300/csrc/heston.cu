@@ -24,8 +24,8 @@
 // Bound: issue (72 % of the slots) and the FMA-heavy pipe (66 %), 176
 // thread-instructions per path-step.  64 sets of 64 strikes, 252 steps, 2^20
 // paths: 110 ms -> 106 with the Philox products of the draw and of the path
-// taken out of the step, 101-104 with one branch region for both paths'
-// exponential steps.
+// taken out of the step, 100-104 with one branch region for both paths'
+// exponential steps, 97.5 at 5 CTAs per SM.
 //
 // nvcc-flags: --fmad=false --ftz=true
 #include <cuda_runtime.h>
