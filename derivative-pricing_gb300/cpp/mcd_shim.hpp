@@ -9,7 +9,7 @@
 //   * functions are not noexcept: a failed GPU call throws mcd::gpu::Error
 //     (the reference has no error channel and "trusts the caller");
 //   * the arithmetic precision is a per-thread setting (mcd::gpu::set_precision,
-//     default FP64 = the reference's arithmetic on the GPU).
+//     default FP64 = the reference's draws and formulas).
 // Every call of a thread goes to one mcd_ctx created on first use (device
 // from MCD_GPU_DEVICE, default 0).
 #pragma once

@@ -14,7 +14,7 @@
 //           toggles of European and Asian price requests.
 //
 // Additions, in new fields only:
-//   "precision": "fp64" (default: the reference's arithmetic) or "fp32";
+//   "precision": "fp64" (default: the reference's formulas in FP64) or "fp32";
 //   "request": "batch"         many contracts in one launch (mcd_price_batch);
 //   "request": "batch_greeks"  price and CRN finite-difference, pathwise and
 //                              likelihood-ratio Greeks of many contracts in one

@@ -562,7 +562,7 @@ __device__ __forceinline__ double pivot_rsqrt(double d) {
 // operands, about 105; on FP32 paths a continuation value one bit off moves
 // exercise decisions (those of paths within FP32 rounding of the boundary) and
 // with them the price by 1e-5.  PREC 0: 65 (fused products, the pivots' own
-// rsqrt, gamma = T R^{-T} h), 12,400 -> 6,000 cycles from the sums to the
+// rsqrt, gamma = T R^{-T} h), 12,400 -> 9,000 cycles from the sums to the
 // coefficients; decisions there would have to tie to 1e-16.  Only the form
 // without a diagonal shift: a matrix that is not positive definite goes to the
 // serial routine.
@@ -1209,11 +1209,13 @@ __global__ void __launch_bounds__(kChunkThreads<PREC>, PREC == 0 ? 1 : 4)
 // recorded and ends the CTA.
 //
 // Bound: a date is a serial chain of products (about 8,000 cycles, the FP64
-// pipe), the CTA's and the contract's folds (9,000), the solve (6,000), two
+// pipe), the CTA's and the contract's folds (9,000), the solve (9,000), two
 // trips through L2 and the exercise tests (5,000).  A put of 131,072 paths and
-// 50 dates: 37 -> 17 us a date, the call 1.92 -> 1.0 ms.  Two CTAs fit an SM,
-// so batches of up to 304 chunks come here; larger ones go date by date, where
-// the chunks of one date fill the GPU and the launches' share is small.
+// 50 dates: 37 -> 17 us a date, the call 1.92 -> 1.0 ms.  Two CTAs fit an SM, so
+// batches of up to 304 chunks come here.  Puts of 50 dates, one launch against a
+// launch per date, ms: one of 5,000 paths 1.10 and 1.53, of 131,072 1.13 and
+// 1.69, of 311,296 1.81 and 2.36; five of 51,200 1.65 and 2.10; a hundred of
+// 3,072 1.65 and 2.22; 300 of 1,000 1.60 and 2.27.
 constexpr int kChainSlots = 5;  // s and the four basis values of a packed path
 struct ChainWarp {
     double f[2][kChainSlots][kWarpPaths];  // packed paths of this date and of the next

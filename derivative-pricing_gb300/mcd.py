@@ -185,7 +185,7 @@ def _engine() -> _Lease:
 
 
 def set_precision(precision: str) -> None:
-    """"fp64" (default, the reference's arithmetic) or "fp32" for this thread."""
+    """"fp64" (default, the reference's draws and formulas in FP64) or "fp32" for this thread."""
     if precision not in ("fp64", "fp32"):
         raise ValueError("precision must be 'fp64' or 'fp32'")
     _tls.precision = precision

@@ -3,7 +3,7 @@
 Function names and argument order follow the reference's Python module
 (bindings/python/src/module.cpp:64-293: ``monte_carlo_european``,
 ``monte_carlo_asian``, ...), with one extra keyword, ``precision`` ("fp64" for
-the reference's arithmetic on the GPU, "fp32" for FP32 paths with FP64
+the reference's draws and formulas in FP64, "fp32" for FP32 paths with FP64
 accumulation).  Every call goes to the GPU: there is no CPU fallback, and
 loading fails loudly when the library has not been built.
 """

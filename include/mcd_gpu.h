@@ -148,7 +148,7 @@ int mcd_price_lookback(mcd_ctx* ctx, double spot, double strike, double rate, do
                        uint64_t path_count, uint64_t seed, const mcd_mc_options* options,
                        int precision, mcd_mc_result* out);
 
-/* ---- batched pricing: one persistent-kernel launch in a CUDA graph ------ */
+/* ---- batched pricing: one persistent-kernel launch ----------------------- */
 /* Host arrays in and out (copies included).  Equivalent to calling the
  * reference pricer once per contract (monte_carlo.cpp:233-338). */
 int mcd_price_batch(mcd_ctx* ctx, const mcd_contract* contracts, size_t n, int precision,
@@ -272,7 +272,7 @@ int mcd_lsm_reprice_frozen(mcd_ctx* ctx, double spot, double strike, double rate
                            int monitoring_points, uint64_t path_count, uint64_t seed,
                            const double* coefficients, const uint8_t* has_coefficients,
                            int exercise_at_inception, int precision, double* price);
-/* Many American contracts (uneven date counts allowed) in one graph launch:
+/* Many American contracts (uneven date counts allowed) in one call:
  * all paths stay resident and the contracts step back in lockstep. */
 int mcd_lsm_batch(mcd_ctx* ctx, const mcd_lsm_contract* contracts, size_t n, int precision,
                   int regression, mcd_lsm_result* results);
