@@ -109,12 +109,12 @@ PATH_KERNEL_SOURCES = ("derivative-pricing_gb300/csrc/gbm_paths.cu",
                        "derivative-pricing_gb300/csrc/device_common.cuh",
                        "derivative-pricing_gb300/csrc/engine.hpp")
 PATH_KERNEL_PROFILE = {
-    "sources": "e907cc1bbe6addaf",
+    "sources": "b03e871022c03809",
     "case_path_steps": 6807363601.0,
     # variant -> smsp__inst_executed.sum of one launch
-    "warp_inst": {"0": 14007048935, "1": 14022687499, "2": 14730401002, "3": 14114297334, "4": 14020495026},
+    "warp_inst": {"0": 14013227156, "1": 14030631398, "2": 14732996643, "3": 14156821798, "4": 14019151174},
     # variant -> dram__bytes_read.sum + dram__bytes_write.sum of one launch
-    "dram_bytes": {"0": 201984, "1": 253440, "2": 498944, "3": 1787392, "4": 162304},
+    "dram_bytes": {"0": 608768, "1": 314112, "2": 746240, "3": 840448, "4": 460288},
 }
 
 

@@ -123,7 +123,7 @@ extern "C" int mcd_price_batch_static(const mcd_contract* contracts, size_t n, i
     if (rc != MCD_OK || n == 0) return rc;
 
     uint64_t total = 0;   // slabs, the limit's unit
-    uint32_t items = 0;   // slabs (FP32) or units (FP64) so far, modulo 2^32
+    uint32_t items = 0;   // items (FP32) or units (FP64) so far, modulo 2^32
     for (size_t i = 0; i < n; ++i) {
         const char* why = mcdg::convert_contract(contracts[i], static_cast<uint32_t>(i), g_stage_contracts[i]);
         if (why) {
@@ -132,7 +132,7 @@ extern "C" int mcd_price_batch_static(const mcd_contract* contracts, size_t n, i
             return report(error_message, error_capacity, MCD_ERR_INVALID_ARGUMENT, text);
         }
         g_stage_prefix[i] = items;
-        items += precision == MCD_PRECISION_FP64 ? g_stage_contracts[i].n_units : g_stage_contracts[i].n_slabs;
+        items += precision == MCD_PRECISION_FP64 ? g_stage_contracts[i].n_units : g_stage_contracts[i].n_items;
         total += g_stage_contracts[i].n_slabs;
         if (total > kStaticMaxSlabs)
             return report(error_message, error_capacity, MCD_ERR_INVALID_ARGUMENT,
@@ -155,10 +155,10 @@ extern "C" int mcd_price_batch_static(const mcd_contract* contracts, size_t n, i
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(d_prefix, g_stage_prefix, sizeof(uint32_t) * (n + 1), cudaMemcpyHostToDevice, s);
     if (e != cudaSuccess) return report_cuda(error_message, error_capacity, e, "stage contracts");
-    // Contracts in ranges whose items fit the partials: all at once in FP32
-    // (the slab limit); FP64 units are smaller than slabs (at most 4096 per
-    // contract below 2^23 paths, slabs above), so a large FP64 batch takes
-    // several launches on the same scratch.
+    // Contracts in ranges whose items fit the partials: FP32 items (at most 64 or
+    // the slabs of a contract) and FP64 units (at most 4096 per contract below
+    // 2^23 paths, slabs above) are smaller than slabs, so a large batch of
+    // small contracts takes several launches on the same scratch.
     for (size_t first = 0; first < n;) {
         size_t end = first + 1;
         while (end < n && g_stage_prefix[end + 1] - g_stage_prefix[first] <= kStaticMaxSlabs) ++end;

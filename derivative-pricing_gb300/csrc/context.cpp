@@ -244,6 +244,22 @@ const char* convert_contract(const mcd_contract& in, uint32_t index, DevContract
     while (out.unit_log < 7 && (in.path_count >> (17 + out.unit_log)) != 0) ++out.unit_log;
     const uint64_t unit = 32ull << out.unit_log;
     out.n_units = static_cast<uint32_t>((in.path_count + unit - 1) / unit);
+    // FP32 items: a CTA's 4096 paths, halved while the contract has at most 256
+    // items of the half and those still hold 131,072 path-steps.  A small book's
+    // time is that of its longest item (4096 paths of 252 dates: 1.9 ms in a CTA
+    // by itself); contracts of more than 2^20 paths keep whole slabs.  Books of
+    // 3, 10, 30, 100, 300, 1000, 4096 contracts of 1e3 to 3e5 paths, ms, whole
+    // slabs against items: priced 1.11, 1.18, 1.78, 2.47, 4.35, 11.7, 54.4 and
+    // 0.72, 0.50, 0.85, 1.46, 4.12, 11.8, 54.7; sensitivities 2.72, 2.85, 3.34,
+    // 4.35, 7.75, 20.8, 93.4 and 1.60, 1.07, 1.52, 2.44, 7.43, 20.4, 91.6.
+    out.item_log = 5;
+    while (out.item_log > 1) {
+        const uint64_t half = 64ull << out.item_log;
+        if (in.path_count > 256 * half || half * static_cast<uint64_t>(out.n_steps) < 131072) break;
+        --out.item_log;
+    }
+    const uint64_t item = 128ull << out.item_log;
+    out.n_items = static_cast<uint32_t>((in.path_count + item - 1) / item);
     out.inv_n = 1.0 / static_cast<double>(out.n_steps);
     fixed_scale(out);
     return nullptr;
@@ -264,19 +280,17 @@ double slab_cost(const DevContract& c) {
     return static_cast<double>(c.n_steps) * per_step * (c.antithetic ? 2.0 : 1.0);
 }
 
-// range_items: 0 for slab items, else the items are FP64 units (the pricer and
-// the Greeks in FP64), at most range_items of them in a range.
-int plan_batch(Ctx& ctx, const mcd_contract* contracts, size_t n, uint64_t range_items, BatchPlan& plan) {
-    const bool units = range_items != 0;
+// range_items: at most that many items in a range (slabs: one range).
+int plan_batch(Ctx& ctx, const mcd_contract* contracts, size_t n, Items kind, uint64_t range_items, BatchPlan& plan) {
     if (n > 0x7FFFFFFF) return ctx.fail(MCD_ERR_INVALID_ARGUMENT, "too many contracts");
     plan.dev.resize(n);
     for (size_t i = 0; i < n; ++i) {
         const int rc = plan_contract(ctx, contracts[i], static_cast<uint32_t>(i), plan.dev[i]);
         if (rc != MCD_OK) return rc;
     }
-    std::stable_sort(plan.dev.begin(), plan.dev.end(), [](const DevContract& a, const DevContract& b) {
-        return slab_cost(a) > slab_cost(b);
-    });
+    auto cost = [&](const DevContract& c) { return slab_cost(c) * (kind == Items::kItems32 ? 1 << c.item_log : 1); };
+    std::stable_sort(plan.dev.begin(), plan.dev.end(),
+                     [&](const DevContract& a, const DevContract& b) { return cost(a) > cost(b); });
     // The prefix counts items modulo 2^32: kernels use differences within a
     // range of contracts, and every range holds at most range_items units (or
     // one contract), so that the partials of a batch of many small contracts
@@ -287,11 +301,12 @@ int plan_batch(Ctx& ctx, const mcd_contract* contracts, size_t n, uint64_t range
     uint32_t items = 0;
     plan.max_items = 0;
     for (size_t i = 0; i < n; ++i) {
-        const uint32_t more = units ? plan.dev[i].n_units : plan.dev[i].n_slabs;
+        const DevContract& c = plan.dev[i];
+        const uint32_t more = kind == Items::kUnits64 ? c.n_units : kind == Items::kItems32 ? c.n_items : c.n_slabs;
         plan.prefix[i] = items;
         slabs += plan.dev[i].n_slabs;
         if (slabs > 0xFFFFFFF0ull) return ctx.fail(MCD_ERR_INVALID_ARGUMENT, "batch too large");
-        if (units && in_range > 0 && in_range + more > range_items) {
+        if (kind != Items::kSlabs && in_range > 0 && in_range + more > range_items) {
             plan.ranges.push_back(static_cast<uint32_t>(i));
             in_range = 0;
         }
@@ -485,7 +500,7 @@ int price_quote(Ctx& ctx, const DevContract& c, mcd_mc_result* result) {
 int price_batch_host(Ctx& ctx, const mcd_contract* contracts, size_t n, int precision,
                      mcd_mc_result* results) {
     BatchPlan& plan = ctx.host_plan;
-    int rc = plan_batch(ctx, contracts, n, precision == 0 ? kRangeItems : 0, plan);
+    int rc = plan_batch(ctx, contracts, n, precision == 0 ? Items::kUnits64 : Items::kItems32, kRangeItems, plan);
     if (rc) return rc;
     if (n == 0) return MCD_OK;
     const DevContract& c0 = plan.dev[0];
@@ -659,7 +674,7 @@ int mcd_price_batch_device(mcd_ctx* handle, const mcd_contract* contracts, size_
         e = cudaMemcpyAsync(host.data(), contracts, sizeof(mcd_contract) * n, cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
         if (e != cudaSuccess) return ctx->cuda_fail(e, "read device contracts");
-        int rc = plan_batch(*ctx, host.data(), n, precision == 0 ? kRangeItems : 0, ctx->device_plan);
+        int rc = plan_batch(*ctx, host.data(), n, precision == 0 ? Items::kUnits64 : Items::kItems32, kRangeItems, ctx->device_plan);
         if (rc) return rc;
         rc = upload_plan(*ctx, ctx->device_plan);
         if (rc) return rc;
@@ -712,7 +727,7 @@ int mcd_autotune(mcd_ctx* handle, const mcd_contract* contracts, size_t n, int p
     if (precision != 0 && precision != 1) return ctx->fail(MCD_ERR_INVALID_ARGUMENT, "bad precision");
     if (n == 0 || !contracts) return ctx->fail(MCD_ERR_INVALID_ARGUMENT, "empty tuning batch");
     BatchPlan plan;
-    int rc = plan_batch(*ctx, contracts, n, precision == 0 ? kRangeItems : 0, plan);
+    int rc = plan_batch(*ctx, contracts, n, precision == 0 ? Items::kUnits64 : Items::kItems32, kRangeItems, plan);
     if (rc) return rc;
     rc = upload_plan(*ctx, plan);
     if (rc) return rc;

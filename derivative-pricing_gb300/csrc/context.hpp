@@ -138,7 +138,9 @@ int plan_contract(Ctx& ctx, const mcd_contract& in, uint32_t index, DevContract&
 int fixed_frac(int n_steps, double drift, double vs);
 void fixed_step(double drift, double vs, int frac, int64_t* hi, uint32_t* lo, uint64_t* scale);
 int64_t fixed_barrier(double log_rel, int frac);
-int plan_batch(Ctx& ctx, const mcd_contract* contracts, size_t n, uint64_t range_items, BatchPlan& plan);
+// What a batch's items are: slabs (Sobol), FP64 units, FP32 items.
+enum class Items { kSlabs, kUnits64, kItems32 };
+int plan_batch(Ctx& ctx, const mcd_contract* contracts, size_t n, Items kind, uint64_t range_items, BatchPlan& plan);
 int price_batch_host(Ctx& ctx, const mcd_contract* contracts, size_t n, int precision,
                      mcd_mc_result* results);
 

@@ -71,6 +71,9 @@ struct DevContract {
     // contract is outside the fixed-point range.
     uint32_t n_units;
     int32_t unit_log, frac;
+    // FP32 paths (gbm_paths.cu, greeks.cu): items of 128 << item_log paths.
+    int32_t item_log;
+    uint32_t n_items;
     uint32_t y_drift_lo;   // drift / ln 2 = (y_drift + y_drift_lo 2^-32) 2^-frac
     int64_t y_drift;
     uint64_t y_vs;         // vs / ln 2, 2^(frac + 3)
@@ -88,7 +91,7 @@ const char* convert_contract(const mcd_contract& in, uint32_t index, DevContract
 // The persistent path kernel over items [0, item_prefix[n_contracts]) (the
 // item count is read on the device, so one captured launch serves every path
 // count of the same number of contracts).
-// Items are slabs of kSlabPaths paths in FP32 and units of 32 << unit_log paths
+// Items are 128 << item_log paths in FP32 and units of 32 << unit_log paths
 // in FP64; `tables` (fixed_tables_device) is for FP64.
 cudaError_t launch_path_kernel(int precision, int variant, int grid, const DevContract* contracts,
                                int n_contracts, const uint32_t* item_prefix, uint32_t* ticket,

@@ -2,12 +2,12 @@
 // barrier, lookback) in FP32 as one persistent kernel, and the merge of both
 // precisions (the FP64 paths are gbm_paths64.cu).
 //
-// Work decomposition.  Every contract's paths are cut into fixed slabs of
-// kSlabPaths = 4096 paths; one (contract, slab) pair is one work item.  The
+// Work decomposition.  Every contract's paths are cut into items of 128 << item_log
+// paths, 4096 or fewer (convert_contract); one (contract, item) pair is one work item.  The
 // host orders contracts longest-first and passes the running item count per
 // contract (item_prefix).  A CTA of 128 threads claims items from a ticket
 // counter (one atomicAdd per item, no waiting) until the list is exhausted.
-// Inside a slab, thread t simulates paths slab*4096 + j*128 + t for
+// Inside an item, thread t simulates paths base + j*128 + t for
 // j = 0..31, so the Philox counters of a warp are consecutive path indices.
 //
 // Determinism.  A slab's Welford triple depends only on the slab: per-thread
@@ -161,11 +161,13 @@ __device__ __forceinline__ double terminal32(const DevContract& c, uint32_t bits
     return c.discount * static_cast<double>(payoff);
 }
 
-// A warp's share of a slab (valid in lane 0); table: the CTA's step table.
+// A warp's share of an item (valid in lane 0), from path base on, `rounds` paths
+// per thread; table: the CTA's step table.
 // Every thread runs every round (the table's refills are CTA barriers); a path
 // past the contract's last one is simulated or skipped, and not counted.
 template <int KIND>
-__device__ Welford slab32(const DevContract& c, const PhiloxKeys& k, PhiloxStep* table, uint64_t base) {
+__device__ Welford slab32(const DevContract& c, const PhiloxKeys& k, PhiloxStep* table, const uint64_t& base,
+                          const int& rounds) {
     unsigned count = 0;
     UnitSums acc;
     auto add = [&](double v) {
@@ -173,8 +175,6 @@ __device__ Welford slab32(const DevContract& c, const PhiloxKeys& k, PhiloxStep*
         acc.add(v);
     };
     const uint32_t path_hi = static_cast<uint32_t>(base >> 32);  // a slab is aligned to its size
-    const uint64_t left = c.path_count - base;
-    const int rounds = left >= kSlabPaths ? kPathsPerThread : static_cast<int>((left + kSlabThreads - 1) / kSlabThreads);
     if constexpr (KIND == kEuropean || KIND == kDigital) {
         const PhiloxStep st = philox_step(0u, path_hi, k);
         for (int j = 0; j < rounds; ++j) {
@@ -228,18 +228,18 @@ __device__ Welford slab32(const DevContract& c, const PhiloxKeys& k, PhiloxStep*
     return acc.reduce(__reduce_add_sync(0xffffffffu, count));
 }
 
-__device__ Welford run_slab(const DevContract& c, PhiloxStep* table, uint64_t base) {
+__device__ Welford run_slab(const DevContract& c, PhiloxStep* table, const uint64_t& base, const int& rounds) {
     const PhiloxKeys k = philox_keys(c.seed);
     switch (c.kind) {
-        case kEuropean: return slab32<kEuropean>(c, k, table, base);
-        case kDigital: return slab32<kDigital>(c, k, table, base);
-        case kAsianArith: return slab32<kAsianArith>(c, k, table, base);
-        case kAsianGeo: return slab32<kAsianGeo>(c, k, table, base);
-        case kAsianCv: return slab32<kAsianCv>(c, k, table, base);
-        case kBarrier: return slab32<kBarrier>(c, k, table, base);
-        case kBarrierBridge: return slab32<kBarrierBridge>(c, k, table, base);
-        case kLookbackFixed: return slab32<kLookbackFixed>(c, k, table, base);
-        default: return slab32<kLookbackFloating>(c, k, table, base);
+        case kEuropean: return slab32<kEuropean>(c, k, table, base, rounds);
+        case kDigital: return slab32<kDigital>(c, k, table, base, rounds);
+        case kAsianArith: return slab32<kAsianArith>(c, k, table, base, rounds);
+        case kAsianGeo: return slab32<kAsianGeo>(c, k, table, base, rounds);
+        case kAsianCv: return slab32<kAsianCv>(c, k, table, base, rounds);
+        case kBarrier: return slab32<kBarrier>(c, k, table, base, rounds);
+        case kBarrierBridge: return slab32<kBarrierBridge>(c, k, table, base, rounds);
+        case kLookbackFixed: return slab32<kLookbackFixed>(c, k, table, base, rounds);
+        default: return slab32<kLookbackFloating>(c, k, table, base, rounds);
     }
 }
 
@@ -249,14 +249,20 @@ __global__ void __launch_bounds__(kSlabThreads, MINB)
                 const uint32_t* __restrict__ item_prefix, uint32_t* __restrict__ ticket,
                 Welford* __restrict__ partials, uint32_t* __restrict__ error_flag) {
     __shared__ uint32_t s_item, s_total;
+    // an item's first path and its paths per thread: in registers they cost the
+    // step loop 1.5 % (72 registers instead of 68)
+    __shared__ uint64_t s_base;
+    __shared__ int s_rounds;
     __shared__ Welford s_warp[kSlabThreads / 32];
     __shared__ DevContract s_contract;
     __shared__ PhiloxStep s_step[kStepTable];
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
-    // The batch's item count is the prefix's last entry (read from memory, so
-    // a captured launch serves every path count of the same contract count).
-    if (threadIdx.x == 0) s_total = item_prefix[n_contracts];
+    // The batch's items are read from the prefix (modulo 2^32, from its first
+    // entry on), so a captured launch serves every path count of the same
+    // contract count.
+    const uint32_t first = item_prefix[0];
+    if (threadIdx.x == 0) s_total = item_prefix[n_contracts] - first;
     for (;;) {
         if (threadIdx.x == 0) s_item = atomicAdd(ticket, 1u);
         __syncthreads();
@@ -267,7 +273,7 @@ __global__ void __launch_bounds__(kSlabThreads, MINB)
         int lo = 0, hi = n_contracts;
         while (hi - lo > 1) {
             const int mid = (lo + hi) >> 1;
-            if (item_prefix[mid] <= item) lo = mid; else hi = mid;
+            if (item_prefix[mid] - first <= item) lo = mid; else hi = mid;
         }
         static_assert(sizeof(DevContract) % 4 == 0 && sizeof(DevContract) / 4 <= kSlabThreads,
                       "contract staging assumes one word per thread");
@@ -276,19 +282,22 @@ __global__ void __launch_bounds__(kSlabThreads, MINB)
                 reinterpret_cast<const uint32_t*>(&contracts[lo])[threadIdx.x];
         __syncthreads();
         const DevContract& c = s_contract;
-        const uint32_t slab = item - item_prefix[lo];
-        if (slab >= c.n_slabs) {  // planning invariant broken: record, skip the item
+        const uint32_t slab = item - (item_prefix[lo] - first);
+        if (slab >= c.n_items) {  // planning invariant broken: record, skip the item
             if (threadIdx.x == 0) atomicOr(error_flag, 1u);
             __syncthreads();
             continue;
         }
-        const Welford w = run_slab(c, s_step, static_cast<uint64_t>(slab) * kSlabPaths);
+        if (threadIdx.x == 0) {
+            s_base = static_cast<uint64_t>(slab) * kSlabThreads << c.item_log;
+            const uint64_t left = c.path_count - s_base, size = static_cast<uint64_t>(kSlabThreads) << c.item_log;
+            s_rounds = static_cast<int>(((left < size ? left : size) + kSlabThreads - 1) / kSlabThreads);
+        }
+        __syncthreads();
+        const Welford w = run_slab(c, s_step, s_base, s_rounds);
         if (lane == 0) s_warp[warp] = w;
         __syncthreads();
-        if (threadIdx.x == 0) {
-            partials[item] = welford_merge(welford_merge(s_warp[0], s_warp[1]),
-                                           welford_merge(s_warp[2], s_warp[3]));
-        }
+        if (threadIdx.x == 0) partials[item] = merge_warps(s_warp[0], s_warp[1], s_warp[2], s_warp[3]);
         __syncthreads();
     }
 }

@@ -341,7 +341,8 @@ __device__ void slab_greeks(const DevContract& c, const DevGreeks& g, const Phil
                             uint64_t base, double (*acc)[kNumGreeks][kSlabThreads], double* pivot, Welford* out) {
     const int t = threadIdx.x, lane = t & 31;
     const uint64_t left = c.path_count - base;
-    const int rounds = left >= kSlabPaths ? kPathsPerThread : static_cast<int>((left + kSlabThreads - 1) / kSlabThreads);
+    const uint64_t size = static_cast<uint64_t>(kSlabThreads) << c.item_log;
+    const int rounds = static_cast<int>(((left < size ? left : size) + kSlabThreads - 1) / kSlabThreads);
     unsigned count = 0;
     for (int j = 0; j < rounds; ++j) {
         const uint64_t path = base + static_cast<uint64_t>(j * kSlabThreads) + t;
@@ -397,8 +398,8 @@ __device__ void run_greeks_slab(const DevContract& c, const DevGreeks& g, Philox
 template <int MINB>
 __global__ void __launch_bounds__(kSlabThreads, MINB)
     greeks_kernel(const DevContract* __restrict__ contracts, const DevGreeks* __restrict__ greeks, int n_contracts,
-                  const uint32_t* __restrict__ item_prefix, uint32_t total_items, uint32_t* __restrict__ ticket,
-                  Welford* __restrict__ partials, uint32_t* __restrict__ error_flag) {
+                  const uint32_t* __restrict__ item_prefix, uint32_t* __restrict__ ticket, Welford* __restrict__ partials,
+                  uint32_t* __restrict__ error_flag) {
     __shared__ uint32_t s_item;
     __shared__ DevContract s_contract;
     __shared__ DevGreeks s_greeks;
@@ -414,35 +415,36 @@ __global__ void __launch_bounds__(kSlabThreads, MINB)
     static_assert(sizeof(DevContract) % 4 == 0 && sizeof(DevGreeks) % 4 == 0 &&
                       (sizeof(DevContract) + sizeof(DevGreeks)) / 4 <= 2 * kSlabThreads,
                   "contract staging assumes at most two words per thread");
+    const uint32_t first = item_prefix[0], total = item_prefix[n_contracts] - first;
     for (;;) {
         if (threadIdx.x == 0) s_item = atomicAdd(ticket, 1u);
         __syncthreads();
         const uint32_t item = s_item;
-        if (item >= total_items) return;
+        if (item >= total) return;
         int lo = 0, hi = n_contracts;
         while (hi - lo > 1) {
             const int mid = (lo + hi) >> 1;
-            if (item_prefix[mid] <= item) lo = mid; else hi = mid;
+            if (item_prefix[mid] - first <= item) lo = mid; else hi = mid;
         }
         for (int i = threadIdx.x; i < static_cast<int>(sizeof(DevContract) / 4); i += kSlabThreads)
             reinterpret_cast<uint32_t*>(&s_contract)[i] = reinterpret_cast<const uint32_t*>(&contracts[lo])[i];
         for (int i = threadIdx.x; i < static_cast<int>(sizeof(DevGreeks) / 4); i += kSlabThreads)
             reinterpret_cast<uint32_t*>(&s_greeks)[i] = reinterpret_cast<const uint32_t*>(&greeks[lo])[i];
         __syncthreads();
-        const uint32_t slab = item - item_prefix[lo];
-        if (slab >= s_contract.n_slabs) {
+        const uint32_t slab = item - (item_prefix[lo] - first);
+        if (slab >= s_contract.n_items) {
             if (threadIdx.x == 0) atomicOr(error_flag, 1u);
             __syncthreads();
             continue;
         }
-        run_greeks_slab(s_contract, s_greeks, s_warp[warp].step, static_cast<uint64_t>(slab) * kSlabPaths, s_acc,
+        run_greeks_slab(s_contract, s_greeks, s_warp[warp].step,
+                        static_cast<uint64_t>(slab) * kSlabThreads << s_contract.item_log, s_acc,
                         s_pivot[warp], s_warp[warp].triple);
         __syncthreads();
         if (threadIdx.x < kNumGreeks) {
             const int i = threadIdx.x;
             partials[static_cast<size_t>(item) * kNumGreeks + i] =
-                welford_merge(welford_merge(s_warp[0].triple[i], s_warp[1].triple[i]),
-                              welford_merge(s_warp[2].triple[i], s_warp[3].triple[i]));
+                merge_warps(s_warp[0].triple[i], s_warp[1].triple[i], s_warp[2].triple[i], s_warp[3].triple[i]);
         }
         __syncthreads();
     }
@@ -466,9 +468,9 @@ __global__ void __launch_bounds__(kMergeThreads)
 
 template <int MINB>
 cudaError_t launch_one(int grid, const DevContract* c, const DevGreeks* g, int n, const uint32_t* prefix,
-                       uint32_t total, uint32_t* ticket, Welford* partials, uint32_t* err, cudaStream_t stream) {
+                       uint32_t* ticket, Welford* partials, uint32_t* err, cudaStream_t stream) {
     cudaGetLastError();
-    greeks_kernel<MINB><<<grid, kSlabThreads, 0, stream>>>(c, g, n, prefix, total, ticket, partials, err);
+    greeks_kernel<MINB><<<grid, kSlabThreads, 0, stream>>>(c, g, n, prefix, ticket, partials, err);
     return cudaGetLastError();
 }
 
@@ -476,12 +478,12 @@ cudaError_t launch_one(int grid, const DevContract* c, const DevGreeks* g, int n
 
 cudaError_t launch_greeks_kernel(int precision, int variant, int grid, const DevContract* contracts,
                                  const DevGreeks* greeks, int n_contracts, const uint32_t* item_prefix,
-                                 uint32_t total_items, uint32_t* ticket, Welford* partials,
-                                 uint32_t* error_flag, const FixedTables* tables, cudaStream_t stream) {
+                                 uint32_t* ticket, Welford* partials, uint32_t* error_flag,
+                                 const FixedTables* tables, cudaStream_t stream) {
     if (precision == 0)
         return launch_greeks64_kernel(grid, contracts, greeks, n_contracts, item_prefix, ticket, partials, error_flag,
                                       tables, stream);
-#define MCD_GREEKS_ARGS grid, contracts, greeks, n_contracts, item_prefix, total_items, ticket, partials, error_flag, stream
+#define MCD_GREEKS_ARGS grid, contracts, greeks, n_contracts, item_prefix, ticket, partials, error_flag, stream
     switch (variant) {
         case 0: return launch_one<2>(MCD_GREEKS_ARGS);
         case 1: return launch_one<4>(MCD_GREEKS_ARGS);

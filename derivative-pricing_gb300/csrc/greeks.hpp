@@ -56,7 +56,7 @@ struct DevGreeks {
 
 cudaError_t launch_greeks_kernel(int precision, int variant, int grid, const DevContract* contracts,
                                  const DevGreeks* greeks, int n_contracts, const uint32_t* item_prefix,
-                                 uint32_t total_items, uint32_t* ticket, Welford* partials,
+                                 uint32_t* ticket, Welford* partials,
                                  uint32_t* error_flag, const FixedTables* tables, cudaStream_t stream);
 cudaError_t launch_greeks64_kernel(int grid, const DevContract* contracts, const DevGreeks* greeks, int n_contracts,
                                    const uint32_t* item_prefix, uint32_t* ticket, Welford* partials,

@@ -45,7 +45,7 @@ int plan_greeks(Ctx& ctx, const mcd_contract* cs, size_t n, int precision, doubl
         if (c.product == MCD_PRODUCT_BARRIER && c.brownian_bridge)
             return ctx.fail(MCD_ERR_UNSUPPORTED, "contract " + std::to_string(i) + ": no Greeks for the Brownian-bridge barrier");
     }
-    int rc = plan_batch(ctx, cs, n, precision == 0 ? kGreeksRangeItems : 0, plan);
+    int rc = plan_batch(ctx, cs, n, precision == 0 ? Items::kUnits64 : Items::kItems32, kGreeksRangeItems, plan);
     if (rc) return rc;
     consts.resize(n);
     for (size_t j = 0; j < n; ++j) {
@@ -142,7 +142,7 @@ int prepare_greeks(Ctx& ctx, int precision, const BatchPlan& plan, const std::ve
     int variant = 0, grid = 0;
     rc = greeks_grid(ctx, precision, variant, grid);
     if (rc) return rc;
-    const GraphKey key{precision, variant, grid, n, plan.max_items, ctx.ext[kGDev].ptr, ctx.ext[kGPrefix].ptr,
+    const GraphKey key{precision, variant, grid, n, 0u, ctx.ext[kGDev].ptr, ctx.ext[kGPrefix].ptr,
                        ctx.ext[kGPart].ptr, ctx.ext[kGOut].ptr};
     if (ctx.greeks_graph && ctx.greeks_key == key && plan.ranges.size() == 2) {
         *out = ctx.greeks_graph;
@@ -167,8 +167,8 @@ int prepare_greeks(Ctx& ctx, int precision, const BatchPlan& plan, const std::ve
         el = cudaMemsetAsync(flags, 0, (r == 0 ? 2 : 1) * sizeof(uint32_t), ctx.stream);
         if (el == cudaSuccess)
             el = launch_greeks_kernel(precision, variant, grid, dev,
-                                      static_cast<const DevGreeks*>(ctx.ext[kGConst].ptr) + first, count, prefix,
-                                      plan.max_items, flags, partials, flags + 1, ctx.tables, ctx.stream);
+                                      static_cast<const DevGreeks*>(ctx.ext[kGConst].ptr) + first, count, prefix, flags,
+                                      partials, flags + 1, ctx.tables, ctx.stream);
         if (el == cudaSuccess)
             el = launch_greeks_merge(dev, count, prefix, partials, static_cast<double*>(ctx.ext[kGOut].ptr), ctx.stream);
     }

@@ -163,7 +163,7 @@ int plan_qmc(Ctx& ctx, const mcd_contract* cs, size_t n, BatchPlan& plan, std::v
         if (c.product >= MCD_PRODUCT_ASIAN && c.monitoring_points > kSobolDims)
             return ctx.fail(MCD_ERR_INVALID_ARGUMENT, who + "monitoring_points must be <= MCD_SOBOL_MAX_DIMS (256)");
     }
-    int rc = plan_batch(ctx, cs, n, 0, plan);
+    int rc = plan_batch(ctx, cs, n, Items::kSlabs, 0, plan);
     if (rc) return rc;
     std::map<int, uint32_t> offset_of;
     programs.clear();

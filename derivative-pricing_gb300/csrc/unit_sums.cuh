@@ -7,6 +7,7 @@
 
 #include <cuda_runtime.h>
 
+#include "device_common.cuh"
 #include "engine.hpp"
 
 namespace mcdg {
@@ -21,6 +22,20 @@ __device__ __forceinline__ Welford unit_triple(uint32_t count, double pivot, dou
     const double m = pow2 ? a * inv : a / static_cast<double>(count);
     const double m2 = fma(-a, m, b);
     return Welford{count, pivot + m, m2 > 0.0 ? m2 : 0.0};
+}
+
+// The triples of a CTA's four warps.  Whole items have a power of two of samples
+// in every warp: the mean of the means and one term of the between-warps
+// variance each, 18 FP64 operations; a chain of three Welford merges takes
+// about 120 (three divisions), by one thread while its CTA waits.
+__device__ __forceinline__ Welford merge_warps(const Welford& a, const Welford& b, const Welford& c, const Welford& d) {
+    if (a.count != b.count || a.count != c.count || a.count != d.count || a.count == 0)
+        return welford_merge(welford_merge(a, b), welford_merge(c, d));
+    const double mean = 0.25 * ((a.mean + b.mean) + (c.mean + d.mean));
+    const double da = a.mean - mean, db = b.mean - mean, dc = c.mean - mean, dd = d.mean - mean;
+    const double between = fma(da, da, fma(db, db, fma(dc, dc, dd * dd)));
+    return Welford{4 * a.count, mean,
+                   fma(static_cast<double>(static_cast<uint32_t>(a.count)), between, (a.m2 + b.m2) + (c.m2 + d.m2))};
 }
 
 // One output.  first() once, by all lanes, with lane 0's sample valid (or no
