@@ -109,12 +109,12 @@ PATH_KERNEL_SOURCES = ("derivative-pricing_gb300/csrc/gbm_paths.cu",
                        "derivative-pricing_gb300/csrc/device_common.cuh",
                        "derivative-pricing_gb300/csrc/engine.hpp")
 PATH_KERNEL_PROFILE = {
-    "sources": "b03e871022c03809",
+    "sources": "f02428902a30f0ab",
     "case_path_steps": 6807363601.0,
     # variant -> smsp__inst_executed.sum of one launch
     "warp_inst": {"0": 14013227156, "1": 14030631398, "2": 14732996643, "3": 14156821798, "4": 14019151174},
     # variant -> dram__bytes_read.sum + dram__bytes_write.sum of one launch
-    "dram_bytes": {"0": 608768, "1": 314112, "2": 746240, "3": 840448, "4": 460288},
+    "dram_bytes": {"0": 357632, "1": 541184, "2": 420864, "3": 885760, "4": 202496},
 }
 
 

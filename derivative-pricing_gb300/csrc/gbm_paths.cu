@@ -7,12 +7,12 @@
 // host orders contracts longest-first and passes the running item count per
 // contract (item_prefix).  A CTA of 128 threads claims items from a ticket
 // counter (one atomicAdd per item, no waiting) until the list is exhausted.
-// Inside an item, thread t simulates paths base + j*128 + t for
-// j = 0..31, so the Philox counters of a warp are consecutive path indices.
+// Inside an item, thread t simulates paths base + j*128 + t for j = 0, 1, ...,
+// so the Philox counters of a warp are consecutive path indices.
 //
-// Determinism.  A slab's Welford triple depends only on the slab: per-thread
+// Determinism.  An item's Welford triple depends only on the item: per-thread
 // shifted sums in j order (unit_sums.cuh), then a fixed warp shuffle tree and a
-// fixed 4-warp tree.  The merge kernel folds a contract's slabs in a fixed tree (merge.cuh).
+// fixed 4-warp tree.  The merge kernel folds a contract's items in a fixed tree (merge.cuh).
 // Grid size and kernel variant (register budget) only decide who
 // computes an item, never the arithmetic, so results are bitwise identical
 // across launch shapes.
@@ -21,14 +21,14 @@
 // scheduler (measured; an FFMA 1.1, and the two do not overlap), so a
 // path-step's 12 wide products, three half products and 16 FP32 operations
 // take 82 cycles; measured 94 on the 4096-contract book.  Products that depend
-// on the draw alone come from a table per slab, those of the path alone are
+// on the draw alone come from a table per item, those of the path alone are
 // taken once per path (PhiloxStep, PhiloxRow): 18 products -> 14.5.  The book
 // 313 -> 253 ms at 8 CTAs per SM (294 before at its best launch shape), of
 // which 7 ms from sums instead of Welford merges in the reductions.  Flushing
 // denormals (--ftz) takes the range tests out of the logarithm and the
 // exponentials (arguments here are normal numbers, the bits stay); the
-// compiler then wants 72 registers: at 5, 6, 7 and 8 CTAs per SM 260, 256, 253
-// and 266 ms on one GPU.
+// compiler then wants about 70 registers: at 5, 6, 7 and 8 CTAs per SM 260, 256,
+// 253 and 266 ms on one GPU.
 //
 // Reference semantics restated per kind (src/pricers/monte_carlo.cpp):
 //   terminal products :135-149, path-dependent loop :154-177, Brownian-bridge
