@@ -109,12 +109,12 @@ PATH_KERNEL_SOURCES = ("derivative-pricing_gb300/csrc/gbm_paths.cu",
                        "derivative-pricing_gb300/csrc/device_common.cuh",
                        "derivative-pricing_gb300/csrc/engine.hpp")
 PATH_KERNEL_PROFILE = {
-    "sources": "f02428902a30f0ab",
+    "sources": "852b8eff9b45756d",
     "case_path_steps": 6807363601.0,
     # variant -> smsp__inst_executed.sum of one launch
-    "warp_inst": {"0": 14013227156, "1": 14030631398, "2": 14732996643, "3": 14156821798, "4": 14019151174},
+    "warp_inst": {"0": 14013206001, "1": 14030673708, "2": 14733038953, "3": 14156864108, "4": 14019130019},
     # variant -> dram__bytes_read.sum + dram__bytes_write.sum of one launch
-    "dram_bytes": {"0": 357632, "1": 541184, "2": 420864, "3": 885760, "4": 202496},
+    "dram_bytes": {"0": 163840, "1": 166656, "2": 764928, "3": 1000192, "4": 462592},
 }
 
 

@@ -71,15 +71,18 @@ struct DevContract {
     // contract is outside the fixed-point range.
     uint32_t n_units;
     int32_t unit_log, frac;
-    // FP32 paths (gbm_paths.cu, greeks.cu): items of 128 << item_log paths.
-    int32_t item_log;
-    uint32_t n_items;
     uint32_t y_drift_lo;   // drift / ln 2 = (y_drift + y_drift_lo 2^-32) 2^-frac
     int64_t y_drift;
     uint64_t y_vs;         // vs / ln 2, 2^(frac + 3)
     int64_t y_barrier;     // log2(H / S0), 2^frac, within +/- 2^61
     double y_bridge;       // -2 (ln 2)^2 / (vol^2 dt), 2^(-2 frac)
     double inv_n;          // 1 / n_steps
+    // FP32 paths (gbm_paths.cu, greeks.cu): items of 128 << item_log paths.
+    // (Last, with padding: the FP64 kernels read pairs of the words above in 16
+    // bytes, and keep the record before 16-byte tables.)
+    int32_t item_log;
+    uint32_t n_items;
+    uint64_t reserved;
 };
 
 // Validates one contract and converts it to the kernel layout; null on
