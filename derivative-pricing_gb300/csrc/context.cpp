@@ -482,6 +482,10 @@ int price_quote(Ctx& ctx, const DevContract& c, mcd_mc_result* result) {
     if (rc) return rc;
     cudaError_t e = cudaStreamSynchronize(ctx.stream);  // staging buffer reuse
     if (e != cudaSuccess) return ctx.cuda_fail(e, "stream sync");
+    // A count that no call has: what is left there if no CTA wrote the result.
+    auto* record = static_cast<volatile DevMcResult*>(ctx.h_stage.ptr);
+    constexpr unsigned long long kNoResult = ~0ull;
+    record->path_count = kNoResult;
     int pair = -1;
     rc = ctx.record_start(ctx.stream, &pair);
     if (rc) return rc;
@@ -493,6 +497,7 @@ int price_quote(Ctx& ctx, const DevContract& c, mcd_mc_result* result) {
     if (e != cudaSuccess) return ctx.cuda_fail(e, "batch execution");
     ctx.collect_timing(false);
     if (rc) return rc;
+    if (record->path_count == kNoResult) return ctx.fail(MCD_ERR_CUDA, "the quote kernel wrote no result");
     std::memcpy(result, ctx.h_stage.ptr, sizeof *result);
     return MCD_OK;
 }
@@ -606,7 +611,11 @@ int mcd_create(int device, mcd_ctx** out) try {
     }
     if ((e = cudaMalloc(reinterpret_cast<void**>(&ctx->d_flags), 64)) != cudaSuccess)
         return init_fail(e, "flags");
-    cudaMemset(ctx->d_flags, 0, 64);
+    // On the context's own stream: it is not ordered after the legacy stream, and
+    // quote64_kernel takes its counter as it finds it.
+    e = cudaMemsetAsync(ctx->d_flags, 0, 64, ctx->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+    if (e != cudaSuccess) return init_fail(e, "reset flags");
     if ((e = fixed_tables_device(&ctx->tables)) != cudaSuccess) return init_fail(e, "fixed-point tables");
     *out = reinterpret_cast<mcd_ctx*>(ctx);
     return MCD_OK;
