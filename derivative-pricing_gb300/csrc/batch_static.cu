@@ -77,12 +77,12 @@ int report_cuda(char* msg, size_t cap, cudaError_t e, const char* where) {
 // device current and size the grids.  Must happen outside any stream capture.
 // With CUDA's lazy module loading (the runtime's default) this is also when
 // the module is loaded on the device and the array's memory is reserved.
-int static_setup(int device, char* msg, size_t cap) {
+int static_setup(int device, cudaStream_t stream, char* msg, size_t cap) {
     if (g_scratch_addr[device]) return MCD_OK;
     void* addr = nullptr;
     cudaError_t e = cudaGetSymbolAddress(&addr, g_batch_scratch);
     if (e != cudaSuccess) return report_cuda(msg, cap, e, "cudaGetSymbolAddress(scratch)");
-    e = mcdg::fixed_tables_device(&g_tables[device]);
+    e = mcdg::fixed_tables_device(&g_tables[device], stream);
     if (e != cudaSuccess) return report_cuda(msg, cap, e, "fixed-point tables");
     int sms = 0;
     e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
@@ -119,7 +119,8 @@ extern "C" int mcd_price_batch_static(const mcd_contract* contracts, size_t n, i
         return report(error_message, error_capacity, MCD_ERR_UNSUPPORTED, "device index too large");
     // A call with n = 0 does the device's set-up only: a caller that reserves
     // the rest of device memory afterwards makes this call first.
-    int rc = static_setup(device, error_message, error_capacity);
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    int rc = static_setup(device, s, error_message, error_capacity);
     if (rc != MCD_OK || n == 0) return rc;
 
     uint64_t total = 0;   // slabs, the limit's unit
@@ -146,7 +147,6 @@ extern "C" int mcd_price_batch_static(const mcd_contract* contracts, size_t n, i
     Welford* d_partials = reinterpret_cast<Welford*>(base + kOffPartials);
     mcd_mc_result* d_results = reinterpret_cast<mcd_mc_result*>(base + kOffResults);
     uint32_t* d_flags = reinterpret_cast<uint32_t*>(base + kOffFlags);
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
 
     // The array keeps the previous call's contents: the ticket and the error
     // word must start at zero; contracts, prefix, partials and results are

@@ -616,7 +616,7 @@ int mcd_create(int device, mcd_ctx** out) try {
     e = cudaMemsetAsync(ctx->d_flags, 0, 64, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) return init_fail(e, "reset flags");
-    if ((e = fixed_tables_device(&ctx->tables)) != cudaSuccess) return init_fail(e, "fixed-point tables");
+    if ((e = fixed_tables_device(&ctx->tables, ctx->stream)) != cudaSuccess) return init_fail(e, "fixed-point tables");
     *out = reinterpret_cast<mcd_ctx*>(ctx);
     return MCD_OK;
 } catch (...) {

@@ -108,8 +108,9 @@ cudaError_t launch_path64_kernel(int variant, int grid, const DevContract* contr
 cudaError_t launch_quote64(int sm_count, const DevContract& c, Welford* partials, uint32_t* done, DevMcResult* result,
                            const FixedTables* tables, cudaStream_t stream);
 // The fixed-point tables of the current device, placed there at the first call
-// (computed once per process, 22 ms).  Not to be called during stream capture.
-cudaError_t fixed_tables_device(const FixedTables** out);
+// (computed once per process, 22 ms) by a copy on `stream` that has ended when the
+// call returns.  Not to be called during stream capture.
+cudaError_t fixed_tables_device(const FixedTables** out, cudaStream_t stream);
 cudaError_t launch_merge_kernel(const DevContract* contracts, int n_contracts,
                                 const uint32_t* item_prefix, const Welford* partials,
                                 void* results /* mcd_mc_result[] */, cudaStream_t stream);

@@ -310,7 +310,7 @@ __global__ void draws64_kernel(uint64_t seed, uint64_t path_begin, uint64_t n_pa
 
 }  // namespace
 
-cudaError_t fixed_tables_device(const FixedTables** out) {
+cudaError_t fixed_tables_device(const FixedTables** out, cudaStream_t stream) {
     constexpr int kDevices = 64;
     static std::mutex lock;
     static void* address[kDevices] = {};
@@ -322,7 +322,11 @@ cudaError_t fixed_tables_device(const FixedTables** out) {
     if (!address[device]) {
         void* p = nullptr;
         e = cudaGetSymbolAddress(&p, g_fixed_tables);
-        if (e == cudaSuccess) e = cudaMemcpy(p, &fixed_tables(), sizeof(FixedTables), cudaMemcpyHostToDevice);
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(p, &fixed_tables(), sizeof(FixedTables), cudaMemcpyHostToDevice, stream);
+        // A copy from pageable memory may return before its last part has arrived,
+        // and launches on other streams do not wait for it.
+        if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
         if (e != cudaSuccess) return e;
         address[device] = p;
     }

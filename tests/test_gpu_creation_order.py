@@ -7,7 +7,10 @@ compares its first call with an idle engine's, byte for byte.
 """
 from __future__ import annotations
 
-import numpy as np
+import os
+import subprocess
+import sys
+
 import pytest
 
 import mcd_gpu as G
@@ -47,3 +50,27 @@ def test_first_quote_of_an_engine_created_behind_queued_work(engine, work):
             got = [e.price_batch(one, "fp64").tobytes() for _ in range(3)]
         assert got == [want] * 3
     torch.cuda.synchronize()
+
+
+_CHILD = """
+import sys
+sys.path[:0] = [%r, %r]
+import torch
+import test_gpu_creation_order as T
+import mcd_gpu as G
+x = torch.rand(1 << 28, device="cuda")
+torch.cuda.synchronize()
+T._busy(x)
+with G.Engine(0) as e:
+    print(e.price_batch(T._contracts(), "fp64").tobytes().hex())
+"""
+
+
+def test_first_call_of_a_process_behind_queued_work(engine):
+    """The process's one copy of the fixed-point tables has ended before the first kernel."""
+    here = os.path.dirname(os.path.abspath(__file__))
+    package = os.path.dirname(os.path.abspath(G.__file__))
+    want = engine.price_batch(_contracts(), "fp64").tobytes().hex()
+    r = subprocess.run([sys.executable, "-c", _CHILD % (here, package)], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr
+    assert r.stdout.strip() == want
