@@ -188,6 +188,23 @@ int plan_qmc(Ctx& ctx, const mcd_contract* cs, size_t n, BatchPlan& plan, std::v
     return MCD_OK;
 }
 
+// The direction words on the context's first use of them, on its own stream: that
+// stream is not ordered after a copy on the legacy one, which may return before
+// it has ended.
+int ensure_directions(Ctx& ctx) {
+    DeviceBuffer& b = ctx.ext[kQDirs];
+    if (b.ptr) return MCD_OK;
+    const std::vector<uint32_t> dirs = sobol_directions();
+    const int rc = ctx.reserve(b, sizeof(uint32_t) * dirs.size(), "sobol directions");
+    if (rc) return rc;
+    const cudaError_t e =
+        cudaMemcpyAsync(b.ptr, dirs.data(), sizeof(uint32_t) * dirs.size(), cudaMemcpyHostToDevice, ctx.stream);
+    if (e == cudaSuccess) return MCD_OK;
+    cudaFree(b.ptr);
+    b = DeviceBuffer{};
+    return ctx.cuda_fail(e, "sobol directions upload");
+}
+
 int qmc_batch(Ctx& ctx, const mcd_contract* cs, size_t n, int precision, mcd_mc_result* results) {
     if (precision != 0 && precision != 1) return ctx.fail(MCD_ERR_INVALID_ARGUMENT, "precision must be 0 (FP64) or 1 (FP32)");
     if (n == 0) return MCD_OK;
@@ -197,15 +214,8 @@ int qmc_batch(Ctx& ctx, const mcd_contract* cs, size_t n, int precision, mcd_mc_
     std::vector<BridgeNode> programs;
     int rc = plan_qmc(ctx, cs, n, plan, consts, programs);
     if (rc) return rc;
-    if (!ctx.ext[kQDirs].ptr) {
-        const std::vector<uint32_t> dirs = sobol_directions();
-        rc = ctx.reserve(ctx.ext[kQDirs], sizeof(uint32_t) * dirs.size(), "sobol directions");
-        if (rc) return rc;
-        cudaError_t e = cudaMemcpy(ctx.ext[kQDirs].ptr, dirs.data(), sizeof(uint32_t) * dirs.size(),
-                                   cudaMemcpyHostToDevice);
-        if (e != cudaSuccess) return ctx.cuda_fail(e, "sobol directions upload");
-    }
-    rc = ctx.reserve(ctx.ext[kQProg], sizeof(BridgeNode) * programs.size(), "bridge programs");
+    rc = ensure_directions(ctx);
+    if (!rc) rc = ctx.reserve(ctx.ext[kQProg], sizeof(BridgeNode) * programs.size(), "bridge programs");
     if (!rc) rc = ctx.reserve(ctx.ext[kQConst], sizeof(DevQmc) * n, "qmc constants");
     if (!rc) rc = ctx.reserve(ctx.ext[kQDev], sizeof(DevContract) * n, "qmc contracts");
     if (!rc) rc = ctx.reserve(ctx.ext[kQPrefix], sizeof(uint32_t) * (n + 1), "qmc prefix");
@@ -348,16 +358,10 @@ int mcd_sobol_points(mcd_ctx* handle, unsigned dim_begin, unsigned n_dims, uint6
         return ctx->fail(MCD_ERR_INVALID_ARGUMENT, "dimensions must be < MCD_SOBOL_MAX_DIMS (256)");
     if (n_indices * n_dims > (1ull << 28)) return ctx->fail(MCD_ERR_INVALID_ARGUMENT, "at most 2^28 points per call");
     if (n_indices == 0 || n_dims == 0) return MCD_OK;
-    if (!ctx->ext[kQDirs].ptr) {
-        const std::vector<uint32_t> dirs = sobol_directions();
-        int rc = ctx->reserve(ctx->ext[kQDirs], sizeof(uint32_t) * dirs.size(), "sobol directions");
-        if (rc) return rc;
-        cudaError_t e = cudaMemcpy(ctx->ext[kQDirs].ptr, dirs.data(), sizeof(uint32_t) * dirs.size(),
-                                   cudaMemcpyHostToDevice);
-        if (e != cudaSuccess) return ctx->cuda_fail(e, "sobol directions upload");
-    }
+    int rc = ensure_directions(*ctx);
+    if (rc) return rc;
     const size_t bytes = sizeof(double) * n_indices * n_dims;
-    int rc = ctx->reserve(ctx->d_scratch, bytes, "sobol output");
+    rc = ctx->reserve(ctx->d_scratch, bytes, "sobol output");
     if (rc) return rc;
     cudaError_t e = launch_sobol_points(static_cast<const uint32_t*>(ctx->ext[kQDirs].ptr), dim_begin, n_dims,
                                         index_begin, n_indices, static_cast<double*>(ctx->d_scratch.ptr), ctx->stream);

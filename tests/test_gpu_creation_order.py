@@ -52,6 +52,16 @@ def test_first_quote_of_an_engine_created_behind_queued_work(engine, work):
     torch.cuda.synchronize()
 
 
+def test_first_sobol_batch_of_an_engine_behind_queued_work(engine, work):
+    c = _contracts()
+    want = engine.qmc_batch(c, "fp32").tobytes()
+    for _ in range(5):
+        with G.Engine(0) as e:
+            _busy(work)
+            assert e.qmc_batch(c, "fp32").tobytes() == want
+    torch.cuda.synchronize()
+
+
 _CHILD = """
 import sys
 sys.path[:0] = [%r, %r]
