@@ -57,6 +57,7 @@ static __device__ __align__(256) unsigned char g_batch_scratch[kStaticScratchByt
 // calls (the device array is shared by all of them).
 std::mutex g_static_lock;
 unsigned char* g_scratch_addr[kStaticMaxDevices] = {};
+unsigned long long g_context[kStaticMaxDevices] = {};  // the CUDA context that the addresses are of
 int g_grid[kStaticMaxDevices][2] = {};  // persistent grid per device and precision
 DevContract g_stage_contracts[kStaticMaxContracts];
 uint32_t g_stage_prefix[kStaticMaxContracts + 1];
@@ -73,14 +74,17 @@ int report_cuda(char* msg, size_t cap, cudaError_t e, const char* where) {
     return e == cudaErrorMemoryAllocation ? MCD_ERR_OUT_OF_MEMORY : MCD_ERR_CUDA;
 }
 
-// First call on a device: resolve the array's device address with that
+// First call on a device, or on one that was reset since: resolve the array's device address with that
 // device current and size the grids.  Must happen outside any stream capture.
 // With CUDA's lazy module loading (the runtime's default) this is also when
 // the module is loaded on the device and the array's memory is reserved.
 int static_setup(int device, cudaStream_t stream, char* msg, size_t cap) {
-    if (g_scratch_addr[device]) return MCD_OK;
+    unsigned long long id = 0;
+    cudaError_t e = mcdg::device_context_id(&id);
+    if (e != cudaSuccess) return report_cuda(msg, cap, e, "CUDA context");
+    if (g_scratch_addr[device] && g_context[device] == id) return MCD_OK;
     void* addr = nullptr;
-    cudaError_t e = cudaGetSymbolAddress(&addr, g_batch_scratch);
+    e = cudaGetSymbolAddress(&addr, g_batch_scratch);
     if (e != cudaSuccess) return report_cuda(msg, cap, e, "cudaGetSymbolAddress(scratch)");
     e = mcdg::fixed_tables_device(&g_tables[device], stream);
     if (e != cudaSuccess) return report_cuda(msg, cap, e, "fixed-point tables");
@@ -94,6 +98,7 @@ int static_setup(int device, cudaStream_t stream, char* msg, size_t cap) {
         g_grid[device][precision] = sms * (blocks > 0 ? blocks : 1);
     }
     g_scratch_addr[device] = static_cast<unsigned char*>(addr);
+    g_context[device] = id;
     return MCD_OK;
 }
 

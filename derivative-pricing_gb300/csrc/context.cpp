@@ -1,5 +1,6 @@
 // context.cpp -- the C ABI (include/mcd_gpu.h): context, validation, batch
 // planning, CUDA-graph capture of the persistent path kernel, autotuner.
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -8,6 +9,7 @@
 #include <cstring>
 #include <numeric>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "context.hpp"
@@ -101,6 +103,36 @@ Ctx::~Ctx() {
 // Planning and graph helpers, shared with the other modules through
 // context.hpp (greeks_api.cpp builds its batches with them).
 namespace mcdg {
+
+cudaError_t device_context_id(unsigned long long* id) {
+    // through the runtime, so that the library loads where there is no driver
+    struct Driver {
+        decltype(&::cuCtxGetCurrent) current = nullptr;
+        decltype(&::cuCtxGetId) number = nullptr;
+        cudaError_t status = cudaSuccess;
+        Driver() {
+            auto find = [&](const char* name, auto& f) {
+                void* p = nullptr;
+                cudaDriverEntryPointQueryResult found = cudaDriverEntryPointSymbolNotFound;
+                if (status == cudaSuccess)
+                    status = cudaGetDriverEntryPointByVersion(name, &p, 12000, cudaEnableDefault, &found);
+                if (status == cudaSuccess && (found != cudaDriverEntryPointSuccess || !p)) status = cudaErrorSymbolNotFound;
+                f = reinterpret_cast<std::remove_reference_t<decltype(f)>>(p);
+            };
+            find("cuCtxGetCurrent", current);
+            find("cuCtxGetId", number);
+        }
+    };
+    static const Driver driver;
+    if (driver.status != cudaSuccess) return driver.status;
+    CUcontext c = nullptr;
+    for (int attempt = 0; attempt < 2; ++attempt) {
+        if (driver.current(&c) == CUDA_SUCCESS && c && driver.number(c, id) == CUDA_SUCCESS) return cudaSuccess;
+        const cudaError_t e = cudaFree(nullptr);  // none yet, or one that was reset
+        if (e != cudaSuccess) return e;
+    }
+    return cudaErrorDeviceUninitialized;
+}
 
 bool finite_all(std::initializer_list<double> xs) {
     for (double x : xs)

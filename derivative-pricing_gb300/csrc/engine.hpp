@@ -107,9 +107,13 @@ cudaError_t launch_path64_kernel(int variant, int grid, const DevContract* contr
 // host memory; one partial per unit, *done zero before and after.
 cudaError_t launch_quote64(int sm_count, const DevContract& c, Welford* partials, uint32_t* done, DevMcResult* result,
                            const FixedTables* tables, cudaStream_t stream);
-// The fixed-point tables of the current device, placed there at the first call
-// (computed once per process, 22 ms) by a copy on `stream` that has ended when the
-// call returns.  Not to be called during stream capture.
+// The number of the current device's CUDA context (set up if there is none yet),
+// another one after every cudaDeviceReset: what the process remembers of a
+// device's memory is good for one number only.
+cudaError_t device_context_id(unsigned long long* id);
+// The fixed-point tables of the current device, placed there at the first call in
+// its context (computed once per process, 22 ms) by a copy on `stream` that has
+// ended when the call returns.  Not to be called during stream capture.
 cudaError_t fixed_tables_device(const FixedTables** out, cudaStream_t stream);
 cudaError_t launch_merge_kernel(const DevContract* contracts, int n_contracts,
                                 const uint32_t* item_prefix, const Welford* partials,

@@ -314,12 +314,15 @@ cudaError_t fixed_tables_device(const FixedTables** out, cudaStream_t stream) {
     constexpr int kDevices = 64;
     static std::mutex lock;
     static void* address[kDevices] = {};
+    static unsigned long long context[kDevices] = {};  // in which the address holds the tables
     int device = 0;
+    unsigned long long id = 0;
     cudaError_t e = cudaGetDevice(&device);
+    if (e == cudaSuccess) e = device_context_id(&id);
     if (e != cudaSuccess) return e;
     if (device < 0 || device >= kDevices) return cudaErrorInvalidDevice;
     std::lock_guard<std::mutex> hold(lock);
-    if (!address[device]) {
+    if (!address[device] || context[device] != id) {
         void* p = nullptr;
         e = cudaGetSymbolAddress(&p, g_fixed_tables);
         if (e == cudaSuccess)
@@ -329,6 +332,7 @@ cudaError_t fixed_tables_device(const FixedTables** out, cudaStream_t stream) {
         if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
         if (e != cudaSuccess) return e;
         address[device] = p;
+        context[device] = id;
     }
     *out = static_cast<const FixedTables*>(address[device]);
     return cudaSuccess;
