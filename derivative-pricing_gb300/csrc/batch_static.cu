@@ -106,7 +106,7 @@ int static_setup(int device, cudaStream_t stream, char* msg, size_t cap) {
 
 extern "C" int mcd_price_batch_static(const mcd_contract* contracts, size_t n, int precision,
                                       mcd_mc_result* results, void* stream, char* error_message,
-                                      size_t error_capacity) {
+                                      size_t error_capacity) try {
     std::lock_guard<std::mutex> lock(g_static_lock);
     if (error_message && error_capacity) error_message[0] = '\0';
     if (precision != MCD_PRECISION_FP64 && precision != MCD_PRECISION_FP32)
@@ -187,4 +187,6 @@ extern "C" int mcd_price_batch_static(const mcd_contract* contracts, size_t n, i
     if (flags[1] != 0)
         return report(error_message, error_capacity, MCD_ERR_CUDA, "path kernel reported an inconsistent work item");
     return MCD_OK;
+} catch (...) {  // nothing here throws but a lock that the system refuses
+    return report(error_message, error_capacity, MCD_ERR_INVALID_ARGUMENT, "internal error");
 }

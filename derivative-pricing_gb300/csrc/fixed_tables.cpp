@@ -12,8 +12,6 @@
 #include "fixed_tables.hpp"
 
 #include <cmath>
-#include <memory>
-#include <mutex>
 
 namespace mcdg {
 
@@ -140,17 +138,18 @@ void fill_log(FixedTables& t) {
 
 }  // namespace
 
+// In static storage: mcd_price_batch_static, which allocates nothing and has no
+// status for a failed allocation here, needs the tables too.
 const FixedTables& fixed_tables() {
-    static std::once_flag once;
-    static std::unique_ptr<FixedTables> tables;
-    std::call_once(once, [] {
-        auto t = std::make_unique<FixedTables>();
-        fill_quantile(*t);
-        fill_exp(*t);
-        fill_log(*t);
-        tables = std::move(t);
-    });
-    return *tables;
+    static FixedTables tables;
+    static const bool filled = [] {
+        fill_quantile(tables);
+        fill_exp(tables);
+        fill_log(tables);
+        return true;
+    }();
+    static_cast<void>(filled);
+    return tables;
 }
 
 }  // namespace mcdg
