@@ -81,7 +81,7 @@ __device__ __forceinline__ MergedResult merge_items(const Welford* __restrict__ 
         const double mean = s1 * fast_rcp64(nd);
         const double m2 = fma(-s1, mean, s2);
         r.mean = shift + mean;
-        if (n > 1 && m2 > 0.0) r.standard_error = fast_sqrt64(m2 * fast_rcp64((nd - 1.0) * nd));
+        if (n > 1 && !(m2 <= 0.0)) r.standard_error = fast_sqrt64(m2 * fast_rcp64((nd - 1.0) * nd));
     }
     return r;
 }

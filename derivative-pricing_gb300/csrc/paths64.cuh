@@ -74,8 +74,10 @@ struct Path64 {
     }
 };
 
-__device__ __forceinline__ double positive_part(double x) {  // (x < 0) ? 0 : x, from the sign bit
-    return __double2hiint(x) < 0 ? 0.0 : x;
+// (x < 0) ? 0 : x by the high word: from 0x80000000 (-0) to 0xFFF00000 (-infinity);
+// a NaN above that stays, as in the comparison's form.
+__device__ __forceinline__ double positive_part(double x) {
+    return static_cast<uint32_t>(__double2hiint(x)) - 0x80000000u <= 0x7FF00000u ? 0.0 : x;
 }
 __device__ __forceinline__ double put_sign(double x, int type) { return type == 0 ? x : -x; }
 

@@ -21,7 +21,7 @@ __device__ __forceinline__ Welford unit_triple(uint32_t count, double pivot, dou
     const double inv = __hiloint2double((1023 - (31 - __clz(static_cast<int>(count)))) << 20, 0);
     const double m = pow2 ? a * inv : a / static_cast<double>(count);
     const double m2 = fma(-a, m, b);
-    return Welford{count, pivot + m, m2 > 0.0 ? m2 : 0.0};
+    return Welford{count, pivot + m, m2 < 0.0 ? 0.0 : m2};  // (NaN stays)
 }
 
 // The triples of a CTA's four warps.  Whole items have a power of two of samples
