@@ -3,13 +3,13 @@
 #pragma once
 
 #include "engine.hpp"
-#include "fp64_fast.cuh"
 
 namespace mcdg {
 
 // A single contract of 1e5 paths has 3125 items, 25 per thread: four loads in
-// flight and the division, square root and last tree cut to 20 FP64 operations
-// take a call's merge from 16 to 9 us (cold); 256 or 512 threads measured the same.
+// flight and a short last tree take a call's merge from 16 to 9 us (cold); 256 or
+// 512 threads measured the same.  The last division and root are IEEE's (0.3 us
+// of a quote's 27 against ones from an FP32 seed, which err by up to a unit).
 constexpr int kMergeThreads = 128;
 
 struct MergedResult {
@@ -78,10 +78,10 @@ __device__ __forceinline__ MergedResult merge_items(const Welford* __restrict__ 
     r.count = n;
     if (n > 0) {
         const double nd = static_cast<double>(n);
-        const double mean = s1 * fast_rcp64(nd);
+        const double mean = s1 / nd;
         const double m2 = fma(-s1, mean, s2);
         r.mean = shift + mean;
-        if (n > 1 && !(m2 <= 0.0)) r.standard_error = fast_sqrt64(m2 * fast_rcp64((nd - 1.0) * nd));
+        if (n > 1 && !(m2 <= 0.0)) r.standard_error = sqrt(m2 / ((nd - 1.0) * nd));
     }
     return r;
 }
