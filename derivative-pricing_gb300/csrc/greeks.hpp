@@ -42,16 +42,15 @@ struct DevGreeks {
     double lr_gamma_scale;     // 1 / (S0^2 vol^2 dt1)
     double sqrt_dt_over_vol, inv_vol, inv_n, inv_spot, inv_2t, mu_over_vol_sqrt_t;
     // FP64 kernel: the vol-bumped states' log2 steps in the contract's units
-    // (DevContract::frac), the barrier seen from the bumped spots, and
+    // (DevContract::frac), the barrier seen from the bumped spots, and the unit
+    // of the draws' running sum
     int64_t y_drift_up, y_drift_dn;
     uint64_t y_vs_up, y_vs_dn;
     uint32_t y_drift_lo_up, y_drift_lo_dn;
     int64_t y_barrier_su, y_barrier_sd;
-    double x_unit;             // ln 2 2^-frac: log-spot per unit
-    double z_unit;             // 1 / (vs / ln 2 2^frac): normals per unit of their sum
-    double dvol_drift;         // drift / vol + vol dt: dlnS_i/dvol = ln(S_i/S0) / vol - i dvol_drift
+    double z_unit;             // 2^(z_shift - 61): the running sum of the normals in normals
     int32_t vol_series;        // |vol-bump exponent| <= 1e-2 on all but > 8-sigma paths: cubic expm1
-    int32_t pad;
+    int32_t z_shift;           // FP64: that sum of n_steps normals (below 6.34 each) stays within 63 bits
 };
 
 cudaError_t launch_greeks_kernel(int precision, int variant, int grid, const DevContract* contracts,

@@ -8,9 +8,10 @@
 // differences (src/greeks/finite_difference.cpp:40-65), likelihood ratio
 // (src/greeks/likelihood_ratio.cpp:33-73, :105-154), pathwise
 // (src/greeks/pathwise.cpp:28-55, :64-147).  Sums that the reference takes per
-// step follow from integer sums: the draws' sum from the log-spot itself, the
-// log-spots' derivatives from ln S_i = drift i + vol sqrt(dt) W_i, and
-// sum i S_i from the prefix sums of S_i.
+// step follow from integer sums: W_i, the running sum of the draws, is one of its
+// own (the log-spot's differs from it by vol sqrt(dt), and would have lost as many
+// of its bits as that is small), the log-spots' derivatives are sqrt(dt) W_i - vol
+// i dt, and sum i S_i follows from the prefix sums of S_i.
 //
 // Bound: issue and the FMA-heavy pipe for barriers, lookbacks and geometric
 // Asians; the FP64 pipe for arithmetic Asians (five operations per step).  1024
@@ -173,7 +174,10 @@ __device__ __forceinline__ void greeks_fixed(GreeksSlot& slot, const FixedShared
     const PhiloxRow row = philox_row(path_lo, 0u, k);
     State<KIND> p, up, dn;
     uint64_t zz_lo = 0, zz_hi = 0;  // sum of z^2, units of 2^-58, split at 32 bits
-    double prefix = 0.0, e_y = 0.0;  // arithmetic Asian: sum of the running sums, sum of S_i / S0 times y_i
+    int64_t w = 0;                   // W_i, units of 2^(z_shift - 61)
+    int64_t wsum_hi = 0;             // geometric Asian: sum of W_i, as Path64's of y
+    uint64_t wsum_lo = 0;
+    double prefix = 0.0, e_w = 0.0;  // arithmetic Asian: sum of the running sums, sum of S_i / S0 times W_i
     FixedNormal z1{};
     for (int d0 = 0; d0 < n; d0 += 32) {
         if (refill || n > 32) {
@@ -197,9 +201,17 @@ __device__ __forceinline__ void greeks_fixed(GreeksSlot& slot, const FixedShared
             const uint64_t zz = mul_hi64(z.mag, z.mag);
             zz_lo += static_cast<uint32_t>(zz);
             zz_hi += zz >> 32;
+            if constexpr (KIND != kEuropean && KIND != kDigital) {
+                const int64_t neg = z.neg;
+                w += (static_cast<int64_t>(z.mag >> g.z_shift) ^ neg) - neg;
+            }
             if constexpr (KIND == kAsianArith) {
                 prefix += p.sum;
-                e_y = fma(p.last, static_cast<double>(p.y), e_y);
+                e_w = fma(p.last, static_cast<double>(w), e_w);
+            }
+            if constexpr (KIND == kAsianGeo) {
+                wsum_hi += w >> 32;
+                wsum_lo += static_cast<uint32_t>(w);
             }
         }
     }
@@ -214,23 +226,22 @@ __device__ __forceinline__ void greeks_fixed(GreeksSlot& slot, const FixedShared
         b.z_sum = b.z1;
         b.zz_excess = b.z1 * b.z1 - 1.0;
     } else {
-        // the log-spot less its drift, in units of the normals' sum
-        const uint64_t un = static_cast<uint64_t>(n);
-        const int64_t drift = static_cast<int64_t>(un) * c.y_drift + static_cast<int64_t>(un * c.y_drift_lo >> 32);
-        b.z_sum = static_cast<double>(p.y - drift) * g.z_unit;
+        b.z_sum = static_cast<double>(w) * g.z_unit;
         b.zz_excess = fma(fma(static_cast<double>(zz_hi), 4294967296.0, static_cast<double>(zz_lo)), 0x1p-58, -nd);
     }
     if constexpr (KIND == kAsianArith || KIND == kAsianGeo) {
         b.avg = average64<KIND>(c, c.spot, s, p);
-        const double x_over_vol = g.x_unit * g.inv_vol;
-        b.last_dvol = b.last * fma(static_cast<double>(p.y), x_over_vol, -nd * g.dvol_drift);
+        const double decay = g.vol * g.dt;  // dlnS_i/dvol = sqrt(dt) W_i - i decay
+        b.last_dvol = b.last * fma(g.sqrt_dt, b.z_sum, -nd * decay);
         if constexpr (KIND == kAsianArith) {
             const double i_s = fma(nd + 1.0, p.sum, -prefix);  // sum of i S_i / S0
-            b.avg_dvol = c.spot * (fma(e_y, x_over_vol, -i_s * g.dvol_drift) * c.inv_n);
+            b.avg_dvol = c.spot * (fma(g.sqrt_dt, e_w * g.z_unit, -i_s * decay) * c.inv_n);
             b.avg_drate = c.spot * (i_s * g.dt * c.inv_n);
         } else {
             const double i_mean = 0.5 * (nd + 1.0);
-            b.avg_dvol = b.avg * fma(p.log_sum() * c.inv_n, x_over_vol, -i_mean * g.dvol_drift);
+            const double w_mean = fma(static_cast<double>(wsum_hi), 4294967296.0, static_cast<double>(wsum_lo)) *
+                                  (g.z_unit * c.inv_n);
+            b.avg_dvol = b.avg * fma(g.sqrt_dt, w_mean, -i_mean * decay);
             b.avg_drate = b.avg * (i_mean * g.dt);
         }
     }

@@ -95,9 +95,8 @@ int plan_greeks(Ctx& ctx, const mcd_contract* cs, size_t n, int precision, doubl
                 g.y_barrier_su = fixed_barrier(g.log_h_rel_up, d.frac);
                 g.y_barrier_sd = fixed_barrier(g.log_h_rel_dn, d.frac);
             }
-            g.x_unit = std::ldexp(1.0 / kInvLn2, -d.frac);
-            g.z_unit = 1.0 / std::ldexp(d.vs * kInvLn2, d.frac);
-            g.dvol_drift = d.drift / in.vol + in.vol * g.dt;
+            while (1.585 * static_cast<double>(d.n_steps) > std::ldexp(1.0, g.z_shift)) ++g.z_shift;  // 6.34 2^61 = 1.585 2^63
+            g.z_unit = std::ldexp(1.0, g.z_shift - 61);
         }
         // The vol-bump exponent is h_vol D - h_vol^2 i dt / 2 with |D| below
         // 8 sqrt(T) + vol T on all but > 8-sigma paths.
