@@ -312,9 +312,40 @@ double slab_cost(const DevContract& c) {
     return static_cast<double>(c.n_steps) * per_step * (c.antithetic ? 2.0 : 1.0);
 }
 
+// Cuts the plan's contracts into ranges of at most range_items items, or one
+// contract (slabs: one range), so that the partials of a batch of many small
+// items stay bounded.  A batch is one range unless it is very large; results do
+// not depend on the ranges.
+void split_ranges(BatchPlan& plan, uint64_t range_items) {
+    plan.ranges.assign(1, 0);
+    plan.max_items = 0;
+    uint64_t in_range = 0;
+    for (size_t i = 0; i < plan.n; ++i) {
+        const uint32_t more = plan.prefix[i + 1] - plan.prefix[i];
+        if (plan.kind != Items::kSlabs && in_range > 0 && in_range + more > range_items) {
+            plan.ranges.push_back(static_cast<uint32_t>(i));
+            in_range = 0;
+        }
+        in_range += more;
+        plan.max_items = std::max(plan.max_items, static_cast<uint32_t>(in_range));
+    }
+    plan.ranges.push_back(static_cast<uint32_t>(plan.n));
+}
+
+int reserve_partials(Ctx& ctx, DeviceBuffer& b, BatchPlan& plan, size_t item_bytes, const char* what) {
+    for (;;) {
+        const int rc = ctx.reserve(b, item_bytes * std::max<size_t>(plan.max_items, 1), what);
+        const uint32_t had = plan.max_items;
+        if (rc != MCD_ERR_OUT_OF_MEMORY || had <= kMinRangeItems) return rc;
+        split_ranges(plan, std::max<uint64_t>(had / 4, kMinRangeItems));
+        if (plan.max_items >= had) return rc;  // slabs, or one contract's items
+    }
+}
+
 // range_items: at most that many items in a range (slabs: one range).
 int plan_batch(Ctx& ctx, const mcd_contract* contracts, size_t n, Items kind, uint64_t range_items, BatchPlan& plan) {
     if (n > 0x7FFFFFFF) return ctx.fail(MCD_ERR_INVALID_ARGUMENT, "too many contracts");
+    plan.kind = kind;
     plan.dev.resize(n);
     for (size_t i = 0; i < n; ++i) {
         const int rc = plan_contract(ctx, contracts[i], static_cast<uint32_t>(i), plan.dev[i]);
@@ -324,31 +355,20 @@ int plan_batch(Ctx& ctx, const mcd_contract* contracts, size_t n, Items kind, ui
     std::stable_sort(plan.dev.begin(), plan.dev.end(),
                      [&](const DevContract& a, const DevContract& b) { return cost(a) > cost(b); });
     // The prefix counts items modulo 2^32: kernels use differences within a
-    // range of contracts, and every range holds at most range_items units (or
-    // one contract), so that the partials of a batch of many small contracts
-    // stay bounded.  A batch is one range unless it is very large.
+    // range of contracts.
     plan.prefix.resize(n + 1);
-    plan.ranges.assign(1, 0);
-    uint64_t slabs = 0, in_range = 0;
+    uint64_t slabs = 0;
     uint32_t items = 0;
-    plan.max_items = 0;
     for (size_t i = 0; i < n; ++i) {
         const DevContract& c = plan.dev[i];
-        const uint32_t more = kind == Items::kUnits64 ? c.n_units : kind == Items::kItems32 ? c.n_items : c.n_slabs;
         plan.prefix[i] = items;
-        slabs += plan.dev[i].n_slabs;
+        slabs += c.n_slabs;
         if (slabs > 0xFFFFFFF0ull) return ctx.fail(MCD_ERR_INVALID_ARGUMENT, "batch too large");
-        if (kind != Items::kSlabs && in_range > 0 && in_range + more > range_items) {
-            plan.ranges.push_back(static_cast<uint32_t>(i));
-            in_range = 0;
-        }
-        in_range += more;
-        items += more;
-        plan.max_items = std::max(plan.max_items, static_cast<uint32_t>(in_range));
+        items += kind == Items::kUnits64 ? c.n_units : kind == Items::kItems32 ? c.n_items : c.n_slabs;
     }
     plan.prefix[n] = items;
-    plan.ranges.push_back(static_cast<uint32_t>(n));
     plan.n = n;
+    split_ranges(plan, range_items);
     return MCD_OK;
 }
 
@@ -385,14 +405,14 @@ struct PlanBuffers {
 
 // Uploads a plan (its ticket and error words zero) into the context's device
 // buffers (async on ctx.stream).
-int upload_plan(Ctx& ctx, const BatchPlan& plan) {
+int upload_plan(Ctx& ctx, BatchPlan& plan) {
     // The device-resident plan shares these buffers; any upload retires it.
     ctx.device_plan_valid = false;
     const size_t n = plan.n;
     PlanBuffers at(nullptr, n);
     int rc = ctx.reserve(ctx.d_plan, at.bytes, "contracts and results");
     if (rc) return rc;
-    rc = ctx.reserve(ctx.d_partials, sizeof(Welford) * std::max<size_t>(plan.max_items, 1), "partials");
+    rc = reserve_partials(ctx, ctx.d_partials, plan, sizeof(Welford), "partials");
     if (rc) return rc;
     // Stage through pinned memory so the copy is truly asynchronous.
     rc = ctx.reserve_host(ctx.h_stage, at.bytes, "pinned staging");

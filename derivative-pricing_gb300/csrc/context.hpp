@@ -22,14 +22,21 @@ struct HostBuffer {
     size_t bytes = 0;
 };
 
+// What a batch's items are: slabs (Sobol), FP64 units, FP32 items.
+enum class Items { kSlabs, kUnits64, kItems32 };
+
 struct BatchPlan {
+    Items kind = Items::kSlabs;
     std::vector<DevContract> dev;    // longest-first
-    std::vector<uint32_t> prefix;    // n + 1 running item counts (slabs or units)
+    std::vector<uint32_t> prefix;    // n + 1 running item counts, modulo 2^32
     std::vector<uint32_t> ranges;    // first contract of each range, then n
     uint32_t max_items = 0;          // items of the largest range
     size_t n = 0;
 };
-constexpr uint64_t kRangeItems = 1ull << 26;  // 1.6 GB of partials
+// Items of a range at most (or one contract's): 100 MB of partials, 860 rounds of
+// the resident warps.
+constexpr uint64_t kRangeItems = 1ull << 22;
+constexpr uint64_t kMinRangeItems = 1ull << 14;  // down to which a lack of memory cuts them
 
 struct LaunchShape {
     int variant = 1;
@@ -138,9 +145,10 @@ int plan_contract(Ctx& ctx, const mcd_contract& in, uint32_t index, DevContract&
 int fixed_frac(int n_steps, double drift, double vs);
 void fixed_step(double drift, double vs, int frac, int64_t* hi, uint32_t* lo, uint64_t* scale);
 int64_t fixed_barrier(double log_rel, int frac);
-// What a batch's items are: slabs (Sobol), FP64 units, FP32 items.
-enum class Items { kSlabs, kUnits64, kItems32 };
 int plan_batch(Ctx& ctx, const mcd_contract* contracts, size_t n, Items kind, uint64_t range_items, BatchPlan& plan);
+// Room for the partials of the plan's largest range, in smaller ranges if the
+// device has no more memory for this one (slabs: one range always).
+int reserve_partials(Ctx& ctx, DeviceBuffer& b, BatchPlan& plan, size_t item_bytes, const char* what);
 int price_batch_host(Ctx& ctx, const mcd_contract* contracts, size_t n, int precision,
                      mcd_mc_result* results);
 

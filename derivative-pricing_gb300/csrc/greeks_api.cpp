@@ -21,7 +21,7 @@ namespace {
 
 enum { kGDev = 21, kGConst = 22, kGPrefix = 23, kGPart = 24, kGOut = 25, kGFlags = 26 };
 
-constexpr uint64_t kGreeksRangeItems = 1ull << 23;  // 2.4 GB of FP64 partials
+constexpr uint64_t kGreeksRangeItems = 1ull << 18;  // 75 MB of partials, 54 rounds of the resident FP64 warps
 
 // Bits of mcd_greeks_result::defined.
 uint32_t defined_bits(int kind) {
@@ -118,16 +118,15 @@ int greeks_grid(Ctx& ctx, int precision, int& variant, int& grid) {
 
 // Uploads the plan and captures (or reuses) the graph: reset ticket and
 // error word, sensitivity kernel, merge.
-int prepare_greeks(Ctx& ctx, int precision, const BatchPlan& plan, const std::vector<DevGreeks>& consts,
+int prepare_greeks(Ctx& ctx, int precision, BatchPlan& plan, const std::vector<DevGreeks>& consts,
                    cudaGraphExec_t* out) {
     const size_t n = plan.n;
     int rc = ctx.reserve(ctx.ext[kGDev], sizeof(DevContract) * n, "greeks contracts");
     if (!rc) rc = ctx.reserve(ctx.ext[kGConst], sizeof(DevGreeks) * n, "greeks constants");
     if (!rc) rc = ctx.reserve(ctx.ext[kGPrefix], sizeof(uint32_t) * (n + 1), "greeks prefix");
-    if (!rc) rc = ctx.reserve(ctx.ext[kGPart], sizeof(Welford) * kNumGreeks * std::max<uint32_t>(plan.max_items, 1),
-                              "greeks partials");
     if (!rc) rc = ctx.reserve(ctx.ext[kGOut], sizeof(double) * kGreeksOutStride * n, "greeks results");
     if (!rc) rc = ctx.reserve(ctx.ext[kGFlags], 256, "greeks flags");
+    if (!rc) rc = reserve_partials(ctx, ctx.ext[kGPart], plan, sizeof(Welford) * kNumGreeks, "greeks partials");
     if (rc) return rc;
     cudaError_t e = cudaMemcpyAsync(ctx.ext[kGDev].ptr, plan.dev.data(), sizeof(DevContract) * n,
                                     cudaMemcpyHostToDevice, ctx.stream);
@@ -183,7 +182,7 @@ int prepare_greeks(Ctx& ctx, int precision, const BatchPlan& plan, const std::ve
     cudaGraphDestroy(graph);
     if (e != cudaSuccess) return ctx.cuda_fail(e, "greeks instantiate");
     ctx.greeks_graph = exec;
-    ctx.greeks_key = key;
+    ctx.greeks_key = plan.ranges.size() == 2 ? key : GraphKey{};  // (its bounds are this batch's)
     *out = exec;
     return MCD_OK;
 }

@@ -90,14 +90,18 @@ int heston_run(Ctx& ctx, const mcd_heston_params* sets, size_t n_sets, const dou
     const uint32_t items_per_set = fp64 ? static_cast<uint32_t>((paths + unit - 1) / unit) : hs[0].n_slabs;
     if (static_cast<uint64_t>(hs[0].n_slabs) * n_sets > 0xFFFFFFF0ull)
         return ctx.fail(MCD_ERR_INVALID_ARGUMENT, "batch too large");
-    // FP64 batches run in ranges of sets, so that the partials stay within 1 GB
-    // (or one set's).
+    // FP64 batches run in ranges of sets, so that the partials stay within 128 MB
+    // (or one set's), or in smaller ranges where the device has no more memory.
     const uint64_t set_bytes = sizeof(Welford) * std::max<uint64_t>(items_per_set, 1) * n_strikes;
-    const size_t per_range = fp64 ? std::min<size_t>(n_sets, std::max<uint64_t>((1ull << 30) / set_bytes, 1)) : n_sets;
+    size_t per_range = fp64 ? std::min<size_t>(n_sets, std::max<uint64_t>((128ull << 20) / set_bytes, 1)) : n_sets;
     int rc = ctx.reserve(ctx.ext[kSets], sizeof(HestonSet) * n_sets, "heston sets");
     if (!rc) rc = ctx.reserve(ctx.ext[kStrikes], sizeof(double) * n_strikes, "strikes");
-    if (!rc) rc = ctx.reserve(ctx.ext[kPartials], set_bytes * per_range, "heston partials");
     if (!rc) rc = ctx.reserve(ctx.ext[kOut], sizeof(mcd_mc_result) * n_sets * n_strikes, "heston results");
+    if (!rc) rc = ctx.reserve(ctx.ext[kPartials], set_bytes * per_range, "heston partials");
+    while (rc == MCD_ERR_OUT_OF_MEMORY && fp64 && per_range > 1) {
+        per_range = (per_range + 3) / 4;
+        rc = ctx.reserve(ctx.ext[kPartials], set_bytes * per_range, "heston partials");
+    }
     if (rc) return rc;
     cudaError_t e = cudaMemcpyAsync(ctx.ext[kSets].ptr, hs.data(), sizeof(HestonSet) * n_sets, cudaMemcpyHostToDevice, ctx.stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(ctx.ext[kStrikes].ptr, strikes, sizeof(double) * n_strikes, cudaMemcpyHostToDevice, ctx.stream);
