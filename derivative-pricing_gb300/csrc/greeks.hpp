@@ -51,6 +51,8 @@ struct DevGreeks {
     double z_unit;             // 2^(z_shift - 61): the running sum of the normals in normals
     int32_t vol_series;        // |vol-bump exponent| <= 1e-2 on all but > 8-sigma paths: cubic expm1
     int32_t z_shift;           // FP64: that sum of n_steps normals (below 6.34 each) stays within 63 bits
+    int32_t wide;              // FP64: the bumped states leave the fixed-point range, whatever the base does
+    int32_t pad;
 };
 
 cudaError_t launch_greeks_kernel(int precision, int variant, int grid, const DevContract* contracts,

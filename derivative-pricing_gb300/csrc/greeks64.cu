@@ -81,8 +81,8 @@ __device__ __forceinline__ void estimators(const DevContract& c, const DevGreeks
 }
 
 // ---------------------------------------------------------------------------
-// Contracts outside the fixed-point range (DevContract::frac = 0): the five
-// states step by step in FP64.
+// Contracts outside the fixed-point range (DevGreeks::wide): the five states step
+// by step in FP64.
 // ---------------------------------------------------------------------------
 __device__ __noinline__ void greeks_wide(const DevContract& c, const DevGreeks& g, uint64_t path,
                                          double (&o)[kNumGreeks]) {
@@ -257,6 +257,34 @@ __device__ __forceinline__ void greeks_fixed(GreeksSlot& slot, const FixedShared
     }
 }
 
+// The pricer's sample where its contract is in the fixed-point range but a bumped
+// state is not.
+template <int KIND>
+__device__ __forceinline__ double price_sample(const DevContract& c, const FixedShared& s,
+                                               const FixedTables* __restrict__ t, uint64_t path) {
+    const PhiloxKeys k = philox_keys(c.seed);
+    const PhiloxRow row = philox_row(static_cast<uint32_t>(path), 0u, k);
+    const uint32_t n = KIND == kEuropean || KIND == kDigital ? 1u : static_cast<uint32_t>(c.n_steps);
+    Path64<KIND> p;
+    for (uint32_t d = 0; d < n; ++d) {
+        const uint32_t bits = philox_word0(row, philox_step(d, static_cast<uint32_t>(path >> 32), k), k);
+        p.step(c, s, c.y_drift + drift_carry(d, c.y_drift_lo) + scaled_normal(normal_fixed(bits, s, t), c.y_vs), 0u);
+    }
+    return c.discount * payoff64<KIND>(c, c.spot, s, p);
+}
+__device__ __noinline__ double price_fixed(const DevContract& c, const FixedShared& s,
+                                           const FixedTables* __restrict__ t, uint64_t path) {
+    switch (c.kind) {
+        case kEuropean: return price_sample<kEuropean>(c, s, t, path);
+        case kDigital: return price_sample<kDigital>(c, s, t, path);
+        case kAsianArith: return price_sample<kAsianArith>(c, s, t, path);
+        case kAsianGeo: return price_sample<kAsianGeo>(c, s, t, path);
+        case kBarrier: return price_sample<kBarrier>(c, s, t, path);
+        case kLookbackFixed: return price_sample<kLookbackFixed>(c, s, t, path);
+        default: return price_sample<kLookbackFloating>(c, s, t, path);
+    }
+}
+
 struct SharedGreeks {
     FixedShared tables;
     GreeksSlot slot[kThreads / 32];
@@ -302,8 +330,9 @@ __global__ void __launch_bounds__(kThreads, 1)
             const uint32_t at = static_cast<uint32_t>(j) * 32u + lane;
             const uint32_t path_lo = static_cast<uint32_t>(base) + at, path_hi = static_cast<uint32_t>(base >> 32);
 #define MCD_GREEKS(K) case K: greeks_fixed<K>(slot, s, t, k, path_lo, path_hi, j == 0, o); break;
-            if (c.frac == 0) {
+            if (slot.g.wide) {
                 greeks_wide(c, slot.g, base + at, o);
+                if (c.frac != 0) o[kGPrice] = price_fixed(c, s, t, base + at);
             } else {
                 switch (c.kind) {
                     MCD_GREEKS(kEuropean)

@@ -49,7 +49,7 @@ int plan_greeks(Ctx& ctx, const mcd_contract* cs, size_t n, int precision, doubl
     if (rc) return rc;
     consts.resize(n);
     for (size_t j = 0; j < n; ++j) {
-        DevContract& d = plan.dev[j];
+        const DevContract& d = plan.dev[j];
         const mcd_contract& in = cs[d.orig_index];
         DevGreeks& g = consts[j];
         std::memset(&g, 0, sizeof g);
@@ -85,9 +85,10 @@ int plan_greeks(Ctx& ctx, const mcd_contract* cs, size_t n, int precision, doubl
         // FP64 kernel: the vol states in the base's units.  A vol bump below
         // 100 % makes the log-spot's bound less than four times the base's,
         // which the two spare bits of the units take; beyond the exponent
-        // range of a double the contract leaves the fixed-point form.
-        if (d.frac != 0 && in.vol * std::sqrt(in.time) * (1.0 + vol_rel) > 8.0) d.frac = 0;
-        if (d.frac != 0) {
+        // range of a double the states leave the fixed-point form (the price
+        // keeps the pricer's).
+        g.wide = d.frac == 0 || in.vol * std::sqrt(in.time) * (1.0 + vol_rel) > 8.0 ? 1 : 0;
+        if (!g.wide) {
             constexpr double kInvLn2 = 1.44269504088896340736;
             fixed_step(g.drift_up, g.vs_up, d.frac, &g.y_drift_up, &g.y_drift_lo_up, &g.y_vs_up);
             fixed_step(g.drift_dn, g.vs_dn, d.frac, &g.y_drift_dn, &g.y_drift_lo_dn, &g.y_vs_dn);
