@@ -8,6 +8,7 @@
 #include <vector>
 
 #include "engine.hpp"
+#include "lsm.hpp"
 #include "mcd_gpu.h"
 
 namespace mcdg {
@@ -122,6 +123,11 @@ struct Ctx {
     LaunchShape greeks_shape[2] = {{1, 0}, {3, 0}};  // FP32: 8 CTAs per SM (64 registers)
     cudaGraphExec_t greeks_graph = nullptr;
     GraphKey greeks_key{};
+
+    // Longstaff-Schwartz, all dates in one launch (lsm.hpp): looks at the others'
+    // progress before a wait gives up, and shared memory per CTA (0: what it needs).
+    uint32_t chain_polls = kLsmChainPolls;
+    size_t chain_shared = 0;
 
     // Training schedule of the learned LSM regression (mcd_lsm_set_mlp_config).
     int mlp_steps_first = 100;

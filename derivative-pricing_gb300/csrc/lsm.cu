@@ -1205,7 +1205,7 @@ __global__ void __launch_bounds__(kChunkThreads<PREC>, PREC == 0 ? 1 : 4)
 // the next date's column and evaluate its basis.  Every operation on a path and
 // every sum is the lockstep form's (the basis is evaluated once for both uses),
 // so prices and policies have its bits.  A CTA waits for its own contract's
-// CTAs only, all of them resident; a wait that runs out (kChainPolls) is
+// CTAs only, all of them resident; a wait that runs out (kLsmChainPolls) is
 // recorded and ends the CTA.
 //
 // Bound: a date is a serial chain of products (about 8,000 cycles, the FP64
@@ -1227,7 +1227,6 @@ struct ChainShared {
     double T[10], poly[4];
     int has;
 };
-constexpr uint32_t kChainPolls = 1u << 22;  // of at least 0.1 us each
 
 __device__ __forceinline__ uint32_t load_acquire(const uint32_t* p) {
     uint32_t v;
@@ -1321,7 +1320,7 @@ __global__ void __launch_bounds__(kLsmThreads64, 2)
     lsm_chain64(const LsmDev* __restrict__ cs, const uint32_t* __restrict__ chunk_contract,
                 const double* __restrict__ store, LsmReg* __restrict__ reg, LsmPartial* __restrict__ part,
                 Welford* __restrict__ final_part, uint32_t* __restrict__ counters /* arrivals, epoch */,
-                uint32_t* __restrict__ need, double kappa_max, double* __restrict__ error,
+                uint32_t* __restrict__ need, double kappa_max, double* __restrict__ error, uint32_t max_polls,
                 const FixedTables* __restrict__ fixed) {
     extern __shared__ __align__(16) unsigned char chain_smem[];
     ChainShared& sh = *reinterpret_cast<ChainShared*>(chain_smem);
@@ -1353,8 +1352,8 @@ __global__ void __launch_bounds__(kLsmThreads64, 2)
         ++seen;
         if (threadIdx.x == 0) {
             uint32_t polls = 0;
-            while (load_acquire(epoch) < seen && ++polls < kChainPolls) {}
-            s_waited = polls < kChainPolls;
+            while (load_acquire(epoch) < seen && ++polls < max_polls) {}
+            s_waited = polls < max_polls;
         }
         __syncthreads();
         const bool ok = s_waited != 0;
@@ -1548,15 +1547,15 @@ cudaError_t lsm_chain64_capacity(int sm_count, uint32_t* chunks) {
 
 cudaError_t launch_lsm_chain64(const LsmDev* c, int n_contracts, const uint32_t* chunk_contract, uint32_t chunk_count,
                                uint32_t total_folds, const double* s_store, LsmReg* reg, LsmPartial* part,
-                               Welford* final_part, uint32_t* counters, double* error, const FixedTables* tables,
-                               cudaStream_t stream) {
+                               Welford* final_part, uint32_t* counters, double* error, uint32_t polls, size_t shared,
+                               const FixedTables* tables, cudaStream_t stream) {
     cudaGetLastError();
     if (chunk_count == 0) return cudaSuccess;
     uint32_t* need = counters + 2 * static_cast<size_t>(n_contracts) + 2 * static_cast<size_t>(total_folds);
     double kappa_max = 1e2;  // as launch_lsm_iteration
-    void* args[] = {&c, &chunk_contract, &s_store, &reg, &part, &final_part, &counters, &need, &kappa_max, &error, &tables};
+    void* args[] = {&c, &chunk_contract, &s_store, &reg, &part, &final_part, &counters, &need, &kappa_max, &error, &polls, &tables};
     return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(lsm_chain64), dim3(chunk_count),
-                                       dim3(kLsmThreads64), args, sizeof(ChainShared), stream);
+                                       dim3(kLsmThreads64), args, shared ? shared : sizeof(ChainShared), stream);
 }
 
 cudaError_t launch_lsm_finish(const LsmDev* c, int n_contracts, const Welford* final_part,

@@ -49,6 +49,7 @@ constexpr int kLsmMinGroupChunks = 16;  // chunks per learned-regression CTA at 
 constexpr int kLsmMaxFolds = 256;       // QR: fold groups per contract at most
 constexpr int kLsmMinFoldChunks = 32;   // QR: chunks per fold group at least
 constexpr uint32_t kLsmChainChunks = 512;  // the one-launch FP64 form folds at most 16 groups of 32 chunks
+constexpr uint32_t kLsmChainPolls = 1u << 22;  // of at least 0.1 us each
 constexpr int kGramPacked = 66 * 67 / 2;  // upper triangle of the 66 x 66 Gram matrix, row-major
 
 // Regression state of one (contract, date): T, the date's preconditioner
@@ -135,12 +136,13 @@ cudaError_t launch_lsm_iteration(int precision, int k, const LsmDev* c, int n_co
                                  const FixedTables* tables, cudaStream_t stream);
 // All dates of an FP64 batch of at most lsm_chain64_capacity chunks, every one
 // resident: counters zeroed as above, *error zero before and not zero after a
-// wait that ran out.
+// wait that ran out (after `polls` looks).  shared: dynamic shared memory per CTA,
+// 0 for what it needs.
 cudaError_t lsm_chain64_capacity(int sm_count, uint32_t* chunks);
 cudaError_t launch_lsm_chain64(const LsmDev* c, int n_contracts, const uint32_t* chunk_contract, uint32_t chunk_count,
                                uint32_t total_folds, const double* s_store, LsmReg* reg, LsmPartial* part,
-                               Welford* final_part, uint32_t* counters, double* error, const FixedTables* tables,
-                               cudaStream_t stream);
+                               Welford* final_part, uint32_t* counters, double* error, uint32_t polls, size_t shared,
+                               const FixedTables* tables, cudaStream_t stream);
 cudaError_t launch_lsm_finish(const LsmDev* c, int n_contracts, const Welford* final_part,
                               double* out /* n x 6: price, se, count, inception, mean, se */,
                               cudaStream_t stream);

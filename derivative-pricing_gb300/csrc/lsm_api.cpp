@@ -242,13 +242,13 @@ int upload_and_run(Ctx& ctx, const LsmPlan& p, int precision, bool frozen, std::
     // An FP64 batch whose chunks are all resident at once walks its dates in one
     // cooperative launch (lsm.cu).  One such launch at a time in the process:
     // another thread's batch meanwhile goes date by date, with the same bits, and
-    // so does this one again if its CTAs gave up waiting for one another.
+    // so does this one again if its CTAs gave up waiting for one another, or if the
+    // launch is refused (a process held to a part of the device, for instance).
     static std::mutex chain_lock;
     std::unique_lock<std::mutex> chain_hold(chain_lock, std::defer_lock);
     uint32_t resident = 0;
     if (precision == 0 && !mlp && chained && p.total_chunks > 0 && chain_hold.try_lock()) {
-        e = lsm_chain64_capacity(ctx.sm_count, &resident);
-        if (e != cudaSuccess) return ctx.cuda_fail(e, "lsm occupancy");
+        if (lsm_chain64_capacity(ctx.sm_count, &resident) != cudaSuccess) cudaGetLastError();  // (resident: 0)
     }
     const bool one_launch = p.total_chunks <= std::min(resident, kLsmChainChunks) && resident > 0;
     if (!one_launch && chain_hold.owns_lock()) chain_hold.unlock();
@@ -302,13 +302,22 @@ int upload_and_run(Ctx& ctx, const LsmPlan& p, int precision, bool frozen, std::
             le = launch_lsm_forward(precision, ctx.sm_count, d_dev, d_map, ch.chunk_first, ch.chunk_count,
                                     ctx.ext[kStore].ptr, ctx.tables, cs);
         if (le == cudaSuccess && j + 1 < chains.size()) le = cudaEventRecord(ctx.ev_stage[j], cs);
-        if (le == cudaSuccess && one_launch)
+        if (le == cudaSuccess && one_launch) {
             le = launch_lsm_chain64(d_dev, static_cast<int>(n), d_map, p.total_chunks, p.total_folds,
                                     static_cast<const double*>(ctx.ext[kStore].ptr),
                                     static_cast<LsmReg*>(ctx.ext[kReg].ptr),
                                     static_cast<LsmPartial*>(ctx.ext[kPartA].ptr),
                                     static_cast<Welford*>(ctx.ext[kFinal].ptr),
-                                    static_cast<uint32_t*>(ctx.ext[kCounters].ptr), d_out + 6 * n, ctx.tables, cs);
+                                    static_cast<uint32_t*>(ctx.ext[kCounters].ptr), d_out + 6 * n, ctx.chain_polls,
+                                    ctx.chain_shared, ctx.tables, cs);
+            if (le != cudaSuccess) {  // refused: nothing of it was queued
+                cudaGetLastError();
+                e = cudaStreamSynchronize(cs);
+                if (e != cudaSuccess) return ctx.cuda_fail(e, "lsm forward");
+                chain_hold.unlock();
+                return upload_and_run(ctx, p, precision, frozen, out, mlp, frozen_nets, frozen_ok, false);
+            }
+        }
         for (int k = 0; k < ch.max_steps && le == cudaSuccess; ++k) {
             if (mlp)
                 le = launch_lsm_mlp_iteration(precision, k, !frozen, d_dev, ch.c_first, ch.c_end, ch.max_steps,
@@ -552,6 +561,15 @@ void assemble_greeks(const mcd_lsm_contract& c, double hs, double hv, bool incep
 }  // namespace
 
 extern "C" {
+
+// Not part of the ABI: limits of the one-launch form, for its tests (0: the
+// usual ones).
+int mcd_test_lsm_chain(mcd_ctx* handle, uint32_t polls, size_t shared_bytes) {
+    MCD_CTX_OR_FAIL(handle, ctx);
+    ctx->chain_polls = polls ? polls : kLsmChainPolls;
+    ctx->chain_shared = shared_bytes;
+    return MCD_OK;
+}
 
 int mcd_lsm_american(mcd_ctx* handle, double spot, double strike, double rate, double carry_yield,
                      double vol, double time, int type, int monitoring_points,
