@@ -19,6 +19,7 @@
 #include <cuda_runtime.h>
 
 #include "engine.hpp"
+#include "fp32_fast.cuh"
 
 namespace mcdg {
 
@@ -251,7 +252,7 @@ __device__ __forceinline__ float fast_rcp(float x) {
 // tail draw (about one in ten) also run the second polynomial.
 __device__ __forceinline__ float upper_arg(float q) {  // w
     const float y = __fmaf_rn(-q, q, q);                          // q (1 - q)
-    return __fmaf_rn(__log2f(y), -0.693147181f, -1.386294361f);   // -ln(4 y)
+    return __fmaf_rn(fast_log2(y), -0.693147181f, -1.386294361f);   // -ln(4 y)
 }
 __device__ __forceinline__ float upper_central(float w) {
     const float t = w - 2.5f;

@@ -24,18 +24,17 @@
 // on the draw alone come from a table per item, those of the path alone are
 // taken once per path (PhiloxStep, PhiloxRow): 18 products -> 14.5.  The book
 // 313 -> 253 ms at 8 CTAs per SM (294 before at its best launch shape), of
-// which 7 ms from sums instead of Welford merges in the reductions.  Flushing
-// denormals (--ftz) takes the range tests out of the logarithm and the
-// exponentials (arguments here are normal numbers, the bits stay); the
-// compiler then wants about 70 registers: at 5, 6, 7 and 8 CTAs per SM 260, 256,
-// 253 and 266 ms on one GPU.
+// which 7 ms from sums instead of Welford merges in the reductions.  Logarithm
+// and exponentials without their range tests (fp32_fast.cuh) left 248 ms at 7
+// CTAs per SM (68 registers); one call, host side included, at 4, 5, 6, 7, 8, 12
+// CTAs: 265, 257, 254, 253, 258, 272 ms.
 //
 // Reference semantics restated per kind (src/pricers/monte_carlo.cpp):
 //   terminal products :135-149, path-dependent loop :154-177, Brownian-bridge
 //   barrier :184-230, control-variate Asian :275-302, antithetic pairing
 //   :73-79; payoffs include/mcd/payoffs/{european,digital,asian,barrier,
 //   lookback}.hpp.
-// nvcc-flags: --fmad=false --ftz=true
+// nvcc-flags: --fmad=false
 #include <cuda_runtime.h>
 
 #include "device_common.cuh"
@@ -91,7 +90,7 @@ struct Pair32 {
             for (int p = 0; p < 2; ++p) {
                 const float x0 = x[p];
                 x[p] = __fmaf_rn(sg, z[p], x[p] + mu);
-                if constexpr (KIND == kAsianArith || KIND == kAsianCv) acc[p] += __expf(x[p]);
+                if constexpr (KIND == kAsianArith || KIND == kAsianCv) acc[p] += fast_exp(x[p]);
                 if constexpr (KIND == kAsianGeo || KIND == kAsianCv) acc2[p] += x[p];
                 if constexpr (KIND == kBarrier || KIND == kBarrierBridge) {
                     const bool crossed = c.up ? x[p] >= lnh : x[p] <= lnh;
@@ -99,7 +98,7 @@ struct Pair32 {
                 }
                 if constexpr (KIND == kBarrierBridge) {
                     if (!breached[p]) {
-                        const float p_cross = __expf(inv_denom * (lnh - x0) * (lnh - x[p]));
+                        const float p_cross = fast_exp(inv_denom * (lnh - x0) * (lnh - x[p]));
                         breached[p] = uniform_from_bits_f32(philox_word0(row_u[p], st, k)) < p_cross;
                     }
                 }
@@ -116,14 +115,14 @@ struct Pair32 {
         const float phi = c.type == 0 ? 1.0f : -1.0f;
         const float s0 = static_cast<float>(c.spot), strike = static_cast<float>(c.strike);
         const float inv_n = 1.0f / static_cast<float>(c.n_steps);
-        const float last = s0 * __expf(x[p]);
+        const float last = s0 * fast_exp(x[p]);
         if constexpr (KIND == kAsianArith || KIND == kAsianGeo) {
-            const float avg = KIND == kAsianArith ? s0 * (acc[p] * inv_n) : s0 * __expf(acc2[p] * inv_n);
+            const float avg = KIND == kAsianArith ? s0 * (acc[p] * inv_n) : s0 * fast_exp(acc2[p] * inv_n);
             const float ref = c.floating ? (last - avg) : (avg - strike);
             return c.discount * static_cast<double>(fmaxf(phi * ref, 0.0f));
         } else if constexpr (KIND == kAsianCv) {
             const float a = s0 * (acc[p] * inv_n);
-            const float g = s0 * __expf(acc2[p] * inv_n);
+            const float g = s0 * fast_exp(acc2[p] * inv_n);
             const double ap = c.discount * static_cast<double>(fmaxf(phi * (a - strike), 0.0f));
             const double gp = c.discount * static_cast<double>(fmaxf(phi * (g - strike), 0.0f));
             return ap - (gp - c.kv_anchor);
@@ -132,11 +131,11 @@ struct Pair32 {
             const bool pays = c.out ? !breached[p] : breached[p];
             return c.discount * static_cast<double>(pays ? vanilla : static_cast<float>(c.rebate));
         } else if constexpr (KIND == kLookbackFixed) {
-            const float v = c.type == 0 ? fmaxf(s0 * __expf(xmax[p]) - strike, 0.0f)
-                                        : fmaxf(strike - s0 * __expf(xmin[p]), 0.0f);
+            const float v = c.type == 0 ? fmaxf(s0 * fast_exp(xmax[p]) - strike, 0.0f)
+                                        : fmaxf(strike - s0 * fast_exp(xmin[p]), 0.0f);
             return c.discount * static_cast<double>(v);
         } else {
-            const float v = c.type == 0 ? (last - s0 * __expf(xmin[p])) : (s0 * __expf(xmax[p]) - last);
+            const float v = c.type == 0 ? (last - s0 * fast_exp(xmin[p])) : (s0 * fast_exp(xmax[p]) - last);
             return c.discount * static_cast<double>(v);
         }
     }
@@ -150,7 +149,7 @@ __device__ __forceinline__ double terminal32(const DevContract& c, uint32_t bits
     const float s0 = static_cast<float>(c.spot), strike = static_cast<float>(c.strike);
     const float z0 = normal_from_bits_f32(bits);
     const float z = neg ? -z0 : z0;
-    const float s = s0 * __expf(__fmaf_rn(sg, z, mu));
+    const float s = s0 * fast_exp(__fmaf_rn(sg, z, mu));
     float payoff;
     if constexpr (KIND == kEuropean) {
         payoff = fmaxf(phi * (s - strike), 0.0f);

@@ -32,9 +32,10 @@
 // former default of 128 registers, 239 ms at its best launch shape (64
 // registers, 8 CTAs per SM), 221 ms with the Philox products of the draw and of
 // the path taken out of the step, transposed warp sums instead of twelve
-// Welford trees, and 8 CTAs per SM as the default.
+// Welford trees, and 8 CTAs per SM as the default, 211 ms with the logarithm and
+// the exponentials of fp32_fast.cuh.
 //
-// nvcc-flags: --fmad=false --ftz=true
+// nvcc-flags: --fmad=false
 #include <cuda_runtime.h>
 
 #include "device_common.cuh"
@@ -51,13 +52,13 @@ __device__ __forceinline__ double dmax(double a, double b) { return (a < b) ? b 
 
 // expm1 for the vol-bump exponents: a short Taylor series where |a| < 1/64
 // (relative error below 2e-12 there; bumps of 1e-4 give |a| ~ 1e-4), else
-// __expf(a) - 1 (relative error ~1e-7 / |a|, used for bumps above ~1 %).
+// fast_exp(a) - 1 (relative error ~1e-7 / |a|, used for bumps above ~1 %).
 __device__ __forceinline__ float expm1_small(float a) {
     if (fabsf(a) < 0.015625f) {
         const float p = __fmaf_rn(__fmaf_rn(__fmaf_rn(a, 1.0f / 120.0f, 1.0f / 24.0f), a, 1.0f / 6.0f), a, 0.5f);
         return __fmaf_rn(p * a, a, a);
     }
-    return __expf(a) - 1.0f;
+    return fast_exp(a) - 1.0f;
 }
 
 // expm1 by its cubic Taylor polynomial, for exponents the host bounds by
@@ -90,7 +91,7 @@ __device__ void greeks32(const DevContract& c, const DevGreeks& g, const PhiloxK
     double v[5];
     if constexpr (KIND == kEuropean || KIND == kDigital) {
         const float z = normal_from_bits_f32(philox_word0(row, philox_step(0u, path_hi, k), k));
-        const float ef = __expf(__fmaf_rn(sg, z, mu));
+        const float ef = fast_exp(__fmaf_rn(sg, z, mu));
         const float s = s0 * ef;  // as the path engine
         float payoff;
         if constexpr (KIND == kEuropean) {
@@ -172,7 +173,7 @@ __device__ void greeks32(const DevContract& c, const DevGreeks& g, const PhiloxK
             e_up = __fmaf_rn(hvf, D, -q);
             e_dn = __fmaf_rn(-hvf, D, -q);
             if constexpr (KIND == kAsianArith) {
-                const float e = __expf(x);
+                const float e = fast_exp(x);
                 acc += e;
                 a_d = __fmaf_rn(e, D, a_d);
                 a_r = __fmaf_rn(e, fi, a_r);
@@ -221,9 +222,9 @@ __device__ void greeks32(const DevContract& c, const DevGreeks& g, const PhiloxK
         }
         // price: the path engine's FP32 payoff
         const float inv_n = 1.0f / static_cast<float>(c.n_steps);
-        const float lastf = s0 * __expf(x);
+        const float lastf = s0 * fast_exp(x);
         if constexpr (KIND == kAsianArith || KIND == kAsianGeo) {
-            const float avg = KIND == kAsianArith ? s0 * (acc * inv_n) : s0 * __expf(acc2 * inv_n);
+            const float avg = KIND == kAsianArith ? s0 * (acc * inv_n) : s0 * fast_exp(acc2 * inv_n);
             const float ref = c.floating ? (lastf - avg) : (avg - strike);
             o[kGPrice] = c.discount * static_cast<double>(fmaxf(phi * ref, 0.0f));
         } else if constexpr (KIND == kBarrier) {
@@ -231,16 +232,16 @@ __device__ void greeks32(const DevContract& c, const DevGreeks& g, const PhiloxK
             const bool pays = c.out ? !br : br;
             o[kGPrice] = c.discount * static_cast<double>(pays ? vanilla : static_cast<float>(c.rebate));
         } else if constexpr (KIND == kLookbackFixed) {
-            const float val = c.type == 0 ? fmaxf(s0 * __expf(xmax) - strike, 0.0f)
-                                          : fmaxf(strike - s0 * __expf(xmin), 0.0f);
+            const float val = c.type == 0 ? fmaxf(s0 * fast_exp(xmax) - strike, 0.0f)
+                                          : fmaxf(strike - s0 * fast_exp(xmin), 0.0f);
             o[kGPrice] = c.discount * static_cast<double>(val);
         } else {
-            const float val = c.type == 0 ? (lastf - s0 * __expf(xmin)) : (s0 * __expf(xmax) - lastf);
+            const float val = c.type == 0 ? (lastf - s0 * fast_exp(xmin)) : (s0 * fast_exp(xmax) - lastf);
             o[kGPrice] = c.discount * static_cast<double>(val);
         }
         // the five states in FP64
         const double n = static_cast<double>(c.n_steps);
-        const double le = static_cast<double>(__expf(x));  // S_n / S0
+        const double le = static_cast<double>(fast_exp(x));  // S_n / S0
         const double em_up_n = static_cast<double>(expm1_small(e_up));
         const double em_dn_n = static_cast<double>(expm1_small(e_dn));
         const double last0 = S0 * le;

@@ -5,6 +5,9 @@
 #include <cuda_runtime.h>
 
 #include "engine.hpp"
+#ifdef __CUDACC__
+#include "fp32_fast.cuh"
+#endif
 
 namespace mcdg {
 
@@ -109,12 +112,12 @@ __host__ __device__ inline void laguerre_poly(const double gamma[4], double poly
 // Every kernel that regenerates stored path values uses these, so they agree
 // bit for bit (FP64: lsm_math.cuh).
 __device__ __forceinline__ float gbm_log_step_f32(float x, float z, float mu, float sg) { return __fmaf_rn(sg, z, x + mu); }
-__device__ __forceinline__ float gbm_spot_f32(float s0, float x) { return s0 * __expf(x); }
+__device__ __forceinline__ float gbm_spot_f32(float s0, float x) { return s0 * fast_exp(x); }
 // FP32 continuation value at S from poly (the FP32 backward pass and the
 // FP32 frozen replay both use this, so their decisions coincide).
 __device__ __forceinline__ float continuation_poly32(float s, float inv_strike, const float p[4]) {
     const float x = s * inv_strike;
-    const float e = __expf(-0.5f * x);
+    const float e = fast_exp(-0.5f * x);
     return e * __fmaf_rn(__fmaf_rn(__fmaf_rn(p[3], x, p[2]), x, p[1]), x, p[0]);
 }
 #endif

@@ -20,7 +20,7 @@
 // sums up to the warp on the FP32 path), chunks merged in order per contract
 // -- the base scenario reproduces the fitted price bit for bit.
 //
-// nvcc-flags: --fmad=false --ftz=true
+// nvcc-flags: --fmad=false
 #include <cuda_runtime.h>
 
 #include "device_common.cuh"
@@ -159,7 +159,7 @@ __device__ void replay32(const LsmDev& c, const FrozenDev& f, const LsmReg* __re
             if (group_live<NS>(live, gi)) {
                 const FrozenScenario& g0 = f.sc[group_lead(gi)];
                 x[gi] = __fmaf_rn(g0.sg_f, z, x[gi] + g0.mu_f);
-                e[gi] = __expf(x[gi]);
+                e[gi] = fast_exp(x[gi]);
             }
         }
 #pragma unroll
@@ -357,7 +357,7 @@ __global__ void __launch_bounds__(kLsmThreads, 6)
 #pragma unroll
             for (int gi = 0; gi < kGroups<NS>; ++gi) {
                 x[gi] = __fmaf_rn(sg[gi], z, x[gi] + mu[gi]);
-                e[gi] = __expf(x[gi]);
+                e[gi] = fast_exp(x[gi]);
             }
 #pragma unroll
             for (int q = 0; q < NS; ++q) {

@@ -42,7 +42,7 @@
 // below the BF16 rounding of the network's own hidden layer.  Every mbarrier
 // wait is bounded (umma.cuh).
 //
-// nvcc-flags: --fmad=false --ftz=true
+// nvcc-flags: --fmad=false
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -337,7 +337,7 @@ __global__ void __launch_bounds__(kBinThreads, 5)
                 if (xx > T(0)) {
                     int b;
                     float t;
-                    locate(ge, __logf(static_cast<float>(se[q]) * inv_kf), b, t);
+                    locate(ge, fast_log(static_cast<float>(se[q]) * inv_kf), b, t);
                     const float2 nb = tab[b];
                     const float cont = __fmaf_rn(t, nb.y, nb.x);
                     if (cont < 0.0f) v = xx;  // predicted time value < 0: exercise
@@ -360,7 +360,7 @@ __global__ void __launch_bounds__(kBinThreads, 5)
                 if (xx > T(0)) {
                     int b;
                     float t;
-                    locate(gd, __logf(static_cast<float>(sd[q]) * inv_kf), b, t);
+                    locate(gd, fast_log(static_cast<float>(sd[q]) * inv_kf), b, t);
                     const float y = static_cast<float>((v - xx) * inv_k);
                     // 32-bit conversions (a 64-bit one would run on the FP64 unit), widened by
                     // integer products: tq in [0, 2^16], |yq| <= 2^24

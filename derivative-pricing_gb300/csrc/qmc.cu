@@ -21,7 +21,7 @@
 // aggregates at once (sum, log-sum, extrema, barrier test, terminal spot), so
 // no path array is kept: one value per tree depth.
 //
-// nvcc-flags: --fmad=false --ftz=true
+// nvcc-flags: --fmad=false
 #include <cuda_runtime.h>
 
 #include <type_traits>
@@ -207,7 +207,7 @@ __device__ __forceinline__ double terminal_qmc32(const DevContract& c, uint32_t 
     const float phi = c.type == 0 ? 1.0f : -1.0f;
     const float s0 = static_cast<float>(c.spot), strike = static_cast<float>(c.strike);
     const float z = normal_from_sobol_f32(x);
-    const float s = s0 * __expf(__fmaf_rn(static_cast<float>(c.vs), z, static_cast<float>(c.drift)));
+    const float s = s0 * fast_exp(__fmaf_rn(static_cast<float>(c.vs), z, static_cast<float>(c.drift)));
     float payoff;
     if (c.kind == kEuropean) {
         payoff = fmaxf(phi * (s - strike), 0.0f);
@@ -224,7 +224,8 @@ __device__ __forceinline__ double terminal_qmc32(const DevContract& c, uint32_t 
 // at a time 282 ms, two 277 (both waiting on bank conflicts of the directions,
 // see add_x), with the bit-major directions and the node fetched one ahead 173,
 // the root taken out of the loop 165, four paths from one row 149 (47
-// instructions per path-step instead of 59, issue 83 % at 5 CTAs per SM).
+// instructions per path-step instead of 59, issue 83 % at 5 CTAs per SM); 146
+// with subnormals flushed in ex2 and lg2 alone (fp32_fast.cuh).
 // The bridge values live in shared memory, one column per thread and path
 // (w[slot * 512 + 128 p]): a node's slots are known only at run time, so a
 // register array would be spilled to local memory.
@@ -249,7 +250,7 @@ __device__ __forceinline__ void quad_qmc32(const DevContract& c, const DevQmc& q
     }
     auto observe = [&](int p, float x) {
         if constexpr (KIND == kAsianArith) {
-            acc[p] += __expf(x);
+            acc[p] += fast_exp(x);
         } else if constexpr (KIND == kAsianGeo) {
             acc[p] += x;
         } else if constexpr (KIND == kBarrier) {
@@ -307,18 +308,18 @@ __device__ __forceinline__ void quad_qmc32(const DevContract& c, const DevQmc& q
     const float inv_n = 1.0f / static_cast<float>(n);
 #pragma unroll
     for (int p = 0; p < kQuad; ++p) {
-        const float last = s0 * __expf(xlast[p]);
+        const float last = s0 * fast_exp(xlast[p]);
         float v;
         if constexpr (KIND == kAsianArith || KIND == kAsianGeo) {
-            const float avg = KIND == kAsianArith ? s0 * (acc[p] * inv_n) : s0 * __expf(acc[p] * inv_n);
+            const float avg = KIND == kAsianArith ? s0 * (acc[p] * inv_n) : s0 * fast_exp(acc[p] * inv_n);
             v = fmaxf(phi * (c.floating ? (last - avg) : (avg - strike)), 0.0f);
         } else if constexpr (KIND == kBarrier) {
             const float vanilla = fmaxf(phi * (last - strike), 0.0f);
             v = (c.out ? !breached[p] : breached[p]) ? vanilla : static_cast<float>(c.rebate);
         } else if constexpr (KIND == kLookbackFixed) {
-            v = c.type == 0 ? fmaxf(s0 * __expf(xmax[p]) - strike, 0.0f) : fmaxf(strike - s0 * __expf(xmin[p]), 0.0f);
+            v = c.type == 0 ? fmaxf(s0 * fast_exp(xmax[p]) - strike, 0.0f) : fmaxf(strike - s0 * fast_exp(xmin[p]), 0.0f);
         } else {
-            v = c.type == 0 ? (last - s0 * __expf(xmin[p])) : (s0 * __expf(xmax[p]) - last);
+            v = c.type == 0 ? (last - s0 * fast_exp(xmin[p])) : (s0 * fast_exp(xmax[p]) - last);
         }
         out[p] = c.discount * static_cast<double>(v);
     }
