@@ -796,12 +796,14 @@ int mcd_autotune(mcd_ctx* handle, const mcd_contract* contracts, size_t n, int p
     double best = 1e300;
     LaunchShape best_shape = saved;
     for (int v = 0; v < kNumVariants; ++v) {
+        if (precision == 0 && (v == 2 || v == 3)) continue;  // variant 1's kernel (launch_path64_kernel)
         int occ = 0;
         cudaError_t e = path_kernel_occupancy(precision, v, &occ);
         if (e != cudaSuccess) return ctx->cuda_fail(e, "occupancy");
         if (occ < 1) continue;
         std::vector<int> cands;
-        for (int c : {occ, (3 * occ + 3) / 4, (occ + 1) / 2, 2 * occ})
+        // (FP64: the one CTA that an SM holds; another would wait for it and load the tables again)
+        for (int c : {occ, (3 * occ + 3) / 4, (occ + 1) / 2, precision == 0 ? occ : 2 * occ})
             if (c >= 1 && std::find(cands.begin(), cands.end(), c) == cands.end()) cands.push_back(c);
         for (int c : cands) {
             ctx->shape[precision] = LaunchShape{v, c};

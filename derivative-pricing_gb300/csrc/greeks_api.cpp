@@ -324,12 +324,13 @@ int mcd_greeks_autotune(mcd_ctx* handle, const mcd_contract* contracts, size_t n
     LaunchShape best_shape = saved;
     std::vector<double> out;
     for (int v = 0; v < kGreeksVariants; ++v) {
+        if (precision == 0 && v != 1) continue;  // FP64 has one kernel, one CTA of it per SM
         int occ = 0;
         cudaError_t e = greeks_kernel_occupancy(precision, v, &occ);
         if (e != cudaSuccess) return ctx->cuda_fail(e, "greeks occupancy");
         if (occ < 1) continue;
         std::vector<int> cands;
-        for (int c : {occ, (occ + 1) / 2, 2 * occ})
+        for (int c : {occ, (occ + 1) / 2, precision == 0 ? occ : 2 * occ})
             if (c >= 1 && std::find(cands.begin(), cands.end(), c) == cands.end()) cands.push_back(c);
         for (int c : cands) {
             ctx->greeks_shape[precision] = LaunchShape{v, c};
