@@ -1,9 +1,11 @@
-// fp32_fast.cuh -- FP32 exponential and logarithm straight from the GPU's ex2 and
-// lg2 with flushed subnormals: without the scaling that serves subnormal arguments
-// and results (a logarithm's argument here is a normal number, and e^x below
-// 2^-126 counts as zero), which cost 1 to 2 % of every FP32 kernel.  Flushing
-// whole files by --ftz=true was as fast, but took spots and strikes below 1.2e-38
-// for zero.
+// fp32_fast.cuh -- FP32 exponential and logarithm of the step loops, straight from
+// the GPU's ex2 and lg2 with flushed subnormals: without the scaling that serves
+// subnormal arguments and results, which cost 1 to 2 % of every FP32 kernel (a
+// logarithm's argument here is a normal number; of a growth factor below 2^-126
+// a path's sums see nothing).  What is evaluated once per path takes __expf,
+// whose subnormal results count: a bumped state may multiply them by as much.
+// Flushing whole files by --ftz=true was no faster, and took spots and strikes
+// below 1.2e-38 for zero.
 #pragma once
 
 #include <cuda_runtime.h>

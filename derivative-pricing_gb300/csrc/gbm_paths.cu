@@ -115,14 +115,14 @@ struct Pair32 {
         const float phi = c.type == 0 ? 1.0f : -1.0f;
         const float s0 = static_cast<float>(c.spot), strike = static_cast<float>(c.strike);
         const float inv_n = 1.0f / static_cast<float>(c.n_steps);
-        const float last = s0 * fast_exp(x[p]);
+        const float last = s0 * __expf(x[p]);
         if constexpr (KIND == kAsianArith || KIND == kAsianGeo) {
-            const float avg = KIND == kAsianArith ? s0 * (acc[p] * inv_n) : s0 * fast_exp(acc2[p] * inv_n);
+            const float avg = KIND == kAsianArith ? s0 * (acc[p] * inv_n) : s0 * __expf(acc2[p] * inv_n);
             const float ref = c.floating ? (last - avg) : (avg - strike);
             return c.discount * static_cast<double>(fmaxf(phi * ref, 0.0f));
         } else if constexpr (KIND == kAsianCv) {
             const float a = s0 * (acc[p] * inv_n);
-            const float g = s0 * fast_exp(acc2[p] * inv_n);
+            const float g = s0 * __expf(acc2[p] * inv_n);
             const double ap = c.discount * static_cast<double>(fmaxf(phi * (a - strike), 0.0f));
             const double gp = c.discount * static_cast<double>(fmaxf(phi * (g - strike), 0.0f));
             return ap - (gp - c.kv_anchor);
@@ -131,11 +131,11 @@ struct Pair32 {
             const bool pays = c.out ? !breached[p] : breached[p];
             return c.discount * static_cast<double>(pays ? vanilla : static_cast<float>(c.rebate));
         } else if constexpr (KIND == kLookbackFixed) {
-            const float v = c.type == 0 ? fmaxf(s0 * fast_exp(xmax[p]) - strike, 0.0f)
-                                        : fmaxf(strike - s0 * fast_exp(xmin[p]), 0.0f);
+            const float v = c.type == 0 ? fmaxf(s0 * __expf(xmax[p]) - strike, 0.0f)
+                                        : fmaxf(strike - s0 * __expf(xmin[p]), 0.0f);
             return c.discount * static_cast<double>(v);
         } else {
-            const float v = c.type == 0 ? (last - s0 * fast_exp(xmin[p])) : (s0 * fast_exp(xmax[p]) - last);
+            const float v = c.type == 0 ? (last - s0 * __expf(xmin[p])) : (s0 * __expf(xmax[p]) - last);
             return c.discount * static_cast<double>(v);
         }
     }
@@ -149,7 +149,7 @@ __device__ __forceinline__ double terminal32(const DevContract& c, uint32_t bits
     const float s0 = static_cast<float>(c.spot), strike = static_cast<float>(c.strike);
     const float z0 = normal_from_bits_f32(bits);
     const float z = neg ? -z0 : z0;
-    const float s = s0 * fast_exp(__fmaf_rn(sg, z, mu));
+    const float s = s0 * __expf(__fmaf_rn(sg, z, mu));
     float payoff;
     if constexpr (KIND == kEuropean) {
         payoff = fmaxf(phi * (s - strike), 0.0f);

@@ -91,7 +91,7 @@ __device__ void greeks32(const DevContract& c, const DevGreeks& g, const PhiloxK
     double v[5];
     if constexpr (KIND == kEuropean || KIND == kDigital) {
         const float z = normal_from_bits_f32(philox_word0(row, philox_step(0u, path_hi, k), k));
-        const float ef = fast_exp(__fmaf_rn(sg, z, mu));
+        const float ef = __expf(__fmaf_rn(sg, z, mu));  // (subnormal too: a bumped state multiplies it by up to 1e38)
         const float s = s0 * ef;  // as the path engine
         float payoff;
         if constexpr (KIND == kEuropean) {
@@ -173,7 +173,8 @@ __device__ void greeks32(const DevContract& c, const DevGreeks& g, const PhiloxK
             e_up = __fmaf_rn(hvf, D, -q);
             e_dn = __fmaf_rn(-hvf, D, -q);
             if constexpr (KIND == kAsianArith) {
-                const float e = fast_exp(x);
+                // with bumps beyond the series a growth factor may be as large as e is small
+                const float e = SER ? fast_exp(x) : __expf(x);
                 acc += e;
                 a_d = __fmaf_rn(e, D, a_d);
                 a_r = __fmaf_rn(e, fi, a_r);
@@ -222,9 +223,9 @@ __device__ void greeks32(const DevContract& c, const DevGreeks& g, const PhiloxK
         }
         // price: the path engine's FP32 payoff
         const float inv_n = 1.0f / static_cast<float>(c.n_steps);
-        const float lastf = s0 * fast_exp(x);
+        const float lastf = s0 * __expf(x);
         if constexpr (KIND == kAsianArith || KIND == kAsianGeo) {
-            const float avg = KIND == kAsianArith ? s0 * (acc * inv_n) : s0 * fast_exp(acc2 * inv_n);
+            const float avg = KIND == kAsianArith ? s0 * (acc * inv_n) : s0 * __expf(acc2 * inv_n);
             const float ref = c.floating ? (lastf - avg) : (avg - strike);
             o[kGPrice] = c.discount * static_cast<double>(fmaxf(phi * ref, 0.0f));
         } else if constexpr (KIND == kBarrier) {
@@ -232,16 +233,16 @@ __device__ void greeks32(const DevContract& c, const DevGreeks& g, const PhiloxK
             const bool pays = c.out ? !br : br;
             o[kGPrice] = c.discount * static_cast<double>(pays ? vanilla : static_cast<float>(c.rebate));
         } else if constexpr (KIND == kLookbackFixed) {
-            const float val = c.type == 0 ? fmaxf(s0 * fast_exp(xmax) - strike, 0.0f)
-                                          : fmaxf(strike - s0 * fast_exp(xmin), 0.0f);
+            const float val = c.type == 0 ? fmaxf(s0 * __expf(xmax) - strike, 0.0f)
+                                          : fmaxf(strike - s0 * __expf(xmin), 0.0f);
             o[kGPrice] = c.discount * static_cast<double>(val);
         } else {
-            const float val = c.type == 0 ? (lastf - s0 * fast_exp(xmin)) : (s0 * fast_exp(xmax) - lastf);
+            const float val = c.type == 0 ? (lastf - s0 * __expf(xmin)) : (s0 * __expf(xmax) - lastf);
             o[kGPrice] = c.discount * static_cast<double>(val);
         }
         // the five states in FP64
         const double n = static_cast<double>(c.n_steps);
-        const double le = static_cast<double>(fast_exp(x));  // S_n / S0
+        const double le = static_cast<double>(__expf(x));  // S_n / S0
         const double em_up_n = static_cast<double>(expm1_small(e_up));
         const double em_dn_n = static_cast<double>(expm1_small(e_dn));
         const double last0 = S0 * le;

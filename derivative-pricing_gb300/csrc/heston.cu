@@ -197,8 +197,8 @@ __global__ void __launch_bounds__(128, 5)
                             }
                         }
                     }
-                    s_terminal32[t] = h32.s0 * fast_exp(x[0]);
-                    s_terminal32b[t] = h32.s0 * fast_exp(x[1]);
+                    s_terminal32[t] = h32.s0 * __expf(x[0]);
+                    s_terminal32b[t] = h32.s0 * __expf(x[1]);
                 }
                 __syncthreads();
                 payout(j, s_terminal32);

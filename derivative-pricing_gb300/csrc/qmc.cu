@@ -207,7 +207,7 @@ __device__ __forceinline__ double terminal_qmc32(const DevContract& c, uint32_t 
     const float phi = c.type == 0 ? 1.0f : -1.0f;
     const float s0 = static_cast<float>(c.spot), strike = static_cast<float>(c.strike);
     const float z = normal_from_sobol_f32(x);
-    const float s = s0 * fast_exp(__fmaf_rn(static_cast<float>(c.vs), z, static_cast<float>(c.drift)));
+    const float s = s0 * __expf(__fmaf_rn(static_cast<float>(c.vs), z, static_cast<float>(c.drift)));
     float payoff;
     if (c.kind == kEuropean) {
         payoff = fmaxf(phi * (s - strike), 0.0f);
@@ -308,18 +308,18 @@ __device__ __forceinline__ void quad_qmc32(const DevContract& c, const DevQmc& q
     const float inv_n = 1.0f / static_cast<float>(n);
 #pragma unroll
     for (int p = 0; p < kQuad; ++p) {
-        const float last = s0 * fast_exp(xlast[p]);
+        const float last = s0 * __expf(xlast[p]);
         float v;
         if constexpr (KIND == kAsianArith || KIND == kAsianGeo) {
-            const float avg = KIND == kAsianArith ? s0 * (acc[p] * inv_n) : s0 * fast_exp(acc[p] * inv_n);
+            const float avg = KIND == kAsianArith ? s0 * (acc[p] * inv_n) : s0 * __expf(acc[p] * inv_n);
             v = fmaxf(phi * (c.floating ? (last - avg) : (avg - strike)), 0.0f);
         } else if constexpr (KIND == kBarrier) {
             const float vanilla = fmaxf(phi * (last - strike), 0.0f);
             v = (c.out ? !breached[p] : breached[p]) ? vanilla : static_cast<float>(c.rebate);
         } else if constexpr (KIND == kLookbackFixed) {
-            v = c.type == 0 ? fmaxf(s0 * fast_exp(xmax[p]) - strike, 0.0f) : fmaxf(strike - s0 * fast_exp(xmin[p]), 0.0f);
+            v = c.type == 0 ? fmaxf(s0 * __expf(xmax[p]) - strike, 0.0f) : fmaxf(strike - s0 * __expf(xmin[p]), 0.0f);
         } else {
-            v = c.type == 0 ? (last - s0 * fast_exp(xmin[p])) : (s0 * fast_exp(xmax[p]) - last);
+            v = c.type == 0 ? (last - s0 * __expf(xmin[p])) : (s0 * __expf(xmax[p]) - last);
         }
         out[p] = c.discount * static_cast<double>(v);
     }
