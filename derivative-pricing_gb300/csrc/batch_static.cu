@@ -28,6 +28,7 @@
 #include <mutex>
 
 #include "engine.hpp"
+#include "items.hpp"
 #include "mcd_gpu.h"
 
 namespace {
@@ -160,10 +161,11 @@ extern "C" int mcd_price_batch_static(const mcd_contract* contracts, size_t n, i
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(d_prefix, g_stage_prefix, sizeof(uint32_t) * (n + 1), cudaMemcpyHostToDevice, s);
     if (e != cudaSuccess) return report_cuda(error_message, error_capacity, e, "stage contracts");
-    // Contracts in ranges whose items fit the partials: FP32 items (at most 64 or
-    // the slabs of a contract) and FP64 units (at most 4096 per contract below
-    // 2^23 paths, slabs above) are smaller than slabs, so a large batch of
-    // small contracts takes several launches on the same scratch.
+    // Contracts in ranges whose items fit the partials: FP32 items (at most 256 or
+    // the slabs of a contract) and FP64 units (at most 4096 per contract, slabs from
+    // 2^24 paths on) are smaller than slabs, so a large batch of small contracts
+    // takes several launches on the same scratch.
+    static_assert(mcdg::kMaxCutItems <= kStaticMaxSlabs && 4096 <= kStaticMaxSlabs, "one contract's items fit the partials");
     for (size_t first = 0; first < n;) {
         size_t end = first + 1;
         while (end < n && g_stage_prefix[end + 1] - g_stage_prefix[first] <= kStaticMaxSlabs) ++end;

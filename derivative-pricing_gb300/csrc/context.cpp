@@ -14,6 +14,7 @@
 
 #include "context.hpp"
 #include "engine.hpp"
+#include "items.hpp"
 #include "mcd_gpu.h"
 
 using namespace mcdg;
@@ -269,29 +270,10 @@ const char* convert_contract(const mcd_contract& in, uint32_t index, DevContract
     out.drift = (in.rate - in.carry_yield - 0.5 * vol * vol) * dt;
     out.vs = vol * std::sqrt(dt);
     out.n_slabs = static_cast<uint32_t>(slabs);
-    // FP64 units: one path per lane up to 131,071 paths (a single call then has
-    // the most warps to spread over the GPU), doubling from there so that a
-    // contract keeps 2048 to 4096 units, up to a slab.
-    out.unit_log = 0;
-    while (out.unit_log < 7 && (in.path_count >> (17 + out.unit_log)) != 0) ++out.unit_log;
-    const uint64_t unit = 32ull << out.unit_log;
-    out.n_units = static_cast<uint32_t>((in.path_count + unit - 1) / unit);
-    // FP32 items: a CTA's 4096 paths, halved while the contract has at most 256
-    // items of the half and those still hold 131,072 path-steps.  A small book's
-    // time is that of its longest item (4096 paths of 252 dates: 1.9 ms in a CTA
-    // by itself); contracts of more than 2^20 paths keep whole slabs.  Books of
-    // 3, 10, 30, 100, 300, 1000, 4096 contracts of 1e3 to 3e5 paths, ms, whole
-    // slabs against items: priced 1.11, 1.18, 1.78, 2.47, 4.35, 11.7, 54.4 and
-    // 0.72, 0.50, 0.85, 1.46, 4.12, 11.8, 54.7; sensitivities 2.72, 2.85, 3.34,
-    // 4.35, 7.75, 20.8, 93.4 and 1.60, 1.07, 1.52, 2.44, 7.43, 20.4, 91.6.
-    out.item_log = 5;
-    while (out.item_log > 1) {
-        const uint64_t half = 64ull << out.item_log;
-        if (in.path_count > 256 * half || half * static_cast<uint64_t>(out.n_steps) < 131072) break;
-        --out.item_log;
-    }
-    const uint64_t item = 128ull << out.item_log;
-    out.n_items = static_cast<uint32_t>((in.path_count + item - 1) / item);
+    out.unit_log = unit_log(in.path_count);
+    out.n_units = static_cast<uint32_t>(unit_count(in.path_count));
+    out.item_log = item_log(in.path_count, out.n_steps);
+    out.n_items = static_cast<uint32_t>(item_count(in.path_count, out.n_steps));
     out.inv_n = 1.0 / static_cast<double>(out.n_steps);
     fixed_scale(out);
     return nullptr;
@@ -428,10 +410,9 @@ int upload_plan(Ctx& ctx, BatchPlan& plan) {
     return MCD_OK;
 }
 
-// Queues a planned batch on a stream: per range, reset ticket and error word
-// (the first range's are zero already when `fresh`), persistent path kernel,
-// merge kernel.  (The error word keeps the last range's value; an inconsistent
-// item shows in every run.)
+// Queues a planned batch on a stream: per range, reset ticket, and before
+// the first the error word (zero already when `fresh`), persistent path kernel,
+// merge kernel.  (The error word gathers all ranges' errors.)
 int enqueue_plan(Ctx& ctx, int precision, int variant, int grid, const BatchPlan& plan, void* results,
                  uint32_t* flags, bool fresh, cudaStream_t stream) {
     cudaGetLastError();  // launches below report their own status only
@@ -457,7 +438,7 @@ int enqueue_plan(Ctx& ctx, int precision, int variant, int grid, const BatchPlan
 // inside the graph.
 int get_graph(Ctx& ctx, int precision, int variant, int grid, const BatchPlan& plan, void* results,
               cudaGraphExec_t* out) {
-    GraphKey key{precision, variant, grid, plan.n, 0u, ctx.d_plan.ptr, nullptr, ctx.d_partials.ptr, results};
+    GraphKey key{precision, variant, grid, plan.n, ctx.d_plan.ptr, nullptr, ctx.d_partials.ptr, results};
     for (auto& g : ctx.graphs) {
         if (g.key == key && g.exec) {
             *out = g.exec;

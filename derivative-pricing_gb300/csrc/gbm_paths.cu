@@ -330,13 +330,10 @@ __global__ void draws_kernel(uint64_t seed, uint64_t path_begin, uint64_t n_path
     const PhiloxKeys k = philox_keys(seed);
     const PhiloxPath pp = philox_path(path_begin + p, static_cast<uint32_t>(stream_id), k);
     const uint32_t bits = philox_word0(pp, draw_begin + d, k);
-    double v;
-    if (stream_id == 0) {
-        v = precision == 0 ? normal_from_bits_f64(bits) : static_cast<double>(normal_from_bits_f32(bits));
-    } else {
-        v = precision == 0 ? uniform_open01_f64(bits) : static_cast<double>(uniform_from_bits_f32(bits));
-    }
-    out[i] = v;
+    // (FP64 normals: draws64_kernel)
+    out[i] = stream_id == 0   ? static_cast<double>(normal_from_bits_f32(bits))
+             : precision == 0 ? uniform_open01_f64(bits)
+                              : static_cast<double>(uniform_from_bits_f32(bits));
 }
 
 template <int MINB>

@@ -153,7 +153,7 @@ int prepare_greeks(Ctx& ctx, int precision, BatchPlan& plan, const std::vector<D
     int variant = 0, grid = 0;
     rc = greeks_grid(ctx, precision, plan.max_items, variant, grid);
     if (rc) return rc;
-    const GraphKey key{precision, variant, grid, n, 0u, ctx.ext[kGDev].ptr, ctx.ext[kGPrefix].ptr,
+    const GraphKey key{precision, variant, grid, n, ctx.ext[kGDev].ptr, ctx.ext[kGPrefix].ptr,
                        ctx.ext[kGPart].ptr, ctx.ext[kGOut].ptr};
     if (ctx.greeks_graph && ctx.greeks_key == key && plan.ranges.size() == 2) {
         *out = ctx.greeks_graph;

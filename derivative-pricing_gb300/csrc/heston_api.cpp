@@ -9,6 +9,7 @@
 
 #include "context.hpp"
 #include "heston.hpp"
+#include "items.hpp"
 #include "mcd_gpu.h"
 
 using namespace mcdg;
@@ -81,13 +82,9 @@ int heston_run(Ctx& ctx, const mcd_heston_params* sets, size_t n_sets, const dou
         const int rc = make_set(ctx, sets[i], steps, paths, seed, i, hs[i]);
         if (rc) return rc;
     }
-    // FP64 units as the GBM pricer's: 32 paths per warp, doubling from 131,072
-    // paths on, up to a slab.
-    int unit_log = 0;
-    while (unit_log < 7 && (paths >> (17 + unit_log)) != 0) ++unit_log;
+    // FP64 units as the GBM pricer's.
     const bool fp64 = precision == 0;
-    const uint64_t unit = 32ull << unit_log;
-    const uint32_t items_per_set = fp64 ? static_cast<uint32_t>((paths + unit - 1) / unit) : hs[0].n_slabs;
+    const uint32_t items_per_set = fp64 ? static_cast<uint32_t>(unit_count(paths)) : hs[0].n_slabs;
     if (static_cast<uint64_t>(hs[0].n_slabs) * n_sets > 0xFFFFFFF0ull)
         return ctx.fail(MCD_ERR_INVALID_ARGUMENT, "batch too large");
     // FP64 batches run in ranges of sets, so that the partials stay within 128 MB
@@ -121,7 +118,7 @@ int heston_run(Ctx& ctx, const mcd_heston_params* sets, size_t n_sets, const dou
         const int k = static_cast<int>(n_strikes);
         e = cudaMemsetAsync(ctx.d_flags, 0, sizeof(uint32_t), ctx.stream);
         if (e == cudaSuccess && items_per_set > 0)
-            e = fp64 ? launch_heston64(grid, d_sets, count, d_strikes, k, type, items_per_set, unit_log, ctx.d_flags,
+            e = fp64 ? launch_heston64(grid, d_sets, count, d_strikes, k, type, items_per_set, unit_log(paths), ctx.d_flags,
                                        partials, ctx.tables, ctx.stream)
                      : launch_heston32(grid, d_sets, count, d_strikes, k, type, items_per_set, ctx.d_flags, partials,
                                        ctx.stream);
