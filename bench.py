@@ -105,16 +105,15 @@ def path_steps(c):
 # of the sources they were measured on.  The roofline below uses them only
 # while the sources still have that digest; otherwise it reports the
 # instruction-based figures as unmeasured (null) rather than stale.
-PATH_KERNEL_SOURCES = ("derivative-pricing_gb300/csrc/gbm_paths.cu",
-                       "derivative-pricing_gb300/csrc/device_common.cuh",
-                       "derivative-pricing_gb300/csrc/engine.hpp")
+PATH_KERNEL_SOURCES = tuple("derivative-pricing_gb300/csrc/" + f for f in (
+    "gbm_paths.cu", "device_common.cuh", "fp32_fast.cuh", "unit_sums.cuh", "merge.cuh", "items.hpp", "engine.hpp"))
 PATH_KERNEL_PROFILE = {
-    "sources": "852b8eff9b45756d",
+    "sources": "214ea717921c6e38",
     "case_path_steps": 6807363601.0,
     # variant -> smsp__inst_executed.sum of one launch
-    "warp_inst": {"0": 14013206001, "1": 14030673708, "2": 14733038953, "3": 14156864108, "4": 14019130019},
+    "warp_inst": {"0": 13811216785, "1": 13830618832, "2": 14486716045, "3": 13908766312, "4": 13818866688},
     # variant -> dram__bytes_read.sum + dram__bytes_write.sum of one launch
-    "dram_bytes": {"0": 163840, "1": 166656, "2": 764928, "3": 1000192, "4": 462592},
+    "dram_bytes": {"0": 162048, "1": 496384, "2": 742912, "3": 951296, "4": 272896},
 }
 
 

@@ -3,7 +3,7 @@
 // precisions (the FP64 paths are gbm_paths64.cu).
 //
 // Work decomposition.  Every contract's paths are cut into items of 128 << item_log
-// paths, 4096 or fewer (convert_contract); one (contract, item) pair is one work item.  The
+// paths, 4096 or fewer (items.hpp); one (contract, item) pair is one work item.  The
 // host orders contracts longest-first and passes the running item count per
 // contract (item_prefix).  A CTA of 128 threads claims items from a ticket
 // counter (one atomicAdd per item, no waiting) until the list is exhausted.
