@@ -41,7 +41,7 @@ constexpr uint64_t kMinRangeItems = 1ull << 14;  // down to which a lack of memo
 
 struct LaunchShape {
     int variant = 1;
-    int ctas_per_sm = 0;  // 0: occupancy limit
+    int ctas_per_sm = 0;  // 0: occupancy limit (Greeks: or what the items need)
 };
 
 // Key of a captured graph.  The kernels read their item counts from the uploaded

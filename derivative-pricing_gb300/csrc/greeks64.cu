@@ -19,7 +19,7 @@
 // between the rounds of a unit, but a call of 1e5 paths (3125 units) is one
 // round of the 4864 resident warps, where 512 threads and 128 registers took
 // two.  Measured: finite-difference European, likelihood-ratio barrier and
-// pathwise Asian of 1e5 paths and 52 dates, one call each, 130 -> 0.39 ms in all
+// pathwise Asian of 1e5 paths and 52 dates, one call each, 130 -> 0.40 ms in all
 // (512, 640, 768, 1024 threads: 0.48, 0.48, 0.42, 0.41 before the units' sums
 // lost their division); 16 contracts of 2e5 paths, Asian 3.09 -> 2.91 ms, barrier
 // 1.91 -> 1.65, lookback 1.66 -> 1.61, European 0.81; largest error against

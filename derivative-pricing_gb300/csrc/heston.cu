@@ -21,7 +21,7 @@
 // compensation, then added in FP64; the groups and slabs are merged in fixed
 // order.  (The FP64 paths are heston64.cu.)
 //
-// Bound: issue (72 % of the slots) and the FMA-heavy pipe (66 %), 176
+// Bound: issue (68 % of the slots) and the FMA-heavy pipe (69 %), 158
 // thread-instructions per path-step.  64 sets of 64 strikes, 252 steps, 2^20
 // paths: 110 ms -> 106 with the Philox products of the draw and of the path
 // taken out of the step, 100-104 with one branch region for both paths'

@@ -15,18 +15,25 @@
  *
  * Precision (mcd_precision):
  *   MCD_PRECISION_FP64  FP64 accuracy on identical draws; prices agree with
- *                       the CPU reference to ~1e-12 relative (GBM pricers and
- *                       Greeks: 64-bit fixed-point paths, exact to 1e-17 per
- *                       draw; elsewhere the reference's operations in FP64).
+ *                       the CPU reference to ~1e-12 relative.  GBM pricers,
+ *                       Greeks and Longstaff-Schwartz: normals and paths in
+ *                       64-bit fixed point, exact to 1e-17 per draw (contracts
+ *                       whose |log2 S/S0| may pass 2^9 are stepped in FP64),
+ *                       the Longstaff-Schwartz basis with a tabulated
+ *                       exponential; Heston: the same normals, the variance
+ *                       step regrouped with integer reciprocal, roots and
+ *                       logarithm; Sobol: the reference's operations in FP64.
  *   MCD_PRECISION_FP32  the same Philox draws (same counters, word 0) turned
  *                       into FP32 normals; paths evolve in FP32 (log space);
  *                       payoffs are accumulated and merged in FP64.
  *
  * Results are bitwise identical for a given precision regardless of launch
- * configuration (grid size, kernel variant): paths are grouped into fixed
- * slabs of MCD_SLAB_PATHS (FP64 GBM pricers: smaller units whose size depends
- * on the contract's path count alone) and every reduction tree is fixed by
- * slab or unit index.
+ * configuration (grid size, kernel variant): paths are grouped by the contract
+ * alone and every reduction tree is fixed by the group's index.  Groups: FP64 GBM
+ * pricers, Greeks and Heston units of 32 to 4096 paths, by the path count; FP32
+ * GBM pricers and Greeks items of 256 to 4096 paths, by path count and dates;
+ * Sobol and FP32 Heston slabs of MCD_SLAB_PATHS; Longstaff-Schwartz chunks of
+ * 1024 paths.
  */
 #ifndef MCD_GPU_H
 #define MCD_GPU_H
@@ -174,8 +181,8 @@ int mcd_batch_invalidate(mcd_ctx* ctx);
  * no mcd_ctx.  It runs the same kernels as mcd_price_batch and returns bitwise
  * the same results; its scratch (contract records, slab partials, device
  * results, ticket and error word) lives in one fixed __device__ array of
- * about 7 MB.  Every GPU that loads the library holds that array until the
- * process exits.  Under CUDA's lazy module loading (the runtime's default)
+ * about 7 MB.  Every GPU that loads the library holds that array, and 0.6 MB of
+ * tables of the FP64 engines, until the process exits (or resets the device).  Under CUDA's lazy module loading (the runtime's default)
  * the array is reserved on a device by the first call there, not when the
  * library is loaded: a caller that then reserves the rest of device memory
  * makes that first call (n = 0 will do) before doing so.
@@ -188,9 +195,10 @@ int mcd_batch_invalidate(mcd_ctx* ctx);
  * results are in `results`.  On failure, a message is written to
  * error_message (if error_capacity > 0).
  *
- * The first call on a device does the set-up for that device (a call with
- * n = 0 does only that): it resolves the array's device address with that
- * device current.  Make that first call before any stream capture.  All calls share the one array, and it keeps
+ * The first call on a device, or on one that was reset since, does the set-up for
+ * that device (a call with n = 0 does only that): it resolves the array's device
+ * address with that device current and fills the tables, by a copy on `stream`.
+ * Make that first call before any stream capture.  All calls share the one array, and it keeps
  * the last call's contents.  Calls that overlapped on the GPU would race on
  * it; this entry point serialises its calls with a process-wide lock and
  * waits for its GPU work before returning, so its own calls never overlap. */
@@ -200,7 +208,8 @@ int mcd_price_batch_static(const mcd_contract* contracts, size_t n, int precisio
 
 /* Launch shape of the persistent path kernel.  variant 0..4 selects the
  * register budget (FP32: __launch_bounds__ min blocks 4/8/12/16/7; FP64:
- * 512/1024/1024/1024/768 threads in the SM's one CTA), ctas_per_sm the
+ * 512/1024/1024/1024/768 threads in the SM's one CTA, each kernel timed once by
+ * the autotuner), ctas_per_sm the
  * grid (SM count x ctas_per_sm).  0 restores the autotuned/default choice.
  * Results do not depend on either. */
 int mcd_set_launch_shape(mcd_ctx* ctx, int precision, int variant, int ctas_per_sm);
@@ -359,7 +368,8 @@ typedef struct {
 int mcd_greeks_batch(mcd_ctx* ctx, const mcd_contract* contracts, size_t n, double spot_bump_rel,
                      double vol_bump_rel, int precision, mcd_greeks_result* results);
 /* Launch shape of the sensitivity kernel (variant 0..3: register budget for
- * 2, 4, 6 or 8 resident CTAs; ctas_per_sm 0 = occupancy limit) and its tuner, which
+ * 2, 4, 6 or 8 resident CTAs, FP64 one kernel for all; ctas_per_sm 0 = as many as
+ * the batch's items need, up to the occupancy limit) and its tuner, which
  * times every candidate on the given batch and keeps the fastest. */
 int mcd_greeks_set_launch_shape(mcd_ctx* ctx, int precision, int variant, int ctas_per_sm);
 int mcd_greeks_autotune(mcd_ctx* ctx, const mcd_contract* contracts, size_t n, double spot_bump_rel,
